@@ -223,8 +223,8 @@ int ensure_grid_work(aldic_ctx *c, long long n) {
   if (n <= c->gw_n && c->gw.x) return OK;
   const long long R = 12;
   int rc;
-  // x r z p(2 buffers) q b diag zz qq ss pp -> 12 * R * n doubles
-  if ((rc = c->gw_vec.ensure(sizeof(double) * 12 * R * n))) return rc;
+  // x r z p(2 buffers) q b diag zz qq ss pp tmp -> 13 * R * n doubles
+  if ((rc = c->gw_vec.ensure(sizeof(double) * 13 * R * n))) return rc;
   c->gw.max_blocks = 148 * 8;
   if ((rc = c->gw_part.ensure(sizeof(double) * 2 * 4 * R * c->gw.max_blocks))) return rc;
   if ((rc = c->gw_mask.ensure(R * n))) return rc;
@@ -241,12 +241,14 @@ int ensure_grid_work(aldic_ctx *c, long long n) {
   c->gw.qq = v + 9 * R * n;
   c->gw.ss = v + 10 * R * n;
   c->gw.pp = v + 11 * R * n;
+  c->gw.tmp = v + 12 * R * n;
   c->gw.part = c->gw_part.as<double>();
   c->gw.mask = c->gw_mask.as<unsigned char>();
   unsigned int *misc = c->gw_misc.as<unsigned int>();
   c->gw.bar = misc;
   c->gw.err = (int *)(misc + 2);
   c->gw.iters_out = (int *)(misc + 3);
+  c->gw.gate = (int *)(misc + 4);
   c->gw_n = n;
   ALDIC_CUDA(cudaMemsetAsync(c->gw_misc.p, 0, 64, c->stream));
   return OK;
@@ -850,12 +852,9 @@ int aldic_localicgn_post(aldic_ctx *c, int M, int N, const int32_t *iters, doubl
   ALDIC_CHECK(bad && dnum, E_NOMEM, "staging buffer allocation failed");
   if ((rc = icgn_flags(M, N, (const int *)ai.dev, bad, dnum, (double *)(dnum + 2), dnum + 4, c->stream)))
     return rc;
-  if ((rc = inpaint_load(c->gw, M, N, 2, au.dev, 2, bad, c->stream, 0))) return rc;
-  if ((rc = inpaint_load(c->gw, M, N, 4, af.dev, 4, bad, c->stream, 2))) return rc;
-  if ((rc = grid_pcg(c->gw, OP_INPAINT, M, N, 6, 0, 0, 1, 0, kRtolInpaint, kMaxitInpaint, c->stream)))
+  if ((rc = inpaint_solve(c->gw, M, N, 6, FieldMap().interleaved(au.dev, 2).interleaved(af.dev, 4, 2), bad,
+                          kRtolInpaint, kMaxitInpaint, c->stream)))
     return rc;
-  if ((rc = inpaint_store(c->gw, M, N, 2, au.dev, 2, c->stream, 0))) return rc;
-  if ((rc = inpaint_store(c->gw, M, N, 4, af.dev, 4, c->stream, 2))) return rc;
   arg_back(c, au); arg_back(c, af);
   int hb = 0;
   ALDIC_CUDA(cudaMemcpyAsync(&hb, dnum, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -877,11 +876,11 @@ int aldic_subpb1_post(aldic_ctx *c, int M, int N, const int32_t *iters, double *
   int *dnum = (int *)c->arena.get(64);
   ALDIC_CHECK(bad && dnum, E_NOMEM, "staging buffer allocation failed");
   if ((rc = subpb1_flags((int)n, (const int *)ai.dev, bad, dnum, c->stream))) return rc;
-  if ((rc = gridfit_load(c->gw, M, N, 2, au.dev, 2, (const int *)ai.dev, c->stream))) return rc;
-  if ((rc = grid_pcg(c->gw, OP_GRIDFIT, M, N, 2, 0, 0, 1, springs_lam2(M, N), kRtolFit, kMaxitFit,
-                     c->stream)))
+  ALDIC_CUDA(cudaMemcpyAsync(c->gw.tmp, au.dev, sizeof(double) * 2 * n, cudaMemcpyDeviceToDevice, c->stream));
+  if ((rc = gridfit_solve(c->gw, M, N, 2, FieldMap().interleaved(c->gw.tmp, 2),
+                          FieldMap().interleaved(au.dev, 2), (const int *)ai.dev, nullptr,
+                          springs_lam2(M, N), kRtolFit, kMaxitFit, false, c->stream)))
     return rc;
-  if ((rc = grid_store(c->gw, M, N, 2, au.dev, 2, c->stream))) return rc;
   arg_back(c, au);
   int hb = 0;
   ALDIC_CUDA(cudaMemcpyAsync(&hb, dnum, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -1193,14 +1192,16 @@ int aldic_gridfit_springs(aldic_ctx *c, int M, int N, int nf, const double *in, 
   if ((rc = ensure_grid_work(c, n))) return rc;
   Arg<double> ai, ao;
   if ((rc = arg_in(c, in, nf * n, ai)) || (rc = arg_out(c, out, nf * n, ao))) return rc;
-  // field-major input: one field of n values after another (stride 1)
-  for (int f = 0; f < nf; ++f)
-    if ((rc = gridfit_load(c->gw, M, N, 1, ai.dev + f * n, 1, nullptr, c->stream, f))) return rc;
-  if ((rc = grid_pcg(c->gw, OP_GRIDFIT, M, N, nf, 0, 0, 1, springs_lam2(M, N), kRtolFit, kMaxitFit,
-                     c->stream)))
+  // field-major: one field of n values after another; out may share in's memory,
+  // which the solve reads while it writes
+  const double *src = ai.dev;
+  if (ao.dev < ai.dev + nf * n && ai.dev < ao.dev + nf * n) {
+    ALDIC_CUDA(cudaMemcpyAsync(c->gw.tmp, ai.dev, sizeof(double) * nf * n, cudaMemcpyDeviceToDevice, c->stream));
+    src = c->gw.tmp;
+  }
+  if ((rc = gridfit_solve(c->gw, M, N, nf, FieldMap().planes(src, nf, n), FieldMap().planes(ao.dev, nf, n),
+                          nullptr, nullptr, springs_lam2(M, N), kRtolFit, kMaxitFit, false, c->stream)))
     return rc;
-  for (int f = 0; f < nf; ++f)
-    if ((rc = grid_store(c->gw, M, N, 1, ao.dev + f * n, 1, c->stream, f))) return rc;
   arg_back(c, ao);
   return check_grid_err(c);
 }
@@ -1213,12 +1214,9 @@ int aldic_inpaint_springs(aldic_ctx *c, int M, int N, int nf, double *z) {
   if ((rc = ensure_grid_work(c, n))) return rc;
   Arg<double> az;
   if ((rc = arg_out(c, z, nf * n, az, true))) return rc;
-  for (int f = 0; f < nf; ++f)
-    if ((rc = inpaint_load(c->gw, M, N, 1, az.dev + f * n, 1, nullptr, c->stream, f))) return rc;
-  if ((rc = grid_pcg(c->gw, OP_INPAINT, M, N, nf, 0, 0, 1, 0, kRtolInpaint, kMaxitInpaint, c->stream)))
+  if ((rc = inpaint_solve(c->gw, M, N, nf, FieldMap().planes(az.dev, nf, n), nullptr, kRtolInpaint,
+                          kMaxitInpaint, c->stream)))
     return rc;
-  for (int f = 0; f < nf; ++f)
-    if ((rc = inpaint_store(c->gw, M, N, 1, az.dev + f * n, 1, c->stream, f))) return rc;
   arg_back(c, az);
   return check_grid_err(c);
 }
@@ -1227,14 +1225,10 @@ static int smooth_dev(aldic_ctx *c, int M, int N, int nf, double *vals) {
   // funSmoothDisp.m:64-101 / funSmoothStrain.m:63-109: twice (gridfit, nanconv)
   int rc;
   const double lam2 = springs_lam2(M, N);
-  for (int pass = 0; pass < 2; ++pass) {
-    if ((rc = gridfit_load(c->gw, M, N, nf, vals, nf, nullptr, c->stream))) return rc;
-    if ((rc = grid_pcg(c->gw, OP_GRIDFIT, M, N, nf, 0, 0, 1, lam2, kRtolFit, kMaxitFit, c->stream)))
-      return rc;
-    if ((rc = nanconv3(c->gw, M, N, nf, c->stream))) return rc;
-    if ((rc = grid_store(c->gw, M, N, nf, vals, nf, c->stream))) return rc;
-  }
-  return OK;
+  const FieldMap v = FieldMap().interleaved(vals, nf), t = FieldMap().interleaved(c->gw.tmp, nf);
+  if ((rc = gridfit_solve(c->gw, M, N, nf, v, t, nullptr, nullptr, lam2, kRtolFit, kMaxitFit, true, c->stream)))
+    return rc;
+  return gridfit_solve(c->gw, M, N, nf, t, v, nullptr, nullptr, lam2, kRtolFit, kMaxitFit, true, c->stream);
 }
 
 int aldic_smooth(aldic_ctx *c, int M, int N, int nf, double *vals) {
@@ -1461,10 +1455,9 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
                          nullptr, nullptr, st, &c->sw)))
       return rc;
     k_mesh_init<<<nb, 256, 0, st>>>(M, N, B.sx, B.sy, B.su, B.sv, B.coords, B.x0, B.y0, B.U0);
-    if ((rc = inpaint_load(c->gw, M, N, 2, B.U0, 2, nullptr, st, 0))) return rc;
-    if ((rc = grid_pcg(c->gw, OP_INPAINT, M, N, 2, 0, 0, 1, 0, kRtolInpaint, kMaxitInpaint, st)))
+    if ((rc = inpaint_solve(c->gw, M, N, 2, FieldMap().interleaved(B.U0, 2), nullptr, kRtolInpaint,
+                            kMaxitInpaint, st)))
       return rc;
-    if ((rc = inpaint_store(c->gw, M, N, 2, B.U0, 2, st, 0))) return rc;
     if (gated) {
       const double *gF = c->given.as<double>();
       const float *conf = (const float *)(gF + 4 * n);
@@ -1485,11 +1478,9 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
     return rc;
   if ((rc = mark(c, 3))) return rc;
   if ((rc = icgn_flags(M, N, B.it1, B.bad, B.ints, B.meanit, B.ints + 1, st))) return rc;
-  if ((rc = inpaint_load(c->gw, M, N, 2, B.U1, 2, B.bad, st, 0))) return rc;
-  if ((rc = inpaint_load(c->gw, M, N, 4, B.F1, 4, B.bad, st, 2))) return rc;
-  if ((rc = grid_pcg(c->gw, OP_INPAINT, M, N, 6, 0, 0, 1, 0, kRtolInpaint, kMaxitInpaint, st))) return rc;
-  if ((rc = inpaint_store(c->gw, M, N, 2, B.U1, 2, st, 0))) return rc;
-  if ((rc = inpaint_store(c->gw, M, N, 4, B.F1, 4, st, 2))) return rc;
+  if ((rc = inpaint_solve(c->gw, M, N, 6, FieldMap().interleaved(B.U1, 2).interleaved(B.F1, 4, 2), B.bad,
+                          kRtolInpaint, kMaxitInpaint, st)))
+    return rc;
   // Section 5
   if ((rc = mark(c, 4))) return rc;
   if (p->smooth && (rc = smooth_dev(c, M, N, 4, B.F1))) return rc;
@@ -1565,12 +1556,14 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
       ALDIC_CUDA(cudaMemcpyAsync(B.U2old, B.U2, sizeof(double) * 2 * n, cudaMemcpyDeviceToDevice, st));
     u2old_current = false;
     if ((rc = subpb1(im, B.coords, n, B.U2, B.F2, B.vdual, B.H21, nullptr, p->winsize, mu, p->tol,
-                     p->precision, B.U1, B.itb, c->queue.as<unsigned int>(), st, B.cache)))
+                     p->precision, c->gw.tmp, B.itb, c->queue.as<unsigned int>(), st, B.cache)))
       return rc;
     // subsets Subpb1 could not solve start the fit from Subproblem 2's U
-    if ((rc = gridfit_load(c->gw, M, N, 2, B.U1, 2, B.itb, st, 0, B.U2))) return rc;
-    if ((rc = grid_pcg(c->gw, OP_GRIDFIT, M, N, 2, 0, 0, 1, lam2, kRtolFit, kMaxitFit, st))) return rc;
-    if ((rc = grid_store(c->gw, M, N, 2, B.U1, 2, st))) return rc;
+    const FieldMap start = FieldMap().interleaved(B.U2, 2);
+    if ((rc = gridfit_solve(c->gw, M, N, 2, FieldMap().interleaved(c->gw.tmp, 2),
+                            FieldMap().interleaved(B.U1, 2), B.itb, &start, lam2, kRtolFit, kMaxitFit,
+                            false, st)))
+      return rc;
     ALDIC_CUDA(cudaMemcpyAsync(B.F1, B.F2, sizeof(double) * 4 * n, cudaMemcpyDeviceToDevice, st));
     if (a < 16) {  // the update norm, and U1old <- U1 in the same pass
       if ((rc = diffnorm_update(B.U1old, B.U1, 2 * n, B.part, B.upd + 16 + a, inv, st))) return rc;
@@ -1713,9 +1706,8 @@ int aldic_qt_frame(aldic_ctx *c, const aldic_qt_frame_params *p, aldic_qt_mesh *
   k_qt_hole<<<nb0, 256, 0, st>>>(n0, sx, sy, su, sv, c->mask.as<double>(), W);
   k_mesh_init<<<nb0, 256, 0, st>>>(nx, ny, sx, sy, su, sv, ucoords, ux0, uy0, U0u);
   if ((rc = ensure_grid_work(c, n0))) return rc;
-  if ((rc = inpaint_load(c->gw, nx, ny, 2, U0u, 2, nullptr, st, 0)) ||
-      (rc = grid_pcg(c->gw, OP_INPAINT, nx, ny, 2, 0, 0, 1, 0, kRtolInpaint, kMaxitInpaint, st)) ||
-      (rc = inpaint_store(c->gw, nx, ny, 2, U0u, 2, st, 0)))
+  if ((rc = inpaint_solve(c->gw, nx, ny, 2, FieldMap().interleaved(U0u, 2), nullptr, kRtolInpaint,
+                          kMaxitInpaint, st)))
     return rc;
   ALDIC_CUDA(cudaStreamSynchronize(st));
   const auto t1 = clk::now();

@@ -22,7 +22,7 @@ namespace aldic {
 namespace {
 
 constexpr int PCG_THREADS = 512;
-constexpr int MAXRHS = 12;
+constexpr int MAXRHS = kMaxFields;
 
 struct PcgArgs {
   double *x, *r, *z, *p0, *p1, *q, *b, *diag, *part;
@@ -36,6 +36,10 @@ struct PcgArgs {
   int *iters_out;
   CsrOp csr;               // OP_CSR
   const double *ata;       // OP_GRIDFIT with scattered data: A'A, 9 coefficients per node
+  // behind a tile solve (PcgTail)
+  const int *gate;
+  FieldMap guess, out;
+  int nreal, conv;
 };
 
 // Scalar Q4 element matrices on a square element of size h with local nodes
@@ -305,6 +309,8 @@ __device__ void global_sums(PcgShared &S, const double *part, int cnt, int block
 template <int OP, int NR>
 __global__ void __launch_bounds__(PCG_THREADS) k_pcg(PcgArgs A) {
   __shared__ PcgShared S;
+  const int gate = A.gate ? *A.gate : 1;
+  if (gate == 0) return;  // the tiles solved it
   if (A.beta_ptr) {
     const double bv = *A.beta_ptr;
 #pragma unroll
@@ -318,6 +324,16 @@ __global__ void __launch_bounds__(PCG_THREADS) k_pcg(PcgArgs A) {
   double *const Zd = A.zz, *const Qd = A.qq, *const Sd = A.ss, *const Pd = A.pp;
   double *Mv[2] = {A.p0, A.p1};
   const long long pstride = (long long)4 * MAXRHS * A.blocks;  // second partials buffer
+  if (OP == OP_GRIDFIT && gate == 2) {
+    // the tiles met infinities: every field from its data again
+#pragma unroll 1
+    for (int f = 0; f < NR; ++f)
+      for (long long k = tid0; k < n; k += stride) {
+        const long long o = f * n + k;
+        X[o] = (!A.mask[o] && f < A.nreal && A.guess.p[0]) ? A.guess.p[f][k * A.guess.stride[f]] : A.b[o];
+      }
+    if (!grid_sync(A.gs, A.blocks)) return;
+  }
   // ---- r = b - A x, u = D^-1 r, directions 0
 #pragma unroll 1
   for (int f = 0; f < NR; ++f) {
@@ -479,6 +495,25 @@ __global__ void __launch_bounds__(PCG_THREADS) k_pcg(PcgArgs A) {
     bool all = true;
     for (int f = 0; f < NR; ++f) all &= (S.done[f] != 0);
     if (!all) atomicExch(A.gs.err, 2);  // not converged within maxit
+  }
+  if ((OP == OP_GRIDFIT || OP == OP_INPAINT) && A.out.p[0]) {
+    if (A.conv && !grid_sync(A.gs, A.blocks)) return;  // it reads the neighbours
+    const double e1 = 0.1353352832366127, e2 = 0.01831563888873418;  // exp(-2), exp(-4)
+#pragma unroll 1
+    for (int f = 0; f < A.nreal; ++f)
+      for (long long k = tid0; k < n; k += stride) {
+        const double *v = X + f * n + k;
+        double s = v[0];
+        if (A.conv) {
+          const int j = (int)k / M, i = (int)k - j * M;
+          const bool l = i > 0, r = i < M - 1, u = j > 0, d = j < A.N - 1;
+          const double ax = (l ? v[-1] : 0.0) + (r ? v[1] : 0.0) + (u ? v[-M] : 0.0) + (d ? v[M] : 0.0);
+          const double dg = (l && u ? v[-M - 1] : 0.0) + (r && u ? v[-M + 1] : 0.0) +
+                            (l && d ? v[M - 1] : 0.0) + (r && d ? v[M + 1] : 0.0);
+          s = (s + e1 * ax + e2 * dg) / (1.0 + e1 * (l + r + u + d) + e2 * ((l + r) * (u + d)));
+        }
+        A.out.p[f][k * A.out.stride[f]] = s;
+      }
   }
 }
 
@@ -819,69 +854,6 @@ __global__ void k_sweep_err_final(const double *__restrict__ part, int nb, int n
   if (lane == 0) err[s] = sqrt(t);
 }
 
-// ------------------------------------------------------------------ loaders
-__global__ void k_gridfit_load(int M, int N, int nf, const double *__restrict__ vals, int stride,
-                               const int *__restrict__ iters, const double *__restrict__ guess,
-                               double *__restrict__ b, double *__restrict__ x,
-                               unsigned char *__restrict__ mask) {
-  const long long n = (long long)M * N;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-       k += (long long)gridDim.x * blockDim.x) {
-    const bool bad = iters && (iters[k] < 0 || iters[k] > 99);
-    for (int f = 0; f < nf; ++f) {
-      const double v = vals[k * stride + f];
-      const bool ok = !bad && !isnan(v);
-      mask[f * n + k] = ok;
-      b[f * n + k] = ok ? v : 0.0;
-      x[f * n + k] = ok ? v : (guess ? guess[k * stride + f] : 0.0);
-    }
-  }
-}
-
-
-__global__ void k_grid_store(int M, int N, int nf, const double *__restrict__ x,
-                             double *__restrict__ vals, int stride) {
-  const long long n = (long long)M * N;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-       k += (long long)gridDim.x * blockDim.x)
-    for (int f = 0; f < nf; ++f) vals[k * stride + f] = x[f * n + k];
-}
-
-__global__ void k_inpaint_load(int M, int N, int nf, const double *__restrict__ vals, int stride,
-                               const unsigned char *__restrict__ badmask,
-                               double *__restrict__ b, double *__restrict__ x,
-                               unsigned char *__restrict__ mask) {
-  // fields [0, nf) of vals land in slots f0.. of the work vectors (the
-  // caller offsets b, x, mask by f0 * n)
-  const long long n = (long long)M * N;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-       k += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(k % M), j = (int)(k / M);
-    for (int f = 0; f < nf; ++f) {
-      auto known = [&](long long q) {
-        return !(badmask && badmask[q]) && !isnan(vals[q * stride + f]);
-      };
-      const bool kn = known(k);
-      mask[f * n + k] = !kn;
-      double bv;
-      int kc = 0;  // known neighbours of an unknown entry
-      if (kn) {
-        bv = vals[k * stride + f];
-      } else {
-        bv = 0.0;
-        if (i > 0 && known(k - 1)) { bv += vals[(k - 1) * stride + f]; ++kc; }
-        if (i < M - 1 && known(k + 1)) { bv += vals[(k + 1) * stride + f]; ++kc; }
-        if (j > 0 && known(k - M)) { bv += vals[(k - M) * stride + f]; ++kc; }
-        if (j < N - 1 && known(k + M)) { bv += vals[(k + M) * stride + f]; ++kc; }
-      }
-      b[f * n + k] = bv;
-      // an unknown entry starts from the mean of its known neighbours (the
-      // solution itself for an isolated one), else from 0
-      x[f * n + k] = kn ? bv : (kc > 0 ? bv / kc : 0.0);
-    }
-  }
-}
-
 // ------------------------------------------------------------------ flags
 __global__ void k_icgn_flags(long long n, const int *__restrict__ it,
                              unsigned char *__restrict__ bad, int *badnum, double *meanit,
@@ -961,31 +933,6 @@ __global__ void k_subpb1_flags(long long n, const int *__restrict__ it,
   }
 }
 
-// nanconv(z, fspecial('gaussian',3,0.5), 'edge', 'nanout') with no NaN input
-__global__ void k_nanconv3(int M, int N, int nf, const double *__restrict__ in,
-                           double *__restrict__ out) {
-  const long long n = (long long)M * N;
-  const double e1 = 0.1353352832366127;   // exp(-2)
-  const double e2 = 0.01831563888873418;  // exp(-4)
-  const double ks = 1.0 + 4.0 * e1 + 4.0 * e2;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n * nf;
-       k += (long long)gridDim.x * blockDim.x) {
-    const long long kk = k % n, f = k / n;
-    const int i = (int)(kk % M), j = (int)(kk / M);
-    double s = 0.0, w = 0.0;
-    for (int dj = -1; dj <= 1; ++dj)
-      for (int di = -1; di <= 1; ++di) {
-        const int ii = i + di, jj = j + dj;
-        if (ii < 0 || ii >= M || jj < 0 || jj >= N) continue;
-        const int d2 = di * di + dj * dj;
-        const double kv = (d2 == 0 ? 1.0 : (d2 == 1 ? e1 : e2)) / ks;
-        s += kv * in[f * n + (long long)jj * M + ii];
-        w += kv;
-      }
-    out[k] = s / w;
-  }
-}
-
 __global__ void k_vsub(const double *a, const double *b, double *o, long long n) {
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x)
@@ -1050,11 +997,11 @@ inline int blocks_for(long long n, int threads = 256) {
 
 int grid_pcg(GridWork &w, int op, int M, int N, int nrhs, double beta, double mu, double h,
              double lam2, double rtol, int maxit, cudaStream_t st, const double *beta_ptr,
-             const double *beta_each, const double *ata) {
+             const double *beta_each, const double *ata, const PcgTail *tail) {
   ALDIC_CHECK(nrhs >= 1 && nrhs <= MAXRHS, E_ARG, "grid_pcg: 1..12 right-hand sides");
   const long long n = (long long)M * N;
   ALDIC_CHECK(n < (1LL << 31), E_ARG, "grid_pcg: more than 2^31 nodes");
-  int dev = 0, sms = 148, per = 1;
+  int dev = 0, sms = 148;
   ALDIC_CUDA(cudaGetDevice(&dev));
   ALDIC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   void *fn = nullptr;
@@ -1072,10 +1019,9 @@ int grid_pcg(GridWork &w, int op, int M, int N, int nrhs, double beta, double mu
   else { ALDIC_PCG_FN(OP_INPAINT) }
 #undef ALDIC_PCG_FN
   const int nr_pad = nrhs <= 2 ? nrhs : (nrhs <= 4 ? 4 : (nrhs <= 6 ? 6 : 12));
-  ALDIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, PCG_THREADS, 0));
   // one block per SM at most: fewer partials and cheaper barriers, while the
   // grid-stride loops still cover every node
-  long long blocks = (long long)sms * (per < 1 ? 1 : (per > 1 ? 1 : per));
+  long long blocks = sms;
   const long long need = (n + PCG_THREADS - 1) / PCG_THREADS;
   if (blocks > need) blocks = need;
   if (blocks > w.max_blocks) blocks = w.max_blocks;
@@ -1097,7 +1043,13 @@ int grid_pcg(GridWork &w, int op, int M, int N, int nrhs, double beta, double mu
   A.beta_ptr = beta_ptr;
   A.csr = CsrOp{};
   A.ata = op == OP_GRIDFIT ? ata : nullptr;
-  ALDIC_CUDA(cudaMemsetAsync(w.bar, 0, 2 * sizeof(unsigned int), st));
+  A.gate = tail ? tail->gate : nullptr;
+  if (tail && tail->guess) A.guess = *tail->guess;
+  if (tail && tail->out) A.out = *tail->out;
+  A.nreal = nrhs;
+  A.conv = tail && tail->conv;
+  if (!tail)  // the tile kernels reset the barrier words themselves
+    ALDIC_CUDA(cudaMemsetAsync(w.bar, 0, 2 * sizeof(unsigned int), st));
   void *args[] = {&A};
   ALDIC_CUDA(cudaLaunchCooperativeKernel(fn, dim3((unsigned)blocks), dim3(PCG_THREADS), args, 0, st));
   return OK;
@@ -1140,6 +1092,9 @@ int csr_pcg(GridWork &w, const CsrOp &op, long long n, int nrhs, double rtol, in
   A.beta_ptr = nullptr;
   A.csr = op;
   A.ata = nullptr;
+  A.gate = nullptr;
+  A.nreal = nrhs;
+  A.conv = 0;
   ALDIC_CUDA(cudaMemsetAsync(w.bar, 0, 2 * sizeof(unsigned int), st));
   void *args[] = {&A};
   ALDIC_CUDA(cudaLaunchCooperativeKernel(fn, dim3((unsigned)blocks), dim3(PCG_THREADS), args, 0, st));
@@ -1284,35 +1239,22 @@ int nodal_strain(int M, int N, double h, const double *U, double *F, cudaStream_
   return OK;
 }
 
-int gridfit_load(GridWork &w, int M, int N, int nf, const double *vals, int stride,
-                 const int *bad_iters, cudaStream_t st, int f0, const double *guess) {
-  const long long n = (long long)M * N;
-  k_gridfit_load<<<blocks_for(n), 256, 0, st>>>(M, N, nf, vals, stride, bad_iters, guess,
-                                                w.b + f0 * n, w.x + f0 * n, w.mask + f0 * n);
-  ALDIC_CUDA(cudaGetLastError());
-  return OK;
+int gridfit_solve(GridWork &w, int M, int N, int nf, const FieldMap &in, const FieldMap &out,
+                  const int *bad, const FieldMap *guess, double lam2, double rtol, int maxit,
+                  bool conv, cudaStream_t st) {
+  int rc = fit_tiles(w, M, N, nf, in, out, bad, guess, lam2, rtol, conv, st);
+  if (rc) return rc;
+  const PcgTail tail{w.gate, guess, &out, conv};
+  return grid_pcg(w, OP_GRIDFIT, M, N, nf, 0, 0, 1, lam2, rtol, maxit, st, nullptr, nullptr, nullptr,
+                  &tail);
 }
 
-int grid_store(const GridWork &w, int M, int N, int nf, double *vals, int stride,
-               cudaStream_t st, int f0) {
-  const long long n = (long long)M * N;
-  k_grid_store<<<blocks_for(n), 256, 0, st>>>(M, N, nf, w.x + f0 * n, vals, stride);
-  ALDIC_CUDA(cudaGetLastError());
-  return OK;
-}
-
-int inpaint_load(GridWork &w, int M, int N, int nf, const double *vals, int stride,
-                 const unsigned char *badmask, cudaStream_t st, int f0) {
-  const long long n = (long long)M * N;
-  k_inpaint_load<<<blocks_for(n), 256, 0, st>>>(M, N, nf, vals, stride, badmask, w.b + f0 * n,
-                                                w.x + f0 * n, w.mask + f0 * n);
-  ALDIC_CUDA(cudaGetLastError());
-  return OK;
-}
-
-int inpaint_store(const GridWork &w, int M, int N, int nf, double *vals, int stride,
-                  cudaStream_t st, int f0) {
-  return grid_store(w, M, N, nf, vals, stride, st, f0);
+int inpaint_solve(GridWork &w, int M, int N, int nf, const FieldMap &vals, const unsigned char *bad,
+                  double rtol, int maxit, cudaStream_t st) {
+  int rc = fill_tiles(w, M, N, nf, vals, bad, rtol, st);
+  if (rc) return rc;
+  const PcgTail tail{w.gate, nullptr, &vals, false};
+  return grid_pcg(w, OP_INPAINT, M, N, nf, 0, 0, 1, 0, rtol, maxit, st, nullptr, nullptr, nullptr, &tail);
 }
 
 int icgn_flags(int M, int N, const int *iters, unsigned char *badmask, int *d_badnum,
@@ -1327,13 +1269,6 @@ int subpb1_flags(int n, const int *iters, unsigned char *badmask, int *d_badnum,
                  cudaStream_t st) {
   k_subpb1_flags<<<1, 1024, 0, st>>>(n, iters, badmask, d_badnum);
   ALDIC_CUDA(cudaGetLastError());
-  return OK;
-}
-
-int nanconv3(GridWork &w, int M, int N, int nf, cudaStream_t st) {
-  const long long n = (long long)M * N;
-  k_nanconv3<<<blocks_for(n * nf), 256, 0, st>>>(M, N, nf, w.x, w.r);
-  ALDIC_CUDA(cudaMemcpyAsync(w.x, w.r, sizeof(double) * n * nf, cudaMemcpyDeviceToDevice, st));
   return OK;
 }
 

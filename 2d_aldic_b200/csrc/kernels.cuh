@@ -76,6 +76,28 @@ int subpb1(const IcgnImages &im, const double *coords, long long n, const double
            cudaStream_t st, const double *cache = nullptr);
 
 // ---- k_grid.cu: node-grid solvers and field kernels on the M x N mesh
+// nf fields of the nodes somewhere in memory: field f of node k at p[f][k stride[f]]
+constexpr int kMaxFields = 12;
+struct FieldMap {
+  double *p[kMaxFields] = {};
+  int stride[kMaxFields] = {};
+  // nf fields interleaved at v (from slot f0 on)
+  FieldMap &interleaved(const double *v, int nf, int f0 = 0) {
+    for (int f = 0; f < nf; ++f) {
+      p[f0 + f] = const_cast<double *>(v) + f;
+      stride[f0 + f] = nf;
+    }
+    return *this;
+  }
+  // nf fields of n values one after the other
+  FieldMap &planes(const double *v, int nf, long long n) {
+    for (int f = 0; f < nf; ++f) {
+      p[f] = const_cast<double *>(v) + f * n;
+      stride[f] = 1;
+    }
+    return *this;
+  }
+};
 struct GridWork {
   // PCG vectors for up to 12 right-hand sides of M*N (x fastest) each; p is
   // two vectors (the second 12*M*N after the first)
@@ -87,6 +109,8 @@ struct GridWork {
   int *err;              // barrier / solver error flag
   int *iters_out;        // PCG iterations used
   int max_blocks;
+  int *gate = nullptr;   // k_local.cu's {gate, ticket}; the ticket is 0 between launches
+  double *tmp = nullptr; // 12 M N doubles no solver touches
 };
 enum GridOp { OP_FE = 0, OP_GRIDFIT = 1, OP_INPAINT = 2, OP_CSR = 3, OP_FD = 4 };
 
@@ -198,13 +222,23 @@ int cnn_patches(const float *f, const float *g, int W, int H, const double *coor
                 void *bf16_out, float *f32_out, cudaStream_t st);
 int cnn_to_init(const float *out, long long n, double *U0, double *F0, float *conf, cudaStream_t st);
 
+// what follows a tile solve of k_local.cu: k_pcg does nothing when *gate is 0,
+// continues from x when 1, and when 2 starts over from the data (and guess
+// where there is none); then it writes the fields of out, convolved with
+// nanconv's 3 x 3 Gaussian if conv
+struct PcgTail {
+  const int *gate;
+  const FieldMap *guess;
+  const FieldMap *out;
+  bool conv;
+};
 // solve op(x) = b for nrhs fields; b and x live in w.b / w.x (field-major)
 // ata (OP_GRIDFIT only, may be NULL): scattered-data A'A as 9 coefficients per
 // node (offsets (di, dj) in row-major 3 x 3 order); the mask is then unused
 int grid_pcg(GridWork &w, int op, int M, int N, int nrhs, double beta, double mu, double h,
              double lam2, double rtol, int maxit, cudaStream_t st,
              const double *beta_ptr = nullptr, const double *beta_each = nullptr,
-             const double *ata = nullptr);
+             const double *ata = nullptr, const PcgTail *tail = nullptr);
 // Subpb2 right-hand side (Subpb2.m:76-159) into w.b (2 fields: u, v)
 int fe_rhs(GridWork &w, int M, int N, double h, double beta, double mu, const double *U,
            const double *F, const double *udual, const double *vdual, cudaStream_t st,
@@ -217,27 +251,30 @@ int fe_rhs_parts(GridWork &w, int M, int N, double h, const double *U, const dou
 int fe_store(const GridWork &w, int M, int N, double *Uhat, cudaStream_t st, int f0 = 0);
 // nodal strain (funGlobal_NodalStrainAvg.m)
 int nodal_strain(int M, int N, double h, const double *U, double *F, cudaStream_t st);
-// gridfit springs: load nf interleaved (stride, offset) fields, NaN = no data;
-// the solve starts from the data and, at nodes without data, from guess (the
-// same layout as vals; 0 where null) -- the solution does not depend on it
-int gridfit_load(GridWork &w, int M, int N, int nf, const double *vals, int stride,
-                 const int *bad_iters, cudaStream_t st, int f0 = 0,
-                 const double *guess = nullptr);
-int grid_store(const GridWork &w, int M, int N, int nf, double *vals, int stride,
-               cudaStream_t st, int f0 = 0);
-// inpaint springs: load nf fields, nodes flagged (NaN or bad) are unknown
-int inpaint_load(GridWork &w, int M, int N, int nf, const double *vals, int stride,
-                 const unsigned char *badmask, cudaStream_t st, int f0 = 0);
-int inpaint_store(const GridWork &w, int M, int N, int nf, double *vals, int stride,
-                  cudaStream_t st, int f0 = 0);
+// gridfit 'springs' of nf fields of node values (NaN, or a status in bad < 0 or
+// > 99: no data) from in to out (not the same memory); the solve starts from
+// the data and, at nodes without data, from guess (0 where null) -- the
+// solution does not depend on it.  conv: followed by nanconv's 3 x 3 Gaussian
+// with edge normalisation.
+int gridfit_solve(GridWork &w, int M, int N, int nf, const FieldMap &in, const FieldMap &out,
+                  const int *bad, const FieldMap *guess, double lam2, double rtol, int maxit,
+                  bool conv, cudaStream_t st);
+// inpaint_nans method 4 of nf fields in place: entries that are NaN or whose
+// node is flagged in bad are replaced
+int inpaint_solve(GridWork &w, int M, int N, int nf, const FieldMap &vals, const unsigned char *bad,
+                  double rtol, int maxit, cudaStream_t st);
+// their tile kernels (k_local.cu)
+int fit_tiles(GridWork &w, int M, int N, int nf, const FieldMap &in, const FieldMap &out,
+              const int *bad, const FieldMap *guess, double lam2, double rtol, bool conv,
+              cudaStream_t st);
+int fill_tiles(GridWork &w, int M, int N, int nf, const FieldMap &vals, const unsigned char *bad,
+               double rtol, cudaStream_t st);
 // LocalICGN.m:117-131 flags; writes badmask and the bad count to d_badnum
 int icgn_flags(int M, int N, const int *iters, unsigned char *badmask, int *d_badnum,
                double *d_meaniters, int *d_nconv, cudaStream_t st, double floor = __builtin_nan(""));
 // Subpb1.m:167-169 flags
 int subpb1_flags(int n, const int *iters, unsigned char *badmask, int *d_badnum,
                  cudaStream_t st);
-// 3x3 Gaussian nanconv with edge normalisation on nf fields (in w.x)
-int nanconv3(GridWork &w, int M, int N, int nf, cudaStream_t st);
 // out = a - b (n elements)
 int vsub(const double *a, const double *b, double *out, long long n, cudaStream_t st);
 // o1 = a1 - b1, o2 = a2 - b2 in one launch

@@ -1,0 +1,103 @@
+"""The tiled node-grid solves (k_local.cu) against the oracle: gridfit springs
+and spring inpainting at tile edges, with nodes without data scattered, in
+clusters a tile can hold, and in regions only the grid-wide solver can take."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(2, 2), (3, 40), (31, 33), (32, 32), (65, 64), (97, 130)]
+
+
+def _data(M, N, nf, seed):
+    r = np.random.default_rng(seed)
+    j, i = np.mgrid[:N, :M]
+    z = np.stack([np.sin(0.1 * (k + 1) * i) + np.cos(0.13 * j + k) for k in range(nf)])
+    return z.reshape(nf, -1) + 0.1 * r.standard_normal((nf, M * N))
+
+
+def _holes(M, N, kind, seed):
+    """Flat mask of missing nodes."""
+    r = np.random.default_rng(seed + 100)
+    m = np.zeros((N, M), bool)
+    if kind == "scattered":
+        m = r.random((N, M)) < 0.01
+    elif kind == "dense":
+        m = r.random((N, M)) < 0.41
+    elif kind == "blocks":
+        for _ in range(max(1, M * N // 600)):
+            x, y = r.integers(0, M), r.integers(0, N)
+            m[y:y + 5, x:x + 6] = True
+    elif kind == "blob":       # wider than a tile and its halo
+        m[N // 8:N - N // 8, M // 8:M - M // 8] = True
+    elif kind == "snake":      # one connected path through several tiles
+        m[::4, :] = True
+        m[:, -1:] = True
+    m[0, 0] = m[N // 2, 0] = m[-1, -1] = False
+    return m.reshape(-1)
+
+
+@pytest.mark.parametrize("M,N", SIZES)
+@pytest.mark.parametrize("kind", ["none", "scattered", "blocks", "blob"])
+def test_gridfit_matches_oracle(aldic, oracle, M, N, kind):
+    z = _data(M, N, 2, M + N)
+    hole = _holes(M, N, kind, M)
+    z[:, hole] = np.nan
+    z[1, :M // 2] = np.nan           # the fields' masks differ
+    if np.isfinite(z).sum(1).min() < 3:
+        pytest.skip("gridfit needs three data")
+    ref = oracle.gridfit_springs(M, N, z)
+    got = aldic.gridfit_springs(M, N, z)
+    # |r| <= 1e-11 |b|; A's smallest eigenvalue is that of springs over the widest
+    # gap between data, lam2 (pi / (2 gap))^2 at least
+    gap = max(M, N) if kind == "blob" else 12
+    lmin = min(1.0, 0.0214 * (np.pi / (2 * gap)) ** 2)
+    tol = 1e-11 * np.linalg.norm(np.nan_to_num(z)) / lmin + 1e-12
+    np.testing.assert_allclose(got, ref, rtol=0, atol=tol)
+
+
+@pytest.mark.parametrize("M,N", SIZES)
+def test_gridfit_in_place_and_infinite_data(aldic, M, N):
+    import torch
+    z = torch.from_numpy(_data(M, N, 2, 3)).cuda()
+    ref = aldic.gridfit_springs(M, N, z)
+    inplace = z.clone()
+    ctx = aldic.default_context()
+    from importlib import import_module
+    lib = import_module("2d_aldic_b200._lib")
+    lib.call("aldic_gridfit_springs", ctx.h, M, N, 2, inplace.data_ptr(), inplace.data_ptr())
+    torch.testing.assert_close(inplace, ref, rtol=0, atol=0)
+    z[0, M * N // 2] = float("inf")  # no finite residual: the fields come back as they were
+    out = aldic.gridfit_springs(M, N, z)
+    torch.testing.assert_close(out[0], z[0], rtol=0, atol=0)
+    np.testing.assert_allclose(out[1].cpu(), ref[1].cpu(), rtol=0, atol=1e-9)
+
+
+@pytest.mark.parametrize("M,N", SIZES + [(243, 61)])
+@pytest.mark.parametrize("kind", ["none", "scattered", "dense", "blocks", "blob", "snake"])
+def test_inpaint_matches_oracle(aldic, oracle, M, N, kind):
+    z = _data(M, N, 1, M + 3 * N)[0]
+    z[_holes(M, N, kind, N)] = np.nan
+    if not np.isfinite(z).any():
+        pytest.skip("nothing known")
+    ref = oracle.inpaint_springs(M, N, z.copy())
+    got = aldic.inpaint_nans(z.reshape(N, M)).reshape(-1)
+    # |r| <= 1e-11 |b|, the Laplacian's smallest eigenvalue on a region of
+    # diameter d at least (pi / (2 d))^2
+    d = {"blob": max(M, N), "snake": M + N, "dense": 60}.get(kind, 8)
+    tol = 1e-11 * 4 * np.linalg.norm(np.nan_to_num(z)) * (2 * d / np.pi) ** 2 + 1e-12
+    np.testing.assert_allclose(got, ref, rtol=0, atol=tol)
+    np.testing.assert_array_equal(got[np.isfinite(z)], z[np.isfinite(z)])
+
+
+@pytest.mark.parametrize("M,N", [(2, 2), (33, 31), (97, 70)])
+@pytest.mark.parametrize("nf", [1, 2, 4])
+def test_smooth_matches_oracle(aldic, oracle, M, N, nf):
+    v = _data(M, N, nf, 5).T.copy()
+    v[_holes(M, N, "blocks", 1)[:, None] & (np.arange(nf) == 0)] = np.nan
+    from importlib import import_module
+    lib = import_module("2d_aldic_b200._lib")
+    got = v.reshape(-1).copy()
+    lib.call("aldic_smooth", aldic.default_context().h, M, N, nf, got.ctypes.data)
+    ref = oracle.smooth_fields(M, N, v.reshape(-1).copy(), nf)
+    np.testing.assert_allclose(got, ref, rtol=0, atol=1e-11 * np.linalg.norm(np.nan_to_num(v)) / (0.0214 * (np.pi / 24) ** 2))

@@ -252,6 +252,7 @@ struct PcgShared {
   double warp_part[PCG_THREADS / 32][4 * MAXRHS];
   double gsum[4 * MAXRHS];
   double alpha[MAXRHS], beta[MAXRHS], gam[MAXRHS], bb[MAXRHS];
+  double op_beta[MAXRHS];  // the operator's beta per right-hand side
   int done[MAXRHS];
 };
 
@@ -306,16 +307,15 @@ __device__ void global_sums(PcgShared &S, const double *part, int cnt, int block
 // diag(A); convergence on the recursive residual, |r| <= rtol |b|.
 // Buffers: x, r, u (= z slot), w (= q slot), m (p0 / p1), the directions
 // zz, qq, ss, pp, 1/diag.
+// (The arguments are never written to: a changed copy of them lived in every
+// thread's local memory, 6 us a launch.)
 template <int OP, int NR>
-__global__ void __launch_bounds__(PCG_THREADS) k_pcg(PcgArgs A) {
+__global__ void __launch_bounds__(PCG_THREADS) k_pcg(const __grid_constant__ PcgArgs A) {
   __shared__ PcgShared S;
   const int gate = A.gate ? *A.gate : 1;
   if (gate == 0) return;  // the tiles solved it
-  if (A.beta_ptr) {
-    const double bv = *A.beta_ptr;
-#pragma unroll
-    for (int f = 0; f < NR; ++f) A.beta[f] = bv;
-  }
+  if (threadIdx.x < NR) S.op_beta[threadIdx.x] = A.beta_ptr ? *A.beta_ptr : A.beta[threadIdx.x];
+  __syncthreads();
   const long long n = (long long)A.M * A.N;
   const int M = A.M;
   const long long tid0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_pcg(PcgArgs A) {
   // ---- r = b - A x, u = D^-1 r, directions 0
 #pragma unroll 1
   for (int f = 0; f < NR; ++f) {
-    const double bt = A.beta[f];
+    const double bt = S.op_beta[f];
     for (long long k = tid0; k < n; k += stride) {
       const int j = (int)k / M, i = (int)k - j * M;  // n < 2^31 (checked at launch)
       const long long o = f * n + k;
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_pcg(PcgArgs A) {
   // ---- w = A u, m = D^-1 w; partials (r,u) (w,u) (r,r) (b,b)
 #pragma unroll 1
   for (int f = 0; f < NR; ++f) {
-    const double bt = A.beta[f];
+    const double bt = S.op_beta[f];
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
     for (long long k = tid0; k < n; k += stride) {
       const int j = (int)k / M, i = (int)k - j * M;  // n < 2^31 (checked at launch)
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_pcg(PcgArgs A) {
         const int f = f0 + q;
         live[q] = f < NR && !S.done[f];
         anylive |= live[q];
-        bt[q] = f < NR ? A.beta[f] : 0.0;
+        bt[q] = f < NR ? S.op_beta[f] : 0.0;
         al[q] = f < NR ? S.alpha[f] : 0.0;
         be[q] = f < NR ? S.beta[f] : 0.0;
       }

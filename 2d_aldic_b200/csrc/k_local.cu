@@ -31,13 +31,14 @@ namespace {
 // result; where |r| > rtol |b| (clusters of nodes without data), k_pcg goes
 // on from it, with the same stopping test as ever.
 //
-// Shape: 64 x 64 region, 32 x 32 tile, 512 threads, a thread marching 8 rows
-// of a column (x, d, b, 1/D in registers; 22 shared loads for 8 nodes).  The
-// launch is bound by shared-memory wavefronts (two per 8-byte warp load).
-// Two fields of 243 x 243 (ncu, cold caches): 20 us, and 9 us for the k_pcg
-// behind it that finds nothing to do, where k_pcg alone took 63 us.
+// Shape: 64 x 64 region, 32 x 32 tile, 1024 threads, a thread marching 4 rows
+// of a column (x, d, b, 1/D in registers; 14 shared loads for 4 nodes).  The
+// launch is bound by latency: a CTA an SM, and two fields of 243 x 243 are 128
+// CTAs, so more threads with fewer rows won (18.6 us under ncu with cold
+// caches, against 22 for 512 threads with 8 rows).  k_pcg alone took 63 us;
+// behind the tiles, with nothing to do, it takes 2.6.
 constexpr int kFitTile = 32, kFitHalo = 16, kFitReg = kFitTile + 2 * kFitHalo, kFitPitch = kFitReg + 2;
-constexpr int kFitRows = 8, kFitThreads = kFitReg * kFitReg / kFitRows;
+constexpr int kFitRows = 4, kFitThreads = kFitReg * kFitReg / kFitRows;
 constexpr int kFitSteps = 12;
 constexpr double kFitRho = 0.15;
 static_assert(kFitHalo >= kFitSteps + 2, "the residual and the convolution read one more ring");
@@ -262,9 +263,8 @@ __global__ void k_fill_load(const __grid_constant__ FillArgs A) {
 // two block barriers instead of a grid barrier.  A cluster that leaves the
 // region, more than kFillCap nodes, or an iteration that does not converge set
 // the gate and keep their start values for k_pcg.  The refill of LocalICGN's
-// six fields (ncu): 146 -> 25 us at 243 x 243 with 0.6 % of the nodes flagged,
-// 450 -> 42 us at 43 x 43 with 41 %, of which 9 us are the k_pcg that finds
-// nothing to do.
+// six fields (ncu): 146 -> 17 us at 243 x 243 with 0.6 % of the nodes flagged,
+// 450 -> 33 us at 43 x 43 with 41 %.
 constexpr int kFillTile = 32, kFillHalo = 24, kFillReg = kFillTile + 2 * kFillHalo;
 constexpr int kFillPitch = kFillReg + 2, kFillWords = 3, kFillThreads = 256;
 constexpr int kFillPer = 8, kFillCap = kFillPer * kFillThreads, kFillMaxit = 4000;

@@ -12,9 +12,9 @@
 //   L3  dense 4096 -> 256, ReLU                y3 [B, 256]
 //   L4  dense 256 -> 8 (FP32)                  out [B, 8]: u/16, v/16,
 //        20 du/dx, 20 dv/dx, 20 du/dy, 20 dv/dy, confidence logit, 0
-// E1, E2, C and L3 run on the tcgen05 GEMM (bf16 operands, FP32
-// accumulation; C as B independent 64 x 64 x 128 products); their backward
-// products are the same GEMM with transposed operands.  The encoder sees
+// The forward pass is two tensor-core kernels (k_net.cu; bf16 operands, FP32
+// accumulation); the backward products run on the tcgen05 GEMM of k_gemm.cu
+// with transposed operands.  The encoder sees
 // both patches as one batch of 2B, so its weight gradients sum over both.
 // Parameters are FP32 masters updated by Adam; bf16 copies feed the GEMMs.
 #include <cuda_bf16.h>
@@ -115,17 +115,6 @@ __global__ void k_f2bf(const float *__restrict__ a, bf16 *__restrict__ b, long l
     b[k] = __float2bfloat16_rn(a[k]);
 }
 
-// out[b][o] = y[b] . W[o] + bias[o] (the FP32 output layer)
-__global__ void k_fc5(const bf16 *__restrict__ y4, const float *__restrict__ W5,
-                      const float *__restrict__ b5, float *__restrict__ out, int B) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= B * cnn::NOUT) return;
-  const int b = t / cnn::NOUT, o = t - b * cnn::NOUT;
-  float s = b5[o];
-  for (int k = 0; k < cnn::K5; ++k) s += __bfloat162float(y4[(long long)b * cnn::K5 + k]) * W5[o * cnn::K5 + k];
-  out[t] = s;
-}
-
 // loss = mean over the batch of sum_i (o_i - t_i)^2 (i < 6) + BCE of the
 // confidence against "translation within 0.5 px"; dout = d loss / d out
 __global__ void k_loss(const float *__restrict__ out, const float *__restrict__ tgt, int B,
@@ -203,19 +192,6 @@ __global__ void k_splitk_sum(const float *__restrict__ part, int splits, long lo
   }
 }
 
-// the split-K partials of a forward layer summed in split order, + bias,
-// ReLU, rounded to bf16 (the epilogue the unsplit product applies)
-__global__ void k_splitk_relu(const float *__restrict__ part, int splits, long long n, int N,
-                              const float *__restrict__ bias, bf16 *__restrict__ out) {
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-       k += (long long)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int z = 0; z < splits; ++z) s += part[(long long)z * n + k];
-    s += bias[k % N];
-    out[k] = __float2bfloat16_rn(s > 0.f ? s : 0.f);
-  }
-}
-
 // Adam (beta1 0.9, beta2 0.999, eps 1e-8) on an FP32 block; optional bf16 copy
 __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
                        float *__restrict__ v, long long n, float lr, float c1, float c2,
@@ -259,7 +235,7 @@ using namespace aldic;
 
 struct aldic_cnn {
   int device = 0;
-  int maxB = 0;
+  int maxB = 0, maxTrain = 0;
   long long steps = 0;
   DevBuf prm, grad, adm, adv, wbf;  // packed FP32 parameters, gradients, Adam moments; bf16 W1-W3
   DevBuf xin, x0, e1, e2, corr, y3, out, dout, dz3, dcorr, de2, dz1, part, err, loss, tgt;
@@ -298,66 +274,45 @@ GemmDst dst(void *p, long long M, long long N, long long ld, int fp32, const flo
   return d;
 }
 
-int ensure(aldic_cnn *c, int B) {
-  if (B <= c->maxB) return OK;
+// buffers of a batch; the backward pass's only when it trains
+int ensure(aldic_cnn *c, int B, bool train) {
   const long long b = B, cells = 2 * b * cnn::CELLS;
   int rc;
-  if ((rc = c->xin.ensure(2 * b * cnn::P * cnn::P * 2)) || (rc = c->x0.ensure(2 * 2 * b * cnn::P * cnn::P)) ||
-      (rc = c->e1.ensure(2 * cells * cnn::C1)) || (rc = c->e2.ensure(2 * cells * cnn::C2)) ||
-      (rc = c->corr.ensure(2 * b * cnn::K3)) || (rc = c->y3.ensure(2 * b * cnn::F3)) ||
-      (rc = c->out.ensure(4 * b * cnn::NOUT)) || (rc = c->dout.ensure(4 * b * cnn::NOUT)) ||
-      (rc = c->dz3.ensure(2 * b * cnn::F3)) || (rc = c->dcorr.ensure(2 * b * cnn::K3)) ||
-      (rc = c->de2.ensure(2 * cells * cnn::C2)) || (rc = c->dz1.ensure(2 * cells * cnn::C1)) ||
-      (rc = c->tgt.ensure(4 * b * 6)))
-    return rc;
-  c->maxB = B;
+  if (B > c->maxB) {
+    if ((rc = c->corr.ensure(2 * b * cnn::K3)) || (rc = c->y3.ensure(2 * b * cnn::F3)) ||
+        (rc = c->out.ensure(4 * b * cnn::NOUT)))
+      return rc;
+    c->maxB = B;
+  }
+  if (train && B > c->maxTrain) {
+    if ((rc = c->x0.ensure(2 * 2 * b * cnn::P * cnn::P)) || (rc = c->e1.ensure(2 * cells * cnn::C1)) ||
+        (rc = c->e2.ensure(2 * cells * cnn::C2)) || (rc = c->dout.ensure(4 * b * cnn::NOUT)) ||
+        (rc = c->dz3.ensure(2 * b * cnn::F3)) || (rc = c->dcorr.ensure(2 * b * cnn::K3)) ||
+        (rc = c->de2.ensure(2 * cells * cnn::C2)) || (rc = c->dz1.ensure(2 * cells * cnn::C1)) ||
+        (rc = c->tgt.ensure(4 * b * 6)))
+      return rc;
+    c->maxTrain = B;
+  }
   return OK;
 }
 
 constexpr float kCorrScale = 0.08838834764831845f;  // 1 / sqrt(128)
 
-int forward(aldic_cnn *c, int B, cudaStream_t st) {
-  int *err = c->err.as<int>();
+// x: the pairs in device memory; train keeps what the backward pass reads
+int forward(aldic_cnn *c, const void *x, int B, bool train, float *out, cudaStream_t st) {
+  const long long b = B;
   int rc;
-  const long long b = B, cells = 2 * b * cnn::CELLS, fs = (long long)cnn::CELLS * cnn::C2;
-  k_split<<<nblk(b * cnn::P * cnn::P), 256, 0, st>>>(c->xin.as<bf16>(), b, c->x0.as<bf16>());
-  ALDIC_CUDA(cudaGetLastError());
-  // E1: 8x8 patch embedding of both patches
-  if ((rc = gemm_bf16(src(c->x0.p, GEMM_PATCH, cells, cnn::K1, 0, cnn::P, cnn::P, 1, cnn::PS),
-                      src(c->Wb(0), GEMM_ROW, cnn::C1, cnn::K1, cnn::K1),
-                      dst(c->e1.p, cells, cnn::C1, cnn::C1, 0, c->Bv(0), 1), 1, err, st)))
-    return rc;
-  // E2: 1x1 (linear)
-  if ((rc = gemm_bf16(src(c->e1.p, GEMM_ROW, cells, cnn::K2, cnn::C1),
-                      src(c->Wb(1), GEMM_ROW, cnn::C2, cnn::K2, cnn::K2),
-                      dst(c->e2.p, cells, cnn::C2, cnn::C2, 0, c->Bv(1), 0), 1, err, st)))
-    return rc;
-  // C: per pair, reference cells x deformed cells
-  GemmDst dc = dst(c->corr.p, cnn::CELLS, cnn::CELLS, cnn::CELLS, 0, nullptr, 0);
-  dc.scale = kCorrScale;
-  dc.bstride = cnn::K3;
-  if ((rc = gemm_bf16(src(c->e2.p, GEMM_ROW, cnn::CELLS, cnn::C2, cnn::C2, 0, 0, 0, 0, fs),
-                      src(c->e2.as<bf16>() + b * fs, GEMM_ROW, cnn::CELLS, cnn::C2, cnn::C2, 0, 0, 0, 0, fs),
-                      dc, 1, err, st, B)))
-    return rc;
-  // L3: K = 4096 on only b / 128 row tiles -- split K eight ways into FP32
-  // partials, then sum, bias and ReLU in one pass
-  {
-    constexpr int kL3Split = 8;
-    const long long n3 = b * cnn::F3;
-    if ((rc = c->part.ensure(sizeof(float) * n3 * kL3Split))) return rc;
-    GemmDst d3 = dst(c->part.p, b, cnn::F3, cnn::F3, 1, nullptr, 0);
-    d3.split_stride = n3;
-    if ((rc = gemm_bf16(src(c->corr.p, GEMM_ROW, b, cnn::K3, cnn::K3),
-                        src(c->Wb(2), GEMM_ROW, cnn::F3, cnn::K3, cnn::K3), d3, kL3Split, err, st)))
-      return rc;
-    k_splitk_relu<<<nblk(n3), 256, 0, st>>>(c->part.as<float>(), kL3Split, n3, cnn::F3, c->Bv(2),
-                                            c->y3.as<bf16>());
+  if (train) {
+    k_split<<<nblk(b * cnn::P * cnn::P), 256, 0, st>>>((const bf16 *)x, b, c->x0.as<bf16>());
     ALDIC_CUDA(cudaGetLastError());
   }
-  k_fc5<<<nblk(b * cnn::NOUT), 256, 0, st>>>(c->y3.as<bf16>(), c->W(3), c->Bv(3), c->out.as<float>(), B);
-  ALDIC_CUDA(cudaGetLastError());
-  return OK;
+  const int splits = net_dense_splits(B);
+  if (splits > 1 && (rc = c->part.ensure(sizeof(float) * b * cnn::F3 * splits))) return rc;
+  if ((rc = net_encode(x, B, c->Wb(0), c->Bv(0), c->Wb(1), c->Bv(1), kCorrScale, c->corr.p,
+                       train ? c->e1.p : nullptr, train ? c->e2.p : nullptr, c->err.as<int>(), st)))
+    return rc;
+  return net_dense(c->corr.p, B, c->Wb(2), c->Bv(2), c->W(3), c->Bv(3), c->y3.p, out, c->part.as<float>(),
+                   c->err.as<int>(), st);
 }
 
 // dW = A . B^T product with split-K, summed into g
@@ -466,21 +421,34 @@ int check_err(aldic_cnn *c, cudaStream_t st) {
   return OK;
 }
 
-// network input: fp32 (host or device) or bf16 (device) patches
-int load_input(aldic_cnn *c, const void *x, int x_bf16, int B, cudaStream_t st) {
+bool on_device(const void *p) {
+  cudaPointerAttributes at;
+  const bool dev = cudaPointerGetAttributes(&at, p) == cudaSuccess &&
+                   (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged);
+  cudaGetLastError();
+  return dev;
+}
+
+// network input: fp32 (host or device) or bf16 patches -> *pairs, in device
+// memory: the caller's own where the kernels can read it (the call waits for
+// them before it returns), else a copy
+int load_input(aldic_cnn *c, const void *x, int x_bf16, int B, const void **pairs, cudaStream_t st) {
   const long long n = (long long)B * cnn::P * cnn::P * 2;
+  const bool dev = on_device(x);
+  if (x_bf16 && dev && (uintptr_t)x % 16 == 0) {
+    *pairs = x;
+    return OK;
+  }
+  int rc;
+  if ((rc = c->xin.ensure(2 * n))) return rc;
+  *pairs = c->xin.p;
   if (x_bf16) {
     ALDIC_CUDA(cudaMemcpyAsync(c->xin.p, x, 2 * n, cudaMemcpyDefault, st));
     return OK;
   }
   DevBuf tmp;
   const float *xd = (const float *)x;
-  cudaPointerAttributes at;
-  const bool dev = cudaPointerGetAttributes(&at, x) == cudaSuccess &&
-                   (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged);
-  cudaGetLastError();
   if (!dev) {
-    int rc;
     if ((rc = tmp.ensure(4 * n))) return rc;
     ALDIC_CUDA(cudaMemcpyAsync(tmp.p, x, 4 * n, cudaMemcpyHostToDevice, st));
     xd = tmp.as<float>();
@@ -596,13 +564,14 @@ int aldic_cnn_train_step(aldic_cnn *c, const void *x, int x_bf16, const float *t
   cudaGetDevice(&prev);
   cudaSetDevice(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = ensure(c, B);
-  if (!rc) rc = load_input(c, x, x_bf16, B, st);
+  const void *pairs = nullptr;
+  int rc = ensure(c, B, true);
+  if (!rc) rc = load_input(c, x, x_bf16, B, &pairs, st);
   if (!rc && cudaMemcpyAsync(c->tgt.p, targets, sizeof(float) * 6 * B, cudaMemcpyDefault, st) != cudaSuccess) {
     set_error("cnn_train_step: target copy failed");
     rc = E_CUDA;
   }
-  if (!rc) rc = forward(c, B, st);
+  if (!rc) rc = forward(c, pairs, B, true, c->out.as<float>(), st);
   if (!rc) {
     cudaMemsetAsync(c->loss.p, 0, sizeof(double), st);
     k_loss<<<(B + 255) / 256, 256, 0, st>>>(c->out.as<float>(), c->tgt.as<float>(), B,
@@ -627,10 +596,12 @@ int aldic_cnn_predict(aldic_cnn *c, const void *x, int x_bf16, int B, void *stre
   cudaGetDevice(&prev);
   cudaSetDevice(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = ensure(c, B);
-  if (!rc) rc = load_input(c, x, x_bf16, B, st);
-  if (!rc) rc = forward(c, B, st);
-  if (!rc && cudaMemcpyAsync(out, c->out.p, 4LL * B * cnn::NOUT, cudaMemcpyDefault, st) != cudaSuccess)
+  const void *pairs = nullptr;
+  int rc = ensure(c, B, false);
+  if (!rc) rc = load_input(c, x, x_bf16, B, &pairs, st);
+  const bool direct = on_device(out) && (uintptr_t)out % 16 == 0;
+  if (!rc) rc = forward(c, pairs, B, false, direct ? out : c->out.as<float>(), st);
+  if (!rc && !direct && cudaMemcpyAsync(out, c->out.p, 4LL * B * cnn::NOUT, cudaMemcpyDefault, st) != cudaSuccess)
     rc = E_CUDA;
   if (!rc) rc = check_err(c, st);
   cudaSetDevice(prev);

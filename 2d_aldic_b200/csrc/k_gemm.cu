@@ -20,16 +20,13 @@
 
 #include "aldic_internal.cuh"
 #include "kernels.cuh"
+#include "tc.cuh"
 
 namespace aldic {
 
 namespace {
 
-constexpr int BM = 128, BK = 64, GEMM_THREADS = 128;
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
+constexpr int BM = TC_M, BK = 64, GEMM_THREADS = 128;
 
 // element address of operand (r, k) for the direct modes (ROW, PATCH)
 __device__ __forceinline__ const __nv_bfloat16 *src_addr(const GemmSrc &S, long long r, long long k) {
@@ -76,73 +73,6 @@ __device__ __forceinline__ void stage(const GemmSrc &S, long long r0, long long 
       }
     }
   }
-}
-
-// K-major, 128-byte swizzle shared-memory matrix descriptor (sm_100 format:
-// start >> 4 in [0,14), LBO 16 B in [16,30), SBO 1024 B (8 rows x 128 B)
-// in [32,46), version 1 in [46,48), layout SWIZZLE_128B = 2 in [61,64))
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
-// kind::f16 instruction descriptor: D F32, A and B BF16, both K-major,
-// N >> 3 in [17,23), M >> 4 in [24,29)
-template <int BN>
-__device__ __forceinline__ uint32_t idesc() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t id,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
-      "l"(da), "l"(db), "r"(id), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0));
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-
-// bounded wait on an mbarrier phase; false after ~2^26 polls
-__device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
-  const uint32_t a = smem_u32(bar);
-  for (uint32_t it = 0; it < (1u << 26); ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred P1;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, P1;\n\t}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (it > 64) __nanosleep(64);
-  }
-  return false;
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-      "%12, %13, %14, %15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 // destination element offset of (m, n)
@@ -196,7 +126,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(GemmSrc A, GemmSrc B, Gem
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base;
-  const uint32_t id = idesc<BN>();
+  const uint32_t id = idesc(BN);
   uint32_t phase[2] = {0, 0};
 
   if (nk > 0) {

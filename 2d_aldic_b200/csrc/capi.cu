@@ -456,8 +456,9 @@ int aldic_set_ref(aldic_ctx *c, const void *img, int dtype, int W, int H, const 
     if ((rc = b->ensure(sizeof(float) * n))) return rc;
   if ((rc = c->gc.ensure(sizeof(float4) * n))) return rc;
   if ((rc = c->gxy.ensure(sizeof(float2) * n))) return rc;
-  if ((rc = c->f_raw.ensure(es * n))) return rc;
-  if ((rc = c->g_raw.ensure(es * n))) return rc;
+  // 16 spare bytes: the search reads whole words around its regions
+  if ((rc = c->f_raw.ensure(es * n + 16))) return rc;
+  if ((rc = c->g_raw.ensure(es * n + 16))) return rc;
   if (c->dtype != dtype || c->W != W || c->H != H) c->have_def = false;
   c->W = W;
   c->H = H;

@@ -8,15 +8,20 @@
 // On 8-bit images every template row's partial correlation is an exact
 // integer in FP32 (<= 65 * 255^2 < 2^24) and is flushed to a 64-bit integer,
 // so the correlation maps are exact; 16-bit images use 32x32->64-bit integer
-// multiply-adds.  The normalised cross-correlation is then formed from those
+// multiply-adds.  That kernel serves floating-point images and the regions
+// too large for the tensor-core one (k_search_mma.cu), which takes 8- and
+// 16-bit images; 8-bit images whose step divides the subset go by tiles
+// (below).  The normalised cross-correlation is then formed from those
 // integers with a fixed FP64 formula (explicit rounding, no contraction)
 // shared with the CPU restatement, which makes argmax and the 1e-3-rounded
 // sub-pixel peak bit-identical to it.
 #include <algorithm>
+#include <type_traits>
 
 #include "aldic_internal.cuh"
 #include "kernels.cuh"
 #include "ncc.cuh"
+#include "search.cuh"
 
 namespace aldic {
 
@@ -50,14 +55,6 @@ template <> struct SearchTraits<double> : SearchTraits<float> {};
 // S = integral sums type of the box sums
 template <bool INT> struct SumT { using type = long long; };
 template <> struct SumT<false> { using type = double; };
-
-struct SearchGeom {
-  int W, H;
-  int gx1, gy1, nx, ny, step;
-  int w, sx, sy;
-  int tw, twp, dw, dh, cr, cc, nsx, dpw, dph;
-  const double *mu;  // device pointer: ROI mean of the deformed image
-};
 
 __host__ __device__ inline size_t align16(size_t v) { return (v + 15) & ~size_t(15); }
 
@@ -334,515 +331,6 @@ __global__ void __launch_bounds__(512) k_search(const T *__restrict__ f, const T
   }
 }
 
-// ---- 8-bit images: byte-packed correlation with __dp4a (exact int32).
-// The padded region is staged once as aligned 32-bit words (4 pixels each);
-// the 4-pixel window starting at any column is one funnel shift of two
-// neighbouring words, and the template row is packed 4 pixels per word.  A
-// thread owns 8 consecutive shifts of one window row: per template word it
-// loads one template word and one region word, forms 8 windows and issues 8
-// dp4a -- 32 exact multiply-adds.
-struct U8Layout {
-  int tw4, dqw;  // template words per row, region words per row (odd pitch)
-  size_t tb, dw, tq, rs, cs, map, red, total;
-  __host__ __device__ U8Layout(const SearchGeom &g) {
-    tw4 = (g.tw + 3) / 4;
-    // words read: up to (nsx-1)*2 + tw4 + 1; the bytes must also hold the
-    // padded region (dw + 2) and the row-sum window (cr + tw)
-    int need = 2 * g.nsx + tw4 + 2;
-    const int nb = (g.cr + g.tw + 3) / 4 + 1;
-    if (need < nb) need = nb;
-    dqw = need | 1;  // odd pitch: the rows a warp touches fall on different banks
-    size_t o = 0;
-    tb = o; o = align16(o + (size_t)g.tw * g.tw);
-    dw = o; o = align16(o + sizeof(unsigned) * g.dph * dqw);
-    tq = o; o = align16(o + sizeof(unsigned) * g.tw * tw4);
-    // window row sums RS, RS2 (dph x cr each); dead once the box sums are
-    // formed, after which the NCC map (cr x cc doubles) reuses the space
-    rs = o;
-    const size_t rsz = sizeof(int) * 2 * g.dph * g.cr, msz = sizeof(double) * g.cr * g.cc;
-    o = align16(o + (rsz > msz ? rsz : msz));
-    map = rs;
-    cs = o; o = align16(o + sizeof(int) * 2 * g.cc * g.cr);  // box sums of D and D^2
-    red = o; o = align16(o + (sizeof(double) + sizeof(int)) * 32 + 64);
-    total = o;
-  }
-};
-
-__device__ __forceinline__ void search_point_u8(const uint8_t *__restrict__ f,
-                                                const uint8_t *__restrict__ g,
-                                                const SearchGeom &G, const int pt,
-                                                double *__restrict__ ox, double *__restrict__ oy,
-                                                double *__restrict__ ou, double *__restrict__ ov,
-                                                double *__restrict__ occ) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const U8Layout L(G);
-  uint8_t *Tb = smem + L.tb;                 // template bytes, tw x tw
-  unsigned *Dw = (unsigned *)(smem + L.dw);  // padded region, dph rows of dqw words
-  const uint8_t *Db = (const uint8_t *)Dw;   // the same, as bytes (row pitch 4*dqw)
-  unsigned *Tq = (unsigned *)(smem + L.tq);
-  int *RS = (int *)(smem + L.rs);
-  int *RS2 = RS + G.dph * G.cr;
-  int *CS = (int *)(smem + L.cs);
-  int *CS2 = CS + G.cc * G.cr;
-  double *map = (double *)(smem + L.map);
-  double *redv = (double *)(smem + L.red);
-  int *redi = (int *)(redv + 32);
-  __shared__ long long s_st, s_st2;
-  __shared__ int colsum_s[72], rowsum_s[72];
-  const double mu = *G.mu;
-  const int ix = pt % G.nx, iy = pt / G.nx;
-  const int ii = G.gx1 + ix * G.step, jj = G.gy1 + iy * G.step;  // 1-based
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const int lane = tid & 31, wid = tid >> 5, nwarp = nth >> 5;
-  const uint8_t *trow0 = f + (long long)(jj - 1) * G.W + (ii - 1);
-  const uint8_t *drow0 = g + (long long)(jj - 1 - G.sy) * G.W + (ii - 1 - G.sx);
-  const int dbp = 4 * L.dqw;  // byte pitch
-  // ---- stage template bytes and the padded region (warp per row, lanes over
-  // columns; 1-pixel zero border at the top/left, zeros beyond the region)
-  for (int ty = wid; ty < G.tw; ty += nwarp)
-    for (int tx = lane; tx < G.tw; tx += 32) Tb[ty * G.tw + tx] = trow0[(long long)ty * G.W + tx];
-  for (int y = wid; y < G.dph; y += nwarp) {
-    const bool rin = y >= 1 && y <= G.dh;
-    const uint8_t *src = drow0 + (long long)(y - 1) * G.W;
-    for (int w4 = lane; w4 < L.dqw; w4 += 32) {
-      unsigned v = 0;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int x = 4 * w4 + k;
-        if (rin && x >= 1 && x <= G.dw) v |= (unsigned)src[x - 1] << (8 * k);
-      }
-      Dw[y * L.dqw + w4] = v;
-    }
-  }
-  __syncthreads();
-  // ---- packed template words, window row sums, template sums
-  for (int ty = wid; ty < G.tw; ty += nwarp)
-    for (int w4 = lane; w4 < L.tw4; w4 += 32) {
-      unsigned v = 0;
-      for (int k = 0; k < 4; ++k) {
-        const int tx = 4 * w4 + k;
-        if (tx < G.tw) v |= (unsigned)Tb[ty * G.tw + tx] << (8 * k);
-      }
-      Tq[ty * L.tw4 + w4] = v;
-    }
-  for (int y = tid; y < G.dph; y += nth) {
-    const uint8_t *row = Db + y * dbp;
-    int s1 = 0, s2 = 0;
-    for (int k = 0; k < G.tw; ++k) {
-      const int v = row[k];
-      s1 += v;
-      s2 += v * v;
-    }
-    for (int a = 0; a < G.cr; ++a) {
-      RS[y * G.cr + a] = s1;
-      RS2[y * G.cr + a] = s2;
-      const int vo = row[a], vi = row[a + G.tw];
-      s1 += vi - vo;
-      s2 += vi * vi - vo * vo;
-    }
-  }
-  for (int i = tid; i < G.tw; i += nth) {
-    int cs = 0, rsum = 0;
-    for (int k = 0; k < G.tw; ++k) {
-      cs += Tb[k * G.tw + i];
-      rsum += Tb[i * G.tw + k];
-    }
-    colsum_s[i] = cs;
-    rowsum_s[i] = rsum;
-  }
-  if (tid < 32) {
-    long long a = 0, a2 = 0;
-    for (int i = tid; i < G.tw * G.tw; i += 32) {
-      const long long v = Tb[i];
-      a += v;
-      a2 += v * v;
-    }
-    a = warp_sum_ll(a);
-    a2 = warp_sum_ll(a2);
-    if (tid == 0) {
-      s_st = a;
-      s_st2 = a2;
-    }
-  }
-  __syncthreads();
-  // ---- box sums of D and D^2 over every window: slide the row sums down
-  for (int a = tid; a < 2 * G.cr; a += nth) {
-    const int col = a < G.cr ? a : a - G.cr;
-    const int *R = a < G.cr ? RS : RS2;
-    int *Cc = a < G.cr ? CS : CS2;
-    int s1 = 0;
-    for (int k = 0; k < G.tw; ++k) s1 += R[k * G.cr + col];
-    for (int b = 0; b < G.cc; ++b) {
-      Cc[b * G.cr + col] = s1;
-      s1 += R[(b + G.tw) * G.cr + col] - R[b * G.cr + col];
-    }
-  }
-  __syncthreads();  // RS is dead from here on; the map takes its place
-  const long long st = s_st, st2 = s_st2;
-  const long long mn = (long long)G.tw * G.tw;
-  const long long out_idx = (long long)iy + (long long)ix * G.ny;
-  if (mn * st2 - st * st == 0) {
-    if (tid == 0) {
-      const double nan = __longlong_as_double(0x7ff8000000000000ll);
-      ox[out_idx] = (ii + ii + G.w) / 2.0;
-      oy[out_idx] = (jj + jj + G.w) / 2.0;
-      ou[out_idx] = nan;
-      ov[out_idx] = nan;
-      occ[out_idx] = nan;
-    }
-    return;
-  }
-  // ---- correlation strips: 8 shifts of one window row per thread
-  const int nstrips = G.cc * G.nsx;
-  for (int sidx = tid; sidx < nstrips; sidx += nth) {
-    const int b = sidx / G.nsx;
-    const int a0 = (sidx % G.nsx) * KX;  // multiple of 8
-    unsigned acc[KX];
-#pragma unroll
-    for (int k = 0; k < KX; ++k) acc[k] = 0u;
-    const int wbase = a0 >> 2;
-    for (int ty = 0; ty < G.tw; ++ty) {
-      const unsigned *trow = Tq + ty * L.tw4;
-      const unsigned *dr = Dw + (b + ty) * L.dqw + wbase;
-      // windows of the word pair (w0, w1) shifted by 1..3 bytes; each step
-      // computes the shifts of (w1, w2) once and hands them to the next step
-      unsigned w0 = dr[0], w1 = dr[1];
-      unsigned s1 = __funnelshift_r(w0, w1, 8), s2 = __funnelshift_r(w0, w1, 16),
-               s3 = __funnelshift_r(w0, w1, 24);
-#pragma unroll 3
-      for (int jw = 0; jw < L.tw4; ++jw) {
-        const unsigned t = trow[jw];
-        const unsigned w2 = dr[jw + 2];
-        const unsigned n1 = __funnelshift_r(w1, w2, 8), n2 = __funnelshift_r(w1, w2, 16),
-                       n3 = __funnelshift_r(w1, w2, 24);
-        acc[0] = __dp4a(t, w0, acc[0]);
-        acc[1] = __dp4a(t, s1, acc[1]);
-        acc[2] = __dp4a(t, s2, acc[2]);
-        acc[3] = __dp4a(t, s3, acc[3]);
-        acc[4] = __dp4a(t, w1, acc[4]);
-        acc[5] = __dp4a(t, n1, acc[5]);
-        acc[6] = __dp4a(t, n2, acc[6]);
-        acc[7] = __dp4a(t, n3, acc[7]);
-        w0 = w1;
-        w1 = w2;
-        s1 = n1;
-        s2 = n2;
-        s3 = n3;
-      }
-    }
-    const bool ring_b = (b == 0 || b == G.cc - 1);
-#pragma unroll
-    for (int k = 0; k < KX; ++k) {
-      const int a = a0 + k;
-      if (a >= G.cr) break;
-      const long long sd = CS[b * G.cr + a], sd2 = CS2[b * G.cr + a];
-      // Only the outermost ring of the cropped map overhangs the region, by
-      // one template column (a = 0: column 0; a = cr-1: column tw-1) and/or
-      // one template row (b = 0 / cc-1), so the padded part is O(1).
-      int st_out = 0;
-      long long n_out = 0;
-      if (ring_b || a == 0 || a == G.cr - 1) {
-        const int oc = a == 0 ? 0 : (a == G.cr - 1 ? G.tw - 1 : -1);
-        const int orow = b == 0 ? 0 : (b == G.cc - 1 ? G.tw - 1 : -1);
-        if (oc >= 0) st_out += colsum_s[oc];
-        if (orow >= 0) st_out += rowsum_s[orow];
-        if (oc >= 0 && orow >= 0) st_out -= Tb[orow * G.tw + oc];
-        const long long nco = oc >= 0, nro = orow >= 0;
-        n_out = nco * G.tw + nro * G.tw - nco * nro;
-      }
-      map[b * G.cr + a] = ncc_combine(mn, st, st2, (long long)acc[k], sd, sd2, st_out, n_out, mu);
-    }
-  }
-  __syncthreads();
-  peak_epilogue(map, G, ii, jj, out_idx, redv, redi, ox, oy, ou, ov, occ);
-}
-
-// ---- 16-bit images: the same strips with __dp2a (16-bit x 8-bit, exact).
-// The padded region is staged as two byte planes (high and low bytes of each
-// pixel) in the word layout of the 8-bit path, the template as 16-bit pairs;
-// with g = 256 gh + gl, sum t g = 256 sum t gh + sum t gl, and __dp2a_lo /
-// __dp2a_hi take the pixel pair at bytes 0-1 / 2-3 of a plane word, so the
-// words at byte offsets 2j, 2j+1, 2j+4, 2j+5 from a strip's first shift give
-// all 8 shifts of template pair j.  Per template row the two 32-bit partial
-// sums (at most 17 pairs of products below 2^25) are folded into a 64-bit
-// total.
-struct U16Layout {
-  int tw4, tp, dqw;  // 4-pixel template groups per row, pair words per row, plane words per row
-  size_t tb, dh, dl, tq, rs, rs2, cs, cs2, map, red, total;
-  __host__ __device__ U16Layout(const SearchGeom &g) {
-    tw4 = (g.tw + 3) / 4;
-    tp = 2 * tw4;
-    int need = 2 * g.nsx + tw4 + 2;
-    const int nb = (g.cr + g.tw + 3) / 4 + 1;
-    if (need < nb) need = nb;
-    dqw = need | 1;
-    size_t o = 0;
-    tb = o; o = align16(o + sizeof(uint16_t) * g.tw * g.tw);
-    dh = o; o = align16(o + sizeof(unsigned) * g.dph * dqw);
-    dl = o; o = align16(o + sizeof(unsigned) * g.dph * dqw);
-    tq = o; o = align16(o + sizeof(unsigned) * g.tw * tp);
-    // window row sums (dead once the box sums are formed: the map reuses them)
-    rs = o;
-    const size_t rsz = (sizeof(int) + sizeof(long long)) * g.dph * g.cr + 16,
-                 msz = sizeof(double) * g.cr * g.cc;
-    rs2 = align16(rs + sizeof(int) * g.dph * g.cr);
-    o = align16(o + (rsz > msz ? rsz : msz));
-    map = rs;
-    cs = o; o = align16(o + sizeof(int) * g.cc * g.cr);
-    cs2 = o; o = align16(o + sizeof(long long) * g.cc * g.cr);
-    red = o; o = align16(o + (sizeof(double) + sizeof(int)) * 32 + 64);
-    total = o;
-  }
-};
-
-__device__ __forceinline__ void search_point_u16(const uint16_t *__restrict__ f,
-                                                 const uint16_t *__restrict__ g,
-                                                 const SearchGeom &G, const int pt,
-                                                 double *__restrict__ ox, double *__restrict__ oy,
-                                                 double *__restrict__ ou, double *__restrict__ ov,
-                                                 double *__restrict__ occ) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const U16Layout L(G);
-  uint16_t *Tb = (uint16_t *)(smem + L.tb);   // template, tw x tw
-  unsigned *Dh = (unsigned *)(smem + L.dh);   // padded region, high bytes, dph rows of dqw words
-  unsigned *Dl = (unsigned *)(smem + L.dl);   // low bytes
-  unsigned *Tq = (unsigned *)(smem + L.tq);   // template pairs, tp words per row
-  int *RS = (int *)(smem + L.rs);
-  long long *RS2 = (long long *)(smem + L.rs2);
-  int *CS = (int *)(smem + L.cs);
-  long long *CS2 = (long long *)(smem + L.cs2);
-  double *map = (double *)(smem + L.map);
-  double *redv = (double *)(smem + L.red);
-  int *redi = (int *)(redv + 32);
-  __shared__ long long s_st, s_st2;
-  __shared__ int colsum_s[72], rowsum_s[72];
-  const double mu = *G.mu;
-  const int ix = pt % G.nx, iy = pt / G.nx;
-  const int ii = G.gx1 + ix * G.step, jj = G.gy1 + iy * G.step;  // 1-based
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const int lane = tid & 31, wid = tid >> 5, nwarp = nth >> 5;
-  const uint16_t *trow0 = f + (long long)(jj - 1) * G.W + (ii - 1);
-  const uint16_t *drow0 = g + (long long)(jj - 1 - G.sy) * G.W + (ii - 1 - G.sx);
-  // ---- stage the template and the region's byte planes (1-pixel zero
-  // border at the top/left, zeros beyond the region)
-  for (int ty = wid; ty < G.tw; ty += nwarp)
-    for (int tx = lane; tx < G.tw; tx += 32) Tb[ty * G.tw + tx] = trow0[(long long)ty * G.W + tx];
-  for (int y = wid; y < G.dph; y += nwarp) {
-    const bool rin = y >= 1 && y <= G.dh;
-    const uint16_t *src = drow0 + (long long)(y - 1) * G.W;
-    for (int w4 = lane; w4 < L.dqw; w4 += 32) {
-      unsigned vh = 0, vl = 0;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int x = 4 * w4 + k;
-        if (rin && x >= 1 && x <= G.dw) {
-          const unsigned v = src[x - 1];
-          vh |= (v >> 8) << (8 * k);
-          vl |= (v & 0xFFu) << (8 * k);
-        }
-      }
-      Dh[y * L.dqw + w4] = vh;
-      Dl[y * L.dqw + w4] = vl;
-    }
-  }
-  __syncthreads();
-  // ---- template pair words, window row sums, template sums
-  for (int ty = wid; ty < G.tw; ty += nwarp)
-    for (int w = lane; w < L.tp; w += 32) {
-      const int tx = 2 * w;
-      const unsigned a = tx < G.tw ? Tb[ty * G.tw + tx] : 0u;
-      const unsigned b = tx + 1 < G.tw ? Tb[ty * G.tw + tx + 1] : 0u;
-      Tq[ty * L.tp + w] = a | (b << 16);
-    }
-  for (int y = tid; y < G.dph; y += nth) {
-    const uint8_t *rh = (const uint8_t *)(Dh + y * L.dqw), *rl = (const uint8_t *)(Dl + y * L.dqw);
-    int s1 = 0;
-    long long s2 = 0;
-    for (int k = 0; k < G.tw; ++k) {
-      const long long v = 256 * rh[k] + rl[k];
-      s1 += (int)v;
-      s2 += v * v;
-    }
-    for (int a = 0; a < G.cr; ++a) {
-      RS[y * G.cr + a] = s1;
-      RS2[y * G.cr + a] = s2;
-      const long long vo = 256 * rh[a] + rl[a], vi = 256 * rh[a + G.tw] + rl[a + G.tw];
-      s1 += (int)(vi - vo);
-      s2 += vi * vi - vo * vo;
-    }
-  }
-  for (int i = tid; i < G.tw; i += nth) {
-    int cs = 0, rsum = 0;
-    for (int k = 0; k < G.tw; ++k) {
-      cs += Tb[k * G.tw + i];
-      rsum += Tb[i * G.tw + k];
-    }
-    colsum_s[i] = cs;
-    rowsum_s[i] = rsum;
-  }
-  if (tid < 32) {
-    long long a = 0, a2 = 0;
-    for (int i = tid; i < G.tw * G.tw; i += 32) {
-      const long long v = Tb[i];
-      a += v;
-      a2 += v * v;
-    }
-    a = warp_sum_ll(a);
-    a2 = warp_sum_ll(a2);
-    if (tid == 0) {
-      s_st = a;
-      s_st2 = a2;
-    }
-  }
-  __syncthreads();
-  // ---- box sums of D and D^2 over every window: slide the row sums down
-  for (int a = tid; a < 2 * G.cr; a += nth) {
-    const int col = a < G.cr ? a : a - G.cr;
-    if (a < G.cr) {
-      int s1 = 0;
-      for (int k = 0; k < G.tw; ++k) s1 += RS[k * G.cr + col];
-      for (int b = 0; b < G.cc; ++b) {
-        CS[b * G.cr + col] = s1;
-        s1 += RS[(b + G.tw) * G.cr + col] - RS[b * G.cr + col];
-      }
-    } else {
-      long long s2 = 0;
-      for (int k = 0; k < G.tw; ++k) s2 += RS2[k * G.cr + col];
-      for (int b = 0; b < G.cc; ++b) {
-        CS2[b * G.cr + col] = s2;
-        s2 += RS2[(b + G.tw) * G.cr + col] - RS2[b * G.cr + col];
-      }
-    }
-  }
-  __syncthreads();  // RS is dead from here on; the map takes its place
-  const long long st = s_st, st2 = s_st2;
-  const long long mn = (long long)G.tw * G.tw;
-  const long long out_idx = (long long)iy + (long long)ix * G.ny;
-  if (mn * st2 - st * st == 0) {
-    if (tid == 0) {
-      const double nan = __longlong_as_double(0x7ff8000000000000ll);
-      ox[out_idx] = (ii + ii + G.w) / 2.0;
-      oy[out_idx] = (jj + jj + G.w) / 2.0;
-      ou[out_idx] = nan;
-      ov[out_idx] = nan;
-      occ[out_idx] = nan;
-    }
-    return;
-  }
-  // ---- correlation strips: 8 shifts of one window row per thread
-  const int nstrips = G.cc * G.nsx;
-  for (int sidx = tid; sidx < nstrips; sidx += nth) {
-    const int b = sidx / G.nsx;
-    const int a0 = (sidx % G.nsx) * KX;  // multiple of 8
-    unsigned long long acc[KX];
-#pragma unroll
-    for (int k = 0; k < KX; ++k) acc[k] = 0ull;
-    const int wbase = a0 >> 2;
-    for (int ty = 0; ty < G.tw; ++ty) {
-      const unsigned *trow = Tq + ty * L.tp;
-      const unsigned *dh = Dh + (b + ty) * L.dqw + wbase, *dl = Dl + (b + ty) * L.dqw + wbase;
-      unsigned ah[KX], al[KX];
-#pragma unroll
-      for (int k = 0; k < KX; ++k) ah[k] = al[k] = 0u;
-      // words w0, w1 of each plane and their 1-byte shift, carried along
-      unsigned h0 = dh[0], h1 = dh[1], l0 = dl[0], l1 = dl[1];
-      unsigned hs = __funnelshift_r(h0, h1, 8), ls = __funnelshift_r(l0, l1, 8);
-#pragma unroll 2
-      for (int m = 0; m < L.tw4; ++m) {
-        const unsigned te = trow[2 * m], to = trow[2 * m + 1];  // template pairs 2m, 2m+1
-        const unsigned h2 = dh[m + 2], l2 = dl[m + 2];
-        const unsigned hn = __funnelshift_r(h1, h2, 8), ln = __funnelshift_r(l1, l2, 8);
-        const unsigned h16 = __funnelshift_r(h0, h1, 16), h24 = __funnelshift_r(h0, h1, 24);
-        const unsigned l16 = __funnelshift_r(l0, l1, 16), l24 = __funnelshift_r(l0, l1, 24);
-        const unsigned h16n = __funnelshift_r(h1, h2, 16), h24n = __funnelshift_r(h1, h2, 24);
-        const unsigned l16n = __funnelshift_r(l1, l2, 16), l24n = __funnelshift_r(l1, l2, 24);
-        // pair 2m: byte offsets 4m + k; words at 4m (h0), 4m+1 (hs), 4m+4 (h1), 4m+5 (hn)
-        ah[0] = __dp2a_lo(te, h0, ah[0]);  al[0] = __dp2a_lo(te, l0, al[0]);
-        ah[2] = __dp2a_hi(te, h0, ah[2]);  al[2] = __dp2a_hi(te, l0, al[2]);
-        ah[1] = __dp2a_lo(te, hs, ah[1]);  al[1] = __dp2a_lo(te, ls, al[1]);
-        ah[3] = __dp2a_hi(te, hs, ah[3]);  al[3] = __dp2a_hi(te, ls, al[3]);
-        ah[4] = __dp2a_lo(te, h1, ah[4]);  al[4] = __dp2a_lo(te, l1, al[4]);
-        ah[6] = __dp2a_hi(te, h1, ah[6]);  al[6] = __dp2a_hi(te, l1, al[6]);
-        ah[5] = __dp2a_lo(te, hn, ah[5]);  al[5] = __dp2a_lo(te, ln, al[5]);
-        ah[7] = __dp2a_hi(te, hn, ah[7]);  al[7] = __dp2a_hi(te, ln, al[7]);
-        // pair 2m+1: byte offsets 4m + 2 + k; words at 4m+2, 4m+3, 4m+6, 4m+7
-        ah[0] = __dp2a_lo(to, h16, ah[0]);  al[0] = __dp2a_lo(to, l16, al[0]);
-        ah[2] = __dp2a_hi(to, h16, ah[2]);  al[2] = __dp2a_hi(to, l16, al[2]);
-        ah[1] = __dp2a_lo(to, h24, ah[1]);  al[1] = __dp2a_lo(to, l24, al[1]);
-        ah[3] = __dp2a_hi(to, h24, ah[3]);  al[3] = __dp2a_hi(to, l24, al[3]);
-        ah[4] = __dp2a_lo(to, h16n, ah[4]);  al[4] = __dp2a_lo(to, l16n, al[4]);
-        ah[6] = __dp2a_hi(to, h16n, ah[6]);  al[6] = __dp2a_hi(to, l16n, al[6]);
-        ah[5] = __dp2a_lo(to, h24n, ah[5]);  al[5] = __dp2a_lo(to, l24n, al[5]);
-        ah[7] = __dp2a_hi(to, h24n, ah[7]);  al[7] = __dp2a_hi(to, l24n, al[7]);
-        h0 = h1; h1 = h2; l0 = l1; l1 = l2; hs = hn; ls = ln;
-      }
-#pragma unroll
-      for (int k = 0; k < KX; ++k) acc[k] += ((unsigned long long)ah[k] << 8) + al[k];
-    }
-    const bool ring_b = (b == 0 || b == G.cc - 1);
-#pragma unroll
-    for (int k = 0; k < KX; ++k) {
-      const int a = a0 + k;
-      if (a >= G.cr) break;
-      const long long sd = CS[b * G.cr + a], sd2 = CS2[b * G.cr + a];
-      int st_out = 0;
-      long long n_out = 0;
-      if (ring_b || a == 0 || a == G.cr - 1) {
-        const int oc = a == 0 ? 0 : (a == G.cr - 1 ? G.tw - 1 : -1);
-        const int orow = b == 0 ? 0 : (b == G.cc - 1 ? G.tw - 1 : -1);
-        if (oc >= 0) st_out += colsum_s[oc];
-        if (orow >= 0) st_out += rowsum_s[orow];
-        if (oc >= 0 && orow >= 0) st_out -= Tb[orow * G.tw + oc];
-        const long long nco = oc >= 0, nro = orow >= 0;
-        n_out = nco * G.tw + nro * G.tw - nco * nro;
-      }
-      map[b * G.cr + a] = ncc_combine(mn, st, st2, (long long)acc[k], sd, sd2, st_out, n_out, mu);
-    }
-  }
-  __syncthreads();
-  peak_epilogue(map, G, ii, jj, out_idx, redv, redi, ox, oy, ou, ov, occ);
-}
-
-__global__ void __launch_bounds__(512) k_search_u16(const uint16_t *__restrict__ f,
-                                                    const uint16_t *__restrict__ g, SearchGeom G,
-                                                    double *__restrict__ ox,
-                                                    double *__restrict__ oy,
-                                                    double *__restrict__ ou,
-                                                    double *__restrict__ ov,
-                                                    double *__restrict__ occ) {
-  for (int pt = blockIdx.x; pt < G.nx * G.ny; pt += gridDim.x) {
-    search_point_u16(f, g, G, pt, ox, oy, ou, ov, occ);
-    __syncthreads();  // the next point restages shared memory
-  }
-}
-
-__global__ void __launch_bounds__(512) k_search_u8(const uint8_t *__restrict__ f,
-                                                   const uint8_t *__restrict__ g, SearchGeom G,
-                                                   double *__restrict__ ox,
-                                                   double *__restrict__ oy,
-                                                   double *__restrict__ ou,
-                                                   double *__restrict__ ov,
-                                                   double *__restrict__ occ) {
-  search_point_u8(f, g, G, blockIdx.x, ox, oy, ou, ov, occ);
-}
-
-// The same over a device-side list of grid points (list[0] entries from
-// list[1]): the points the tiled search hands back.
-__global__ void __launch_bounds__(512) k_search_u8_list(const uint8_t *__restrict__ f,
-                                                        const uint8_t *__restrict__ g,
-                                                        SearchGeom G, const int *__restrict__ list,
-                                                        double *__restrict__ ox,
-                                                        double *__restrict__ oy,
-                                                        double *__restrict__ ou,
-                                                        double *__restrict__ ov,
-                                                        double *__restrict__ occ) {
-  const int n = list[0];
-  for (int i = blockIdx.x; i < n; i += gridDim.x) {
-    search_point_u8(f, g, G, list[1 + i], ox, oy, ou, ov, occ);
-    __syncthreads();
-  }
-}
-
 // ---- 8-bit images, tiled: step a multiple of 4 that divides the subset size.
 // Neighbouring subsets overlap (step 8 of a 33 px window: every pixel lies in
 // 16 windows), so the per-point kernel above recomputes each product
@@ -900,15 +388,6 @@ struct TileArgs {
   int off_g, off_ti, off_ra, off_rb, off_rc, off_sub;
 };
 
-__device__ __forceinline__ unsigned fkey(float x) {  // order-preserving float -> unsigned
-  const unsigned u = __float_as_uint(x);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float fkey_inv(unsigned k) {
-  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
-}
-
-// template pixels of entry (a, b) whose partner lies beyond the search region
 __device__ __forceinline__ void tile_pad(const TileSub &S, int a, int b, int cr, int cc, int tw,
                                          long long *st_out, long long *n_out) {
   const int nco = (a == 0) || (a == cr - 1), nro = (b == 0) || (b == cc - 1);
@@ -1253,49 +732,59 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_search_tile(const TileArgs 
 // shared memory, vertical sums per column, a prefix sum per row.
 constexpr int kTabX = 128, kTabY = 32;
 
-__global__ void __launch_bounds__(256) k_box_tab(const uint8_t *__restrict__ g, int W, int H,
+template <typename T>
+__global__ void __launch_bounds__(256) k_box_tab(const T *__restrict__ g, int W, int H,
                                                  int tw, long long mn, int x0, int x1, int y0,
                                                  int y1, uint4 *__restrict__ tab) {
   extern __shared__ __align__(16) unsigned char sm[];
   const int bx = x0 + blockIdx.x * kTabX, by = y0 + blockIdx.y * kTabY;
   const int nc = kTabX + tw - 1, nr = kTabY + tw - 1, np = nc + 1;
-  uint8_t *G = sm;
-  unsigned *P1 = reinterpret_cast<unsigned *>(sm + align16((size_t)nr * nc));
-  unsigned *P2 = P1 + kTabY * np;
+  using Sq = typename std::conditional<sizeof(T) == 1, unsigned, unsigned long long>::type;
+  Sq *P2 = reinterpret_cast<Sq *>(sm);
+  unsigned *P1 = reinterpret_cast<unsigned *>(P2 + kTabY * np);
+  T *G = reinterpret_cast<T *>(P1 + kTabY * np);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   for (int i = tid; i < nr * nc; i += 256) {
     const int r = i / nc, c = i - r * nc, yy = by + r, xx = bx + c;
-    G[i] = (yy < H && xx < W) ? g[(long long)yy * W + xx] : (uint8_t)0;
+    G[i] = (yy < H && xx < W) ? g[(long long)yy * W + xx] : (T)0;
   }
   __syncthreads();
   for (int c = tid; c < nc; c += 256) {  // vertical sums, column c, rows oy .. oy+tw-1
-    unsigned s1 = 0, s2 = 0;
+    unsigned s1 = 0;
+    Sq s2 = 0;
     for (int r = 0; r < tw; ++r) {
-      const unsigned v = G[r * nc + c];
-      s1 += v;
+      const Sq v = G[r * nc + c];
+      s1 += (unsigned)v;
       s2 += v * v;
     }
     for (int oy = 0; oy < kTabY; ++oy) {
       P1[oy * np + c + 1] = s1;
       P2[oy * np + c + 1] = s2;
       if (oy + 1 < kTabY) {
-        const unsigned vo = G[oy * nc + c], vi = G[(oy + tw) * nc + c];
-        s1 += vi - vo;
+        const Sq vo = G[oy * nc + c], vi = G[(oy + tw) * nc + c];
+        s1 += (unsigned)(vi - vo);
         s2 += vi * vi - vo * vo;
       }
     }
   }
   __syncthreads();
   for (int oy = wid; oy < kTabY; oy += 8) {  // prefix sums along each row, a warp a row
-    unsigned *q1 = P1 + oy * np, *q2 = P2 + oy * np;
-    if (lane == 0) q1[0] = q2[0] = 0;
-    unsigned c1 = 0, c2 = 0;
+    unsigned *q1 = P1 + oy * np;
+    Sq *q2 = P2 + oy * np;
+    if (lane == 0) {
+      q1[0] = 0;
+      q2[0] = 0;
+    }
+    unsigned c1 = 0;
+    Sq c2 = 0;
     for (int c0 = 1; c0 <= nc; c0 += 32) {
       const int c = c0 + lane;
-      unsigned v1 = c <= nc ? q1[c] : 0u, v2 = c <= nc ? q2[c] : 0u;
+      unsigned v1 = c <= nc ? q1[c] : 0u;
+      Sq v2 = c <= nc ? q2[c] : (Sq)0;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const unsigned t1 = __shfl_up_sync(0xffffffffu, v1, o), t2 = __shfl_up_sync(0xffffffffu, v2, o);
+        const unsigned t1 = __shfl_up_sync(0xffffffffu, v1, o);
+        const Sq t2 = __shfl_up_sync(0xffffffffu, v2, o);
         if (lane >= o) {
           v1 += t1;
           v2 += t2;
@@ -1314,10 +803,12 @@ __global__ void __launch_bounds__(256) k_box_tab(const uint8_t *__restrict__ g, 
     const int oy = i / kTabX, ox = i - oy * kTabX, x = bx + ox, y = by + oy;
     if (x > x1 || y > y1) continue;
     const unsigned s1 = P1[oy * np + ox + tw] - P1[oy * np + ox];
-    const unsigned s2 = P2[oy * np + ox + tw] - P2[oy * np + ox];
+    const Sq s2 = P2[oy * np + ox + tw] - P2[oy * np + ox];
     const long long c0 = mn * (long long)s2 - (long long)s1 * s1;
-    tab[(long long)y * W + x] =
-        make_uint4(s1, s2, c0 > 0 ? __float_as_uint(rsqrtf((float)c0)) : 0u, 0u);
+    const unsigned rs = c0 > 0 ? __float_as_uint(rsqrtf((float)c0)) : 0u;
+    tab[(long long)y * W + x] = sizeof(T) == 1
+                                    ? make_uint4(s1, (unsigned)s2, rs, 0u)
+                                    : make_uint4(s1, (unsigned)s2, (unsigned)((unsigned long long)s2 >> 32), rs);
   }
 }
 
@@ -1666,8 +1157,7 @@ TileBufs tile_bufs(char *base, int W, int H, int nx, int ny, const int search[2]
 
 // tiled 8-bit search; false in *used when the geometry has no tiled kernel
 int tile_search(const uint8_t *f, const uint8_t *g, const SearchGeom &G, SearchWork &sw,
-                double *x, double *y, double *u, double *v, double *cc, int threads_pt,
-                size_t smem_pt, cudaStream_t st, bool *used) {
+                double *x, double *y, double *u, double *v, double *cc, cudaStream_t st, bool *used) {
   *used = false;
   TilePlan P;
   if (G.step % 4 || G.w % G.step || !tile_shape(G.step, G.w, G.sx, G.sy, P)) return OK;
@@ -1681,14 +1171,7 @@ int tile_search(const uint8_t *f, const uint8_t *g, const SearchGeom &G, SearchW
   uint4 *tab = B.tab;
   int *fb = B.fb;
   const long long mn = (long long)G.tw * G.tw;
-  // full windows of every shift of every point (outer ring included)
-  const int x0 = px1 - G.sx - 1, x1 = px1 + (G.nx - 1) * G.step + G.sx + 1;
-  const int y0 = py1 - G.sy - 1, y1 = py1 + (G.ny - 1) * G.step + G.sy + 1;
-  const size_t smt = align16((size_t)(kTabY + G.tw - 1) * (kTabX + G.tw - 1)) +
-                     2 * sizeof(unsigned) * kTabY * (kTabX + G.tw);
-  ALDIC_CUDA(cudaFuncSetAttribute(k_box_tab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt));
-  k_box_tab<<<dim3((x1 - x0 + kTabX) / kTabX, (y1 - y0 + kTabY) / kTabY), 256, smt, st>>>(
-      g, G.W, G.H, G.tw, mn, x0, x1, y0, y1, tab);
+  if ((rc = box_table<uint8_t>(g, G, tab, st))) return rc;
   ALDIC_CUDA(cudaMemsetAsync(fb, 0, sizeof(int), st));
   TileArgs A{};
   A.f = f; A.g = g; A.tab = tab; A.cmap = B.cmap; A.subs = B.subs; A.ringw = B.ringw;
@@ -1704,10 +1187,8 @@ int tile_search(const uint8_t *f, const uint8_t *g, const SearchGeom &G, SearchW
   const int pb = (int)std::min<long long>((npts + kPeakWarps - 1) / kPeakWarps, 148 * 16);
   k_search_peak<<<pb, kPeakWarps * 32, 0, st>>>(K);
   ALDIC_CUDA(cudaGetLastError());
-  // the points handed back: per-point kernel over the device-side list
-  const int nb = (int)std::min<long long>(npts, 296);
-  k_search_u8_list<<<nb, threads_pt, smem_pt, st>>>(f, g, G, fb, x, y, u, v, cc);
-  ALDIC_CUDA(cudaGetLastError());
+  // the points handed back: the per-point kernel over the device-side list
+  if ((rc = search_mma<uint8_t>(f, g, G, tab, fb, x, y, u, v, cc, st))) return rc;
   *used = true;
   return OK;
 }
@@ -1829,7 +1310,6 @@ __global__ void k_qfactor(const T *__restrict__ f, const T *__restrict__ g, Sear
   }
 }
 
-constexpr size_t kSmemMax = 227 * 1024;
 constexpr int kBigBlocks = 296;  // CTAs (and global work slots) of the big-region search
 
 // Search regions too large for shared memory: the per-point kernel with its
@@ -1881,30 +1361,29 @@ int launch_search(const void *f, const void *g, const SearchGeom &G, double *x, 
   if (threads > 512) threads = 512;
   const int npts = G.nx * G.ny;
   if (npts == 0) return OK;
-  if (sizeof(T) == 1 && !(U8Layout(G).total <= kSmemMax && G.tw <= 72)) {
-    const int rc = launch_big<T>(f, g, G, x, y, u, v, cc, st, sw);
-    if (rc) return rc;
-  } else if (sizeof(T) == 1) {
-    U8Layout L(G);
-    ALDIC_CUDA(cudaFuncSetAttribute(k_search_u8, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)L.total));
-    ALDIC_CUDA(cudaFuncSetAttribute(k_search_u8_list,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+  // 8 bit by tiles where one is built for the geometry (2048 x 2048, 32/8/+-16:
+  // 1.2 ms against 2.6 ms point by point on the tensor cores), else the tensor
+  // cores whatever the geometry: against the dot product kernels before, 1100 x
+  // 900, subset/step/zone 28/7/13 8 bit 0.68 against 0.76 ms, 50/25/30 0.22
+  // against 0.44; 16 bit 16/8/10 0.53 against 0.66, 50/25/30 0.26 against 1.16;
+  // 320 x 340, 20/10/20 8 bit 0.119 against 0.127 ms
+  if (sizeof(T) <= 2 && search_mma_fits(G, sizeof(T))) {
     bool tiled = false;
-    if (sw) {
-      const int rc = tile_search((const uint8_t *)f, (const uint8_t *)g, G, *sw, x, y, u, v, cc,
-                                 threads, L.total, st, &tiled);
+    if (sizeof(T) == 1 && sw) {
+      const int rc = tile_search((const uint8_t *)f, (const uint8_t *)g, G, *sw, x, y, u, v, cc, st, &tiled);
       if (rc) return rc;
     }
-    if (!tiled)
-      k_search_u8<<<npts, threads, L.total, st>>>((const uint8_t *)f, (const uint8_t *)g, G, x,
-                                                   y, u, v, cc);
-  } else if (sizeof(T) == 2 && U16Layout(G).total <= kSmemMax && G.tw <= 72) {
-    const U16Layout L(G);
-    ALDIC_CUDA(cudaFuncSetAttribute(k_search_u16, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)L.total));
-    k_search_u16<<<npts, threads, L.total, st>>>((const uint16_t *)f, (const uint16_t *)g, G, x, y,
-                                                  u, v, cc);
+    using Px = typename std::conditional<sizeof(T) == 1, uint8_t, uint16_t>::type;
+    if (!tiled) {
+      ALDIC_CHECK(sw != nullptr, E_ARG, "integer search: the context's work memory is needed");
+      const int srch[2] = {G.sx, G.sy};
+      int rc = search_work_ensure(*sw, G.W, G.H, G.nx, G.ny, srch);
+      if (rc) return rc;
+      uint4 *tab = tile_bufs(sw->buf.as<char>(), G.W, G.H, G.nx, G.ny, srch).tab;
+      if ((rc = box_table<Px>((const Px *)g, G, tab, st)) ||
+          (rc = search_mma<Px>((const Px *)f, (const Px *)g, G, tab, nullptr, x, y, u, v, cc, st)))
+        return rc;
+    }
   } else {
     SmemLayout<V, S> L(G);
     if (L.total > kSmemMax) {
@@ -1930,6 +1409,22 @@ int launch_search(const void *f, const void *g, const SearchGeom &G, double *x, 
 }
 
 }  // namespace
+
+template <typename T>
+int box_table(const T *g, const SearchGeom &G, uint4 *tab, cudaStream_t st) {
+  // the windows of every shift of every point, the outer ring's included
+  const int px1 = G.gx1 - 1, py1 = G.gy1 - 1;
+  const int x0 = std::max(0, px1 - G.sx - 1), x1 = px1 + (G.nx - 1) * G.step + G.sx + 1;
+  const int y0 = std::max(0, py1 - G.sy - 1), y1 = py1 + (G.ny - 1) * G.step + G.sy + 1;
+  const size_t np = kTabX + G.tw;
+  const size_t smt = kTabY * np * (sizeof(T) == 1 ? 8 : 12) +
+                     align16(sizeof(T) * (kTabY + G.tw - 1) * (kTabX + G.tw - 1));
+  ALDIC_CUDA(cudaFuncSetAttribute(k_box_tab<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt));
+  k_box_tab<T><<<dim3((x1 - x0 + kTabX) / kTabX, (y1 - y0 + kTabY) / kTabY), 256, smt, st>>>(
+      g, G.W, G.H, G.tw, (long long)G.tw * G.tw, x0, x1, y0, y1, tab);
+  ALDIC_CUDA(cudaGetLastError());
+  return OK;
+}
 
 int search_dims(int W, int H, const int gridx[2], const int gridy[2], int winsize, int step,
                 const int search[2], int *nx, int *ny, int *gx1o, int *gy1o) {
@@ -1967,9 +1462,8 @@ template <typename T>
 size_t big_bytes(const SearchGeom &G) {
   using Tr = SearchTraits<T>;
   using S = typename SumT<Tr::integer>::type;
-  const bool small = sizeof(T) == 1 ? (U8Layout(G).total <= kSmemMax && G.tw <= 72)
-                                    : ((sizeof(T) == 2 && U16Layout(G).total <= kSmemMax && G.tw <= 72) ||
-                                       SmemLayout<typename Tr::V, S>(G).total <= kSmemMax);
+  const bool small = (sizeof(T) <= 2 && search_mma_fits(G, sizeof(T))) ||
+                     SmemLayout<typename Tr::V, S>(G).total <= kSmemMax;
   if (small) return 0;
   const int npts = G.nx * G.ny;
   return SmemLayout<typename Tr::V, S>(G, true).slot * (size_t)(npts < kBigBlocks ? npts : kBigBlocks);

@@ -9,6 +9,22 @@ namespace aldic {
 
 constexpr int TC_M = 128;  // rows of a tile (lanes of tensor memory)
 
+// One lane of a converged warp.  tcgen05 products take their operands from
+// uniform registers: a warp that runs its issuing loop as a whole, with values
+// that are uniform as the compiler sees them (uniform() of what it cannot know),
+// and issues under elect_one() takes 30 cycles a product; the same loop under
+// `if (threadIdx.x == 0)` took 62.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "elect.sync _|P, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(p));
+  return p;
+}
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -57,20 +73,21 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
                : "memory");
 }
 
-// bounded wait on an mbarrier phase; false after ~2^26 polls
+// bounded wait on an mbarrier phase; false after a few seconds.  Each try may
+// suspend the thread for a microsecond: polling without it took a fifth of an
+// SM's issue slots where a dozen warps wait.
 __device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
   const uint32_t a = smem_u32(bar);
-  for (uint32_t it = 0; it < (1u << 26); ++it) {
+  for (uint32_t it = 0; it < (1u << 22); ++it) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred P1;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2, %3;\n\t"
         "selp.b32 %0, 1, 0, P1;\n\t}\n"
         : "=r"(done)
-        : "r"(a), "r"(parity)
+        : "r"(a), "r"(parity), "r"(1000)
         : "memory");
     if (done) return true;
-    if (it > 64) __nanosleep(64);
   }
   return false;
 }
@@ -134,6 +151,21 @@ __device__ __forceinline__ void tmem_st_16x16(uint32_t taddr, const uint32_t r[8
   asm volatile(
       "tcgen05.st.sync.aligned.16x128b.x4.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};\n" ::"r"(r[0]),
       "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr)
+      : "memory");
+}
+// 8 columns of the warp's 32 lanes, a lane a thread; the caller waits
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t r[8]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};\n" ::"r"(r[0]),
+      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t r[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+      "%11, %12, %13, %14, %15};\n" ::"r"(r[0]),
+      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() {

@@ -125,7 +125,8 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(GemmSrc A, GemmSrc B, Gem
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_base;
+  const uint32_t tmem = uniform(tmem_base), smem0 = uniform(smem_u32(smem));
+  const bool issuer = uniform(warp) == 0;
   const uint32_t id = idesc(BN);
   uint32_t phase[2] = {0, 0};
 
@@ -136,14 +137,16 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(GemmSrc A, GemmSrc B, Gem
     __syncthreads();
     for (int t = 0; t < nk; ++t) {
       const int buf = t & 1;
-      unsigned char *sa = smem + buf * STAGE;
-      if (tid == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t da = sdesc(smem_u32(sa)), db = sdesc(smem_u32(sa + A_BYTES));
+      if (issuer) {
+        tc_after_sync();
+        const uint64_t da = sdesc(smem0 + buf * STAGE), db = sdesc(smem0 + buf * STAGE + A_BYTES);
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk)  // +32 B per K = 16 step: +2 in the address field
-          mma_bf16(tmem, da + 2 * kk, db + 2 * kk, id, (t > 0 || kk > 0) ? 1u : 0u);
-        mma_commit(&bar[buf]);
+          for (int kk = 0; kk < BK / 16; ++kk)  // +32 B per K = 16 step: +2 in the address field
+            mma_bf16(tmem, da + 2 * kk, db + 2 * kk, id, (t > 0 || kk > 0) ? 1u : 0u);
+          mma_commit(&bar[buf]);
+        }
+        __syncwarp();
       }
       if (t + 1 < nk) {
         const int nb = (t + 1) & 1;

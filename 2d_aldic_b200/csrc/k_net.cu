@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kEncBlock, 2) k_encode(const __grid_constant__
     }
   };
   int b = blockIdx.x;
-  const bool issuer = warp == kEncThreads / 32;
+  const bool issuer = uniform(warp) == kEncThreads / 32;
   tc_before_sync();
   __syncthreads();
   tc_after_sync();
@@ -142,9 +142,11 @@ __global__ void __launch_bounds__(kEncBlock, 2) k_encode(const __grid_constant__
   if (!issuer) stage();
   smem_to_async();
   __syncthreads();
-  const uint32_t tD = S.tmem, tC = tD + 128, tE = tD + 192;
+  const uint32_t tD = uniform(S.tmem), tC = tD + 128, tE = tD + 192;
+  const uint32_t sA0 = uniform(smem_u32(S.A0)), sW1 = uniform(smem_u32(S.W1));
+  const uint32_t sW2 = uniform(smem_u32(S.W2[0])), sG = uniform(smem_u32(S.G[0]));
   auto embed = [&]() {
-    const uint64_t da = sdesc(smem_u32(S.A0)), db = sdesc(smem_u32(S.W1));
+    const uint64_t da = sdesc(sA0), db = sdesc(sW1);
 #pragma unroll
     for (int k = 0; k < 4; ++k) mma_bf16(tD, da + 2 * k, db + 2 * k, idesc(128), k > 0);
     mma_commit(&S.bar[0]);
@@ -203,19 +205,20 @@ __global__ void __launch_bounds__(kEncBlock, 2) k_encode(const __grid_constant__
     // the copy never came; nothing else is under way
   } else if (issuer) {
     uint32_t got = 0;  // parity of the last copy waited for
-    if (lane == 0) {
+    if (elect_one()) {
       embed();
       if (b + (int)gridDim.x < A.B) load(b + gridDim.x);
     }
+    __syncwarp();
     const int b0 = b;
     for (; b < A.B; b += gridDim.x) {
       __syncthreads();
       if (S.failed) break;
-      if (lane == 0) {
-        tc_after_sync();
+      tc_after_sync();
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          mma_bf16_ta(tD, tE + 8 * k, sdesc(smem_u32(S.W2[k >> 2])) + 2 * (k & 3), idesc(128), k > 0);
+          mma_bf16_ta(tD, tE + 8 * k, sdesc(sW2 + (k >> 2) * (128 * 128)) + 2 * (k & 3), idesc(128), k > 0);
         mma_commit(&S.bar[1]);
         if (b > b0) {  // the previous pair's correlation; `out` is free again at the next barrier
           store(b - gridDim.x);
@@ -225,15 +228,16 @@ __global__ void __launch_bounds__(kEncBlock, 2) k_encode(const __grid_constant__
       __syncwarp();
       __syncthreads();
       if (S.failed) break;
-      if (lane == 0) {
-        tc_after_sync();
+      tc_after_sync();
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          mma_bf16_ta(tC, tE + 8 * k, sdesc(smem_u32(S.G[k >> 2])) + 2 * (k & 3), idesc(64), k > 0);
+          mma_bf16_ta(tC, tE + 8 * k, sdesc(sG + (k >> 2) * (kCells * 128)) + 2 * (k & 3), idesc(64), k > 0);
         mma_commit(&S.bar[2]);
         if (b + (int)gridDim.x < A.B) embed();
         if (b + 2 * (int)gridDim.x < A.B) load(b + 2 * gridDim.x);
       }
+      __syncwarp();
       got ^= 1;
     }
     // after a failed wait: the copy under way must land before the CTA ends
@@ -346,7 +350,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_dense(const __grid_constan
   tc_before_sync();
   __syncthreads();
   tc_after_sync();
-  const uint32_t tD = S.tmem;
+  const uint32_t tD = uniform(S.tmem);
   if (warp == 0) {
     if (lane == 0) {
       int k = 0;
@@ -367,23 +371,25 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_dense(const __grid_constan
       for (int q = k > kDenseStages ? k - kDenseStages : 0; q < k; ++q)
         if (!bar_wait(&S.full[q % kDenseStages], (q / kDenseStages) & 1)) S.failed = 1;
     }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      for (int k = 0; k < A.steps; ++k) {
-        const int s = k % kDenseStages;
-        if (!bar_wait(&S.full[s], (k / kDenseStages) & 1)) {
-          S.failed = 1;
-          break;
-        }
-        tc_after_sync();
-        const uint64_t da = sdesc(smem_u32(ring + s * kDenseStage));
-        const uint64_t db = sdesc(smem_u32(ring + s * kDenseStage + 128 * 128));
+  } else if (uniform(warp) == 1) {
+    const uint32_t base = uniform(smem_u32(ring));
+    for (int k = 0; k < A.steps; ++k) {
+      const int s = k % kDenseStages;
+      if (!__all_sync(0xffffffffu, bar_wait(&S.full[s], (k / kDenseStages) & 1))) {
+        S.failed = 1;
+        break;
+      }
+      tc_after_sync();
+      const uint64_t da = sdesc(base + s * kDenseStage), db = sdesc(base + s * kDenseStage + 128 * 128);
+      if (elect_one()) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) mma_bf16(tD, da + 2 * q, db + 2 * q, idesc(kF), k > 0 || q > 0);
         mma_commit(&S.empty[s]);
       }
-      mma_commit(&S.done);
+      __syncwarp();
     }
+    if (elect_one()) mma_commit(&S.done);
+    __syncwarp();
   } else {
     const bool ok = __all_sync(0xffffffffu, bar_wait(&S.done, 0) && !*(volatile int *)&S.failed);
     if (!ok) S.failed = 1;

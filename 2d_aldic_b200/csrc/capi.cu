@@ -907,11 +907,10 @@ int aldic_subpb2(aldic_ctx *c, int M, int N, double step, double beta, double mu
   if ((rc = fdm_ensure(c->fdm, FDM_FE, M, N, step, c->stream))) return rc;
   if ((rc = fe_rhs(c->gw, M, N, step, beta, mu, au.dev, af.dev, aud.dev, avd.dev, c->stream)))
     return rc;
-  if ((rc = fdm_solve(c->fdm, 2, c->gw.b, c->gw.x, c->gw.r, mu, beta, nullptr, nullptr, c->stream)))
+  if ((rc = fdm_solve(c->fdm, 2, c->gw.b, c->gw.x, c->gw.r, mu, beta, nullptr, nullptr, c->stream, ao.dev)))
     return rc;
-  if ((rc = fe_store(c->gw, M, N, ao.dev, c->stream))) return rc;
   arg_back(c, ao);
-  return check_grid_err(c);
+  return finish(c, true);  // the direct solve has no status to read
 }
 
 int aldic_qt_mesh_generate(int n0, const double *coords, int ne0, const int32_t *elems,
@@ -1496,11 +1495,12 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
               : fe_rhs(c->gw, M, N, h, beta, mu, B.U1, B.F1, B.udual, B.vdual, st, beta_ptr, f0);
   };
   // the direct fast-diagonalisation solve (fdm.cu; bases set up before capture)
-  auto pcg = [&](int nr, const double *beta_ptr, const double *beta_each) {
-    return fdm_solve(c->fdm, nr, c->gw.b, c->gw.x, c->gw.r, mu, 0.0, beta_each, beta_ptr, st);
-  };
-  auto store = [&](int f0) {
-    return fd ? fd_store(c->gw, M, N, B.U1, B.U2, st, f0) : fe_store(c->gw, M, N, B.U2, st, f0);
+  // of the system at *beta into U2
+  auto solve = [&](const double *beta_ptr) {
+    int rc2 = rhs(0, beta_ptr, 0);
+    if (!rc2)
+      rc2 = fdm_solve(c->fdm, 2, c->gw.b, c->gw.x, c->gw.r, mu, 0.0, nullptr, beta_ptr, st, fd ? nullptr : B.U2);
+    return rc2 || !fd ? rc2 : fd_store(c->gw, M, N, B.U1, B.U2, st, 0);
   };
   auto strain = [&]() {
     return fd ? fd_strain(M, N, h, B.U2, B.F2, st) : nodal_strain(M, N, h, B.U2, B.F2, st);
@@ -1521,7 +1521,7 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
     }
     if (fd) {
       // the six systems of the sweep in one launch (12 right-hand sides)
-      if ((rc = pcg(12, nullptr, be))) return rc;
+      if ((rc = fdm_solve(c->fdm, 12, c->gw.b, c->gw.x, c->gw.r, mu, 0.0, be, nullptr, st))) return rc;
     } else {
       // the right-hand side is linear in beta: its two parts, transformed
       // once, give the six systems' solutions
@@ -1531,7 +1531,7 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
     }
     if (fd) {
       for (int k = 0; k < 6; ++k) {
-        if ((rc = store(2 * k))) return rc;
+        if ((rc = fd_store(c->gw, M, N, B.U1, B.U2, st, 2 * k))) return rc;
         if ((rc = strain())) return rc;
         if ((rc = vdiffnorm(B.U1, B.U2, 2 * n, B.part, B.err + k, st))) return rc;
         if ((rc = vdiffnorm(B.F1, B.F2, 4 * n, B.part, B.err + 6 + k, st))) return rc;
@@ -1543,8 +1543,7 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
     }
     k_beta_select<<<1, 1, 0, st>>>(B.err, base, B.beta, fd ? h : 0.0);
   }
-  if ((rc = rhs(0, B.beta, 0)) || (rc = pcg(2, B.beta, nullptr)) || (rc = store(0)) || (rc = strain()))
-    return rc;
+  if ((rc = solve(B.beta)) || (rc = strain())) return rc;
   if (p->smooth && (rc = smooth_dev(c, M, N, 4, B.F2))) return rc;
   if ((rc = dual(0))) return rc;
   ALDIC_CUDA(cudaMemcpyAsync(B.U1old, B.U1, sizeof(double) * 2 * n, cudaMemcpyDeviceToDevice, st));
@@ -1572,7 +1571,7 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
       ALDIC_CUDA(cudaMemcpyAsync(B.U1old, B.U1, sizeof(double) * 2 * n, cudaMemcpyDeviceToDevice, st));
     }
     if (p->smooth && (rc = smooth_dev(c, M, N, 2, B.U1))) return rc;
-    if ((rc = rhs(0, B.beta, 0)) || (rc = pcg(2, B.beta, nullptr)) || (rc = store(0))) return rc;
+    if ((rc = solve(B.beta))) return rc;
     if (p->smooth && (rc = smooth_dev(c, M, N, 2, B.U2))) return rc;
     if ((rc = strain())) return rc;
     if (p->smooth && (rc = smooth_dev(c, M, N, 4, B.F2))) return rc;

@@ -24,7 +24,7 @@
 // Householder tridiagonalisation and implicit symmetric QR steps with
 // Wilkinson shifts of L^-1 K L^-T -- Golub and Van Loan, Matrix
 // Computations, 4th ed., algorithms 8.3.1 and 8.3.2) and kept on the device;
-// the products run as FP64 CUDA-core tiles.  The solution is exact up to
+// the products run as tiles on the FP64 tensor instruction.  The solution is exact up to
 // rounding (about 1e-13 relative), where an iterative solve stops at a
 // residual of 1e-11.
 #include <algorithm>
@@ -195,30 +195,42 @@ int tridiagonal_qr(int n, std::vector<double> &d, std::vector<double> &e, std::v
 }
 
 // ---------------------------------------------------------------- device: FP64 products
-// 64 x 64 outputs per 256-thread CTA, 4 x 4 per thread taken strided (rows
-// ty + 16 i, columns tx + 16 j), so a warp's shared-memory reads of a k row
-// are 16 consecutive doubles (one wavefront, broadcast to the two row
-// groups) and each thread does 16 FMA per 8 loads.  The operand tiles of
-// 32-wide K chunks go to shared memory by cp.async (no register round trip),
-// double-buffered so that chunk c + 1 arrives while chunk c is multiplied.
-constexpr int TR = 64, TC = 64, KC = 32, GT = 256, LDT = TR + 1;
-// Products with fewer tiles than SMs (the 2-field solves: 32 tiles at 243^2)
-// split K into up to kMaxSplit slices written to a partial buffer and summed
-// in a fixed order by k_fdm_reduce (deterministic, no atomics).
-constexpr int kMaxSplit = 4, kFdmPart = 8;  // partial capacity: kFdmPart fields of M N
-constexpr int kBuf = 2 * KC * LDT;                              // doubles per buffer (A + B)
-constexpr int kSmem = 2 * kBuf * (int)sizeof(double);           // two buffers: 66 560 B
+// TILE x TILE outputs a CTA on the FP64 tensor instruction (m8n8k4), a warp
+// 16 x 8 (TILE 32) or 32 x 16 (TILE 64).  K runs in chunks
+// of 32 through a ring of three buffers filled by cp.async; an operand lies in
+// shared memory the way it does in global memory (k fast or row/column fast),
+// lines of TILE or 32 doubles 4 further apart than they are long, so that the
+// 4 x 4 doubles a half warp reads of a fragment are in 16 different bank pairs.
+//
+// What bounds it: these products are small (243 x 243 x 243 and two fields in a
+// frame), so the time goes to filling the chip and to latency, not to the 64
+// multiply-adds a cycle and SM.  32 x 32 tiles make 128 CTAs of that product
+// where 64 x 64 ones made 32, which had K split four ways and a second launch
+// to add the slices.  A product of 243 x 243 and two fields takes 9 us against
+// 16 with its sum; the fragments need 3 shared loads for 512 multiply-adds a
+// warp where a 4 x 4 register tile needs 8.  Addresses are stepped, not formed
+// from (line, k) at every copy: that alone was 18 us a product.
+constexpr int KC = 32, GT = 256, kFdmStages = 3;
+// 64 x 64 tiles, which read half the operand bytes a multiply-add, from two
+// full waves of them on
+constexpr int kFdmBig = 296;
+constexpr int kFdmCluster = 8, kFdmChainTiles = 8;
+template <int TILE> struct FdmTile {
+  static constexpr int mi = TILE / 16, ni = TILE / 32;  // m8 and n8 fragments a warp
+  static constexpr int LT = TILE + 4, LK = KC + 4; // line pitch: row/column fast, k fast
+  static constexpr int oper = TILE * LK > KC * LT ? TILE * LK : KC * LT;  // doubles an operand
+  static constexpr int smem = kFdmStages * 2 * oper * (int)sizeof(double);
+};
 
-__device__ __forceinline__ void cp_async8(double *dst, const double *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
 }
 
 struct GemmArgs {
@@ -234,147 +246,160 @@ struct GemmArgs {
   double mu;
   double beta[12];
   const double *beta_ptr;  // if set, beta = *beta_ptr for every batch entry
-  // split K: slice s of batch entry b writes P[(s batch + b) R Cn + r Cn + c]
-  int splits;
-  double *P;
 };
 
-// stage K chunk [k0, k0 + KC) of the A and B tiles into buffer `buf`
-// (zeros outside the operands)
-__device__ __forceinline__ void stage_chunk(const GemmArgs &g, const double *A, const double *B,
-                                            int r0, int c0, int k0, double *buf, bool a_rfast,
-                                            bool b_cfast) {
-  double *As = buf, *Bs = buf + KC * LDT;
-#pragma unroll 4
-  for (int e = threadIdx.x; e < TR * KC; e += GT) {
-    const int rr = a_rfast ? (e & (TR - 1)) : (e >> 5), kk = a_rfast ? (e >> 6) : (e & (KC - 1));
-    const int r = r0 + rr, k = k0 + kk;
-    double *d = As + kk * LDT + rr;
-    if (r < g.R && k < g.K) cp_async8(d, A + (long long)r * g.sar + (long long)k * g.sak);
-    else *d = 0.0;
+// One operand's TILE lines (line l, k at src[l sl + k sk]) on their way to
+// shared memory, KC of k at a time; fast: the lines are adjacent in memory.  A
+// thread copies the same TILE KC / 256 places of every chunk, zeros beyond the
+// operand.
+template <int TILE>
+struct Stage {
+  using T = FdmTile<TILE>;
+  static constexpr int each = TILE * KC / GT;
+  const double *src;    // of its first place
+  long long next, adv;  // to its next place, to the next chunk
+  int l, k, dl, dk, dst, dnext;
+  __device__ __forceinline__ Stage(const double *base, long long sl, long long sk, int l0, bool fast) {
+    const int t = threadIdx.x;
+    const int ll = fast ? t % TILE : t / KC;
+    k = fast ? t / TILE : t % KC;
+    l = l0 + ll;
+    dl = fast ? 0 : GT / KC;
+    dk = fast ? GT / TILE : 0;
+    dst = fast ? k * T::LT + ll : ll * T::LK + k;
+    dnext = fast ? dk * T::LT : dl * T::LK;
+    src = base + l * sl + k * sk;
+    next = dl * sl + dk * sk;
+    adv = KC * sk;
   }
-#pragma unroll 4
-  for (int e = threadIdx.x; e < TC * KC; e += GT) {
-    const int cc = b_cfast ? (e & (TC - 1)) : (e >> 5), kk = b_cfast ? (e >> 6) : (e & (KC - 1));
-    const int c = c0 + cc, k = k0 + kk;
-    double *d = Bs + kk * LDT + cc;
-    if (c < g.Cn && k < g.K) cp_async8(d, B + (long long)k * g.sbk + (long long)c * g.sbc);
-    else *d = 0.0;
+  __device__ __forceinline__ void copy(double *buf, int lines, int K) {
+    const unsigned to = (unsigned)__cvta_generic_to_shared(buf + dst);
+#pragma unroll
+    for (int i = 0; i < each; ++i) {
+      const bool in = l + i * dl < lines && k + i * dk < K;
+      const double *p = in ? src + i * next : src0;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(to + 8u * (unsigned)(i * dnext)), "l"(p),
+                   "r"(in ? 8 : 0)
+                   : "memory");
+    }
+    src += adv;
+    k += KC;
   }
-  cp_async_commit();
-}
+  const double *src0 = nullptr;  // a valid address, not read
+};
 
-__global__ void __launch_bounds__(GT) k_fdm_gemm(GemmArgs g) {
-  extern __shared__ double sm[];
-  const int nb = gridDim.z / g.splits;
-  const int b = blockIdx.z % nb, sp = blockIdx.z / nb;
-  const int r0 = blockIdx.y * TR, c0 = blockIdx.x * TC;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+template <int TILE>
+__device__ __forceinline__ void fdm_tile(const GemmArgs &g, int b, int r0, int c0, double *sm) {
+  using T = FdmTile<TILE>;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const double *A = g.A + (long long)b * g.sab;
   const double *B = g.B + (long long)b * g.sbb;
-  double acc[4][4] = {};
-  const bool a_rfast = g.sar <= g.sak, b_cfast = g.sbc <= g.sbk;
-  // this slice's K range, in whole chunks
-  const int nall = (g.K + KC - 1) / KC, per = (nall + g.splits - 1) / g.splits;
-  const int ch0 = sp * per, ch1 = ch0 + per < nall ? ch0 + per : nall;
-  if (ch0 < ch1) stage_chunk(g, A, B, r0, c0, ch0 * KC, sm, a_rfast, b_cfast);
-  for (int ch = ch0; ch < ch1; ++ch) {
-    if (ch + 1 < ch1) {
-      stage_chunk(g, A, B, r0, c0, (ch + 1) * KC, sm + ((ch + 1 - ch0) & 1) * kBuf, a_rfast,
-                  b_cfast);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+  const bool af = g.sar <= g.sak, bf = g.sbc <= g.sbk;
+  const int nch = (g.K + KC - 1) / KC;
+  Stage<TILE> sa(A, g.sar, g.sak, r0, af), sb(B, g.sbc, g.sbk, c0, bf);
+  sa.src0 = A;
+  sb.src0 = B;
+  auto stage = [&](int ch) {
+    if (ch < nch) {
+      double *buf = sm + (ch % kFdmStages) * 2 * T::oper;
+      sa.copy(buf, g.R, g.K);
+      sb.copy(buf + T::oper, g.Cn, g.K);
     }
-    __syncthreads();
-    const double *As = sm + ((ch - ch0) & 1) * kBuf, *Bs = As + KC * LDT;
-    const int kc = g.K - ch * KC < KC ? g.K - ch * KC : KC;
-#pragma unroll 8
-    for (int kk = 0; kk < kc; ++kk) {
-      const double *ar = As + kk * LDT + ty, *br = Bs + kk * LDT + tx;
-      double a[4], bb[4];
+    cp_async_commit();
+  };
+  // the warp's part of the tile; a lane's row/column (lane / 4) and k (lane % 4) of a fragment
+  const int wr = (warp >> 2) * (TILE / 2), wc = (warp & 3) * (TILE / 4);
+  const int al = af ? 1 : T::LK, ak = af ? T::LT : 1, bl = bf ? 1 : T::LK, bk = bf ? T::LT : 1;
+  const int oa = (wr + (lane >> 2)) * al + (lane & 3) * ak, ob = (wc + (lane >> 2)) * bl + (lane & 3) * bk;
+  double acc[T::mi][T::ni][2] = {};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = ar[16 * i];
+  for (int ch = 0; ch < kFdmStages - 1; ++ch) stage(ch);
+  for (int ch = 0; ch < nch; ++ch) {
+    cp_async_wait<kFdmStages - 2>();
+    __syncthreads();  // chunk ch is in; the buffer of chunk ch - 1 is free
+    stage(ch + kFdmStages - 1);
+    const double *As = sm + (ch % kFdmStages) * 2 * T::oper + oa, *Bs = As - oa + T::oper + ob;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) bb[j] = br[16 * j];
+    for (int kk = 0; kk < KC; kk += 4) {
+      double fa[T::mi], fb[T::ni];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < T::mi; ++i) fa[i] = As[8 * i * al + kk * ak];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], bb[j], acc[i][j]);
+      for (int j = 0; j < T::ni; ++j) fb[j] = Bs[8 * j * bl + kk * bk];
+#pragma unroll
+      for (int i = 0; i < T::mi; ++i)
+#pragma unroll
+        for (int j = 0; j < T::ni; ++j) mma_f64(acc[i][j], fa[i], fb[j]);
     }
-    __syncthreads();  // this buffer is restaged by the next round
-  }
-  if (g.splits > 1) {
-    double *P = g.P + ((long long)sp * nb + b) * g.R * g.Cn;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = r0 + ty + 16 * i;
-      if (r >= g.R) continue;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = c0 + tx + 16 * j;
-        if (c < g.Cn) P[(long long)r * g.Cn + c] = acc[i][j];
-      }
-    }
-    return;
   }
   const double beta = g.beta_ptr ? *g.beta_ptr : g.beta[b < 12 ? b : 11];
   double *C = g.C + (long long)b * g.scb;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = r0 + ty + 16 * i;
+  for (int i = 0; i < T::mi; ++i) {
+    const int r = r0 + wr + 8 * i + (lane >> 2);
     if (r >= g.R) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = c0 + tx + 16 * j;
-      if (c >= g.Cn) continue;
-      double v = acc[i][j];
-      if (g.scale) v /= beta * (g.lr[r] + g.lc[c]) + g.mu;
-      C[(long long)r * g.scr + (long long)c * g.scc] = v;
-    }
+    for (int j = 0; j < T::ni; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = c0 + wc + 8 * j + 2 * (lane & 3) + e;
+        if (c >= g.Cn) continue;
+        double v = acc[i][j][e];
+        if (g.scale) v /= beta * (g.lr[r] + g.lc[c]) + g.mu;
+        C[(long long)r * g.scr + (long long)c * g.scc] = v;
+      }
   }
 }
 
-// the kernel's dynamic shared memory (above the 48 KB default) on the current
+template <int TILE>
+__global__ void __launch_bounds__(GT) k_fdm_gemm(const __grid_constant__ GemmArgs g) {
+  extern __shared__ double sm[];
+  fdm_tile<TILE>(g, blockIdx.z, blockIdx.y * TILE, blockIdx.x * TILE, sm);
+}
+
+// The four products of a small solve in one launch: a cluster of eight CTAs
+// takes the 32 x 32 tiles of a product in turn and meets at the cluster's
+// barrier (a few hundred cycles, where a launch costs some 2 us).
+struct FdmChain {
+  GemmArgs g[4];
+  int batch;
+};
+__global__ void __launch_bounds__(GT) __cluster_dims__(kFdmCluster, 1, 1)
+    k_fdm_chain(const __grid_constant__ FdmChain ch) {
+  extern __shared__ double sm[];
+#pragma unroll 1
+  for (int q = 0; q < 4; ++q) {
+    const GemmArgs &g = ch.g[q];
+    const int tc = (g.Cn + 31) / 32, tr = (g.R + 31) / 32;
+    for (int t = blockIdx.x; t < tc * tr * ch.batch; t += kFdmCluster) {
+      fdm_tile<32>(g, t / (tc * tr), t % (tc * tr) / tc * 32, t % tc * 32, sm);
+      __syncthreads();  // the ring is refilled
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  }
+}
+
+// the kernels' dynamic shared memory (above the 48 KB default) on the current
 // device; set by fdm_ensure, ahead of any stream capture
 int gemm_setup() {
-  ALDIC_CUDA(cudaFuncSetAttribute(k_fdm_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  ALDIC_CUDA(cudaFuncSetAttribute(k_fdm_gemm<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, FdmTile<32>::smem));
+  ALDIC_CUDA(cudaFuncSetAttribute(k_fdm_gemm<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, FdmTile<64>::smem));
+  ALDIC_CUDA(cudaFuncSetAttribute(k_fdm_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, FdmTile<32>::smem));
   return OK;
 }
 
-// the split-K slices of every output summed in slice order, then the epilogue
-__global__ void k_fdm_reduce(GemmArgs g, int batch) {
-  const long long rc = (long long)g.R * g.Cn, n = rc * batch;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int b = (int)(i / rc);
-    const long long e = i - (long long)b * rc;
-    const int r = (int)(e / g.Cn), c = (int)(e - (long long)r * g.Cn);
-    double v = 0.0;
-    for (int s = 0; s < g.splits; ++s) v += g.P[((long long)s * batch + b) * rc + e];
-    if (g.scale) {
-      const double beta = g.beta_ptr ? *g.beta_ptr : g.beta[b < 12 ? b : 11];
-      v /= beta * (g.lr[r] + g.lc[c]) + g.mu;
-    }
-    g.C[(long long)b * g.scb + (long long)r * g.scr + (long long)c * g.scc] = v;
-  }
-}
-
-int gemm(GemmArgs g, int batch, double *part, cudaStream_t st) {
-  const int tiles = ((g.Cn + TC - 1) / TC) * ((g.R + TR - 1) / TR) * batch;
-  int sp = 1;
-  while (sp < kMaxSplit && tiles * sp < 148 && (sp + 1) * batch <= kFdmPart) ++sp;
-  g.splits = sp;
-  g.P = part;
-  dim3 grid((unsigned)((g.Cn + TC - 1) / TC), (unsigned)((g.R + TR - 1) / TR), (unsigned)(batch * sp));
-  k_fdm_gemm<<<grid, GT, kSmem, st>>>(g);
+template <int TILE>
+int gemm_tile(const GemmArgs &g, int batch, cudaStream_t st) {
+  const dim3 grid((unsigned)((g.Cn + TILE - 1) / TILE), (unsigned)((g.R + TILE - 1) / TILE), (unsigned)batch);
+  k_fdm_gemm<TILE><<<grid, GT, FdmTile<TILE>::smem, st>>>(g);
   ALDIC_CUDA(cudaGetLastError());
-  if (sp > 1) {
-    const long long n = (long long)g.R * g.Cn * batch;
-    k_fdm_reduce<<<(unsigned)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184), 256, 0, st>>>(g, batch);
-    ALDIC_CUDA(cudaGetLastError());
-  }
   return OK;
+}
+long long gemm_tiles(int R, int Cn, int batch, int tile) {
+  return (long long)((Cn + tile - 1) / tile) * ((R + tile - 1) / tile) * batch;
+}
+int gemm(const GemmArgs &g, int batch, cudaStream_t st) {
+  return gemm_tiles(g.R, g.Cn, batch, 64) >= kFdmBig ? gemm_tile<64>(g, batch, st) : gemm_tile<32>(g, batch, st);
 }
 
 }  // namespace
@@ -436,18 +461,16 @@ int fdm_basis_1d(int type, int n, double h, double *V, double *lam) {
 }
 
 int fdm_ensure(FdmBasis &B, int type, int M, int N, double h, cudaStream_t st) {
-  int rc0 = gemm_setup();
-  if (rc0) return rc0;
   if (B.type == type && B.M == M && B.N == N && B.h == h && B.buf.p) return OK;
   ALDIC_CHECK(M >= 1 && N >= 1, E_ARG, "fdm: empty grid");
   std::vector<double> host((size_t)M * M + (size_t)N * N + M + N);
   double *Vx = host.data(), *Vy = Vx + (size_t)M * M, *lx = Vy + (size_t)N * N, *ly = lx + M;
   int rc;
+  if ((rc = gemm_setup())) return rc;
   if ((rc = fdm_basis_1d(type, M, h, Vx, lx))) return rc;
   if ((rc = fdm_basis_1d(type, N, h, Vy, ly))) return rc;
   B.type = -1;
-  const size_t nbasis = host.size();
-  if ((rc = B.buf.ensure(sizeof(double) * (nbasis + (size_t)kFdmPart * M * N)))) return rc;
+  if ((rc = B.buf.ensure(sizeof(double) * host.size()))) return rc;
   ALDIC_CUDA(cudaMemcpyAsync(B.buf.p, host.data(), sizeof(double) * host.size(),
                              cudaMemcpyHostToDevice, st));
   ALDIC_CUDA(cudaStreamSynchronize(st));  // the host vector goes out of scope
@@ -456,7 +479,6 @@ int fdm_ensure(FdmBasis &B, int type, int M, int N, double h, cudaStream_t st) {
   B.Vy = d + (size_t)M * M;
   B.lx = B.Vy + (size_t)N * N;
   B.ly = B.lx + M;
-  B.part = d + nbasis;
   B.type = type;
   B.M = M;
   B.N = N;
@@ -465,40 +487,51 @@ int fdm_ensure(FdmBasis &B, int type, int M, int N, double h, cudaStream_t st) {
 }
 
 int fdm_solve(const FdmBasis &B, int nrhs, const double *b, double *x, double *tmp, double mu,
-              double beta, const double *beta_each, const double *beta_ptr, cudaStream_t st) {
+              double beta, const double *beta_each, const double *beta_ptr, cudaStream_t st,
+              double *inter) {
   ALDIC_CHECK(B.buf.p && nrhs >= 1 && nrhs <= 12, E_ARG, "fdm solve: bad arguments");
   const int M = B.M, N = B.N;
   const long long n = (long long)M * N;
-  GemmArgs g{};
+  FdmChain ch{};
+  ch.batch = nrhs;
+  GemmArgs &g = ch.g[0];
   g.mu = mu;
   for (int f = 0; f < 12; ++f) g.beta[f] = (beta_each && f < nrhs) ? beta_each[f] : beta;
   g.beta_ptr = beta_ptr;
-  int rc;
+  g.R = N; g.Cn = M;
+  for (int q = 1; q < 4; ++q) ch.g[q] = g;
   // field f as an N x M matrix (row j = node row y, column i = x): B_f[j][i] = b[f n + j M + i]
-  // 1. T = B_f Vx  -> tmp
-  g.A = b; g.sab = n; g.sar = M; g.sak = 1;
-  g.B = B.Vx; g.sbb = 0; g.sbk = M; g.sbc = 1;
-  g.C = tmp; g.scb = n; g.scr = M; g.scc = 1;
-  g.R = N; g.Cn = M; g.K = M; g.scale = 0;
-  if ((rc = gemm(g, nrhs, B.part, st))) return rc;
-  // 2. C = Vy' T, C[q][p] /= beta (ly[q] + lx[p]) + mu  -> x
-  g.A = B.Vy; g.sab = 0; g.sar = 1; g.sak = N;
-  g.B = tmp; g.sbb = n; g.sbk = M; g.sbc = 1;
-  g.C = x; g.scb = n; g.scr = M; g.scc = 1;
-  g.R = N; g.Cn = M; g.K = N; g.scale = 1; g.lr = B.ly; g.lc = B.lx;
-  if ((rc = gemm(g, nrhs, B.part, st))) return rc;
-  // 3. S = C Vx'  -> tmp
-  g.A = x; g.sab = n; g.sar = M; g.sak = 1;
-  g.B = B.Vx; g.sbb = 0; g.sbk = 1; g.sbc = M;
-  g.C = tmp; g.scb = n; g.scr = M; g.scc = 1;
-  g.R = N; g.Cn = M; g.K = M; g.scale = 0;
-  if ((rc = gemm(g, nrhs, B.part, st))) return rc;
-  // 4. X = Vy S  -> x
-  g.A = B.Vy; g.sab = 0; g.sar = N; g.sak = 1;
-  g.B = tmp; g.sbb = n; g.sbk = M; g.sbc = 1;
-  g.C = x; g.scb = n; g.scr = M; g.scc = 1;
-  g.R = N; g.Cn = M; g.K = N; g.scale = 0;
-  return gemm(g, nrhs, B.part, st);
+  auto set = [&](int q, const double *A, long long sab, long long sar, long long sak, const double *Bm,
+                 long long sbb, long long sbk, long long sbc, double *C, int K) {
+    GemmArgs &p = ch.g[q];
+    p.A = A; p.sab = sab; p.sar = sar; p.sak = sak;
+    p.B = Bm; p.sbb = sbb; p.sbk = sbk; p.sbc = sbc;
+    p.C = C; p.scb = n; p.scr = M; p.scc = 1;
+    p.K = K;
+  };
+  set(0, b, n, M, 1, B.Vx, 0, M, 1, tmp, M);     // T = B_f Vx
+  set(1, B.Vy, 0, 1, N, tmp, n, M, 1, x, N);     // C = Vy' T, C[q][p] /= beta (ly[q] + lx[p]) + mu
+  ch.g[1].scale = 1; ch.g[1].lr = B.ly; ch.g[1].lc = B.lx;
+  set(2, x, n, M, 1, B.Vx, 0, 1, M, tmp, M);     // S = C Vx'
+  set(3, B.Vy, 0, N, 1, tmp, n, M, 1, x, N);     // X = Vy S
+  if (inter) {
+    ch.g[3].C = inter;
+    ch.g[3].scb = 1; ch.g[3].scr = (long long)nrhs * M; ch.g[3].scc = nrhs;
+  }
+  // One launch while the cluster has a tile a CTA: a whole aldic_subpb2 at 43 x 43
+  // takes 42.6 us this way and 58 us with four launches; with two rounds of
+  // tiles (61 x 97, 55.4 us) it is no faster than four launches of 128 x 128
+  // (53.7 us).
+  if (gemm_tiles(N, M, nrhs, 32) <= kFdmChainTiles) {
+    k_fdm_chain<<<kFdmCluster, GT, FdmTile<32>::smem, st>>>(ch);
+    ALDIC_CUDA(cudaGetLastError());
+    return OK;
+  }
+  for (int q = 0; q < 4; ++q) {
+    const int rc = gemm(ch.g[q], nrhs, st);
+    if (rc) return rc;
+  }
+  return OK;
 }
 
 // The beta sweep's eigen-domain solutions from the two transformed
@@ -539,13 +572,13 @@ int fdm_solve_sweep(const FdmBasis &B, const double beta[6], const double *b, do
   g.B = B.Vx; g.sbb = 0; g.sbk = M; g.sbc = 1;
   g.C = tmp; g.scb = n; g.scr = M; g.scc = 1;
   g.R = N; g.Cn = M; g.K = M; g.scale = 0;
-  if ((rc = gemm(g, 4, B.part, st))) return rc;
+  if ((rc = gemm(g, 4, st))) return rc;
   // 2. C = Vy' T, unscaled -> tmp fields 4-7
   g.A = B.Vy; g.sab = 0; g.sar = 1; g.sak = N;
   g.B = tmp; g.sbb = n; g.sbk = M; g.sbc = 1;
   g.C = tmp + 4 * n; g.scb = n; g.scr = M; g.scc = 1;
   g.R = N; g.Cn = M; g.K = N; g.scale = 0;
-  if ((rc = gemm(g, 4, B.part, st))) return rc;
+  if ((rc = gemm(g, 4, st))) return rc;
   // the six systems' scaled eigen-domain solutions -> x fields 0-11
   SweepBetas be;
   for (int k = 0; k < 6; ++k) be.v[k] = beta[k];
@@ -557,13 +590,13 @@ int fdm_solve_sweep(const FdmBasis &B, const double beta[6], const double *b, do
   g.B = B.Vx; g.sbb = 0; g.sbk = 1; g.sbc = M;
   g.C = tmp; g.scb = n; g.scr = M; g.scc = 1;
   g.R = N; g.Cn = M; g.K = M; g.scale = 0;
-  if ((rc = gemm(g, 12, B.part, st))) return rc;
+  if ((rc = gemm(g, 12, st))) return rc;
   // 4. X = Vy S -> x
   g.A = B.Vy; g.sab = 0; g.sar = N; g.sak = 1;
   g.B = tmp; g.sbb = n; g.sbk = M; g.sbc = 1;
   g.C = x; g.scb = n; g.scr = M; g.scc = 1;
   g.R = N; g.Cn = M; g.K = N; g.scale = 0;
-  return gemm(g, 12, B.part, st);
+  return gemm(g, 12, st);
 }
 
 }  // namespace aldic

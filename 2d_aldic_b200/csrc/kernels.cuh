@@ -120,8 +120,8 @@ enum { FDM_FE = 0, FDM_FD = 1 };
 struct FdmBasis {
   int type = -1, M = 0, N = 0;
   double h = 0.0;
-  DevBuf buf;  // Vx (M x M), Vy (N x N), lx (M), ly (N), split-K partials (kFdmPart M N)
-  double *Vx = nullptr, *Vy = nullptr, *lx = nullptr, *ly = nullptr, *part = nullptr;
+  DevBuf buf;  // Vx (M x M), Vy (N x N), lx (M), ly (N)
+  double *Vx = nullptr, *Vy = nullptr, *lx = nullptr, *ly = nullptr;
   void release() {
     buf.release();
     type = -1;
@@ -135,9 +135,12 @@ int fdm_basis_1d(int type, int n, double h, double *V, double *lam);
 int fdm_ensure(FdmBasis &B, int type, int M, int N, double h, cudaStream_t st);
 // x_f = A_f^-1 b_f for the nrhs fields of M*N values (x fastest) at b, x;
 // A_f = beta_f (Kx (+) Ky) + mu Mx (x) My with beta_f = *beta_ptr if given,
-// else beta_each[f] if given, else beta; tmp: nrhs*M*N doubles
+// else beta_each[f] if given, else beta; tmp: nrhs*M*N doubles.  With `inter`
+// the solution goes there, field f of node k at inter[nrhs k + f], and x is
+// only workspace.
 int fdm_solve(const FdmBasis &B, int nrhs, const double *b, double *x, double *tmp, double mu,
-              double beta, const double *beta_each, const double *beta_ptr, cudaStream_t st);
+              double beta, const double *beta_each, const double *beta_ptr, cudaStream_t st,
+              double *inter = nullptr);
 // the beta sweep's six systems at once from the two right-hand-side parts
 // (b fields 0-1: beta part, 2-3: mu part): x fields 2q, 2q + 1 solve
 // (beta[q] K + mu M) x = beta[q] b_beta + mu b_mu; tmp holds 12 fields
@@ -257,7 +260,7 @@ int fe_rhs(GridWork &w, int M, int N, double h, double beta, double mu, const do
 int fe_rhs_parts(GridWork &w, int M, int N, double h, const double *U, const double *F,
                  const double *udual, const double *vdual, cudaStream_t st);
 // interleave w.x (2 fields from slot f0) into Uhat
-int fe_store(const GridWork &w, int M, int N, double *Uhat, cudaStream_t st, int f0 = 0);
+int fe_store(const GridWork &w, int M, int N, double *Uhat, cudaStream_t st);
 // nodal strain (funGlobal_NodalStrainAvg.m)
 int nodal_strain(int M, int N, double h, const double *U, double *F, cudaStream_t st);
 // gridfit 'springs' of nf fields of node values (NaN, or a status in bad < 0 or

@@ -1052,6 +1052,9 @@ int csr_pcg(GridWork &w, const CsrOp &op, long long n, int nrhs, double rtol, in
             cudaStream_t st, const double *beta_each, double mu) {
   ALDIC_CHECK(nrhs >= 1 && nrhs <= 6, E_ARG, "csr_pcg: 1..6 right-hand sides");
   ALDIC_CHECK(n >= 1 && n < (1LL << 31), E_ARG, "csr_pcg: bad size");
+  bool ran = false;
+  const int rc = cluster_csr(w, op, n, nrhs, rtol, maxit, beta_each, mu, st, &ran);
+  if (rc || ran) return rc;
   int dev = 0, sms = 148;
   ALDIC_CUDA(cudaGetDevice(&dev));
   ALDIC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

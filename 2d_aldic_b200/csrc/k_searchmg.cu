@@ -1284,8 +1284,10 @@ int search_mg_fit(GridWork &gw, MgWork &w, MgData &d, const MgGrid &grid, int nf
     ALDIC_CUDA(cudaMemsetAsync(gw.x, 0, sizeof(double) * nr * ng, st));
     ALDIC_CUDA(cudaMemsetAsync(gw.mask, 1, (size_t)nr * ng, st));
     const double lam2 = (NA / NR) * (NA / NR);
-    if ((rc = grid_pcg(gw, OP_GRIDFIT, nx, ny, nr, 0.0, 0.0, 1.0, lam2, 1e-13, 20000, st, nullptr,
-                       nullptr, data)))
+    bool ran = false;
+    if ((rc = cluster_ata(gw, data, nx, ny, nr, lam2, 1e-13, 20000, st, &ran))) return rc;
+    if (!ran && (rc = grid_pcg(gw, OP_GRIDFIT, nx, ny, nr, 0.0, 0.0, 1.0, lam2, 1e-13, 20000, st, nullptr,
+                               nullptr, data)))
       return rc;
     for (int m = 0; m < nr; ++m)
       ALDIC_CUDA(cudaMemcpyAsync(out + (size_t)mem[m] * ng, gw.x + (size_t)m * ng, sizeof(double) * ng,

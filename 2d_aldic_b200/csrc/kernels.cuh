@@ -181,6 +181,13 @@ struct CsrOp {
 };
 int csr_pcg(GridWork &w, const CsrOp &op, long long n, int nrhs, double rtol, int maxit,
             cudaStream_t st, const double *beta_each = nullptr, double mu = 0.0);
+// The same solves, and those of the scattered gridfit system (A'A of 9
+// coefficients a node and springs lam2, right-hand sides w.b, start w.x), by a
+// cluster a field (k_cluster.cu); *ran says whether the system was of a size for it
+int cluster_csr(GridWork &w, const CsrOp &op, long long n, int nrhs, double rtol, int maxit,
+                const double *beta_each, double mu, cudaStream_t st, bool *ran);
+int cluster_ata(GridWork &w, const double *ata, int M, int N, int nrhs, double lam2, double rtol, int maxit,
+                cudaStream_t st, bool *ran);
 
 // ---- BF16 tensor-core GEMM (k_gemm.cu): D = A . B^T over K
 enum GemmMode { GEMM_ROW = 0, GEMM_PATCH = 1, GEMM_TRANS = 2, GEMM_PATCHT = 3 };

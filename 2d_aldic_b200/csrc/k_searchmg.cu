@@ -8,12 +8,14 @@
 //   * summed-area tables of f, f^2, g, g^2 (exact 64-bit for integer images)
 //     give every window sum of the normalised cross-correlation in O(1);
 //   * level 1: normxcorr2 of the whole f ROI against the g ROI for every
-//     shift by an FP64 FFT cross-correlation (own radix-2 kernels: rows in
-//     shared memory, tiled transposes; the two real transforms packed into
-//     one complex one), then an argmax reduction and findpeak's 3x3 fit;
+//     shift by an FP64 FFT cross-correlation (own kernels: radix 8 in
+//     registers, tiled transposes; the two real inputs packed into one
+//     complex row, two real output rows into one; the NCC map is formed and
+//     searched by the last transform), then findpeak's 3x3 fit;
 //   * intermediate levels: the 13 x 14 cropped map of every region from
-//     exact integer products -- CTAs over (region, 8-row band, 256-column
-//     tile), each thread a register window over 13 horizontal shifts;
+//     exact integer products -- CTAs over (region, row band, 256-column
+//     tile), each thread a register window over 13 horizontal shifts, packed
+//     byte products for integer images;
 //   * last level: the full (2a+9) x (2b+9) map of every region in shared
 //     memory (for compute_qFactor), with register-blocked strips of 8 shifts.
 // Host side: the region bookkeeping of funIntegerSearchMg.m (splits, border
@@ -93,101 +95,150 @@ __device__ __forceinline__ double combine(long long mn, S st, S st2, S stdv, S s
 
 // ------------------------------------------------------------ summed-area tables
 // sat[0..3] = f, f^2, g, g^2, each (W+1) x (H+1), row 0 and column 0 zero.
-// Pass 1: one block per image row, block-wide scan along x.
+// Bound by the writes of the tables (32 bytes a pixel, 134 MB at 2048 x 2048):
+// they are written once.  (Rows, then columns in place in two passes moved them
+// five times, 208 us; this takes 94 us.)
+// Pass 1: sums of each column over chunks of kSatChunk rows, read from the images.
+constexpr int kSatChunk = 16;
 template <typename P>
-__global__ void k_sat_rows(const P *__restrict__ f, const P *__restrict__ g, int W, int H,
-                           typename MgT<P>::S *__restrict__ sat) {
+__global__ void k_sat_chunks(const P *__restrict__ f, const P *__restrict__ g, int W, int H,
+                             typename MgT<P>::S *__restrict__ tot) {
   using S = typename MgT<P>::S;
-  const int y = blockIdx.x;  // image row -> table row y + 1
-  const int q = blockIdx.y;  // 0 f, 1 f^2, 2 g, 3 g^2
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, ch = blockIdx.y, nch = gridDim.y;
+  if (x >= W) return;
+  const int y0 = ch * kSatChunk, y1 = min(H, y0 + kSatChunk);
+  S a[4] = {0, 0, 0, 0};
+  for (int y = y0; y < y1; ++y) {
+    const S u = (S)f[(long long)y * W + x], v = (S)g[(long long)y * W + x];
+    a[0] += u;
+    a[1] += u * u;
+    a[2] += v;
+    a[3] += v * v;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) tot[((long long)q * nch + ch) * W + x] = a[q];
+}
+// Pass 2: each chunk's entry becomes the column's sum above the chunk.
+template <typename S>
+__global__ void k_sat_above(S *__restrict__ tot, int W, int nch) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= W) return;
+  S *p = tot + (long long)blockIdx.y * nch * W + x;
+  S acc = 0;
+  for (int c0 = 0; c0 < nch; c0 += 8) {
+    S v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = c0 + e < nch ? p[(long long)(c0 + e) * W] : S(0);
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (c0 + e < nch) {
+        p[(long long)(c0 + e) * W] = acc;
+        acc += v[e];
+      }
+  }
+}
+// Pass 3: the rows of a chunk: running column sums in registers, scanned along x
+// a warp a kSatSpan columns, the warps' totals and those of the columns to the
+// left through shared memory.
+constexpr int kSatThreads = 256, kSatItems = 8, kSatSpan = 32 * kSatItems;
+template <typename P>
+__global__ void __launch_bounds__(kSatThreads)
+    k_sat_fill(const P *__restrict__ f, const P *__restrict__ g, int W, int H,
+               const typename MgT<P>::S *__restrict__ tot, typename MgT<P>::S *__restrict__ sat) {
+  using S = typename MgT<P>::S;
+  constexpr int kWarps = kSatThreads / 32;
+  __shared__ S warp_tot[2][kWarps], left[kSatChunk];
+  const int q = blockIdx.y, ch = blockIdx.x, nch = gridDim.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const P *img = q < 2 ? f : g;
   const bool sq = q & 1;
-  const long long W1 = W + 1, plane = W1 * (H + 1);
-  S *row = sat + q * plane + (long long)(y + 1) * W1;
-  __shared__ S wsum[32];
-  __shared__ S carry;
-  if (threadIdx.x == 0) {
-    carry = 0;
-    row[0] = 0;
-    if (y == 0) sat[q * plane] = 0;
+  const long long W1 = W + 1;
+  S *out = sat + q * W1 * (H + 1);
+  const int y0 = ch * kSatChunk, rows = min(H - y0, kSatChunk);
+  if (ch == 0)
+    for (int x = threadIdx.x; x <= W; x += kSatThreads) out[x] = 0;
+  if (threadIdx.x < rows) {
+    left[threadIdx.x] = 0;
+    out[(y0 + 1 + threadIdx.x) * W1] = 0;
   }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int x0 = 0; x0 < W; x0 += blockDim.x) {
-    const int x = x0 + threadIdx.x;
-    S v = 0;
-    if (x < W) {
-      const S p = (S)img[(long long)y * W + x];
-      v = sq ? p * p : p;
+  for (int x0 = 0; x0 < W; x0 += kWarps * kSatSpan) {
+    S col[kSatItems];
+    const int xw = x0 + warp * kSatSpan + lane;
+#pragma unroll
+    for (int e = 0; e < kSatItems; ++e) {
+      const int x = xw + 32 * e;
+      col[e] = x < W ? tot[((long long)q * nch + ch) * W + x] : S(0);
     }
-    for (int o = 1; o < 32; o <<= 1) {
-      const S t = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += t;
-    }
-    if (lane == 31) wsum[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-      S t = lane < nw ? wsum[lane] : 0;
-      for (int o = 1; o < 32; o <<= 1) {
-        const S u = __shfl_up_sync(0xffffffffu, t, o);
-        if (lane >= o) t += u;
+    P next[kSatItems];  // the row to come, on its way during this one's scan
+    auto fetch = [&](int r) {
+#pragma unroll
+      for (int e = 0; e < kSatItems; ++e) {
+        const int x = xw + 32 * e;
+        next[e] = r < rows && x < W ? img[(long long)(y0 + r) * W + x] : P(0);
       }
-      if (lane < nw) wsum[lane] = t;
+    };
+    fetch(0);
+    __syncthreads();  // left is set
+    for (int r = 0; r < rows; ++r) {
+      S v[kSatItems], run = 0;
+      S px[kSatItems];
+#pragma unroll
+      for (int e = 0; e < kSatItems; ++e) px[e] = (S)next[e];
+      fetch(r + 1);
+#pragma unroll
+      for (int e = 0; e < kSatItems; ++e) {
+        col[e] += sq ? px[e] * px[e] : px[e];
+        S t = col[e];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const S n = __shfl_up_sync(0xffffffffu, t, o);
+          if (lane >= o) t += n;
+        }
+        v[e] = run + t;
+        run += __shfl_sync(0xffffffffu, t, 31);
+      }
+      if (lane == 0) warp_tot[r & 1][warp] = run;
+      __syncthreads();
+      S before = left[r];
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) before += w < warp ? warp_tot[r & 1][w] : S(0);
+#pragma unroll
+      for (int e = 0; e < kSatItems; ++e) {
+        const int x = xw + 32 * e;
+        if (x < W) out[(y0 + 1 + r) * W1 + x + 1] = before + v[e];
+      }
+      if (x0 + kWarps * kSatSpan < W) {  // the row's sum so far, for the columns to come
+        __syncthreads();
+        if (threadIdx.x == kSatThreads - 1) left[r] = before + v[kSatItems - 1];
+      }
     }
     __syncthreads();
-    const S base = carry + (wid ? wsum[wid - 1] : 0);
-    if (x < W) row[x + 1] = base + v;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = base + v;
-    __syncthreads();
   }
-  // first table row (zeros) for columns > 0
-  if (y == 0)
-    for (int x = threadIdx.x; x < W; x += blockDim.x) sat[q * plane + x + 1] = 0;
-}
-
-// Pass 2: columns, in chunks of rows: scan each chunk, then add the totals
-// of the chunks above.
-constexpr int kSatChunk = 64;
-template <typename S>
-__global__ void k_sat_cols_chunk(S *__restrict__ sat, int W, int H, S *__restrict__ tot) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int q = blockIdx.z, ch = blockIdx.y;
-  const long long W1 = W + 1, plane = W1 * (H + 1);
-  if (x > W) return;
-  S *p = sat + q * plane;
-  const int y0 = 1 + ch * kSatChunk, y1 = min(H + 1, y0 + kSatChunk);
-  S acc = 0;
-  for (int y = y0; y < y1; ++y) {
-    acc += p[(long long)y * W1 + x];
-    p[(long long)y * W1 + x] = acc;
-  }
-  tot[((long long)q * gridDim.y + ch) * W1 + x] = acc;
-}
-template <typename S>
-__global__ void k_sat_cols_fix(S *__restrict__ sat, int W, int H, const S *__restrict__ tot) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int q = blockIdx.z, ch = blockIdx.y;
-  const long long W1 = W + 1, plane = W1 * (H + 1);
-  if (x > W || ch == 0) return;
-  S off = 0;
-  for (int c = 0; c < ch; ++c) off += tot[((long long)q * gridDim.y + c) * W1 + x];
-  S *p = sat + q * plane;
-  const int y0 = 1 + ch * kSatChunk, y1 = min(H + 1, y0 + kSatChunk);
-  for (int y = y0; y < y1; ++y) p[(long long)y * W1 + x] += off;
 }
 
 // ------------------------------------------------------------ FFT (FP64)
-// Stockham autosort transform of one row in shared memory: passes of radix
-// 8 (a radix-2 or radix-4 pass first when log2 L is not a multiple of 3),
-// each thread loading R values L/R apart, twiddling, an R-point DFT in
-// registers and writing them Ns apart -- natural order in and out, no
-// bit reversal.  Twiddles come from a table of exp(-2 pi i t / L).
-__global__ void k_fft_twiddle(double2 *tw, int L) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= L) return;
+// Stockham autosort transform of one row, a CTA of L / 8 threads a row: passes
+// of radix 8 (a radix-2 or radix-4 pass first when log2 L is not a multiple of
+// 3), every thread eight values in registers: read L/R apart, twiddled, an
+// R-point DFT, handed on Ns apart through shared memory (entry e at e + e/8, so
+// that no pass has a bank conflict) -- natural order in and out, no bit reversal.
+// The first pass reads and the last writes what the caller gives, so a row is
+// not staged.  Twiddles come from a table laid out as the passes read them:
+// exp(-2 pi i k q / 8 Ns) at (q - 1) Ns + k of the pass.
+// What bounds it at 4096: three exchanges of 128 KB a row through shared memory,
+// some 3000 cycles, and as many of FP64; two CTAs an SM overlap them with the
+// loads.  A pass over 4096 rows took 450 us with staged rows, 8-way conflicts
+// and one CTA an SM; 123 us now (half of its rows zeros that are not read).
+__global__ void k_fft_twiddle(double2 *tw, int L, int logL) {
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int rem = logL % 3;
+  int at = t, Ns = rem == 1 ? 2 : rem == 2 ? 4 : 8;
+  for (; Ns < L && at >= 7 * Ns; Ns *= 8) at -= 7 * Ns;
+  if (Ns >= L) return;
+  const int q = 1 + at / Ns, k = at % Ns;
   double s, c;
-  sincospi(2.0 * (double)k / (double)L, &s, &c);
-  tw[k] = make_double2(c, -s);  // exp(-2 pi i k / L)
+  sincospi(2.0 * (double)(k * q) / (8.0 * Ns), &s, &c);
+  tw[t] = make_double2(c, -s);
 }
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
@@ -200,8 +251,8 @@ __device__ __forceinline__ double2 cmi(double2 a, bool inv) {
   return inv ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x);
 }
 
-template <int R>
-__device__ __forceinline__ void dft_reg(double2 *a, bool inv) {
+template <int R, bool inv>
+__device__ __forceinline__ void dft_reg(double2 *a) {
   if constexpr (R == 2) {
     const double2 t = a[0];
     a[0] = cadd(t, a[1]);
@@ -240,177 +291,206 @@ __device__ __forceinline__ void dft_reg(double2 *a, bool inv) {
   }
 }
 
-// index groups per thread in a radix-R pass: every value of an 8192-point
-// row is held in registers by the 512 threads between read and write
-template <int R> struct FftJ { static constexpr int J = kMaxFFT / (R * 512); };
+__device__ __forceinline__ int fft_pos(int e) { return e + (e >> 3); }
+__host__ __device__ inline int fft_threads(int L) { return L / 8 < 32 ? 32 : L / 8; }
+inline size_t fft_smem(int L) { return sizeof(double2) * (size_t)(L + L / 8 + 1); }
 
-template <int R>
-__device__ void stockham_pass(double2 *s, int L, int Ns, const double2 *__restrict__ tw, bool inv) {
-  constexpr int kFftJ = FftJ<R>::J;
-  const int nj = L / R, tstep = L / (Ns * R);
-  double2 v[kFftJ][R];
+template <int R, bool INV, bool FIRST, bool LAST, typename Load, typename Store>
+__device__ __forceinline__ void stockham_pass(double2 *s, int L, int Ns, const double2 *__restrict__ tw, Load load,
+                                              Store store) {
+  constexpr int G = 8 / R;  // groups a thread
+  const int nj = L / R;
+  double2 v[G][R];
 #pragma unroll
-  for (int t = 0; t < kFftJ; ++t) {
+  for (int t = 0; t < G; ++t) {
     const int j = threadIdx.x + t * blockDim.x;
     if (j < nj) {
 #pragma unroll
-      for (int q = 0; q < R; ++q) v[t][q] = s[j + q * nj];
+      for (int q = 0; q < R; ++q) v[t][q] = FIRST ? load(j + q * nj) : s[fft_pos(j + q * nj)];
     }
   }
-  __syncthreads();
+  if (!FIRST) __syncthreads();
 #pragma unroll
-  for (int t = 0; t < kFftJ; ++t) {
+  for (int t = 0; t < G; ++t) {
     const int j = threadIdx.x + t * blockDim.x;
     if (j < nj) {
-      const int k = j % Ns;
+      const int k = j & (Ns - 1);
+      if (!FIRST) {
 #pragma unroll
-      for (int q = 1; q < R; ++q) {
-        double2 w = __ldg(&tw[k * q * tstep]);
-        if (inv) w.y = -w.y;
-        v[t][q] = cmul(v[t][q], w);
+        for (int q = 1; q < R; ++q) {
+          double2 w = __ldg(&tw[(q - 1) * Ns + k]);
+          if (INV) w.y = -w.y;
+          v[t][q] = cmul(v[t][q], w);
+        }
       }
-      dft_reg<R>(v[t], inv);
-      const int base = (j / Ns) * Ns * R + k;
+      dft_reg<R, INV>(v[t]);
+      const int base = (j - k) * R + k;
 #pragma unroll
-      for (int q = 0; q < R; ++q) s[base + q * Ns] = v[t][q];
+      for (int q = 0; q < R; ++q) {
+        if (LAST) store(base + q * Ns, v[t][q]);
+        else s[fft_pos(base + q * Ns)] = v[t][q];
+      }
     }
   }
-  __syncthreads();
+  if (!LAST) __syncthreads();
 }
 
-// the whole row: s[0..L) in natural order, L = 2^logL <= 8192
-__device__ void fft_smem(double2 *s, int L, int logL, const double2 *__restrict__ tw, bool inv) {
-  int Ns = 1;
-  const int rem = logL % 3;
-  if (rem == 1) { stockham_pass<2>(s, L, Ns, tw, inv); Ns *= 2; }
-  else if (rem == 2) { stockham_pass<4>(s, L, Ns, tw, inv); Ns *= 4; }
-  while (Ns < L) { stockham_pass<8>(s, L, Ns, tw, inv); Ns *= 8; }
+// a row of L = 2^logL <= 8192 entries from load(e) to store(e, value)
+template <bool INV, typename Load, typename Store>
+__device__ __forceinline__ void fft_row(double2 *s, int L, int logL, const double2 *__restrict__ tw, Load load,
+                                        Store store) {
+  const int rem = logL % 3, R0 = rem == 1 ? 2 : rem == 2 ? 4 : 8;
+  if (L == R0) {
+    if (rem == 1) stockham_pass<2, INV, true, true>(s, L, 1, tw, load, store);
+    else if (rem == 2) stockham_pass<4, INV, true, true>(s, L, 1, tw, load, store);
+    else stockham_pass<8, INV, true, true>(s, L, 1, tw, load, store);
+    return;
+  }
+  if (rem == 1) stockham_pass<2, INV, true, false>(s, L, 1, tw, load, store);
+  else if (rem == 2) stockham_pass<4, INV, true, false>(s, L, 1, tw, load, store);
+  else stockham_pass<8, INV, true, false>(s, L, 1, tw, load, store);
+  int Ns = R0;
+  for (; Ns * 8 < L; Ns *= 8) {
+    stockham_pass<8, INV, false, false>(s, L, Ns, tw, load, store);
+    tw += 7 * Ns;
+  }
+  stockham_pass<8, INV, false, true>(s, L, Ns, tw, load, store);
 }
 
-// Level-1 forward row transforms with the packing fused: row y < b holds
-// z(x) = (f - mean f) + i (g - mu) over the ROI, zero beyond; rows >= b are
-// zero (their transform too).
+// Level 1 packs its two real inputs into one complex row,
+// z(x) = (f - mean f) + i (g - mu) over the ROI and zero beyond; rows y < b only.
 template <typename P>
-__global__ void __launch_bounds__(512) k_fft_pack_rows(const P *__restrict__ f, const P *__restrict__ g, int W, int H,
-                                int x1, int y1, int a, int b, const typename MgT<P>::S *__restrict__ sat,
-                                const double *__restrict__ mu_g, double2 *__restrict__ Z, int L,
-                                int logL, const double2 *__restrict__ tw) {
+__global__ void __launch_bounds__(1024)
+    k_fft_pack_rows(const P *__restrict__ f, const P *__restrict__ g, int W, int H, int x1, int y1, int a, int b,
+                    const typename MgT<P>::S *__restrict__ sat, const double *__restrict__ mu_g,
+                    double2 *__restrict__ Z, int L, int logL, const double2 *__restrict__ tw) {
   extern __shared__ double2 s[];
   const int y = blockIdx.x;
   double2 *row = Z + (long long)y * L;
-  if (y >= b) {
-    for (int x = threadIdx.x; x < L; x += blockDim.x) row[x] = make_double2(0.0, 0.0);
-    return;
-  }
-  const long long W1 = W + 1;
+  const long long W1 = W + 1, o = (long long)(y1 - 1 + y) * W + (x1 - 1);
   const double st = (double)rect_sum(sat, (int)W1, x1 - 1, x1 - 1 + a, y1 - 1, y1 - 1 + b);
   const double mean_t = st / ((double)a * (double)b);
   const double mu = *mu_g;
-  for (int x = threadIdx.x; x < L; x += blockDim.x) {
-    double2 z = make_double2(0.0, 0.0);
-    if (x < a) {
-      const long long o = (long long)(y1 - 1 + y) * W + (x1 - 1 + x);
-      z = make_double2((double)f[o] - mean_t, (double)g[o] - mu);
-    }
-    s[x] = z;
-  }
-  __syncthreads();
-  fft_smem(s, L, logL, tw, false);
-  for (int x = threadIdx.x; x < L; x += blockDim.x) row[x] = s[x];
+  fft_row<false>(
+      s, L, logL, tw,
+      [&](int x) { return x < a ? make_double2((double)f[o + x] - mean_t, (double)g[o + x] - mu) : make_double2(0.0, 0.0); },
+      [&](int x, double2 v) { row[x] = v; });
 }
 
-template <bool INV>
-__global__ void __launch_bounds__(512) k_fft_rows(double2 *__restrict__ Z, int L, int logL,
-                                                  const double2 *__restrict__ tw, int row0, int row1) {
+// columns [kx][ky], in place; entries from `len` on are zeros that nobody wrote
+__global__ void __launch_bounds__(1024)
+    k_fft_cols(double2 *__restrict__ Z, int L, int logL, const double2 *__restrict__ tw, int len) {
   extern __shared__ double2 s[];
-  const int y = blockIdx.x;
-  if (y >= row0 && y < row1) return;  // rows nobody reads
-  double2 *row = Z + (long long)y * L;
-  for (int x = threadIdx.x; x < L; x += blockDim.x) s[x] = row[x];
-  __syncthreads();
-  fft_smem(s, L, logL, tw, INV);
-  for (int x = threadIdx.x; x < L; x += blockDim.x) row[x] = s[x];
+  double2 *row = Z + (long long)blockIdx.x * L;
+  fft_row<false>(s, L, logL, tw, [&](int y) { return y < len ? row[y] : make_double2(0.0, 0.0); },
+                 [&](int y, double2 v) { row[y] = v; });
 }
 
-// out (C x R) = in (R x C)^T
-__global__ void k_transpose_c(const double2 *__restrict__ in, double2 *__restrict__ out, int R,
-                              int Cn) {
+// The correlation's spectrum and its inverse along y: with Z = F + i G (F, G
+// transforms of the two real inputs), F(k) = (Z(k) + conj Z(-k)) / 2, G(k) =
+// (Z(k) - conj Z(-k)) / 2i, and sum_p t(p) d(p + s) has the transform conj(F) G.
+// The correlation is real, so kx beyond P1 / 2 is the conjugate of P1 - kx and not
+// formed.  Z is [kx][ky], C [kx][oy].
+__global__ void __launch_bounds__(1024)
+    k_fft_spectrum(const double2 *__restrict__ Z, double2 *__restrict__ C, int P1, int L, int logL,
+                   const double2 *__restrict__ tw) {
+  extern __shared__ double2 s[];
+  const int kx = blockIdx.x;
+  const double2 *zk = Z + (long long)kx * L, *zm = Z + (long long)((P1 - kx) & (P1 - 1)) * L;
+  double2 *row = C + (long long)kx * L;
+  fft_row<true>(
+      s, L, logL, tw,
+      [&](int ky) {
+        const double2 z = zk[ky], w = zm[(L - ky) & (L - 1)];
+        const double2 F = make_double2(0.5 * (z.x + w.x), 0.5 * (z.y - w.y));
+        const double2 Gm = make_double2(z.x - w.x, z.y + w.y);  // Z(k) - conj Z(-k)
+        const double2 G = make_double2(0.5 * Gm.y, -0.5 * Gm.x);
+        return make_double2(F.x * G.x + F.y * G.y, F.x * G.y - F.y * G.x);
+      },
+      [&](int y, double2 v) { row[y] = v; });
+}
+
+// out (C x R, rows ldo apart) = in (R x C, rows ldi apart)^T
+__global__ void k_transpose_c(const double2 *__restrict__ in, double2 *__restrict__ out, int R, int Cn, int ldi,
+                              int ldo) {
   __shared__ double2 t[32][33];
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const int r = r0 + k, c = c0 + threadIdx.x;
-    if (r < R && c < Cn) t[k][threadIdx.x] = in[(long long)r * Cn + c];
+    if (r < R && c < Cn) t[k][threadIdx.x] = in[(long long)r * ldi + c];
   }
   __syncthreads();
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const int c = c0 + k, r = r0 + threadIdx.x;
-    if (r < R && c < Cn) out[(long long)c * R + r] = t[threadIdx.x][k];
-  }
-}
-
-// Spectrum of the correlation: with Z = F + i G (F, G transforms of the two
-// real inputs), F(k) = (Z(k) + conj Z(-k)) / 2, G(k) = (Z(k) - conj Z(-k)) / 2i,
-// and sum_p t(p) d(p + s) has the transform conj(F) G.  Z is [kx][ky].
-__global__ void k_mg_spectrum(const double2 *__restrict__ Z, double2 *__restrict__ Cs, int P1,
-                              int P2) {
-  const long long n = (long long)P1 * P2;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int kx = (int)(e / P2), ky = (int)(e - (long long)kx * P2);
-    const long long m = (long long)((P1 - kx) & (P1 - 1)) * P2 + ((P2 - ky) & (P2 - 1));
-    const double2 z = Z[e], w = Z[m];
-    const double2 F = make_double2(0.5 * (z.x + w.x), 0.5 * (z.y - w.y));
-    const double2 Gm = make_double2(z.x - w.x, z.y + w.y);  // Z(k) - conj Z(-k)
-    const double2 G = make_double2(0.5 * Gm.y, -0.5 * Gm.x);
-    Cs[e] = make_double2(F.x * G.x + F.y * G.y, F.x * G.y - F.y * G.x);
+    if (r < R && c < Cn) out[(long long)c * ldo + r] = t[threadIdx.x][k];
   }
 }
 
 // Level-1 normalised cross-correlation at map entry e of the (2a-1) x (2b-1)
 // map (column-major, rows = x shifts): D offset (ox, oy) of the template.
-template <bool INT, typename S>
+template <typename S>
 struct L1Args {
-  const S *sat;          // g, g^2 planes used
+  const S *sat;          // the four tables
+  long long plane;       // one table's entries
   int W1, gx0, gy0;      // table row length, 0-based ROI origin
   int a, b;
   long long mn;
-  S st, st2;             // template sums
-  const double2 *c;      // [oy][ox] cyclic correlation, unscaled
-  int P1, P2;
+  double *c;             // correlation, unscaled: row oy + b - 1, column ox mod P1
+  int P1;
   double inv;            // 1 / (P1 P2)
-  double mu;
+  const double *mu;
+  bool narrow;           // mn sum(g^2) < 2^63
 };
 
-template <bool INT, typename S>
-__device__ double l1_ncc(const L1Args<INT, S> &A, const S *satg, const S *satg2, long long e) {
-  const int nr = 2 * A.a - 1;
-  const int i = (int)(e % nr), j = (int)(e / nr);
-  const int ox = i - (A.a - 1), oy = j - (A.b - 1);
-  const int x0 = max(0, ox), x1 = min(A.a, A.a + ox), y0 = max(0, oy), y1 = min(A.b, A.b + oy);
-  if (x1 <= x0 || y1 <= y0) return 0.0;
-  const long long n_in = (long long)(x1 - x0) * (y1 - y0), n_pad = A.mn - n_in;
-  const S sd = rect_sum(satg, A.W1, A.gx0 + x0, A.gx0 + x1, A.gy0 + y0, A.gy0 + y1);
-  const S sd2 = rect_sum(satg2, A.W1, A.gx0 + x0, A.gx0 + x1, A.gy0 + y0, A.gy0 + y1);
-  const double cv = A.c[(long long)(oy & (A.P2 - 1)) * A.P1 + (ox & (A.P1 - 1))].x * A.inv;
-  const double num = (double)A.mn * cv;
-  double denT, C0, Cc = 0.0;
-  if constexpr (INT) {
-    typedef __int128 Wd;
-    denT = (double)((Wd)A.mn * (long long)A.st2 - (Wd)(long long)A.st * (long long)A.st);
-    C0 = (double)((Wd)A.mn * (long long)sd2 - (Wd)(long long)sd * (long long)sd);
-    if (n_pad > 0)
-      Cc = A.mu * ((double)((Wd)n_pad * (A.mn - n_pad)) * A.mu - 2.0 * (double)((Wd)(long long)sd * n_pad));
+// what every entry shares
+template <typename S>
+struct L1Consts {
+  S st, st2;
+  double denT, mu;
+};
+template <typename S>
+__device__ __forceinline__ L1Consts<S> l1_consts(const L1Args<S> &A) {
+  L1Consts<S> K;
+  K.st = rect_sum(A.sat, A.W1, A.gx0, A.gx0 + A.a, A.gy0, A.gy0 + A.b);
+  K.st2 = rect_sum(A.sat + A.plane, A.W1, A.gx0, A.gx0 + A.a, A.gy0, A.gy0 + A.b);
+  if constexpr (std::is_integral<S>::value)
+    K.denT = (double)((__int128)A.mn * K.st2 - (__int128)K.st * K.st);
+  else
+    K.denT = (double)A.mn * K.st2 - K.st * K.st;
+  K.mu = *A.mu;
+  return K;
+}
+// window part of the denominator; n_in entries of the window lie in the region
+template <typename S>
+__device__ __forceinline__ double l1_den(const L1Args<S> &A, double mu, S sd, S sd2, long long n_in) {
+  const long long n_pad = A.mn - n_in;
+  double C0, Cc = 0.0;
+  if constexpr (std::is_integral<S>::value) {
+    C0 = A.narrow ? (double)(A.mn * sd2 - sd * sd) : (double)((__int128)A.mn * sd2 - (__int128)sd * sd);
+    if (n_pad > 0) Cc = mu * ((double)((__int128)n_pad * n_in) * mu - 2.0 * (double)((__int128)sd * n_pad));
   } else {
-    denT = (double)A.mn * (double)A.st2 - (double)A.st * (double)A.st;
-    C0 = (double)A.mn * (double)sd2 - (double)sd * (double)sd;
-    if (n_pad > 0)
-      Cc = A.mu * ((double)n_pad * (double)(A.mn - n_pad) * A.mu - 2.0 * ((double)sd * (double)n_pad));
+    C0 = (double)A.mn * sd2 - sd * sd;
+    if (n_pad > 0) Cc = mu * ((double)n_pad * (double)n_in * mu - 2.0 * (sd * (double)n_pad));
   }
-  const double den = C0 + Cc;
+  return C0 + Cc;
+}
+__device__ __forceinline__ double l1_r(double num, double denT, double den) {
   if (!(den > 0.0)) return 0.0;
   double r = num / sqrt(denT * den);
   if (fabs(r) - 1.0 > kSqrtEps) r = 0.0;
   return r;
+}
+
+// NCC at shift (ox, oy) from the stored correlation
+template <typename S>
+__device__ double l1_ncc(const L1Args<S> &A, const L1Consts<S> &K, int ox, int oy) {
+  const int x0 = max(0, ox), x1 = min(A.a, A.a + ox), y0 = max(0, oy), y1 = min(A.b, A.b + oy);
+  if (x1 <= x0 || y1 <= y0) return 0.0;
+  const S *satg = A.sat + 2 * A.plane;
+  const S sd = rect_sum(satg, A.W1, A.gx0 + x0, A.gx0 + x1, A.gy0 + y0, A.gy0 + y1);
+  const S sd2 = rect_sum(satg + A.plane, A.W1, A.gx0 + x0, A.gx0 + x1, A.gy0 + y0, A.gy0 + y1);
+  const double cv = A.c[(long long)(oy + A.b - 1) * A.P1 + (ox & (A.P1 - 1))] * A.inv;
+  return l1_r((double)A.mn * cv, K.denT, l1_den(A, K.mu, sd, sd2, (long long)(x1 - x0) * (y1 - y0)));
 }
 
 __device__ __forceinline__ void argmax_merge(double &bv, long long &bi, double v, long long i) {
@@ -419,55 +499,108 @@ __device__ __forceinline__ void argmax_merge(double &bv, long long &bi, double v
     bi = i;
   }
 }
-
-template <bool INT, typename S>
-__global__ void k_mg_l1_argmax(L1Args<INT, S> A, const S *__restrict__ satg,
-                               const S *__restrict__ satg2, double *__restrict__ pv,
-                               long long *__restrict__ pi) {
-  const long long nm = (long long)(2 * A.a - 1) * (2 * A.b - 1);
-  double bv = -1e300;
-  long long bi = 0x7fffffffffffffffll;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nm;
-       e += (long long)gridDim.x * blockDim.x)
-    argmax_merge(bv, bi, l1_ncc(A, satg, satg2, e), e);
+__device__ __forceinline__ void argmax_warp(double &bv, long long &bi) {
+#pragma unroll
   for (int o = 16; o > 0; o >>= 1)
     argmax_merge(bv, bi, __shfl_xor_sync(0xffffffffu, bv, o), __shfl_xor_sync(0xffffffffu, bi, o));
+}
+
+// The last inverse transform, along x, two rows oy at once (the correlation is
+// real: row oy in the real part, oy + 1 in the imaginary part), and the maximum
+// over the two rows' map entries.  The window sums of a row need two table rows,
+// and one varying column of them; the root and the division are formed only
+// where num^2 reaches the thread's best entry so far.  C is [oy mod P2][kx] with
+// rows ldc apart.
+template <typename S>
+__global__ void __launch_bounds__(1024)
+    k_fft_ncc(const double2 *__restrict__ C, int ldc, int P2, const __grid_constant__ L1Args<S> A, int logL,
+              const double2 *__restrict__ tw, double *__restrict__ pv, long long *__restrict__ pi) {
+  extern __shared__ double2 s[];
   __shared__ double sv[32];
   __shared__ long long si[32];
+  const int L = A.P1, rows = 2 * A.b - 1;
+  const int r0 = 2 * blockIdx.x, two = r0 + 1 < rows;
+  const double2 *ca = C + (long long)((r0 - (A.b - 1)) & (P2 - 1)) * ldc;
+  const double2 *cb = C + (long long)((r0 + 1 - (A.b - 1)) & (P2 - 1)) * ldc;
+  fft_row<true>(
+      s, L, logL, tw,
+      [&](int kx) {
+        const bool up = kx <= L / 2;
+        const int k = up ? kx : L - kx;
+        const double2 u = ca[k], v = two ? cb[k] : make_double2(0.0, 0.0);
+        return up ? make_double2(u.x - v.y, u.y + v.x) : make_double2(u.x + v.y, v.x - u.y);
+      },
+      [&](int x, double2 v) { s[fft_pos(x)] = v; });
+  __syncthreads();
+  const L1Consts<S> K = l1_consts(A);
+  double bv = -1e300;
+  long long bi = 0x7fffffffffffffffll;
+  for (int h = 0; h <= two; ++h) {
+    const int r = r0 + h, oy = r - (A.b - 1), y0 = max(0, oy), y1 = min(A.b, A.b + oy);
+    const S *g0 = A.sat + 2 * A.plane + (long long)(A.gy0 + y0) * A.W1 + A.gx0;
+    const S *g1 = g0 + (long long)(y1 - y0) * A.W1;
+    const S *q0 = g0 + A.plane, *q1 = g1 + A.plane;
+    const S ga = g1[A.a] - g0[A.a], gz = g1[0] - g0[0], qa = q1[A.a] - q0[A.a], qz = q1[0] - q0[0];
+    double *crow = A.c + (long long)r * L;
+    for (int x = threadIdx.x; x < L; x += blockDim.x) {
+      const double2 cc = s[fft_pos(x)];
+      const double c = h ? cc.y : cc.x;
+      crow[x] = c;
+      const int ox = x < A.a ? x : x - L;
+      if (ox <= -A.a) continue;  // no entry of the map
+      const int e = ox >= 0 ? ox : A.a + ox;  // the window's inner edge
+      const S ge = g1[e] - g0[e], qe = q1[e] - q0[e];
+      const S sd = ox >= 0 ? ga - ge : ge - gz, sd2 = ox >= 0 ? qa - qe : qe - qz;
+      const double den = l1_den(A, K.mu, sd, sd2, (long long)(A.a - abs(ox)) * (y1 - y0));
+      const double num = (double)A.mn * (c * A.inv);
+      if (bv > 0.0 && (!(num > 0.0) || num * num < bv * bv * (1.0 - 1e-12) * (K.denT * den))) continue;
+      argmax_merge(bv, bi, l1_r(num, K.denT, den), (long long)r * (2 * A.a - 1) + (ox + A.a - 1));
+    }
+  }
+  argmax_warp(bv, bi);
   if ((threadIdx.x & 31) == 0) {
     sv[threadIdx.x >> 5] = bv;
     si[threadIdx.x >> 5] = bi;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) argmax_merge(bv, bi, sv[k], si[k]);
-    pv[blockIdx.x] = bv;
-    pi[blockIdx.x] = bi;
+  if (threadIdx.x < 32) {
+    const bool in = threadIdx.x < blockDim.x / 32;
+    bv = in ? sv[threadIdx.x] : -1e300;
+    bi = in ? si[threadIdx.x] : 0x7fffffffffffffffll;
+    argmax_warp(bv, bi);
+    if (threadIdx.x == 0) {
+      pv[blockIdx.x] = bv;
+      pi[blockIdx.x] = bi;
+    }
   }
 }
 
-// out = {row, col, max_f} of findpeak over the level-1 map
-template <bool INT, typename S>
-__global__ void k_mg_l1_peak(L1Args<INT, S> A, const S *__restrict__ satg,
-                             const S *__restrict__ satg2, const double *__restrict__ pv,
+// out = {row, col, max_f} of findpeak over the level-1 map, {constant template}; one warp
+template <typename S>
+__global__ void k_mg_l1_peak(const __grid_constant__ L1Args<S> A, const double *__restrict__ pv,
                              const long long *__restrict__ pi, int np, double *__restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  const int lane = threadIdx.x;
   double bv = -1e300;
   long long bi = 0x7fffffffffffffffll;
-  for (int k = 0; k < np; ++k) argmax_merge(bv, bi, pv[k], pi[k]);
+  for (int k = lane; k < np; k += 32) argmax_merge(bv, bi, pv[k], pi[k]);
+  argmax_warp(bv, bi);
+  const L1Consts<S> K = l1_consts(A);
   const int nr = 2 * A.a - 1, nc = 2 * A.b - 1;
   const int r = (int)(bi % nr), c = (int)(bi / nr);
   double rp = r + 1, cp = c + 1, mf = bv;
   if (!(r == 0 || r == nr - 1 || c == 0 || c == nc - 1)) {
+    const double mine = lane < 9 ? l1_ncc(A, K, r + lane % 3 - 1 - (A.a - 1), c + lane / 3 - 1 - (A.b - 1)) : 0.0;
     double u9[9];
-    for (int dc = -1; dc <= 1; ++dc)
-      for (int dr = -1; dr <= 1; ++dr)
-        u9[(dc + 1) * 3 + dr + 1] = l1_ncc(A, satg, satg2, (long long)(c + dc) * nr + (r + dr));
+#pragma unroll
+    for (int q = 0; q < 9; ++q) u9[q] = __shfl_sync(0xffffffffu, mine, q);
     findpeak_fit9(u9, r, c, &rp, &cp, &mf);
   }
-  out[0] = rp;
-  out[1] = cp;
-  out[2] = mf;
+  if (lane == 0) {
+    out[0] = rp;
+    out[1] = cp;
+    out[2] = mf;
+    out[3] = K.denT > 0.0 ? 0.0 : 1.0;
+  }
 }
 
 // ------------------------------------------------------------ intermediate levels
@@ -481,6 +614,140 @@ template <typename P> struct CropCfg {
   static constexpr int SW = sizeof(typename MgT<P>::V) == 8 ? 8 : 16;
   static constexpr int TILE = kSegs * SW;
 };
+
+// Four pixels of a row as the words of its byte planes (16 bit: high, low), zeros
+// outside columns [lo, hi); row points at column 0.  A word that lies inside is
+// read as aligned words (the images have spare bytes behind them).
+template <typename P>
+__device__ __forceinline__ void four_pixels(const P *row, int x, int lo, int hi, uint32_t w[sizeof(P)]) {
+  if (x >= lo && x + 4 <= hi) {
+    const uintptr_t at = (uintptr_t)(row + x);
+    const uint32_t *q = (const uint32_t *)(at & ~(uintptr_t)3);
+    const uint32_t sh = 8 * (uint32_t)(at & 3);
+    if constexpr (sizeof(P) == 1) {
+      w[0] = __funnelshift_r(q[0], q[1], sh);
+    } else {
+      const uint32_t v0 = __funnelshift_r(q[0], q[1], sh), v1 = __funnelshift_r(q[1], q[2], sh);
+      w[0] = __byte_perm(v0, v1, 0x7531);
+      w[1] = __byte_perm(v0, v1, 0x6420);
+    }
+    return;
+  }
+#pragma unroll
+  for (int p = 0; p < (int)sizeof(P); ++p) w[p] = 0;
+  for (int e = 0; e < 4; ++e)
+    if (x + e >= lo && x + e < hi) {
+      const uint32_t v = row[x + e];
+#pragma unroll
+      for (int p = 0; p < (int)sizeof(P); ++p) w[p] |= ((v >> (8 * (sizeof(P) - 1 - p))) & 255u) << (8 * e);
+    }
+}
+
+// The sums of products of byte planes: one (8 bit) or high x high, the mixed two,
+// low x low (16 bit), each exact in 32 bits.
+template <int PL>
+struct PlaneSums {
+  uint32_t s[PL == 1 ? 1 : 3];
+  __device__ __forceinline__ void add(const uint32_t t[PL], const uint32_t d[PL]) {
+    if constexpr (PL == 1) {
+      s[0] = __dp4a(t[0], d[0], s[0]);
+    } else {
+      s[0] = __dp4a(t[0], d[0], s[0]);
+      s[1] = __dp4a(t[0], d[1], s[1]);
+      s[1] = __dp4a(t[1], d[0], s[1]);
+      s[2] = __dp4a(t[1], d[1], s[2]);
+    }
+  }
+  __device__ __forceinline__ unsigned long long total() const {
+    if constexpr (PL == 1) return s[0];
+    return ((unsigned long long)s[0] << 16) + ((unsigned long long)s[1] << 8) + s[PL == 1 ? 0 : 2];
+  }
+};
+
+// The crop's sums of 8- and 16-bit images, four products an instruction: bands
+// of 32 rows and 256 columns in shared memory as packed words, a thread one y
+// shift and 16 columns, its region words shifted to the four byte offsets in
+// registers for all 13 x shifts.  In a region narrower than the tile the spare
+// threads take every second, fourth ... row.  All levels of a 2048 x 2048 search
+// (3.8 G products): 171 us, 815 us with one product an instruction and
+// 16-way bank conflicts.
+constexpr int kBandI = 32, kTileI = 256;
+template <typename P>
+__global__ void __launch_bounds__(224) k_mg_crop_int(const P *__restrict__ f, const P *__restrict__ g, int W,
+                                                     const MgReg *__restrict__ regs,
+                                                     unsigned long long *__restrict__ acc) {
+  constexpr int PL = sizeof(P), TW = kTileI / 4, DW = TW + 4, DR = kBandI + kCropC - 1;
+  __shared__ __align__(16) uint32_t Ts[PL][kBandI][TW], Ds[PL][DR][DW];
+  const MgReg R = regs[blockIdx.x];
+  if (!R.valid) return;
+  const int q0 = blockIdx.y * kBandI, x0 = blockIdx.z * kTileI;
+  if (q0 >= R.b || x0 >= R.a) return;
+  const int nq = min(kBandI, R.b - q0), nx = min(kTileI, R.a - x0);
+  const int dwid = R.a + 10, dhgt = R.b + 10;
+  const int words = (nx + 15) / 16 * 4;  // of a template row, whole segments
+  for (int e = threadIdx.x; e < nq * words; e += blockDim.x) {
+    const int qq = e / words, m = e - qq * words;
+    uint32_t w[PL];
+    four_pixels(f + (long long)(R.ty - 1 + q0 + qq) * W + (R.tx - 1 + x0), 4 * m, 0, nx, w);
+#pragma unroll
+    for (int p = 0; p < PL; ++p) Ts[p][qq][m] = w[p];
+  }
+  const int dwords = words + 4, drows = nq + kCropC - 1;
+  for (int e = threadIdx.x; e < drows * dwords; e += blockDim.x) {
+    const int r = e / dwords, m = e - r * dwords, yl = q0 - 1 + r;  // region row
+    uint32_t w[PL] = {};
+    if (yl >= 0 && yl < dhgt) {
+      // column c of the tile is the region's x0 - 1 + c
+      const P *row = g + (long long)(R.dy - 1 + yl) * W + (R.dx - 1);
+      four_pixels(row, x0 - 1 + 4 * m, 0, dwid, w);
+    }
+#pragma unroll
+    for (int p = 0; p < PL; ++p) Ds[p][r][m] = w[p];
+  }
+  __syncthreads();
+  const int oyi = threadIdx.x / kSegs, lane16 = threadIdx.x % kSegs;  // oy = oyi - 1
+  int ns = 1;  // segments, a power of two
+  while (ns < words / 4) ns <<= 1;
+  const int seg = lane16 & (ns - 1), every = kSegs / ns;
+  PlaneSums<PL> s[kCropR] = {};
+  if (4 * seg < words) {
+    for (int qq = lane16 / ns; qq < nq; qq += every) {
+      uint32_t t[PL][4], d[PL][8];
+#pragma unroll
+      for (int p = 0; p < PL; ++p) {
+        *(uint4 *)t[p] = *(const uint4 *)&Ts[p][qq][4 * seg];
+        *(uint4 *)d[p] = *(const uint4 *)&Ds[p][qq + oyi][4 * seg];
+        *(uint4 *)(d[p] + 4) = *(const uint4 *)&Ds[p][qq + oyi][4 * seg + 4];
+      }
+#pragma unroll
+      for (int sh = 0; sh < 4; ++sh) {
+        uint32_t v[7][PL];
+#pragma unroll
+        for (int j = 0; j < 7; ++j)
+#pragma unroll
+          for (int p = 0; p < PL; ++p) v[j][p] = sh ? __funnelshift_r(d[p][j], d[p][j + 1], 8 * sh) : d[p][j];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t ti[PL];
+#pragma unroll
+          for (int p = 0; p < PL; ++p) ti[p] = t[p][i];
+#pragma unroll
+          for (int m = 0; m < 4; ++m)
+            if (4 * m + sh < kCropR) s[4 * m + sh].add(ti, v[i + m]);
+        }
+      }
+    }
+  }
+  // the 16 threads of a y shift: at most 32 x 256 products of 2^16, twice
+  const unsigned half = 0xffffu << (threadIdx.x & 16);
+#pragma unroll
+  for (int k = 0; k < kCropR; ++k) {
+#pragma unroll
+    for (uint32_t &v : s[k].s) v = __reduce_add_sync(half, v);
+    const unsigned long long v = s[k].total();
+    if (lane16 == 0 && v) atomicAdd(&acc[(long long)blockIdx.x * kCrop + oyi * kCropR + k], v);
+  }
+}
 
 template <typename P>
 __global__ void __launch_bounds__(224) k_mg_crop(const P *__restrict__ f, const P *__restrict__ g,
@@ -547,6 +814,16 @@ __global__ void __launch_bounds__(224) k_mg_crop(const P *__restrict__ f, const 
   }
 }
 
+// first maximum of a crop, by one warp
+__device__ __forceinline__ int crop_max(const double *map) {
+  const int lane = threadIdx.x & 31;
+  double bv = map[lane];
+  long long bi = lane;
+  for (int e = lane + 32; e < kCrop; e += 32) argmax_merge(bv, bi, map[e], e);
+  argmax_warp(bv, bi);
+  return (int)bi;
+}
+
 // NCC of the 182 crop entries from the products and the window sums, then
 // findpeak: res[region] = {u offset, v offset, Phi, ok}.
 template <typename P>
@@ -595,18 +872,13 @@ __global__ void k_mg_crop_peak(const MgReg *__restrict__ regs, int W, int H,
     map[e] = r;
   }
   __syncthreads();
+  if (threadIdx.x >= 32) return;
+  if (s_flat) {
+    if (threadIdx.x == 0) o[3] = 0.0;
+    return;
+  }
+  const int im = crop_max(map);
   if (threadIdx.x == 0) {
-    if (s_flat) {
-      o[3] = 0.0;
-      return;
-    }
-    int im = 0;
-    double mv = map[0];
-    for (int e = 1; e < kCrop; ++e)
-      if (map[e] > mv) {
-        mv = map[e];
-        im = e;
-      }
     double rp, cp, mf;
     findpeak_fit(map, kCropR, kCropC, im, &rp, &cp, &mf);
     o[0] = __dsub_rn(rp, 7.0);
@@ -620,6 +892,14 @@ __global__ void k_mg_crop_peak(const MgReg *__restrict__ regs, int W, int H,
 // One CTA per region: the full normxcorr2 map (2a+9) x (2b+9) in shared
 // memory, compute_qFactor over it, findpeak on its 13 x 14 crop.
 // res[region] = {u offset, v offset, Phi, ok, PCE, 1/entropy}.
+// k_mg_full's operands of integer images as words: of a template row, of a region
+// row, and the zero columns before the region's first (strips start at shifts a
+// multiple of kStrip from -(a - 1), so each starts a word)
+struct FullWords {
+  int tw, dw, pad;
+  __host__ __device__ explicit FullWords(int a) : tw((a + 3) / 4), dw((2 * a + 12) / 4 + 3), pad(a - 1) {}
+};
+
 template <typename P>
 __global__ void __launch_bounds__(256) k_mg_full(const P *__restrict__ f, const P *__restrict__ g,
                                                  int W, int H, const MgReg *__restrict__ regs,
@@ -628,7 +908,8 @@ __global__ void __launch_bounds__(256) k_mg_full(const P *__restrict__ f, const 
                                                  double *__restrict__ res) {
   using S = typename MgT<P>::S;
   using V = typename MgT<P>::V;
-  using A = typename MgT<P>::A;  // u8: <= 80 * 80 * 255^2 < 2^32
+  using A = typename MgT<P>::A;
+  constexpr int PL = MgT<P>::integer ? sizeof(P) : 1;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[64];
   __shared__ int hist[30];
@@ -641,19 +922,40 @@ __global__ void __launch_bounds__(256) k_mg_full(const P *__restrict__ f, const 
   }
   const int a = R.a, b = R.b, dw = a + 10, dh = b + 10;
   const int fr = a + dw - 1, fc = b + dh - 1, nm = fr * fc;
-  // template rows padded with 8 zero columns, region rows with kStrip zero
-  // columns on the left and kStrip + 8 on the right
-  const int TP = a + 8, DP = dw + 2 * kStrip + 8;
   double *map = (double *)smem;
+  // floats: template rows padded with 8 zero columns, region rows with kStrip zero
+  // columns on the left and kStrip + 8 on the right.  Integers: words of a byte
+  // plane, template rows from column 0, region rows so that every strip's first
+  // shift starts a word; zeros around
+  const int TP = a + 8, DP = dw + 2 * kStrip + 8;
   V *Ts = (V *)(map + nm);
   V *Ds = Ts + TP * b;
-  for (int e = threadIdx.x; e < TP * b; e += blockDim.x) {
-    const int ty = e / TP, tx = e - ty * TP;
-    Ts[e] = tx < a ? (V)f[(long long)(R.ty - 1 + ty) * W + (R.tx - 1 + tx)] : (V)0;
-  }
-  for (int e = threadIdx.x; e < dh * DP; e += blockDim.x) {
-    const int yy = e / DP, xx = e - yy * DP - kStrip;
-    Ds[e] = (xx >= 0 && xx < dw) ? (V)g[(long long)(R.dy - 1 + yy) * W + (R.dx - 1 + xx)] : (V)0;
+  const FullWords FW(a);
+  uint32_t *const Tw = (uint32_t *)(map + nm), *const Dw = Tw + PL * b * FW.tw;
+  if constexpr (MgT<P>::integer) {
+    for (int e = threadIdx.x; e < b * FW.tw; e += blockDim.x) {
+      const int ty = e / FW.tw, m = e - ty * FW.tw;
+      uint32_t w[PL];
+      four_pixels(f + (long long)(R.ty - 1 + ty) * W + (R.tx - 1), 4 * m, 0, a, w);
+#pragma unroll
+      for (int p = 0; p < PL; ++p) Tw[p * b * FW.tw + e] = w[p];
+    }
+    for (int e = threadIdx.x; e < dh * FW.dw; e += blockDim.x) {
+      const int yy = e / FW.dw, m = e - yy * FW.dw;
+      uint32_t w[PL];
+      four_pixels(g + (long long)(R.dy - 1 + yy) * W + (R.dx - 1), 4 * m - FW.pad, 0, dw, w);
+#pragma unroll
+      for (int p = 0; p < PL; ++p) Dw[p * dh * FW.dw + e] = w[p];
+    }
+  } else {
+    for (int e = threadIdx.x; e < TP * b; e += blockDim.x) {
+      const int ty = e / TP, tx = e - ty * TP;
+      Ts[e] = tx < a ? (V)f[(long long)(R.ty - 1 + ty) * W + (R.tx - 1 + tx)] : (V)0;
+    }
+    for (int e = threadIdx.x; e < dh * DP; e += blockDim.x) {
+      const int yy = e / DP, xx = e - yy * DP - kStrip;
+      Ds[e] = (xx >= 0 && xx < dw) ? (V)g[(long long)(R.dy - 1 + yy) * W + (R.dx - 1 + xx)] : (V)0;
+    }
   }
   if (threadIdx.x < 30) hist[threadIdx.x] = 0;
   const int W1 = W + 1;
@@ -674,48 +976,115 @@ __global__ void __launch_bounds__(256) k_mg_full(const P *__restrict__ f, const 
   }
   const double mu = *mu_g;
   __syncthreads();
-  // strips of kStrip consecutive x shifts (map rows) at one y shift; the
-  // template columns run in chunks of 8 over zero-padded rows, so the 8 x 8
-  // products of a chunk are fully unrolled in registers
-  const int nsr = (fr + kStrip - 1) / kStrip, nstrips = nsr * fc;
-  for (int sI = threadIdx.x; sI < nstrips; sI += blockDim.x) {
-    const int j = sI / nsr, i0 = (sI - j * nsr) * kStrip;
-    const int oy = j - (b - 1), ox0 = i0 - (a - 1);
-    const int ty0 = max(0, -oy), ty1 = min(b, dh - oy);
-    const int txa = max(0, -(ox0 + kStrip - 1)), txb = min(a, dw - ox0);
-    A s[kStrip];
+  // NCC of map entry (i, j) from its sum of products
+  auto entry = [&](int i, int j, S stdv) {
+    const int ox = i - (a - 1), oy = j - (b - 1);
+    const int tx0 = max(0, -ox), tx1 = min(a, dw - ox), ty0 = max(0, -oy), ty1 = min(b, dh - oy);
+    if (tx1 <= tx0 || ty1 <= ty0) return 0.0;
+    const long long n_in = (long long)(tx1 - tx0) * (ty1 - ty0);
+    const S st_in = rect_sum(sf, W1, tx0i + tx0, tx0i + tx1, ty0i + ty0, ty0i + ty1);
+    const S sd = rect_sum(sg, W1, dx0i + tx0 + ox, dx0i + tx1 + ox, dy0i + ty0 + oy, dy0i + ty1 + oy);
+    const S sd2 = rect_sum(sg2, W1, dx0i + tx0 + ox, dx0i + tx1 + ox, dy0i + ty0 + oy, dy0i + ty1 + oy);
+    // at most 80 x 80 pixels: 64-bit products hold
+    if constexpr (MgT<P>::integer)
+      return ncc_combine(mn, st, st2, stdv, sd, sd2, st - st_in, mn - n_in, mu);
+    else
+      return combine<S>(mn, st, st2, stdv, sd, sd2, st - st_in, mn - n_in, mu);
+  };
+  // strips of kStrip consecutive x shifts (map rows) at one y shift
+  const int nsr = (fr + kStrip - 1) / kStrip;
+  if constexpr (MgT<P>::integer) {
+    // Four products an instruction (4096 regions of 33 x 33: the kernel 0.60 ms,
+    // 1.64 ms with one): per template word one new region word, three
+    // shifted ones (the other three are the last word's) and eight dp4a.  The
+    // y shifts t and t + b + 10 (t < b - 1) overlap t + 1 and b - 1 - t rows: a
+    // thread takes both, so each has the same b rows, and the 11 full ones alone.
+    unsigned long long *const raw = (unsigned long long *)map;
+    const int nv = b + 10;
+    for (int sI = threadIdx.x; sI < nsr * nv; sI += blockDim.x) {
+      const int i0 = sI / nv * kStrip, v = sI % nv, ox0 = i0 - (a - 1);
+      const bool pair = v < b - 1;
+      const int r1 = pair ? v + 1 : b;  // rows of the first y shift
+      const int wa = max(0, -(ox0 + kStrip - 1)) >> 2, wb = (min(a, dw - ox0) + 3) >> 2;
+      PlaneSums<PL> s[kStrip] = {};
+      int j = v, ty = pair ? b - 1 - v : max(0, (b - 1) - v);
+      const int dcol = (FW.pad + ox0) >> 2;  // the region word of template word 0
+      for (int r = 0; r < b; ++r, ++ty) {
+        if (r == r1) {  // on to the second y shift
 #pragma unroll
-    for (int k = 0; k < kStrip; ++k) s[k] = 0;
-    for (int ty = ty0; ty < ty1; ++ty) {
-      const V *tr = Ts + ty * TP;
-      const V *dr = Ds + (ty + oy) * DP + kStrip + ox0;  // dr[tx + k]: region x = tx + ox0 + k
-      for (int tx = txa; tx < txb; tx += 8) {
-        V tv[8], dv[15];
+          for (int k = 0; k < kStrip; ++k) {
+            if (i0 + k < fr) raw[(long long)j * fr + i0 + k] = s[k].total();
+            s[k] = PlaneSums<PL>{};
+          }
+          j = v + b + 10;
+          ty = 0;
+        }
+        const uint32_t *tr = Tw + ty * FW.tw;
+        const uint32_t *dr = Dw + (ty + j - (b - 1)) * FW.dw + dcol;
+        uint32_t d0[PL], d1[PL], lo[4][PL];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) tv[q] = tr[tx + q];
+        for (int p = 0; p < PL; ++p) {
+          d0[p] = dr[p * dh * FW.dw + wa];
+          d1[p] = dr[p * dh * FW.dw + wa + 1];
+          lo[0][p] = d0[p];
 #pragma unroll
-        for (int q = 0; q < 15; ++q) dv[q] = dr[tx + q];
+          for (int e = 1; e < 4; ++e) lo[e][p] = __funnelshift_r(d0[p], d1[p], 8 * e);
+        }
+        for (int m = wa; m < wb; ++m) {
+          uint32_t t[PL], hi[4][PL];
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
+          for (int p = 0; p < PL; ++p) {
+            t[p] = tr[p * b * FW.tw + m];
+            const uint32_t d2 = dr[p * dh * FW.dw + m + 2];
+            hi[0][p] = d1[p];
 #pragma unroll
-          for (int k = 0; k < kStrip; ++k) s[k] += (A)tv[q] * (A)dv[q + k];
+            for (int e = 1; e < 4; ++e) hi[e][p] = __funnelshift_r(d1[p], d2, 8 * e);
+            d1[p] = d2;
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            s[e].add(t, lo[e]);
+            s[e + 4].add(t, hi[e]);
+#pragma unroll
+            for (int p = 0; p < PL; ++p) lo[e][p] = hi[e][p];
+          }
+        }
       }
+#pragma unroll
+      for (int k = 0; k < kStrip; ++k)
+        if (i0 + k < fr) raw[(long long)j * fr + i0 + k] = s[k].total();
     }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nm; e += blockDim.x) map[e] = entry(e % fr, e / fr, (S)raw[e]);
+  } else {
+    // the template columns run in chunks of 8 over zero-padded rows, so the 8 x 8
+    // products of a chunk are fully unrolled in registers
+    for (int sI = threadIdx.x; sI < nsr * fc; sI += blockDim.x) {
+      const int j = sI / nsr, i0 = (sI - j * nsr) * kStrip;
+      const int oy = j - (b - 1), ox0 = i0 - (a - 1);
+      const int ty0 = max(0, -oy), ty1 = min(b, dh - oy);
+      const int txa = max(0, -(ox0 + kStrip - 1)), txb = min(a, dw - ox0);
+      A s[kStrip];
 #pragma unroll
-    for (int k = 0; k < kStrip; ++k) {
-      const int i = i0 + k;
-      if (i >= fr) break;
-      const int ox = ox0 + k;
-      const int tx0 = max(0, -ox), tx1 = min(a, dw - ox);
-      double r = 0.0;
-      if (tx1 > tx0 && ty1 > ty0) {
-        const long long n_in = (long long)(tx1 - tx0) * (ty1 - ty0);
-        const S st_in = rect_sum(sf, W1, tx0i + tx0, tx0i + tx1, ty0i + ty0, ty0i + ty1);
-        const S sd = rect_sum(sg, W1, dx0i + tx0 + ox, dx0i + tx1 + ox, dy0i + ty0 + oy, dy0i + ty1 + oy);
-        const S sd2 = rect_sum(sg2, W1, dx0i + tx0 + ox, dx0i + tx1 + ox, dy0i + ty0 + oy, dy0i + ty1 + oy);
-        r = combine<S>(mn, st, st2, (S)s[k], sd, sd2, st - st_in, mn - n_in, mu);
+      for (int k = 0; k < kStrip; ++k) s[k] = 0;
+      for (int ty = ty0; ty < ty1; ++ty) {
+        const V *tr = Ts + ty * TP;
+        const V *dr = Ds + (ty + oy) * DP + kStrip + ox0;  // dr[tx + k]: region x = tx + ox0 + k
+        for (int tx = txa; tx < txb; tx += 8) {
+          V tv[8], dv[15];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) tv[q] = tr[tx + q];
+#pragma unroll
+          for (int q = 0; q < 15; ++q) dv[q] = dr[tx + q];
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+#pragma unroll
+            for (int k = 0; k < kStrip; ++k) s[k] += (A)tv[q] * (A)dv[q + k];
+        }
       }
-      map[(long long)j * fr + i] = r;
+#pragma unroll
+      for (int k = 0; k < kStrip; ++k)
+        if (i0 + k < fr) map[(long long)j * fr + i0 + k] = entry(i0 + k, j, (S)s[k]);
     }
   }
   __syncthreads();
@@ -771,28 +1140,27 @@ __global__ void __launch_bounds__(256) k_mg_full(const P *__restrict__ f, const 
     crop[e] = map[(long long)(b - 2 + c) * fr + (a - 2 + r)];
   }
   __syncthreads();
-  if (tid == 0) {
+  if (tid < 32) {
     const double n = (double)nm;
-    o[4] = (peak * peak) / (sumsq / n);
-    double ent = 0;
-    for (int k = 0; k < 30; ++k) {
-      const double p = hist[k] / n;
-      if (p > 0) ent += p * log(1.0 / p);
+    // the entropy's terms a lane each, added in their order
+    double term = 0.0;
+    if (tid < 30) {
+      const double p = hist[tid] / n;
+      if (p > 0) term = p * log(1.0 / p);
     }
-    o[5] = 1.0 / ent;
-    int im = 0;
-    double mv = crop[0];
-    for (int e = 1; e < kCrop; ++e)
-      if (crop[e] > mv) {
-        mv = crop[e];
-        im = e;
-      }
-    double rp, cp, mf;
-    findpeak_fit(crop, kCropR, kCropC, im, &rp, &cp, &mf);
-    o[0] = __dsub_rn(rp, 7.0);
-    o[1] = __dsub_rn(cp, 7.0);
-    o[2] = mf;
-    o[3] = 1.0;
+    double ent = 0;
+    for (int k = 0; k < 30; ++k) ent += __shfl_sync(0xffffffffu, term, k);
+    const int im = crop_max(crop);
+    if (tid == 0) {
+      o[4] = (peak * peak) / (sumsq / n);
+      o[5] = 1.0 / ent;
+      double rp, cp, mf;
+      findpeak_fit(crop, kCropR, kCropC, im, &rp, &cp, &mf);
+      o[0] = __dsub_rn(rp, 7.0);
+      o[1] = __dsub_rn(cp, 7.0);
+      o[2] = mf;
+      o[3] = 1.0;
+    }
   }
 }
 
@@ -900,11 +1268,12 @@ int run_levels(MgWork &w, const P *f, const P *g, int W, int H, const double *mu
   // summed-area tables
   const int nch = (H + kSatChunk - 1) / kSatChunk;
   if ((rc = w.sat.ensure(sizeof(S) * 4 * plane))) return rc;
-  if ((rc = w.tot.ensure(sizeof(S) * 4 * (size_t)nch * W1))) return rc;
+  if ((rc = w.tot.ensure(sizeof(S) * 4 * (size_t)nch * W))) return rc;
   S *sat = w.sat.as<S>();
-  k_sat_rows<P><<<dim3(H, 4), 256, 0, st>>>(f, g, W, H, sat);
-  k_sat_cols_chunk<S><<<dim3((unsigned)((W1 + 127) / 128), nch, 4), 128, 0, st>>>(sat, W, H, w.tot.as<S>());
-  k_sat_cols_fix<S><<<dim3((unsigned)((W1 + 127) / 128), nch, 4), 128, 0, st>>>(sat, W, H, w.tot.as<S>());
+  const unsigned cols = (unsigned)((W + 127) / 128);
+  k_sat_chunks<P><<<dim3(cols, nch), 128, 0, st>>>(f, g, W, H, w.tot.as<S>());
+  k_sat_above<S><<<dim3(cols, 4), 128, 0, st>>>(w.tot.as<S>(), W, nch);
+  k_sat_fill<P><<<dim3(nch, 4), kSatThreads, 0, st>>>(f, g, W, H, w.tot.as<S>(), sat);
   ALDIC_CUDA(cudaGetLastError());
 
   // ---- level 1: whole ROI (funIntegerSearchMg.m:9-35)
@@ -923,77 +1292,53 @@ int run_levels(MgWork &w, const P *f, const P *g, int W, int H, const double *mu
               "multigrid search: the ROI is wider than 4096 px");
   if (P1 < 2) { P1 = 2; l1 = 1; }
   if (P2 < 2) { P2 = 2; l2 = 1; }
-  if ((rc = w.fft.ensure(sizeof(double2) * 2 * (size_t)P1 * P2))) return rc;
+  // the second plane also holds P2 rows of P1 / 2 + 8
+  const size_t zn = (size_t)P1 * P2 + 8 * (size_t)P2;
+  if ((rc = w.fft.ensure(sizeof(double2) * 2 * zn))) return rc;
   if ((rc = w.tw.ensure(sizeof(double2) * (size_t)(P1 + P2)))) return rc;
-  double2 *Z0 = w.fft.as<double2>(), *Z1 = Z0 + (size_t)P1 * P2;
+  double2 *Z0 = w.fft.as<double2>(), *Z1 = Z0 + zn;
   double2 *tw1 = w.tw.as<double2>(), *tw2 = tw1 + P1;
-  k_fft_twiddle<<<(P1 + 255) / 256, 256, 0, st>>>(tw1, P1);
-  k_fft_twiddle<<<(P2 + 255) / 256, 256, 0, st>>>(tw2, P2);
-  const size_t sm1 = sizeof(double2) * P1, sm2 = sizeof(double2) * P2;
-  const size_t smx = std::max(sm1, sm2);
-  ALDIC_CUDA(cudaFuncSetAttribute(k_fft_pack_rows<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
-  ALDIC_CUDA(cudaFuncSetAttribute(k_fft_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
-  ALDIC_CUDA(cudaFuncSetAttribute(k_fft_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
-  const int fth = 512;
-  // rows: [y][x] (P2 rows of P1)
-  k_fft_pack_rows<P><<<P2, fth, sm1, st>>>(f, g, W, H, gx[0], gy[0], a, b, sat, mu_g, Z0, P1, l1, tw1);
-  k_transpose_c<<<dim3((P1 + 31) / 32, (P2 + 31) / 32), dim3(32, 8), 0, st>>>(Z0, Z1, P2, P1);
-  k_fft_rows<false><<<P1, fth, sm2, st>>>(Z1, P2, l2, tw2, 0, 0);               // [kx][ky]
-  k_mg_spectrum<<<1184, 256, 0, st>>>(Z1, Z0, P1, P2);
-  k_fft_rows<true><<<P1, fth, sm2, st>>>(Z0, P2, l2, tw2, 0, 0);                // [kx][oy]
-  k_transpose_c<<<dim3((P2 + 31) / 32, (P1 + 31) / 32), dim3(32, 8), 0, st>>>(Z0, Z1, P1, P2);
-  // [oy][kx]: only rows oy in [-(b-1), b-1] (mod P2) are read
-  k_fft_rows<true><<<P2, fth, sm1, st>>>(Z1, P1, l1, tw1, b, P2 - (b - 1));      // [oy][ox]
-  ALDIC_CUDA(cudaGetLastError());
-  L1Args<MgT<P>::integer, S> L1;
+  k_fft_twiddle<<<(P1 + 255) / 256, 256, 0, st>>>(tw1, P1, l1);
+  k_fft_twiddle<<<(P2 + 255) / 256, 256, 0, st>>>(tw2, P2, l2);
+  const size_t sm1 = fft_smem(P1), sm2 = fft_smem(P2);
+  const int th1 = fft_threads(P1), th2 = fft_threads(P2);
+  ALDIC_CUDA(cudaFuncSetAttribute(k_fft_pack_rows<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
+  ALDIC_CUDA(cudaFuncSetAttribute(k_fft_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
+  ALDIC_CUDA(cudaFuncSetAttribute(k_fft_spectrum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
+  ALDIC_CUDA(cudaFuncSetAttribute(k_fft_ncc<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
+  L1Args<S> L1;
   L1.sat = sat;
+  L1.plane = plane;
   L1.W1 = (int)W1;
   L1.gx0 = gx[0] - 1;
   L1.gy0 = gy[0] - 1;
   L1.a = a;
   L1.b = b;
   L1.mn = (long long)a * b;
-  L1.c = Z1;
+  L1.c = (double *)Z0;  // free by then
   L1.P1 = P1;
-  L1.P2 = P2;
   L1.inv = 1.0 / ((double)P1 * (double)P2);
-  // template sums and mu on the host (two small reads)
-  S sums[4];
-  {
-    S c4[2][4];
-    const S *sf = sat, *sf2 = sat + plane;
-    const long long xo0 = gx[0] - 1, yo0 = gy[0] - 1;
-    const long long idx[4] = {yo0 * W1 + xo0, yo0 * W1 + xo0 + a, (yo0 + b) * W1 + xo0,
-                              (yo0 + b) * W1 + xo0 + a};
-    for (int k = 0; k < 4; ++k) {
-      ALDIC_CUDA(cudaMemcpyAsync(&c4[0][k], sf + idx[k], sizeof(S), cudaMemcpyDeviceToHost, st));
-      ALDIC_CUDA(cudaMemcpyAsync(&c4[1][k], sf2 + idx[k], sizeof(S), cudaMemcpyDeviceToHost, st));
-    }
-    double mu_h = 0;
-    ALDIC_CUDA(cudaMemcpyAsync(&mu_h, mu_g, sizeof(double), cudaMemcpyDeviceToHost, st));
-    ALDIC_CUDA(cudaStreamSynchronize(st));
-    for (int q = 0; q < 2; ++q) sums[q] = c4[q][3] - c4[q][1] - c4[q][2] + c4[q][0];
-    L1.mu = mu_h;
-  }
-  L1.st = sums[0];
-  L1.st2 = sums[1];
-  bool flat;
-  if constexpr (MgT<P>::integer)
-    flat = ((__int128)L1.mn * (long long)L1.st2 - (__int128)(long long)L1.st * (long long)L1.st) == 0;
-  else
-    flat = !((double)L1.mn * (double)L1.st2 - (double)L1.st * (double)L1.st > 0.0);
-  ALDIC_CHECK(!flat, E_ARG, "multigrid search: the ROI of the reference image is constant");
-  const int nblk = 148 * 8;
-  if ((rc = w.part.ensure((sizeof(double) + sizeof(long long)) * nblk + 64))) return rc;
+  L1.mu = mu_g;
+  const double most = sizeof(P) == 1 ? 255.0 : 65535.0;
+  L1.narrow = (double)L1.mn * (double)L1.mn * most * most < 9e18;
+  const int np = (2 * b - 1 + 1) / 2, half = P1 / 2 + 1, ldc = P1 / 2 + 8;
+  if ((rc = w.part.ensure((sizeof(double) + sizeof(long long)) * np + 64))) return rc;
   double *pv = w.part.as<double>();
-  long long *pi = (long long *)(pv + nblk);
-  double *peak = (double *)(pi + nblk);
-  k_mg_l1_argmax<MgT<P>::integer, S><<<nblk, 256, 0, st>>>(L1, sat + 2 * plane, sat + 3 * plane, pv, pi);
-  k_mg_l1_peak<MgT<P>::integer, S><<<1, 32, 0, st>>>(L1, sat + 2 * plane, sat + 3 * plane, pv, pi, nblk, peak);
+  long long *pi = (long long *)(pv + np);
+  double *peak = (double *)(pi + np);
+  const dim3 tb(32, 8);
+  k_fft_pack_rows<P><<<b, th1, sm1, st>>>(f, g, W, H, gx[0], gy[0], a, b, sat, mu_g, Z0, P1, l1, tw1);  // [y][kx]
+  k_transpose_c<<<dim3((P1 + 31) / 32, (b + 31) / 32), tb, 0, st>>>(Z0, Z1, b, P1, P1, P2);
+  k_fft_cols<<<P1, th2, sm2, st>>>(Z1, P2, l2, tw2, b);                                                 // [kx][ky]
+  k_fft_spectrum<<<half, th2, sm2, st>>>(Z1, Z0, P1, P2, l2, tw2);                                      // [kx][oy]
+  k_transpose_c<<<dim3((P2 + 31) / 32, (half + 31) / 32), tb, 0, st>>>(Z0, Z1, half, P2, P2, ldc);
+  k_fft_ncc<S><<<np, th1, sm1, st>>>(Z1, ldc, P2, L1, l1, tw1, pv, pi);                                 // [oy][ox]
+  k_mg_l1_peak<S><<<1, 32, 0, st>>>(L1, pv, pi, np, peak);
   ALDIC_CUDA(cudaGetLastError());
-  double pk3[3];
+  double pk3[4];
   ALDIC_CUDA(cudaMemcpyAsync(pk3, peak, sizeof(pk3), cudaMemcpyDeviceToHost, st));
   ALDIC_CUDA(cudaStreamSynchronize(st));
+  ALDIC_CHECK(pk3[3] == 0.0, E_ARG, "multigrid search: the ROI of the reference image is constant");
   const double ut = pk3[0] - a, vt = pk3[1] - b;
   out.l1_u = ut;
   out.l1_v = vt;
@@ -1071,16 +1416,26 @@ int run_levels(MgWork &w, const P *f, const P *g, int W, int H, const double *mu
                         sizeof(typename MgT<P>::V) *
                             ((size_t)(amax + 8) * bmax + (size_t)dhm * (dwm + 2 * kStrip + 8)) + 16;
       ALDIC_CHECK(sm <= 200 * 1024, E_ARG, "multigrid search: last-level map too large for shared memory");
-      ALDIC_CUDA(cudaFuncSetAttribute(k_mg_full<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-      if (amax > 0) k_mg_full<P><<<n, 256, sm, st>>>(f, g, W, H, dr, sat, mu_g, dres);
+      size_t use = sm;
+      if constexpr (MgT<P>::integer) {  // operands as packed words: less than that
+        const FullWords fw(amax);
+        use = sizeof(double) * (size_t)(amax + dwm - 1) * (bmax + dhm - 1) +
+              sizeof(P) * sizeof(uint32_t) * ((size_t)bmax * fw.tw + (size_t)dhm * fw.dw) + 16;
+      }
+      ALDIC_CUDA(cudaFuncSetAttribute(k_mg_full<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)use));
+      if (amax > 0) k_mg_full<P><<<n, 256, use, st>>>(f, g, W, H, dr, sat, mu_g, dres);
     } else {
       if ((rc = w.acc.ensure(sizeof(G) * (size_t)kCrop * n))) return rc;
       ALDIC_CUDA(cudaMemsetAsync(w.acc.p, 0, sizeof(G) * (size_t)kCrop * n, st));
       if (amax > 0) {
-        constexpr int kTile = CropCfg<P>::TILE;
-        const dim3 grid(n, (bmax + kBand - 1) / kBand, (amax + kTile - 1) / kTile);
+        constexpr bool kInt = MgT<P>::integer;
+        constexpr int kTile = kInt ? kTileI : CropCfg<P>::TILE, kRows = kInt ? kBandI : kBand;
+        const dim3 grid(n, (bmax + kRows - 1) / kRows, (amax + kTile - 1) / kTile);
         ALDIC_CHECK(grid.y <= 65535 && grid.z <= 65535, E_ARG, "multigrid search: region too large");
-        k_mg_crop<P><<<grid, 224, 0, st>>>(f, g, W, dr, w.acc.as<G>());
+        if constexpr (kInt)
+          k_mg_crop_int<P><<<grid, 224, 0, st>>>(f, g, W, dr, w.acc.as<G>());
+        else
+          k_mg_crop<P><<<grid, 224, 0, st>>>(f, g, W, dr, w.acc.as<G>());
         k_mg_crop_peak<P><<<n, 192, 0, st>>>(dr, W, H, sat, w.acc.as<G>(), mu_g, dres);
       }
     }

@@ -505,10 +505,8 @@ static int prep_def(aldic_ctx *c) {
   int rc = roi_stats(c->g_raw.p, c->dtype, c->W, c->roi, st + 2, c->isums.as<unsigned long long>(),
                      c->part.as<double>(), c->stream);
   if (rc) return rc;
-  if ((rc = normalize(c->g_raw.p, c->dtype, (long long)c->W * c->H, st + 2, c->g64.as<double>(),
-                      c->g32.as<float>(), c->stream)))
-    return rc;
-  return row_cubic(c->g64.as<double>(), c->W, c->H, c->gc.as<float4>(), c->stream);
+  return normalize_cubic(c->g_raw.p, c->dtype, c->W, c->H, st + 2, c->g64.as<double>(), c->g32.as<float>(),
+                         c->gc.as<float4>(), c->stream);
 }
 
 int aldic_set_def(aldic_ctx *c, const void *img, int dtype) {
@@ -543,9 +541,8 @@ int aldic_set_stats(aldic_ctx *c, const double stats[4]) {
   if ((rc = grad_pairs(c->gx32.as<float>(), c->gy32.as<float>(), n, c->gxy.as<float2>(), c->stream)))
     return rc;
   // the deformed image with stats[2..3] (not prep_def, which takes them from the ROI)
-  if ((rc = normalize(c->g_raw.p, c->dtype, n, st + 2, c->g64.as<double>(), c->g32.as<float>(),
-                      c->stream)) ||
-      (rc = row_cubic(c->g64.as<double>(), c->W, c->H, c->gc.as<float4>(), c->stream)))
+  if ((rc = normalize_cubic(c->g_raw.p, c->dtype, c->W, c->H, st + 2, c->g64.as<double>(), c->g32.as<float>(),
+                            c->gc.as<float4>(), c->stream)))
     return rc;
   return finish(c, true);
 }

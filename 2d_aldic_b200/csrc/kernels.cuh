@@ -17,6 +17,8 @@ int gradient(const double *f, const double *mask, int W, int H, double *gx64, do
              float *gx32, float *gy32, cudaStream_t st);
 // row-cubic coefficients of the FP64 image g: W H float4, q[y W + x] =
 // (a0, a1, a2, a3) of row y's Keys cubic on floor column x
+int normalize_cubic(const void *img, int dtype, int W, int H, const double *d_stats, double *o64, float *o32,
+                    float4 *q, cudaStream_t st);
 int row_cubic(const double *g, int W, int H, float4 *q, cudaStream_t st);
 // q[i] = (gx[i], gy[i]), n float2
 int grad_pairs(const float *gx, const float *gy, long long n, float2 *q, cudaStream_t st);

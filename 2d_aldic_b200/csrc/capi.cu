@@ -249,6 +249,7 @@ int ensure_grid_work(aldic_ctx *c, long long n) {
   c->gw.err = (int *)(misc + 2);
   c->gw.iters_out = (int *)(misc + 3);
   c->gw.gate = (int *)(misc + 4);
+  c->gw.ticket = misc + 8;
   c->gw_n = n;
   ALDIC_CUDA(cudaMemsetAsync(c->gw_misc.p, 0, 64, c->stream));
   return OK;
@@ -1487,14 +1488,17 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
   // interior nodes (main_ALDIC.m:243-278): solve into fields f0, f0 + 1,
   // store U2, strain F2
   const bool fd = p->subpb2_fd != 0;
-  auto rhs = [&](double beta, const double *beta_ptr, int f0) {
-    return fd ? fd_rhs(c->gw, M, N, h, beta, mu, B.U1, B.F1, B.udual, B.vdual, st, beta_ptr, f0)
-              : fe_rhs(c->gw, M, N, h, beta, mu, B.U1, B.F1, B.udual, B.vdual, st, beta_ptr, f0);
+  auto rhs = [&](double beta, const double *beta_ptr, int f0, const double *F) {
+    return fd ? fd_rhs(c->gw, M, N, h, beta, mu, B.U1, F, B.udual, B.vdual, st, beta_ptr, f0)
+              : fe_rhs(c->gw, M, N, h, beta, mu, B.U1, F, B.udual, B.vdual, st, beta_ptr, f0);
   };
+  // strain, duals, update norm and F1's copy of a global step in one launch; the
+  // finite-difference step and smoothing keep them apart
+  const bool tail = !fd && !p->smooth;
   // the direct fast-diagonalisation solve (fdm.cu; bases set up before capture)
-  // of the system at *beta into U2
-  auto solve = [&](const double *beta_ptr) {
-    int rc2 = rhs(0, beta_ptr, 0);
+  // of the system at *beta with Subproblem 1's strains F into U2
+  auto solve = [&](const double *beta_ptr, const double *F) {
+    int rc2 = rhs(0, beta_ptr, 0, F);
     if (!rc2)
       rc2 = fdm_solve(c->fdm, 2, c->gw.b, c->gw.x, c->gw.r, mu, 0.0, nullptr, beta_ptr, st, fd ? nullptr : B.U2);
     return rc2 || !fd ? rc2 : fd_store(c->gw, M, N, B.U1, B.U2, st, 0);
@@ -1514,7 +1518,7 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
     double be[12], b6[6];
     for (int k = 0; k < 6; ++k) {
       be[2 * k] = be[2 * k + 1] = b6[k] = bl[k] * base;
-      if (fd && (rc = rhs(bl[k] * base, nullptr, 2 * k))) return rc;
+      if (fd && (rc = rhs(bl[k] * base, nullptr, 2 * k, B.F1))) return rc;
     }
     if (fd) {
       // the six systems of the sweep in one launch (12 right-hand sides)
@@ -1530,8 +1534,8 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
       for (int k = 0; k < 6; ++k) {
         if ((rc = fd_store(c->gw, M, N, B.U1, B.U2, st, 2 * k))) return rc;
         if ((rc = strain())) return rc;
-        if ((rc = vdiffnorm(B.U1, B.U2, 2 * n, B.part, B.err + k, st))) return rc;
-        if ((rc = vdiffnorm(B.F1, B.F2, 4 * n, B.part, B.err + 6 + k, st))) return rc;
+        if ((rc = vdiffnorm(c->gw, B.U1, B.U2, 2 * n, B.part, B.err + k, st))) return rc;
+        if ((rc = vdiffnorm(c->gw, B.F1, B.F2, 4 * n, B.part, B.err + 6 + k, st))) return rc;
       }
     } else {
       // store, nodal strain and both norms of every candidate in one pass
@@ -1540,9 +1544,16 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
     }
     k_beta_select<<<1, 1, 0, st>>>(B.err, base, B.beta, fd ? h : 0.0);
   }
-  if ((rc = solve(B.beta)) || (rc = strain())) return rc;
-  if (p->smooth && (rc = smooth_dev(c, M, N, 4, B.F2))) return rc;
-  if ((rc = dual(0))) return rc;
+  if ((rc = solve(B.beta, B.F1))) return rc;
+  if (tail) {
+    if ((rc = fe_tail(c->gw, M, N, h, B.U1, B.U2, B.F1, B.F2, B.udual, B.vdual, false, nullptr, nullptr, nullptr,
+                      0.0, st)))
+      return rc;
+  } else {
+    if ((rc = strain())) return rc;
+    if (p->smooth && (rc = smooth_dev(c, M, N, 4, B.F2))) return rc;
+    if ((rc = dual(0))) return rc;
+  }
   ALDIC_CUDA(cudaMemcpyAsync(B.U1old, B.U1, sizeof(double) * 2 * n, cudaMemcpyDeviceToDevice, st));
   // Section 6: ADMM iterations
   if ((rc = mark(c, 5))) return rc;
@@ -1561,19 +1572,26 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
                             FieldMap().interleaved(B.U1, 2), B.itb, &start, lam2, kRtolFit, kMaxitFit,
                             false, st)))
       return rc;
-    ALDIC_CUDA(cudaMemcpyAsync(B.F1, B.F2, sizeof(double) * 4 * n, cudaMemcpyDeviceToDevice, st));
+    if (!tail) ALDIC_CUDA(cudaMemcpyAsync(B.F1, B.F2, sizeof(double) * 4 * n, cudaMemcpyDeviceToDevice, st));
     if (a < 16) {  // the update norm, and U1old <- U1 in the same pass
-      if ((rc = diffnorm_update(B.U1old, B.U1, 2 * n, B.part, B.upd + 16 + a, inv, st))) return rc;
+      if ((rc = diffnorm_update(c->gw, B.U1old, B.U1, 2 * n, B.part, B.upd + 16 + a, inv, st))) return rc;
     } else {
       ALDIC_CUDA(cudaMemcpyAsync(B.U1old, B.U1, sizeof(double) * 2 * n, cudaMemcpyDeviceToDevice, st));
     }
     if (p->smooth && (rc = smooth_dev(c, M, N, 2, B.U1))) return rc;
-    if ((rc = solve(B.beta))) return rc;
+    if ((rc = solve(B.beta, tail ? B.F2 : B.F1))) return rc;
+    if (tail) {  // U2 is not written again before the next Subpb1
+      if ((rc = fe_tail(c->gw, M, N, h, B.U1, B.U2, B.F1, B.F2, B.udual, B.vdual, true, B.U2old, B.part,
+                        a < 16 ? B.upd + a : nullptr, inv, st)))
+        return rc;
+      u2old_current = a < 16;
+      continue;
+    }
     if (p->smooth && (rc = smooth_dev(c, M, N, 2, B.U2))) return rc;
     if ((rc = strain())) return rc;
     if (p->smooth && (rc = smooth_dev(c, M, N, 4, B.F2))) return rc;
     if (a < 16) {  // U2 is not written again before the next Subpb1
-      if ((rc = diffnorm_update(B.U2old, B.U2, 2 * n, B.part, B.upd + a, inv, st))) return rc;
+      if ((rc = diffnorm_update(c->gw, B.U2old, B.U2, 2 * n, B.part, B.upd + a, inv, st))) return rc;
       u2old_current = true;
     }
     if ((rc = dual(1))) return rc;   // FE resets the duals, FD accumulates (main_ALDIC.m:434-441)
@@ -1823,8 +1841,8 @@ int aldic_qt_frame(aldic_ctx *c, const aldic_qt_frame_params *p, aldic_qt_mesh *
   if ((rc = qt_subpb2_sweep(m, c->gw, betas, mu, Q.U1, Q.F1, st))) return rc;
   for (int k = 0; k < 3; ++k) {
     if ((rc = qt_store_candidate(m, c->gw, k, Q.U2, st)) || (rc = qt_strain(m, Q.U2, Q.F2, st)) ||
-        (rc = vdiffnorm(Q.U1, Q.U2, 2 * n, part, nrm + k, st)) ||
-        (rc = vdiffnorm(Q.F1, Q.F2, 4 * n, part, nrm + 4 + k, st)))
+        (rc = vdiffnorm(c->gw, Q.U1, Q.U2, 2 * n, part, nrm + k, st)) ||
+        (rc = vdiffnorm(c->gw, Q.F1, Q.F2, 4 * n, part, nrm + 4 + k, st)))
       return rc;
   }
   double hn[8];
@@ -1861,8 +1879,8 @@ int aldic_qt_frame(aldic_ctx *c, const aldic_qt_frame_params *p, aldic_qt_mesh *
       return rc;
     k_qt_keep_dirichlet<<<nb, 256, 0, st>>>(n, kind, Q.F1, Q.F2);
     // the update norms, each old vector refreshed in the same pass
-    if ((rc = diffnorm_update(Q.U2old, Q.U2, 2 * n, part, nrm + 8, 1.0, st)) ||
-        (rc = diffnorm_update(Q.U1old, Q.U1, 2 * n, part, nrm + 9, 1.0, st)))
+    if ((rc = diffnorm_update(c->gw, Q.U2old, Q.U2, 2 * n, part, nrm + 8, 1.0, st)) ||
+        (rc = diffnorm_update(c->gw, Q.U1old, Q.U1, 2 * n, part, nrm + 9, 1.0, st)))
       return rc;
     if ((rc = vsub2(Q.F2, Q.F1, Q.ud, 4 * n, Q.U2, Q.U1, Q.vd, 2 * n, st))) return rc;
     double hv[2];

@@ -48,10 +48,6 @@ struct PcgArgs {
 // u and v separately, beta*DN'DN) and mass (h^2/36)[4 2 1 2; ...]
 // (mu*N'N).  Their node-pair sums give the 9-point stencil below.
 
-// local node index -> (di, dj) offset from the element's first node
-__device__ __forceinline__ int lx(int a) { return (a == 1 || a == 2) ? 1 : 0; }
-__device__ __forceinline__ int ly(int a) { return (a >= 2) ? 1 : 0; }
-
 // FE stencil weights on a square-element grid: the element matrices above
 // summed over the elements two nodes share.  kap[0] centre, [1] axial, [2]
 // diagonal; the coefficient of neighbour (di, dj) of node (i, j) is
@@ -700,57 +696,26 @@ __global__ void k_fe_store(long long n, const double *__restrict__ x, double *__
   }
 }
 
-// ------------------------------------------------------------------ nodal strain
-// funGlobal_NodalStrainAvg.m:51-144: per element, DN*U at the 2x2 Gauss points
-// in the order (-,-), (+,-), (+,+), (-,+); extrapolated to the corners with
-// the matrix of :105-108; averaged over the elements sharing a node.  Output
-// slots per node are [du/dx, du/dy, dv/dx, dv/dy] as written at :123-137.
-// The nodal strain of node (i, j); ld(q, &u, &v) reads the displacement of
-// node q.
-template <class Load>
+// funGlobal_NodalStrainAvg.m at node (i, j): the mean over its elements of the
+// strain that the 2 x 2 Gauss points extrapolate to the corner.  On a square
+// bilinear element that is the corner's own gradient, the difference along the
+// edge, so the mean is the mean of the differences to either side.  out: du/dx,
+// du/dy, dv/dx, dv/dy.
+template <typename Load>
 __device__ __forceinline__ void nodal_strain_node(int M, int N, double h, int i, int j,
                                                   const Load &ld, double out[4]) {
-  const double r3 = 0.5773502691896257;  // 1/sqrt(3)
-  const double s3 = 1.7320508075688772;
-  const double gks[4] = {-r3, r3, r3, -r3}, get_[4] = {-r3, -r3, r3, r3};
-  const double E[4][4] = {{1 + 0.5 * s3, -0.5, 1 - 0.5 * s3, -0.5},
-                          {-0.5, 1 + 0.5 * s3, -0.5, 1 - 0.5 * s3},
-                          {1 - 0.5 * s3, -0.5, 1 + 0.5 * s3, -0.5},
-                          {-0.5, 1 - 0.5 * s3, -0.5, 1 + 0.5 * s3}};
-  double acc[4] = {0, 0, 0, 0};
-  int cnt = 0;
-  for (int ej = j - 1; ej <= j; ++ej)
-    for (int ei = i - 1; ei <= i; ++ei) {
-      if (ei < 0 || ei >= M - 1 || ej < 0 || ej >= N - 1) continue;
-      const int la = (i - ei) + (j - ej) * 3 - 2 * (i - ei) * (j - ej);
-      double ue[8];
-      for (int lb = 0; lb < 4; ++lb) {
-        const long long q = (long long)(ej + ly(lb)) * M + (ei + lx(lb));
-        ld(q, &ue[2 * lb], &ue[2 * lb + 1]);
-      }
-      double G[4][4];
-      for (int g = 0; g < 4; ++g) {
-        const double ksi = gks[g], eta = get_[g];
-        const double dks[4] = {-(1 - eta) / 4, (1 - eta) / 4, (1 + eta) / 4, -(1 + eta) / 4};
-        const double det_[4] = {-(1 - ksi) / 4, -(1 + ksi) / 4, (1 + ksi) / 4, (1 - ksi) / 4};
-        double v[4] = {0, 0, 0, 0};
-        for (int a = 0; a < 4; ++a) {
-          const double gx = (2.0 / h) * dks[a], gy = (2.0 / h) * det_[a];
-          v[0] += gx * ue[2 * a];
-          v[1] += gy * ue[2 * a];
-          v[2] += gx * ue[2 * a + 1];
-          v[3] += gy * ue[2 * a + 1];
-        }
-        for (int c = 0; c < 4; ++c) G[g][c] = v[c];
-      }
-      for (int c = 0; c < 4; ++c) {
-        double s = 0.0;
-        for (int g = 0; g < 4; ++g) s += E[la][g] * G[g][c];
-        acc[c] += s;
-      }
-      cnt++;
-    }
-  for (int c = 0; c < 4; ++c) out[c] = acc[c] / cnt;
+  const long long k = (long long)j * M + i;
+  const bool l = i > 0, r = i < M - 1, d = j > 0, u = j < N - 1;
+  double a[2], b[2];
+  ld(r ? k + 1 : k, &a[0], &a[1]);
+  ld(l ? k - 1 : k, &b[0], &b[1]);
+  const double sx = 1.0 / (h * (l + r)), sy = 1.0 / (h * (d + u));
+  out[0] = (a[0] - b[0]) * sx;
+  out[2] = (a[1] - b[1]) * sx;
+  ld(u ? k + M : k, &a[0], &a[1]);
+  ld(d ? k - M : k, &b[0], &b[1]);
+  out[1] = (a[0] - b[0]) * sy;
+  out[3] = (a[1] - b[1]) * sy;
 }
 
 __global__ void k_nodal_strain(int M, int N, double h, const double *__restrict__ U,
@@ -848,63 +813,65 @@ __global__ void k_sweep_err_final(const double *__restrict__ part, int nb, int n
 }
 
 // ------------------------------------------------------------------ flags
-__global__ void k_icgn_flags(long long n, const int *__restrict__ it,
-                             unsigned char *__restrict__ bad, int *badnum, double *meanit,
-                             int *nconv, double floor) {
-  __shared__ long long sh[32][3];
-  __shared__ double shd[32];
-  __shared__ double s_mean, s_thr;
+// The counts, the sum and the sum of squares of the evaluations are whole numbers,
+// so one pass gives mean and deviation; four subsets a load, four loads in flight
+// (one block: 59049 subsets in 21 us, three passes of single loads took 25).
+__global__ void __launch_bounds__(1024)
+    k_icgn_flags(long long n, const int *__restrict__ it, unsigned char *__restrict__ bad, int *badnum,
+                 double *meanit, int *nconv, double floor) {
+  __shared__ long long sh[5][32];
+  __shared__ double s_thr;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  long long cb = 0, c102 = 0, sg = 0, ng = 0;
-  for (long long k = threadIdx.x; k < n; k += blockDim.x) {
-    const int v = it[k];
-    const bool b1 = v < 0 || v > 99;
-    cb += b1;
-    c102 += (v == 102);
-    if (!b1) {
-      sg += v;
-      ng++;
-    }
+  const long long n4 = ((uintptr_t)it & 15) == 0 ? n / 4 : 0;
+  long long c[5] = {0, 0, 0, 0, 0};  // flagged, masked; sum, squares and count of the others
+  auto count = [&](int v) {
+    const bool b = v < 0 || v > 99;
+    c[0] += b;
+    c[1] += v == 102;
+    c[2] += b ? 0 : v;
+    c[3] += b ? 0 : v * v;
+    c[4] += !b;
+  };
+#pragma unroll 4
+  for (long long k = threadIdx.x; k < n4; k += blockDim.x) {
+    const int4 v = ((const int4 *)it)[k];
+    count(v.x);
+    count(v.y);
+    count(v.z);
+    count(v.w);
   }
-  cb = warp_sum_ll(cb); c102 = warp_sum_ll(c102); sg = warp_sum_ll(sg); ng = warp_sum_ll(ng);
-  if (lane == 0) { sh[wid][0] = cb; sh[wid][1] = c102; sh[wid][2] = sg; shd[wid] = (double)ng; }
+  for (long long k = 4 * n4 + threadIdx.x; k < n; k += blockDim.x) count(it[k]);
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    c[q] = warp_sum_ll(c[q]);
+    if (lane == 0) sh[q][wid] = c[q];
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    long long a = 0, b = 0, c = 0, d = 0;
-    for (int w = 0; w < nw; ++w) { a += sh[w][0]; b += sh[w][1]; c += sh[w][2]; d += (long long)shd[w]; }
-    *badnum = (int)(a - b);
-    *nconv = (int)d;
-    s_mean = d ? (double)c / (double)d : __longlong_as_double(0x7ff8000000000000ll);
-    *meanit = s_mean;
-    sh[0][0] = d;
-  }
-  __syncthreads();
-  const long long ngood = sh[0][0];
-  const double m = s_mean;
-  double ss = 0.0;
-  for (long long k = threadIdx.x; k < n; k += blockDim.x) {
-    const int v = it[k];
-    if (!(v < 0 || v > 99)) ss += (v - m) * (v - m);
-  }
-  ss = warp_sum(ss);
-  __syncthreads();
-  if (lane == 0) shd[wid] = ss;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < nw; ++w) t += shd[w];
-    const double sd = ngood > 1 ? sqrt(t / (double)(ngood - 1))
-                                : (ngood == 1 ? 0.0 : __longlong_as_double(0x7ff8000000000000ll));
+    long long t[5] = {0, 0, 0, 0, 0};
+    for (int w = 0; w < nw; ++w)
+      for (int q = 0; q < 5; ++q) t[q] += sh[q][w];
+    const double nan = __longlong_as_double(0x7ff8000000000000ll), d = (double)t[4];
+    *badnum = (int)(t[0] - t[1]);
+    *nconv = (int)t[4];
+    const double m = t[4] ? (double)t[2] / d : nan;
+    *meanit = m;
+    const double sd = t[4] > 1 ? sqrt((double)(t[4] * t[3] - t[2] * t[2]) / d / (double)(t[4] - 1))
+                               : (t[4] == 1 ? 0.0 : nan);
     // Subpb1Quadtree.m:180 raises the threshold to at least `floor`
     // (MATLAB's max ignores a NaN); NaN floor = LocalICGN.m:128-131
     s_thr = isnan(floor) ? m + 0.15 * sd : fmax(m + 0.15 * sd, floor);
   }
   __syncthreads();
   const double thr = s_thr;
-  for (long long k = threadIdx.x; k < n; k += blockDim.x) {
-    const int v = it[k];
-    bad[k] = (v < 0 || v > 99 || (double)v > thr) ? 1 : 0;
+  auto flag = [&](int v) { return (unsigned char)((v < 0 || v > 99 || (double)v > thr) ? 1 : 0); };
+  const long long b4 = ((uintptr_t)bad & 3) == 0 ? n4 : 0;
+#pragma unroll 4
+  for (long long k = threadIdx.x; k < b4; k += blockDim.x) {
+    const int4 v = ((const int4 *)it)[k];
+    ((uchar4 *)bad)[k] = make_uchar4(flag(v.x), flag(v.y), flag(v.z), flag(v.w));
   }
+  for (long long k = 4 * b4 + threadIdx.x; k < n; k += blockDim.x) bad[k] = flag(it[k]);
 }
 
 __global__ void k_subpb1_flags(long long n, const int *__restrict__ it,
@@ -944,7 +911,42 @@ __global__ void k_vsub2(const double *a1, const double *b1, double *o1, long lon
 
 // block partials of |a - b|^2; with copy, a <- b as it goes (the caller's
 // "old" vector refreshed in the same pass)
-__global__ void k_diffnorm_part(double *a, const double *b, long long n, double *part, bool copy) {
+// *res = sqrt(sum of the blocks' s) * scale: the last block to arrive adds the
+// partials in their order, so the result does not depend on which it is
+__device__ __forceinline__ void norm_finish(double s, double *part, unsigned int *ticket, double *res,
+                                            double scale) {
+  __shared__ double sh[32];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  s = warp_sum(s);
+  if (lane == 0) sh[warp] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < nw; ++w) t += sh[w];
+    part[blockIdx.x] = t;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double t = 0.0;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) t += __ldcg(part + k);
+  t = warp_sum(t);
+  if (lane == 0) sh[warp] = t;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double u = 0.0;
+    for (int w = 0; w < nw; ++w) u += sh[w];
+    *res = sqrt(u) * scale;
+    *ticket = 0u;
+  }
+}
+
+// |a - b| * scale, and with `copy` a = b
+__global__ void k_diffnorm(double *a, const double *b, long long n, double *part, unsigned int *ticket,
+                           double *res, double scale, bool copy) {
   double s = 0.0;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x) {
@@ -953,31 +955,50 @@ __global__ void k_diffnorm_part(double *a, const double *b, long long n, double 
     s += d * d;
     if (copy) a[k] = bk;
   }
-  s = warp_sum(s);
-  __shared__ double sh[32];
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
-    part[blockIdx.x] = t;
-  }
+  norm_finish(s, part, ticket, res, scale);
 }
 
-// one 256-thread block: strided partial sums, then a fixed-order tree;
-// res = sqrt(sum) * scale
-__global__ void k_diffnorm_final(const double *part, int np, double *res, double scale) {
-  double t = 0.0;
-  for (int k = threadIdx.x; k < np; k += blockDim.x) t += part[k];
-  t = warp_sum(t);
-  __shared__ double sh[32];
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double u = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) u += sh[w];
-    *res = sqrt(u) * scale;
+// What follows a finite-element global step, a node at a time: F1 takes the
+// strains that Subproblem 1 held (F2 so far), F2 those of the new U2; the duals
+// F2 - F1 and U2 - U1; with `res` the update norm |U2old - U2| * scale, and U2old
+// takes U2.  (Five launches of 2 to 5 us each before.)
+struct FeTail {
+  const double *U1, *U2;
+  double *F1, *F2, *ud, *vd, *U2old;
+  bool keep;  // F1 := F2 first
+  double *part, *res;
+  unsigned int *ticket;
+  double scale;
+};
+__global__ void k_fe_tail(int M, int N, double h, const __grid_constant__ FeTail A) {
+  const long long n = (long long)M * N;
+  double s = 0.0;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
+       k += (long long)gridDim.x * blockDim.x) {
+    double out[4];
+    nodal_strain_node(M, N, h, (int)(k % M), (int)(k / M),
+                      [&](long long q, double *u, double *v) {
+                        *u = A.U2[2 * q];
+                        *v = A.U2[2 * q + 1];
+                      },
+                      out);
+    for (int c = 0; c < 4; ++c) {
+      const double f1 = A.keep ? A.F2[4 * k + c] : A.F1[4 * k + c];
+      if (A.keep) A.F1[4 * k + c] = f1;
+      A.F2[4 * k + c] = out[c];
+      A.ud[4 * k + c] = out[c] - f1;
+    }
+    for (int c = 0; c < 2; ++c) {
+      const double u2 = A.U2[2 * k + c];
+      A.vd[2 * k + c] = u2 - A.U1[2 * k + c];
+      if (A.res) {
+        const double d = A.U2old[2 * k + c] - u2;
+        s += d * d;
+        A.U2old[2 * k + c] = u2;
+      }
+    }
   }
+  if (A.res) norm_finish(s, A.part, A.ticket, A.res, A.scale);
 }
 
 inline int blocks_for(long long n, int threads = 256) {
@@ -1295,20 +1316,23 @@ int vsub2(const double *a1, const double *b1, double *o1, long long n1, const do
   return OK;
 }
 
-int vdiffnorm(const double *a, const double *b, long long n, double *part, double *res,
+int vdiffnorm(const GridWork &w, const double *a, const double *b, long long n, double *part, double *res,
               cudaStream_t st) {
-  const int nb = 148;
-  k_diffnorm_part<<<nb, 256, 0, st>>>(const_cast<double *>(a), b, n, part, false);
-  k_diffnorm_final<<<1, 256, 0, st>>>(part, nb, res, 1.0);
+  k_diffnorm<<<148, 256, 0, st>>>(const_cast<double *>(a), b, n, part, w.ticket, res, 1.0, false);
   ALDIC_CUDA(cudaGetLastError());
   return OK;
 }
-
-int diffnorm_update(double *old, const double *cur, long long n, double *part, double *res,
+int diffnorm_update(const GridWork &w, double *old, const double *cur, long long n, double *part, double *res,
                     double scale, cudaStream_t st) {
-  const int nb = 148;
-  k_diffnorm_part<<<nb, 256, 0, st>>>(old, cur, n, part, true);
-  k_diffnorm_final<<<1, 256, 0, st>>>(part, nb, res, scale);
+  k_diffnorm<<<148, 256, 0, st>>>(old, cur, n, part, w.ticket, res, scale, true);
+  ALDIC_CUDA(cudaGetLastError());
+  return OK;
+}
+int fe_tail(const GridWork &w, int M, int N, double h, const double *U1, const double *U2, double *F1, double *F2,
+            double *ud, double *vd, bool keep, double *U2old, double *part, double *res, double scale,
+            cudaStream_t st) {
+  const FeTail A{U1, U2, F1, F2, ud, vd, U2old, keep, part, res, w.ticket, scale};
+  k_fe_tail<<<blocks_for((long long)M * N), 256, 0, st>>>(M, N, h, A);
   ALDIC_CUDA(cudaGetLastError());
   return OK;
 }

@@ -113,6 +113,7 @@ struct GridWork {
   int max_blocks;
   int *gate = nullptr;   // k_local.cu's {gate, ticket}; the ticket is 0 between launches
   double *tmp = nullptr; // 12 M N doubles no solver touches
+  unsigned int *ticket = nullptr;  // of the norms' last block; 0 between launches
 };
 enum GridOp { OP_FE = 0, OP_GRIDFIT = 1, OP_INPAINT = 2, OP_CSR = 3, OP_FD = 4 };
 
@@ -301,16 +302,22 @@ int vsub(const double *a, const double *b, double *out, long long n, cudaStream_
 // o1 = a1 - b1, o2 = a2 - b2 in one launch
 int vsub2(const double *a1, const double *b1, double *o1, long long n1, const double *a2,
           const double *b2, double *o2, long long n2, cudaStream_t st);
-// ||a - b||_2 into *res (deterministic)
 // the beta sweep's errors |U1 - U2_c| -> err[c], |F1 - F2_c| -> err[6 + c] for
 // the nc <= 6 FE candidates in fields (2c, 2c + 1) of x; part holds npart doubles
 int sweep_err(int M, int N, int nc, double h, const double *x, const double *U1,
               const double *F1, double *part, int npart, double *err, cudaStream_t st);
-int vdiffnorm(const double *a, const double *b, long long n, double *part, double *res,
+// *res = |a - b| (part: 148 doubles; the same bits every time)
+int vdiffnorm(const GridWork &w, const double *a, const double *b, long long n, double *part, double *res,
               cudaStream_t st);
-// res = |old - cur| * scale (part: 148 doubles), and old <- cur in the same pass
-int diffnorm_update(double *old, const double *cur, long long n, double *part, double *res,
+// res = |old - cur| * scale, and old <- cur in the same pass
+int diffnorm_update(const GridWork &w, double *old, const double *cur, long long n, double *part, double *res,
                     double scale, cudaStream_t st);
+// after a finite-element global step: F1 <- F2 (if keep), F2 = strain of U2, ud =
+// F2 - F1, vd = U2 - U1, and where res is given *res = |U2old - U2| * scale with
+// U2old <- U2 (part: 1184 doubles)
+int fe_tail(const GridWork &w, int M, int N, double h, const double *U1, const double *U2, double *F1, double *F2,
+            double *ud, double *vd, bool keep, double *U2old, double *part, double *res, double scale,
+            cudaStream_t st);
 
 // ---- multigrid integer search (k_searchmg.cu, funIntegerSearchMg.m)
 struct MgWork {

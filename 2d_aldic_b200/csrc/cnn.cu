@@ -142,60 +142,92 @@ __global__ void k_loss(const float *__restrict__ out, const float *__restrict__ 
   if ((threadIdx.x & 31) == 0 && l != 0.0) atomicAdd(loss, l / B);
 }
 
-// output-layer backward: dW, db (thread per (o, k) / o), dz = (dout . W) * (y > 0)
-__global__ void k_fc5_back(const float *__restrict__ dout, const bf16 *__restrict__ y4,
-                           const float *__restrict__ W5, int B, float *__restrict__ gW5,
-                           float *__restrict__ gb5, bf16 *__restrict__ dz4) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long nW = (long long)cnn::NOUT * cnn::K5;
-  if (t < nW) {
-    const int o = (int)(t / cnn::K5), k = (int)(t - (long long)o * cnn::K5);
-    float s = 0.f;
-    for (int b = 0; b < B; ++b) s += dout[b * cnn::NOUT + o] * __bfloat162float(y4[(long long)b * cnn::K5 + k]);
-    gW5[t] = s;
-  } else if (t < nW + cnn::NOUT) {
-    const int o = (int)(t - nW);
-    float s = 0.f;
-    for (int b = 0; b < B; ++b) s += dout[b * cnn::NOUT + o];
-    gb5[o] = s;
-  } else if (t < nW + cnn::NOUT + (long long)B * cnn::K5) {
-    const long long q = t - nW - cnn::NOUT;
-    const int b = (int)(q / cnn::K5), k = (int)(q - (long long)b * cnn::K5);
-    float s = 0.f;
-    for (int o = 0; o < cnn::NOUT; ++o) s += dout[b * cnn::NOUT + o] * W5[o * cnn::K5 + k];
-    dz4[q] = __float2bfloat16_rn(__bfloat162float(y4[q]) > 0.f ? s : 0.f);
+// output-layer backward.  Blocks 0 .. 31: dW of output o and 64 of its inputs, a
+// quarter of the batch a thread, the quarters added in order (db of o likewise); the
+// others: dz = (dout . W) *
+// (y > 0), an entry a thread.
+constexpr int kBackW = cnn::NOUT * cnn::K5 / 64;
+__global__ void __launch_bounds__(256)
+    k_fc5_back(const float *__restrict__ dout, const bf16 *__restrict__ y4, const float *__restrict__ W5, int B,
+               float *__restrict__ gW5, float *__restrict__ gb5, bf16 *__restrict__ dz4) {
+  __shared__ float sh[2][256];
+  if (blockIdx.x < kBackW) {
+    const int o = blockIdx.x / (cnn::K5 / 64), k = blockIdx.x % (cnn::K5 / 64) * 64 + (threadIdx.x & 63);
+    const int part = threadIdx.x >> 6, per = (B + 3) / 4, b1 = min(B, (part + 1) * per);
+    float s = 0.f, t = 0.f;
+#pragma unroll 16
+    for (int b = part * per; b < b1; ++b) {
+      const float d = dout[b * cnn::NOUT + o];
+      s += d * __bfloat162float(y4[(long long)b * cnn::K5 + k]);
+      t += d;
+    }
+    sh[0][threadIdx.x] = s;
+    sh[1][threadIdx.x] = t;
+    __syncthreads();
+    if (part) return;
+    for (int e = 1; e < 4; ++e) {
+      s += sh[0][64 * e + threadIdx.x];
+      t += sh[1][64 * e + threadIdx.x];
+    }
+    gW5[o * cnn::K5 + k] = s;
+    if (k == 0) gb5[o] = t;
+    return;
   }
+  const long long q = (long long)(blockIdx.x - kBackW) * 256 + threadIdx.x;
+  if (q >= (long long)B * cnn::K5) return;
+  const int b = (int)(q / cnn::K5), k = (int)(q - (long long)b * cnn::K5);
+  float s = 0.f;
+  for (int o = 0; o < cnn::NOUT; ++o) s += dout[b * cnn::NOUT + o] * W5[o * cnn::K5 + k];
+  dz4[q] = __float2bfloat16_rn(__bfloat162float(y4[q]) > 0.f ? s : 0.f);
 }
 
-// column sums of a rows x cols bf16 matrix (bias gradients), fixed order
-__global__ void k_colsum(const bf16 *__restrict__ a, long long rows, int cols, float *__restrict__ out) {
-  const int c = blockIdx.x;
-  __shared__ float red[32];
-  float s = 0.f;
-  for (long long r = threadIdx.x; r < rows; r += blockDim.x) s += __bfloat162float(a[r * cols + c]);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    out[c] = t;
+// Column sums of a rows x cols bf16 matrix (bias gradients): a block a run of
+// rows, a thread two columns of every 512 / cols-th row, the blocks' sums added in
+// their order by k_splitk_sum.  (A block a column read two bytes a row: 26 us for
+// 32768 x 128, 9 us now.)
+constexpr int kColBlocks = 128;
+__global__ void __launch_bounds__(256)
+    k_colsum(const bf16 *__restrict__ a, long long rows, int cols, float *__restrict__ part) {
+  __shared__ float2 sh[256];
+  const int pairs = cols / 2, each = 256 / pairs, c = threadIdx.x % pairs, r0 = threadIdx.x / pairs;
+  const long long per = (rows + gridDim.x - 1) / gridDim.x;
+  const long long y0 = blockIdx.x * per, y1 = y0 + per < rows ? y0 + per : rows;
+  float2 s = make_float2(0.f, 0.f);
+#pragma unroll 8
+  for (long long y = y0 + r0; y < y1; y += each) {
+    const float2 v = __bfloat1622float2(*(const __nv_bfloat162 *)(a + y * cols + 2 * c));
+    s.x += v.x;
+    s.y += v.y;
   }
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  if (r0) return;
+  for (int e = 1; e < each; ++e) {
+    s.x += sh[e * pairs + c].x;
+    s.y += sh[e * pairs + c].y;
+  }
+  *(float2 *)(part + (long long)blockIdx.x * cols + 2 * c) = s;
 }
 
 __global__ void k_splitk_sum(const float *__restrict__ part, int splits, long long n, float *__restrict__ out) {
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x) {
     float s = 0.f;
+#pragma unroll 32
     for (int z = 0; z < splits; ++z) s += part[(long long)z * n + k];
     out[k] = s;
   }
 }
 
-// Adam (beta1 0.9, beta2 0.999, eps 1e-8) on an FP32 block; optional bf16 copy
+// Adam (beta1 0.9, beta2 0.999, eps 1e-8) on the packed FP32 parameters, and the
+// bf16 copies of the tensor-core layers' weights: those of layer l lie from off[l]
+// on, in the copy from to[l] on
+struct AdamLayers {
+  long long off[cnn::NL - 1], len[cnn::NL - 1], to[cnn::NL - 1];
+};
 __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
-                       float *__restrict__ v, long long n, float lr, float c1, float c2,
-                       bf16 *__restrict__ wb) {
+                       float *__restrict__ v, long long n, float lr, float c1, float c2, bf16 *__restrict__ wb,
+                       const AdamLayers L) {
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x) {
     const float gk = g[k];
@@ -204,7 +236,9 @@ __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float
     v[k] = vk;
     const float wk = w[k] - lr * (mk * c1) / (sqrtf(vk * c2) + 1e-8f);
     w[k] = wk;
-    if (wb) wb[k] = __float2bfloat16_rn(wk);
+#pragma unroll
+    for (int l = 0; l < cnn::NL - 1; ++l)
+      if (k >= L.off[l] && k < L.off[l] + L.len[l]) wb[L.to[l] + k - L.off[l]] = __float2bfloat16_rn(wk);
   }
 }
 
@@ -238,7 +272,12 @@ struct aldic_cnn {
   int maxB = 0, maxTrain = 0;
   long long steps = 0;
   DevBuf prm, grad, adm, adv, wbf;  // packed FP32 parameters, gradients, Adam moments; bf16 W1-W3
-  DevBuf xin, x0, e1, e2, corr, y3, out, dout, dz3, dcorr, de2, dz1, part, err, loss, tgt;
+  // the gradient of W3 (nine tenths of all) leaves on its own stream from the
+  // moment it is there
+  cudaStream_t copies = nullptr;
+  cudaEvent_t w3_ready = nullptr;
+  DevBuf xin, x0, e1, e2, corr, y3, out, dout, dz3, dcorr, de2, dz1, part, err, tgt;
+  double *loss_ptr() const { return (double *)(err.as<char>() + 8); }
   float *W(int l) const { return prm.as<float>() + off_w(l); }
   float *Bv(int l) const { return prm.as<float>() + off_w(l) + cnn::NW[l]; }
   float *gW(int l) const { return grad.as<float>() + off_w(l); }
@@ -302,10 +341,6 @@ constexpr float kCorrScale = 0.08838834764831845f;  // 1 / sqrt(128)
 int forward(aldic_cnn *c, const void *x, int B, bool train, float *out, cudaStream_t st) {
   const long long b = B;
   int rc;
-  if (train) {
-    k_split<<<nblk(b * cnn::P * cnn::P), 256, 0, st>>>((const bf16 *)x, b, c->x0.as<bf16>());
-    ALDIC_CUDA(cudaGetLastError());
-  }
   const int splits = net_dense_splits(B);
   if (splits > 1 && (rc = c->part.ensure(sizeof(float) * b * cnn::F3 * splits))) return rc;
   if ((rc = net_encode(x, B, c->Wb(0), c->Bv(0), c->Wb(1), c->Bv(1), kCorrScale, c->corr.p,
@@ -318,25 +353,35 @@ int forward(aldic_cnn *c, const void *x, int B, bool train, float *out, cudaStre
 // dW = A . B^T product with split-K, summed into g
 int weight_grad(aldic_cnn *c, const GemmSrc &A, const GemmSrc &Bm, float *g, cudaStream_t st) {
   const long long kt = (A.kdim + 63) / 64;
-  int splits = (int)(kt / 8);
-  splits = splits < 1 ? 1 : (splits > 64 ? 64 : splits);
+  int splits = (int)(kt / 4);
+  splits = splits < 1 ? 1 : (splits > 128 ? 128 : splits);
   const long long n = A.rows * Bm.rows;
   int rc;
-  if ((rc = c->part.ensure(sizeof(float) * n * splits))) return rc;
-  GemmDst d = dst(c->part.p, A.rows, Bm.rows, Bm.rows, 1, nullptr, 0);
+  if (splits > 1 && (rc = c->part.ensure(sizeof(float) * n * splits))) return rc;
+  GemmDst d = dst(splits > 1 ? c->part.p : g, A.rows, Bm.rows, Bm.rows, 1, nullptr, 0);
   d.split_stride = n;
   if ((rc = gemm_bf16(A, Bm, d, splits, c->err.as<int>(), st))) return rc;
-  k_splitk_sum<<<nblk(n), 256, 0, st>>>(c->part.as<float>(), splits, n, g);
+  if (splits > 1) k_splitk_sum<<<nblk(n), 256, 0, st>>>(c->part.as<float>(), splits, n, g);
   ALDIC_CUDA(cudaGetLastError());
   return OK;
 }
 
-int backward(aldic_cnn *c, int B, cudaStream_t st) {
+// g = column sums of the rows x cols matrix a
+int bias_grad(aldic_cnn *c, const void *a, long long rows, int cols, float *g, cudaStream_t st) {
+  int rc;
+  const int blocks = rows < kColBlocks ? (int)rows : kColBlocks;
+  if ((rc = c->part.ensure(sizeof(float) * kColBlocks * cols))) return rc;
+  k_colsum<<<blocks, 256, 0, st>>>((const bf16 *)a, rows, cols, c->part.as<float>());
+  k_splitk_sum<<<nblk(cols), 256, 0, st>>>(c->part.as<float>(), blocks, cols, g);
+  ALDIC_CUDA(cudaGetLastError());
+  return OK;
+}
+
+int backward(aldic_cnn *c, const void *x, int B, cudaStream_t st) {
   int *err = c->err.as<int>();
   const long long b = B, cells = 2 * b * cnn::CELLS, fs = (long long)cnn::CELLS * cnn::C2;
   int rc;
-  const long long t5 = (long long)cnn::NOUT * cnn::K5 + cnn::NOUT + b * cnn::K5;
-  k_fc5_back<<<(unsigned)((t5 + 255) / 256), 256, 0, st>>>(c->dout.as<float>(), c->y3.as<bf16>(),
+  k_fc5_back<<<(unsigned)(kBackW + (b * cnn::K5 + 255) / 256), 256, 0, st>>>(c->dout.as<float>(), c->y3.as<bf16>(),
                                                            c->W(3), B, c->gW(3), c->gB(3),
                                                            c->dz3.as<bf16>());
   ALDIC_CUDA(cudaGetLastError());
@@ -344,7 +389,8 @@ int backward(aldic_cnn *c, int B, cudaStream_t st) {
   if ((rc = weight_grad(c, src(c->dz3.p, GEMM_TRANS, cnn::F3, b, cnn::F3),
                         src(c->corr.p, GEMM_TRANS, cnn::K3, b, cnn::K3), c->gW(2), st)))
     return rc;
-  k_colsum<<<cnn::F3, 256, 0, st>>>(c->dz3.as<bf16>(), b, cnn::F3, c->gB(2));
+  if (cudaEventRecord(c->w3_ready, st) != cudaSuccess) return E_CUDA;
+  if ((rc = bias_grad(c, c->dz3.p, b, cnn::F3, c->gB(2), st))) return rc;
   if ((rc = gemm_bf16(src(c->dz3.p, GEMM_ROW, b, cnn::F3, cnn::F3),
                       src(c->Wb(2), GEMM_TRANS, cnn::K3, cnn::F3, cnn::K3),
                       dst(c->dcorr.p, b, cnn::K3, cnn::K3, 0, nullptr, 0), 1, err, st)))
@@ -367,37 +413,35 @@ int backward(aldic_cnn *c, int B, cudaStream_t st) {
   if ((rc = weight_grad(c, src(c->de2.p, GEMM_TRANS, cnn::C2, cells, cnn::C2),
                         src(c->e1.p, GEMM_TRANS, cnn::K2, cells, cnn::C1), c->gW(1), st)))
     return rc;
-  k_colsum<<<cnn::C2, 256, 0, st>>>(c->de2.as<bf16>(), cells, cnn::C2, c->gB(1));
+  if ((rc = bias_grad(c, c->de2.p, cells, cnn::C2, c->gB(1), st))) return rc;
   if ((rc = gemm_bf16(src(c->de2.p, GEMM_ROW, cells, cnn::C2, cnn::C2),
                       src(c->Wb(1), GEMM_TRANS, cnn::K2, cnn::C2, cnn::K2),
                       dst(c->dz1.p, cells, cnn::C1, cnn::C1, 0, nullptr, 0, GEMM_ROW, c->e1.p), 1, err,
                       st)))
     return rc;
   // E1
+  k_split<<<nblk(b * cnn::P * cnn::P), 256, 0, st>>>((const bf16 *)x, b, c->x0.as<bf16>());
+  ALDIC_CUDA(cudaGetLastError());
   if ((rc = weight_grad(c, src(c->dz1.p, GEMM_TRANS, cnn::C1, cells, cnn::C1),
                         src(c->x0.p, GEMM_PATCHT, cnn::K1, cells, 0, cnn::P, cnn::P, 1, cnn::PS),
                         c->gW(0), st)))
     return rc;
-  k_colsum<<<cnn::C1, 256, 0, st>>>(c->dz1.as<bf16>(), cells, cnn::C1, c->gB(0));
-  ALDIC_CUDA(cudaGetLastError());
-  return OK;
+  return bias_grad(c, c->dz1.p, cells, cnn::C1, c->gB(0), st);
 }
 
 int adam(aldic_cnn *c, float lr, cudaStream_t st) {
   c->steps++;
   const float c1 = 1.f / (1.f - powf(0.9f, (float)c->steps));
   const float c2 = 1.f / (1.f - powf(0.999f, (float)c->steps));
-  for (int l = 0; l < cnn::NL; ++l) {
-    const long long o = aldic_cnn::off_w(l), n = cnn::NW[l] + cnn::NB[l];
-    float *w = c->prm.as<float>() + o;
-    // weights (bf16 copy for the tensor-core layers), then biases
-    k_adam<<<nblk(cnn::NW[l]), 256, 0, st>>>(w, c->grad.as<float>() + o, c->adm.as<float>() + o,
-                                             c->adv.as<float>() + o, cnn::NW[l], lr, c1, c2,
-                                             l < cnn::NL - 1 ? c->Wb(l) : nullptr);
-    k_adam<<<1, 256, 0, st>>>(w + cnn::NW[l], c->grad.as<float>() + o + cnn::NW[l],
-                              c->adm.as<float>() + o + cnn::NW[l], c->adv.as<float>() + o + cnn::NW[l],
-                              n - cnn::NW[l], lr, c1, c2, nullptr);
+  AdamLayers L;
+  for (int l = 0; l < cnn::NL - 1; ++l) {
+    L.off[l] = aldic_cnn::off_w(l);
+    L.len[l] = cnn::NW[l];
+    L.to[l] = c->Wb(l) - c->wbf.as<bf16>();
   }
+  const long long n = cnn::n_params();
+  k_adam<<<nblk(n), 256, 0, st>>>(c->prm.as<float>(), c->grad.as<float>(), c->adm.as<float>(), c->adv.as<float>(), n,
+                                  lr, c1, c2, c->wbf.as<bf16>(), L);
   ALDIC_CUDA(cudaGetLastError());
   return OK;
 }
@@ -409,11 +453,16 @@ int sync_bf16(aldic_cnn *c, cudaStream_t st) {
   return OK;
 }
 
-int check_err(aldic_cnn *c, cudaStream_t st) {
-  int e = 0;
-  ALDIC_CUDA(cudaMemcpyAsync(&e, c->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+// the error word, and the loss that lies beside it
+int check_err(aldic_cnn *c, cudaStream_t st, double *loss = nullptr) {
+  struct {
+    int e, pad;
+    double loss;
+  } h = {};
+  ALDIC_CUDA(cudaMemcpyAsync(&h, c->err.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   ALDIC_CUDA(cudaStreamSynchronize(st));
-  if (e) {
+  if (loss) *loss = h.loss;
+  if (h.e) {
     cudaMemsetAsync(c->err.p, 0, sizeof(int), st);
     set_error("cnn: a tensor-core wait timed out");
     return E_TIMEOUT;
@@ -480,11 +529,17 @@ int aldic_cnn_create(int device, unsigned long long seed, aldic_cnn **out) {
   for (int l = 0; l < cnn::NL - 1; ++l) nwb += cnn::NW[l];
   int rc;
   if ((rc = c->prm.ensure(4 * np)) || (rc = c->grad.ensure(4 * np)) || (rc = c->adm.ensure(4 * np)) ||
-      (rc = c->adv.ensure(4 * np)) || (rc = c->wbf.ensure(2 * nwb)) || (rc = c->err.ensure(64)) ||
-      (rc = c->loss.ensure(64))) {
+      (rc = c->adv.ensure(4 * np)) || (rc = c->wbf.ensure(2 * nwb)) || (rc = c->err.ensure(64))) {
     delete c;
     cudaSetDevice(prev);
     return rc;
+  }
+  if (cudaStreamCreateWithFlags(&c->copies, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->w3_ready, cudaEventDisableTiming) != cudaSuccess) {
+    delete c;
+    cudaSetDevice(prev);
+    set_error("cnn_create: stream creation failed");
+    return E_CUDA;
   }
   // He-normal weights (std sqrt(2 / fan_in)), zero biases, seeded
   std::vector<float> h(np, 0.f);
@@ -520,8 +575,10 @@ int aldic_cnn_destroy(aldic_cnn *c) {
   cudaDeviceSynchronize();
   DevBuf *b[] = {&c->prm, &c->grad, &c->adm, &c->adv, &c->wbf, &c->xin, &c->x0, &c->e1, &c->e2,
                  &c->corr, &c->y3, &c->out, &c->dout, &c->dz3, &c->dcorr, &c->de2, &c->dz1,
-                 &c->part, &c->err, &c->loss, &c->tgt};
+                 &c->part, &c->err, &c->tgt};
   for (auto *x : b) x->release();
+  if (c->copies) cudaStreamDestroy(c->copies);
+  if (c->w3_ready) cudaEventDestroy(c->w3_ready);
   cudaSetDevice(prev);
   delete c;
   return OK;
@@ -573,19 +630,33 @@ int aldic_cnn_train_step(aldic_cnn *c, const void *x, int x_bf16, const float *t
   }
   if (!rc) rc = forward(c, pairs, B, true, c->out.as<float>(), st);
   if (!rc) {
-    cudaMemsetAsync(c->loss.p, 0, sizeof(double), st);
+    cudaMemsetAsync(c->loss_ptr(), 0, sizeof(double), st);
     k_loss<<<(B + 255) / 256, 256, 0, st>>>(c->out.as<float>(), c->tgt.as<float>(), B,
-                                           c->dout.as<float>(), c->loss.as<double>());
-    rc = backward(c, B, st);
+                                           c->dout.as<float>(), c->loss_ptr());
+    rc = backward(c, pairs, B, st);
   }
   if (!rc && lr > 0) rc = adam(c, lr, st);
-  if (!rc && grads)
-    if (cudaMemcpyAsync(grads, c->grad.p, 4 * cnn::n_params(), cudaMemcpyDefault, st) != cudaSuccess) rc = E_CUDA;
+  if (!rc && grads) {
+    // W3's gradient while the rest of the step runs (a copy to pageable memory
+    // takes 0.24 ms and holds this thread, so all else is launched by now), then
+    // what lies before and after it
+    const long long o = aldic_cnn::off_w(2), e = o + cnn::NW[2], n = cnn::n_params();
+    const float *g = c->grad.as<float>();
+    if (cudaStreamWaitEvent(c->copies, c->w3_ready, 0) != cudaSuccess ||
+        cudaMemcpyAsync(grads + o, g + o, 4 * (e - o), cudaMemcpyDefault, c->copies) != cudaSuccess ||
+        cudaMemcpyAsync(grads, g, 4 * o, cudaMemcpyDefault, st) != cudaSuccess ||
+        cudaMemcpyAsync(grads + e, g + e, 4 * (n - e), cudaMemcpyDefault, st) != cudaSuccess ||
+        cudaStreamSynchronize(c->copies) != cudaSuccess) {
+      set_error("cnn_train_step: copying the gradients failed");
+      rc = E_CUDA;
+    }
+  }
   if (!rc && out)
     if (cudaMemcpyAsync(out, c->out.p, 4LL * B * cnn::NOUT, cudaMemcpyDefault, st) != cudaSuccess) rc = E_CUDA;
-  if (!rc && loss)
-    if (cudaMemcpyAsync(loss, c->loss.p, sizeof(double), cudaMemcpyDefault, st) != cudaSuccess) rc = E_CUDA;
-  if (!rc) rc = check_err(c, st);
+  const bool dev = loss && on_device(loss);
+  if (!rc && dev)
+    if (cudaMemcpyAsync(loss, c->loss_ptr(), sizeof(double), cudaMemcpyDefault, st) != cudaSuccess) rc = E_CUDA;
+  if (!rc) rc = check_err(c, st, dev ? nullptr : loss);
   cudaSetDevice(prev);
   return rc;
 }

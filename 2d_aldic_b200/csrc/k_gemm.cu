@@ -2,13 +2,14 @@
 // the learned initial guess: D[M x N] = A[M x K] . B[N x K]^T (+ bias, ReLU,
 // mask), FP32 accumulation in tensor memory.
 //
-// One CTA (4 warps) owns a 128 x BN tile.  Per 64-wide K step both operand
+// One CTA (8 warps) owns a 128 x BN tile.  Per 64-wide K step both operand
 // tiles are staged in shared memory in the K-major 128-byte-swizzle layout
 // (8 rows x 128 B atoms, 16-B chunk c of row r at chunk c ^ (r & 7)); one
 // thread issues four tcgen05.mma (K = 16 each) on shared-memory descriptors
 // and commits them to an mbarrier, while all threads stage the next K step
 // into the other buffer.  The epilogue reads the accumulator with
-// tcgen05.ld (warp w owns TMEM lanes 32w..32w+31 = tile rows) and applies
+// tcgen05.ld (warp w reads TMEM lanes 32 (w % 4) on = tile rows, half of the
+// columns) and applies
 // bias / ReLU / a ReLU mask.  Operands are read through small address
 // generators so that the same kernel serves the forward pass (rows or
 // non-overlapping patch im2col of an NHWC tensor) and both backward
@@ -26,7 +27,7 @@ namespace aldic {
 
 namespace {
 
-constexpr int BM = TC_M, BK = 64, GEMM_THREADS = 128;
+constexpr int BM = TC_M, BK = 64, GEMM_THREADS = 256;
 
 // element address of operand (r, k) for the direct modes (ROW, PATCH)
 __device__ __forceinline__ const __nv_bfloat16 *src_addr(const GemmSrc &S, long long r, long long k) {
@@ -56,20 +57,35 @@ __device__ __forceinline__ void stage(const GemmSrc &S, long long r0, long long 
     }
   } else {
     // transposed operand: element (r, k) is source element (k, r) of a ROW
-    // or PATCH source; 8 consecutive r are one 16-B source chunk
+    // or PATCH source.  A thread takes 8 x 8 elements, a 16-byte chunk of each of
+    // eight k, transposes them in registers and writes a chunk of each of eight r
+    // (element by element this was 64 two-byte stores with bank conflicts, three
+    // quarters of a weight gradient's time).
     GemmSrc T = S;
     T.mode = S.mode == GEMM_TRANS ? GEMM_ROW : GEMM_PATCH;
-    for (int q = tid; q < BK * (R / 8); q += GEMM_THREADS) {
-      const int k = q / (R / 8), g = q - k * (R / 8);
-      const long long gk = k0 + k, gr = r0 + 8 * g;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (gk < S.kdim && gr < S.rows) v = *reinterpret_cast<const uint4 *>(src_addr(T, gk, gr));
-      const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&v);
-      const int c = k >> 3, off = (k & 7) * 2;
+    for (int q = tid; q < (BK / 8) * (R / 8); q += GEMM_THREADS) {
+      const int c = q / (R / 8), g = q - c * (R / 8);
+      const long long gr = r0 + 8 * g;
+      uint4 v[8];
 #pragma unroll
       for (int t = 0; t < 8; ++t) {
-        const int r = 8 * g + t;
-        *reinterpret_cast<__nv_bfloat16 *>(tile + r * 128 + ((c ^ (r & 7)) << 4) + off) = e[t];
+        const long long gk = k0 + 8 * c + t;
+        v[t] = make_uint4(0, 0, 0, 0);
+        if (gk < S.kdim && gr < S.rows) v[t] = *reinterpret_cast<const uint4 *>(src_addr(T, gk, gr));
+      }
+      // word w of v[t]: elements r = 2w, 2w + 1 at k = 8c + t
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const uint32_t e[8] = {(&v[0].x)[w], (&v[1].x)[w], (&v[2].x)[w], (&v[3].x)[w],
+                               (&v[4].x)[w], (&v[5].x)[w], (&v[6].x)[w], (&v[7].x)[w]};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = 8 * g + 2 * w + h;
+          const uint32_t sel = h ? 0x7632 : 0x5410;
+          *reinterpret_cast<uint4 *>(tile + r * 128 + ((c ^ (r & 7)) << 4)) =
+              make_uint4(__byte_perm(e[0], e[1], sel), __byte_perm(e[2], e[3], sel), __byte_perm(e[4], e[5], sel),
+                         __byte_perm(e[6], e[7], sel));
+        }
       }
     }
   }
@@ -173,13 +189,15 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(GemmSrc A, GemmSrc B, Gem
   if (failed) {
     if (tid == 0) atomicExch(err, 3);
   } else {
-    // epilogue: row r = 32 * warp + lane of the tile
-    const long long m = m0 + 32 * warp + lane;
+    // epilogue: row r = 32 * (warp % 4) + lane of the tile, the upper warps its
+    // right half
+    const int wq = warp & 3;
+    const long long m = m0 + 32 * wq + lane;
     const bool base_aligned = ((uintptr_t)D.p & 15) == 0 && ((uintptr_t)D.mask & 15) == 0;
-    for (int c0 = 0; c0 < BN; c0 += 16) {
+    for (int c0 = (warp >> 2) * (BN / 2), ce = c0 + BN / 2; c0 < ce; c0 += 16) {
       float v[16];
       if (nk > 0) {
-        tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
+        tmem_ld16(tmem + ((uint32_t)(32 * wq) << 16) + (uint32_t)c0, v);
       } else {
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = 0.f;
@@ -291,8 +309,12 @@ int gemm_bf16(const GemmSrc &A, const GemmSrc &B, const GemmDst &D, int splits, 
   ALDIC_CHECK(batches == 1 || (A.bstride % 8 == 0 && B.bstride % 8 == 0), E_ARG,
               "gemm: batch strides must keep 16-byte alignment");
   ALDIC_CHECK(D.mode == GEMM_ROW || (D.ps > 0 && D.C > 0), E_ARG, "gemm: bad output geometry");
-  if (B.rows <= 64) return launch_gemm<64>(A, B, D, splits, batches, err, st);
-  if (B.rows <= 128) return launch_gemm<128>(A, B, D, splits, batches, err, st);
+  // the widest tile that leaves no SM idle: a training step's products of 256 x
+  // 4096 took 74 us on 32 CTAs of 128 x 256 and 26 us on 128 of 128 x 64
+  const long long rows = (A.rows + BM - 1) / BM * (batches > 1 ? batches : splits);
+  auto fills = [&](int bn) { return rows * ((B.rows + bn - 1) / bn) >= 148; };
+  if (B.rows <= 64 || !fills(128)) return launch_gemm<64>(A, B, D, splits, batches, err, st);
+  if (B.rows <= 128 || !fills(256)) return launch_gemm<128>(A, B, D, splits, batches, err, st);
   return launch_gemm<256>(A, B, D, splits, batches, err, st);
 }
 

@@ -1348,6 +1348,17 @@ int launch_big(const void *f, const void *g, const SearchGeom &G, double *x, dou
   return OK;
 }
 
+// Whether 8-bit tiles are the faster way for a geometry that has them: a tile's
+// cost goes with the shifts times the pixels a point adds (step^2 and the halo), a
+// point's on the tensor cores hardly changes with the shifts.  Both measured at 1100
+// x 900, tiles against tensor cores in us: subset 32, step 16, zone 8 210/221, 16
+// 292/245, 24 489/266; step 8, zone 16 429/641, 24 671/715, 40 1399/1015; subset 24,
+// step 8, zone 24 614/661; subset 16, step 8, zone 20 462/588; step 4, zone 12
+// 623/1640: even where shifts x step^3 is 1.6 to 1.9 million, 2.4 for subset 16.
+bool tiles_pay(const SearchGeom &G) {
+  return (double)G.cr * G.cc * G.step * G.step * G.step < (G.w < 24 ? 2.5e6 : 1.85e6);
+}
+
 template <typename T>
 int launch_search(const void *f, const void *g, const SearchGeom &G, double *x, double *y,
                   double *u, double *v, double *cc, double *pce, double *ppe, cudaStream_t st,
@@ -1361,15 +1372,15 @@ int launch_search(const void *f, const void *g, const SearchGeom &G, double *x, 
   if (threads > 512) threads = 512;
   const int npts = G.nx * G.ny;
   if (npts == 0) return OK;
-  // 8 bit by tiles where one is built for the geometry (2048 x 2048, 32/8/+-16:
-  // 1.2 ms against 2.6 ms point by point on the tensor cores), else the tensor
-  // cores whatever the geometry: against the dot product kernels before, 1100 x
+  // 8 bit by tiles where one is built for the geometry and pays (2048 x 2048,
+  // 32/8/+-16: 1.2 ms against 2.6 ms point by point on the tensor cores), else the
+  // tensor cores whatever the geometry: against the dot product kernels before, 1100 x
   // 900, subset/step/zone 28/7/13 8 bit 0.68 against 0.76 ms, 50/25/30 0.22
   // against 0.44; 16 bit 16/8/10 0.53 against 0.66, 50/25/30 0.26 against 1.16;
   // 320 x 340, 20/10/20 8 bit 0.119 against 0.127 ms
   if (sizeof(T) <= 2 && search_mma_fits(G, sizeof(T))) {
     bool tiled = false;
-    if (sizeof(T) == 1 && sw) {
+    if (sizeof(T) == 1 && sw && tiles_pay(G)) {
       const int rc = tile_search((const uint8_t *)f, (const uint8_t *)g, G, *sw, x, y, u, v, cc, st, &tiled);
       if (rc) return rc;
     }

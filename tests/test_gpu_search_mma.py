@@ -49,6 +49,14 @@ def test_plan_edges_bit_exact(aldic, oracle, synth, dtype, w, step, s):
     _check(aldic, oracle, *_images(oracle, synth, dtype, W, H, 51), w, step, s)
 
 
+@pytest.mark.parametrize("w,step,s", [(32, 16, 9), (32, 16, 10), (32, 8, 28), (32, 8, 29), (24, 8, 29), (16, 8, 33),
+                                      (16, 8, 34)])
+def test_tiles_or_points_bit_exact(aldic, oracle, synth, w, step, s):
+    """8-bit geometries with a tile on either side of the line up to which the tiles pay."""
+    W, H = 2 * w + 2 * s + 9 * step + 3, 2 * w + 2 * s + 8 * step + 5
+    _check(aldic, oracle, *_images(oracle, synth, np.uint8, W, H, 57), w, step, s)
+
+
 @pytest.mark.parametrize("level", [0, 77, 255])
 @pytest.mark.parametrize("dtype", [np.uint8, np.uint16])
 def test_flat_and_tied_regions_bit_exact(aldic, oracle, synth, dtype, level):

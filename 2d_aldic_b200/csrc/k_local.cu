@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(kFillThreads, 2) k_fill_tile(const __grid_cons
       S.r[at[q]] = r[q];
     }
   __syncthreads();
-  double gam = 0.0, alpha = 0.0, beta = 0.0, bnorm = 0.0;
+  double alpha = 0.0, beta = 0.0, gi = 0.0, ai = 0.0, bnorm = 0.0;
   bool done = false;
   for (int it = 0; it < kFillMaxit; ++it) {
     apply(r, w);
@@ -487,13 +487,13 @@ __global__ void __launch_bounds__(kFillThreads, 2) k_fill_tile(const __grid_cons
       done = true;
       break;
     }
-    if (it == 0) {
-      alpha = tot[0] / tot[1];
-    } else {
-      beta = tot[0] / gam;
-      alpha = tot[0] / (tot[1] - beta * tot[0] / alpha);
-    }
-    gam = tot[0];
+    // gi, ai: 1 / gamma and 1 / alpha of the iteration before, formed beside its
+    // alpha, so one division is in the chain
+    beta = it == 0 ? 0.0 : tot[0] * gi;
+    const double t = tot[1] - beta * tot[0] * ai;
+    alpha = tot[0] / t;
+    gi = 1.0 / tot[0];
+    ai = t * gi;
 #pragma unroll
     for (int q = 0; q < kFillPer; ++q)
       if (q * kFillThreads < cnt) {

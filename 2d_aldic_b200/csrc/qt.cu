@@ -613,48 +613,78 @@ __device__ __forceinline__ double grads(const double dk[8], const double de[8], 
   return det;
 }
 
-// one thread per (element, local row a): row a of the scalar 8x8 element
+// Row a of the scalar 8x8 element
 // matrix sum_gp detJ (beta grad Na . grad Nb + mu Na Nb) and the row's
 // right-hand sides (the duals are multiplied by zero in the reference)
-__global__ void k_qt_elem(int ne, const int *__restrict__ E, const double *__restrict__ cx,
-                          const double *__restrict__ cy, double beta, double mu,
-                          const double *__restrict__ U, const double *__restrict__ F,
-                          double *__restrict__ ke, double *__restrict__ be) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= 8LL * ne) return;
-  const int e = (int)(t >> 3), a = (int)(t & 7);
-  int nd[8];
-  double px[8], py[8], d[4];
+// 32 elements a CTA.  First a thread per element and Gauss point: shape functions,
+// gradients, Jacobian and the point's U, to shared memory; then a thread per
+// element and node: its row of the matrix and its two entries of the right-hand side
+// over the four points in their order.  (With a thread per row forming everything
+// for itself, eight times over, 51 us at 15000 elements; 18 us.)
+constexpr int kElemCta = 32;
+struct ElemPoint {
+  double N[8], dx[8], dy[8], J, uu, vv;
+};
+__global__ void __launch_bounds__(8 * kElemCta)
+    k_qt_elem(int ne, const int *__restrict__ E, const double *__restrict__ cx,
+              const double *__restrict__ cy, double beta, double mu,
+              const double *__restrict__ U, const double *__restrict__ F,
+              double *__restrict__ ke, double *__restrict__ be) {
+  extern __shared__ __align__(16) unsigned char elem_raw[];
+  ElemPoint *pts = (ElemPoint *)elem_raw;  // [element][point]
+  const int e0 = blockIdx.x * kElemCta;
+  if (threadIdx.x < 4 * kElemCta) {
+    const int e = e0 + threadIdx.x / 4, g = threadIdx.x & 3;
+    if (e < ne) {
+      int nd[8];
+      double px[8], py[8], d[4];
 #pragma unroll
-  for (int s = 0; s < 8; ++s) {
-    nd[s] = E[e * 8 + s];
-    px[s] = nd[s] >= 0 ? cx[nd[s]] : 0.0;
-    py[s] = nd[s] >= 0 ? cy[nd[s]] : 0.0;
-  }
+      for (int s = 0; s < 8; ++s) {
+        nd[s] = E[e * 8 + s];
+        px[s] = nd[s] >= 0 ? cx[nd[s]] : 0.0;
+        py[s] = nd[s] >= 0 ? cy[nd[s]] : 0.0;
+      }
 #pragma unroll
-  for (int s = 0; s < 4; ++s) d[s] = nd[4 + s] >= 0 ? 1.0 : 0.0;
-  double K[8] = {0, 0, 0, 0, 0, 0, 0, 0}, bu = 0, bv = 0;
-  if (nd[a] >= 0) {
-    const int ka = nd[a];
-    const double F0 = F[4 * ka], F1 = F[4 * ka + 1], F2 = F[4 * ka + 2], F3 = F[4 * ka + 3];
-#pragma unroll 1
-    for (int g = 0; g < 4; ++g) {
+      for (int s = 0; s < 4; ++s) d[s] = nd[4 + s] >= 0 ? 1.0 : 0.0;
       const double ksi = (g & 1) ? kG : -kG, eta = (g & 2) ? kG : -kG;
       double N[8], dk[8], de[8], dx[8], dy[8];
       shape8(ksi, eta, d, N, dk, de);
-      const double J = grads(dk, de, px, py, dx, dy);
+      ElemPoint &P = pts[threadIdx.x];
+      P.J = grads(dk, de, px, py, dx, dy);
       double uu = 0, vv = 0;
 #pragma unroll
-      for (int s = 0; s < 8; ++s)
+      for (int s = 0; s < 8; ++s) {
+        P.N[s] = N[s];
+        P.dx[s] = dx[s];
+        P.dy[s] = dy[s];
         if (nd[s] >= 0) {
           uu += N[s] * U[2 * nd[s]];
           vv += N[s] * U[2 * nd[s] + 1];
         }
+      }
+      P.uu = uu;
+      P.vv = vv;
+    }
+  }
+  __syncthreads();
+  const int el = threadIdx.x >> 3, a = threadIdx.x & 7, e = e0 + el;
+  if (e >= ne) return;
+  double K[8] = {0, 0, 0, 0, 0, 0, 0, 0}, bu = 0, bv = 0;
+  const int ka = E[e * 8 + a];
+  if (ka >= 0) {
+    const double F0 = F[4 * ka], F1 = F[4 * ka + 1], F2 = F[4 * ka + 2], F3 = F[4 * ka + 3];
+    bool has[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) has[s] = E[e * 8 + s] >= 0;
+#pragma unroll 1
+    for (int g = 0; g < 4; ++g) {
+      const ElemPoint &P = pts[4 * el + g];
+      const double Na = P.N[a], dxa = P.dx[a], dya = P.dy[a], J = P.J;
 #pragma unroll
       for (int s = 0; s < 8; ++s)
-        if (nd[s] >= 0) K[s] += J * (beta * (dx[a] * dx[s] + dy[a] * dy[s]) + mu * N[a] * N[s]);
-      bu += J * (beta * (dx[a] * F0 + dy[a] * F2) + mu * N[a] * uu);
-      bv += J * (beta * (dx[a] * F1 + dy[a] * F3) + mu * N[a] * vv);
+        if (has[s]) K[s] += J * (beta * (dxa * P.dx[s] + dya * P.dy[s]) + mu * Na * P.N[s]);
+      bu += J * (beta * (dxa * F0 + dya * F2) + mu * Na * P.uu);
+      bv += J * (beta * (dxa * F1 + dya * F3) + mu * Na * P.vv);
     }
   }
 #pragma unroll
@@ -1047,7 +1077,7 @@ int qt_subpb2(aldic_qt_mesh &m, GridWork &w, double beta, double mu, const doubl
   if ((rc = qt_upload(m, st))) return rc;
   const int n = m.n, ne = m.ne;
   const double *cx = m.d_coords.as<double>(), *cy = cx + n;
-  k_qt_elem<<<nblk(8LL * ne), 256, 0, st>>>(ne, m.d_elems.as<int>(), cx, cy, beta, mu, U, F,
+  k_qt_elem<<<(ne + kElemCta - 1) / kElemCta, 8 * kElemCta, kElemCta * 4 * sizeof(ElemPoint), st>>>(ne, m.d_elems.as<int>(), cx, cy, beta, mu, U, F,
                                             m.d_ke.as<double>(), m.d_be.as<double>());
   k_qt_gather<<<nblk(n), 256, 0, st>>>(n, m.d_iptr.as<int>(), m.d_inc.as<int>(), m.d_ipos.as<int>(),
                                        m.d_row.as<int>(), m.d_ke.as<double>(), m.d_be.as<double>(),
@@ -1072,7 +1102,7 @@ int qt_subpb2_sweep(aldic_qt_mesh &m, GridWork &w, const double beta[3], double 
   // stiffness part (beta 1, mu 0) into d_val and b fields 0-1, mass part
   // (beta 0, mu 1) into d_valM and b fields 2-3
   for (int part = 0; part < 2; ++part) {
-    k_qt_elem<<<nblk(8LL * ne), 256, 0, st>>>(ne, m.d_elems.as<int>(), cx, cy, part ? 0.0 : 1.0,
+    k_qt_elem<<<(ne + kElemCta - 1) / kElemCta, 8 * kElemCta, kElemCta * 4 * sizeof(ElemPoint), st>>>(ne, m.d_elems.as<int>(), cx, cy, part ? 0.0 : 1.0,
                                               part ? 1.0 : 0.0, U, F, m.d_ke.as<double>(),
                                               m.d_be.as<double>());
     k_qt_gather<<<nblk(n), 256, 0, st>>>(n, m.d_iptr.as<int>(), m.d_inc.as<int>(),

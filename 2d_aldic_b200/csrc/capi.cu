@@ -903,9 +903,7 @@ int aldic_subpb2(aldic_ctx *c, int M, int N, double step, double beta, double mu
       (rc = arg_out(c, Uhat, 2 * n, ao)))
     return rc;
   if ((rc = fdm_ensure(c->fdm, FDM_FE, M, N, step, c->stream))) return rc;
-  if ((rc = fe_rhs(c->gw, M, N, step, beta, mu, au.dev, af.dev, aud.dev, avd.dev, c->stream)))
-    return rc;
-  if ((rc = fdm_solve(c->fdm, 2, c->gw.b, c->gw.x, c->gw.r, mu, beta, nullptr, nullptr, c->stream, ao.dev)))
+  if ((rc = fe_solve(c->fdm, c->gw, step, beta, mu, nullptr, au.dev, af.dev, aud.dev, avd.dev, ao.dev, c->stream)))
     return rc;
   arg_back(c, ao);
   return finish(c, true);  // the direct solve has no status to read
@@ -1488,20 +1486,16 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
   // interior nodes (main_ALDIC.m:243-278): solve into fields f0, f0 + 1,
   // store U2, strain F2
   const bool fd = p->subpb2_fd != 0;
-  auto rhs = [&](double beta, const double *beta_ptr, int f0, const double *F) {
-    return fd ? fd_rhs(c->gw, M, N, h, beta, mu, B.U1, F, B.udual, B.vdual, st, beta_ptr, f0)
-              : fe_rhs(c->gw, M, N, h, beta, mu, B.U1, F, B.udual, B.vdual, st, beta_ptr, f0);
-  };
   // strain, duals, update norm and F1's copy of a global step in one launch; the
   // finite-difference step and smoothing keep them apart
   const bool tail = !fd && !p->smooth;
   // the direct fast-diagonalisation solve (fdm.cu; bases set up before capture)
   // of the system at *beta with Subproblem 1's strains F into U2
   auto solve = [&](const double *beta_ptr, const double *F) {
-    int rc2 = rhs(0, beta_ptr, 0, F);
-    if (!rc2)
-      rc2 = fdm_solve(c->fdm, 2, c->gw.b, c->gw.x, c->gw.r, mu, 0.0, nullptr, beta_ptr, st, fd ? nullptr : B.U2);
-    return rc2 || !fd ? rc2 : fd_store(c->gw, M, N, B.U1, B.U2, st, 0);
+    if (!fd) return fe_solve(c->fdm, c->gw, h, 0.0, mu, beta_ptr, B.U1, F, B.udual, B.vdual, B.U2, st);
+    int rc2 = fd_rhs(c->gw, M, N, h, 0.0, mu, B.U1, F, B.udual, B.vdual, st, beta_ptr, 0);
+    if (!rc2) rc2 = fdm_solve(c->fdm, 2, c->gw.b, c->gw.x, c->gw.r, mu, 0.0, nullptr, beta_ptr, st);
+    return rc2 ? rc2 : fd_store(c->gw, M, N, B.U1, B.U2, st, 0);
   };
   auto strain = [&]() {
     return fd ? fd_strain(M, N, h, B.U2, B.F2, st) : nodal_strain(M, N, h, B.U2, B.F2, st);
@@ -1518,7 +1512,8 @@ int frame_device(aldic_ctx *c, const aldic_frame_params *p, const FrameBufs &B, 
     double be[12], b6[6];
     for (int k = 0; k < 6; ++k) {
       be[2 * k] = be[2 * k + 1] = b6[k] = bl[k] * base;
-      if (fd && (rc = rhs(bl[k] * base, nullptr, 2 * k, B.F1))) return rc;
+      if (fd && (rc = fd_rhs(c->gw, M, N, h, bl[k] * base, mu, B.U1, B.F1, B.udual, B.vdual, st, nullptr, 2 * k)))
+        return rc;
     }
     if (fd) {
       // the six systems of the sweep in one launch (12 right-hand sides)

@@ -33,6 +33,7 @@
 
 #include "../../include/aldic_b200.h"
 #include "aldic_internal.cuh"
+#include "fe_node.cuh"
 #include "kernels.cuh"
 
 namespace aldic {
@@ -357,16 +358,34 @@ __global__ void __launch_bounds__(GT) k_fdm_gemm(const __grid_constant__ GemmArg
   fdm_tile<TILE>(g, blockIdx.z, blockIdx.y * TILE, blockIdx.x * TILE, sm);
 }
 
-// The four products of a small solve in one launch: a cluster of eight CTAs
-// takes the 32 x 32 tiles of a product in turn and meets at the cluster's
+// The four products of a small solve in one launch, and before them the
+// right-hand side of the finite-element step: a cluster of eight CTAs takes the
+// nodes, then the 32 x 32 tiles of each product in turn and meets at the cluster's
 // barrier (a few hundred cycles, where a launch costs some 2 us).
 struct FdmChain {
   GemmArgs g[4];
   int batch;
+  // the right-hand side's inputs (null U: it is there), two fields of M N at b
+  const double *U, *F, *ud, *vd;
+  double *b;
+  double h;
 };
 __global__ void __launch_bounds__(GT) __cluster_dims__(kFdmCluster, 1, 1)
     k_fdm_chain(const __grid_constant__ FdmChain ch) {
   extern __shared__ double sm[];
+  auto meet = []() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  };
+  if (ch.U) {
+    const int M = ch.g[0].Cn, N = ch.g[0].R, n = M * N;
+    const double beta = ch.g[0].beta_ptr ? *ch.g[0].beta_ptr : ch.g[0].beta[0], mu = ch.g[0].mu;
+    for (int k = blockIdx.x * GT + threadIdx.x; k < n; k += kFdmCluster * GT) {
+      const FeParts p = fe_rhs_node(M, N, ch.h, k % M, k / M, ch.U, ch.F, ch.ud, ch.vd);
+      ch.b[k] = beta * p.ku + mu * p.mu;
+      ch.b[n + k] = beta * p.kv + mu * p.mv;
+    }
+    meet();
+  }
 #pragma unroll 1
   for (int q = 0; q < 4; ++q) {
     const GemmArgs &g = ch.g[q];
@@ -375,7 +394,7 @@ __global__ void __launch_bounds__(GT) __cluster_dims__(kFdmCluster, 1, 1)
       fdm_tile<32>(g, t / (tc * tr), t % (tc * tr) / tc * 32, t % tc * 32, sm);
       __syncthreads();  // the ring is refilled
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    meet();
   }
 }
 
@@ -486,10 +505,11 @@ int fdm_ensure(FdmBasis &B, int type, int M, int N, double h, cudaStream_t st) {
   return OK;
 }
 
-int fdm_solve(const FdmBasis &B, int nrhs, const double *b, double *x, double *tmp, double mu,
-              double beta, const double *beta_each, const double *beta_ptr, cudaStream_t st,
-              double *inter) {
-  ALDIC_CHECK(B.buf.p && nrhs >= 1 && nrhs <= 12, E_ARG, "fdm solve: bad arguments");
+namespace {
+
+// the products of fdm_solve
+FdmChain solve_chain(const FdmBasis &B, int nrhs, const double *b, double *x, double *tmp, double mu, double beta,
+                     const double *beta_each, const double *beta_ptr, double *inter) {
   const int M = B.M, N = B.N;
   const long long n = (long long)M * N;
   FdmChain ch{};
@@ -518,20 +538,50 @@ int fdm_solve(const FdmBasis &B, int nrhs, const double *b, double *x, double *t
     ch.g[3].C = inter;
     ch.g[3].scb = 1; ch.g[3].scr = (long long)nrhs * M; ch.g[3].scc = nrhs;
   }
+  return ch;
+}
+
+bool one_launch(const FdmBasis &B, int nrhs) {
   // One launch while the cluster has a tile a CTA: a whole aldic_subpb2 at 43 x 43
-  // takes 42.6 us this way and 58 us with four launches; with two rounds of
+  // takes 38.8 us this way and 58 us with five launches; with two rounds of
   // tiles (61 x 97, 55.4 us) it is no faster than four launches of 128 x 128
   // (53.7 us).
-  if (gemm_tiles(N, M, nrhs, 32) <= kFdmChainTiles) {
-    k_fdm_chain<<<kFdmCluster, GT, FdmTile<32>::smem, st>>>(ch);
-    ALDIC_CUDA(cudaGetLastError());
-    return OK;
-  }
+  return gemm_tiles(B.N, B.M, nrhs, 32) <= kFdmChainTiles;
+}
+
+int run_chain(const FdmChain &ch, cudaStream_t st) {
+  k_fdm_chain<<<kFdmCluster, GT, FdmTile<32>::smem, st>>>(ch);
+  ALDIC_CUDA(cudaGetLastError());
+  return OK;
+}
+
+}  // namespace
+
+int fdm_solve(const FdmBasis &B, int nrhs, const double *b, double *x, double *tmp, double mu,
+              double beta, const double *beta_each, const double *beta_ptr, cudaStream_t st,
+              double *inter) {
+  ALDIC_CHECK(B.buf.p && nrhs >= 1 && nrhs <= 12, E_ARG, "fdm solve: bad arguments");
+  const FdmChain ch = solve_chain(B, nrhs, b, x, tmp, mu, beta, beta_each, beta_ptr, inter);
+  if (one_launch(B, nrhs)) return run_chain(ch, st);
   for (int q = 0; q < 4; ++q) {
     const int rc = gemm(ch.g[q], nrhs, st);
     if (rc) return rc;
   }
   return OK;
+}
+
+int fe_solve(const FdmBasis &B, GridWork &w, double h, double beta, double mu, const double *beta_ptr,
+             const double *U, const double *F, const double *ud, const double *vd, double *Uhat, cudaStream_t st) {
+  ALDIC_CHECK(B.buf.p && B.type == FDM_FE, E_ARG, "fe solve: no basis");
+  FdmChain ch = solve_chain(B, 2, w.b, w.x, w.r, mu, beta, nullptr, beta_ptr, Uhat);
+  if (one_launch(B, 2)) {
+    ch.U = U; ch.F = F; ch.ud = ud; ch.vd = vd;
+    ch.b = w.b;
+    ch.h = h;
+    return run_chain(ch, st);
+  }
+  const int rc = fe_rhs(w, B.M, B.N, h, beta, mu, U, F, ud, vd, st, beta_ptr, 0);
+  return rc ? rc : fdm_solve(B, 2, w.b, w.x, w.r, mu, beta, nullptr, beta_ptr, st, Uhat);
 }
 
 // The beta sweep's eigen-domain solutions from the two transformed

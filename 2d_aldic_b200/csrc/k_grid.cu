@@ -15,6 +15,7 @@
 #include <cooperative_groups.h>
 
 #include "aldic_internal.cuh"
+#include "fe_node.cuh"
 #include "kernels.cuh"
 
 namespace aldic {
@@ -514,12 +515,10 @@ __global__ void __launch_bounds__(PCG_THREADS) k_pcg(const __grid_constant__ Pcg
 }
 
 // ------------------------------------------------------------------ Subpb2 RHS
-// Subpb2.m:88-149 per node, gathered from its (up to 4) elements.  The 3 x 3
-// Gauss rule there is exact for these integrands, so their values are used
-// (nine evaluations an element cost 8.4 us at 243 x 243, this 7 us).
-// NB right-hand sides at once (the beta sweep: one per beta, the same
-// operations for each as a single one), and the solve's start x = U with every
-// entry unknown: fields (2q, 2q + 1) of b and x for beta[q].
+// Subpb2.m:88-149 per node (fe_node.cuh).  NB right-hand sides at once (the beta
+// sweep: one per beta, the same operations for each as a single one), and the
+// solve's start x = U with every entry unknown: fields (2q, 2q + 1) of b and x for
+// beta[q].
 struct FeBetas {
   double v[6], m[6];  // beta and mu of each right-hand side
 };
@@ -531,46 +530,14 @@ __global__ void k_fe_rhs(int M, int N, double h, FeBetas be, const double *beta_
                          unsigned char *__restrict__ mask) {
   if (beta_ptr) be.v[0] = *beta_ptr;
   const long long n = (long long)M * N;
-  const double ha = 0.5 * h, mh = h * h / 36.0;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(k % M), j = (int)(k / M);
-    // F - W with the column order [4a-3, 4a-1, 4a-2, 4a] of Subpb2.m:88-91
-    const double fw0 = F[4 * k + 0] - ud[4 * k + 0];
-    const double fw1 = F[4 * k + 2] - ud[4 * k + 2];
-    const double fw2 = F[4 * k + 1] - ud[4 * k + 1];
-    const double fw3 = F[4 * k + 3] - ud[4 * k + 3];
-    double bu[NB], bv[NB];
-#pragma unroll
-    for (int q = 0; q < NB; ++q) bu[q] = bv[q] = 0.0;
-    for (int ej = j - 1; ej <= j; ++ej)
-      for (int ei = i - 1; ei <= i; ++ei) {
-        if (ei < 0 || ei >= M - 1 || ej < 0 || ej >= N - 1) continue;
-        // the element's integrals: of the node's shape function times each
-        // node's (h^2/9, /18, /36: itself, along an edge, across) and of its
-        // gradient (+-h/2)
-        double nu = 0.0, nv = 0.0;
-#pragma unroll
-        for (int dj = 0; dj < 2; ++dj)
-#pragma unroll
-          for (int di = 0; di < 2; ++di) {
-            const long long q = (long long)(ej + dj) * M + (ei + di);
-            const double w = (ei + di == i ? 2.0 : 1.0) * (ej + dj == j ? 2.0 : 1.0);
-            nu += w * (U[2 * q] - vd[2 * q]);
-            nv += w * (U[2 * q + 1] - vd[2 * q + 1]);
-          }
-        const double gx = ei == i ? -ha : ha, gy = ej == j ? -ha : ha;
-#pragma unroll
-        for (int q = 0; q < NB; ++q) {
-          bu[q] += be.v[q] * (gx * fw0 + gy * fw1) + be.m[q] * (mh * nu);
-          bv[q] += be.v[q] * (gx * fw2 + gy * fw3) + be.m[q] * (mh * nv);
-        }
-      }
+    const FeParts p = fe_rhs_node(M, N, h, (int)(k % M), (int)(k / M), U, F, ud, vd);
     const double u0 = U[2 * k], v0 = U[2 * k + 1];
 #pragma unroll
     for (int q = 0; q < NB; ++q) {
-      b[2 * q * n + k] = bu[q];
-      b[(2 * q + 1) * n + k] = bv[q];
+      b[2 * q * n + k] = be.v[q] * p.ku + be.m[q] * p.mu;
+      b[(2 * q + 1) * n + k] = be.v[q] * p.kv + be.m[q] * p.mv;
       x[2 * q * n + k] = u0;
       x[(2 * q + 1) * n + k] = v0;
       mask[2 * q * n + k] = 1;

@@ -270,6 +270,10 @@ int fe_rhs(GridWork &w, int M, int N, double h, double beta, double mu, const do
 int fe_rhs_parts(GridWork &w, int M, int N, double h, const double *U, const double *F,
                  const double *udual, const double *vdual, cudaStream_t st);
 // interleave w.x (2 fields from slot f0) into Uhat
+// The finite-element Subproblem 2 at beta (*beta_ptr if given): right-hand side and
+// direct solve (basis B of the mesh), Uhat interleaved; w.b, w.x, w.r are used
+int fe_solve(const FdmBasis &B, GridWork &w, double h, double beta, double mu, const double *beta_ptr,
+             const double *U, const double *F, const double *ud, const double *vd, double *Uhat, cudaStream_t st);
 int fe_store(const GridWork &w, int M, int N, double *Uhat, cudaStream_t st);
 // nodal strain (funGlobal_NodalStrainAvg.m)
 int nodal_strain(int M, int N, double h, const double *U, double *F, cudaStream_t st);

@@ -52,7 +52,7 @@ __device__ __forceinline__ uint32_t swz(int r, int c) { return r * 128 + ((c ^ (
 // KB each) and the weights (48 KB) are there.  The pair's 16 KB are loaded a
 // pair ahead, and the next embedding is issued with the correlation.  Eight
 // warps do the epilogues; a ninth only issues the products.
-// Tensor memory: D 128, C 64, E 64 columns.  16384 pairs: 174 us (ncu), against
+// Tensor memory: D 128, C 64, E 64 columns.  16384 pairs: 164 us (ncu), against
 // 62 us for their 24 KB each at the copy rate and 68 us for the products; a
 // pair's chain of three products and three epilogues is what is left (two CTAs
 // an SM hide half of it; 512 epilogue threads a CTA measured 6 % slower).  The

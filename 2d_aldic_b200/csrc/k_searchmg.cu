@@ -97,7 +97,7 @@ __device__ __forceinline__ double combine(long long mn, S st, S st2, S stdv, S s
 // sat[0..3] = f, f^2, g, g^2, each (W+1) x (H+1), row 0 and column 0 zero.
 // Bound by the writes of the tables (32 bytes a pixel, 134 MB at 2048 x 2048):
 // they are written once.  (Rows, then columns in place in two passes moved them
-// five times, 208 us; this takes 94 us.)
+// five times, 208 us; this takes 77 us.)
 // Pass 1: sums of each column over chunks of kSatChunk rows, read from the images.
 constexpr int kSatChunk = 16;
 template <typename P>
@@ -125,12 +125,12 @@ __global__ void k_sat_above(S *__restrict__ tot, int W, int nch) {
   if (x >= W) return;
   S *p = tot + (long long)blockIdx.y * nch * W + x;
   S acc = 0;
-  for (int c0 = 0; c0 < nch; c0 += 8) {
-    S v[8];
+  for (int c0 = 0; c0 < nch; c0 += 32) {
+    S v[32];  // all on their way at once
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = c0 + e < nch ? p[(long long)(c0 + e) * W] : S(0);
+    for (int e = 0; e < 32; ++e) v[e] = c0 + e < nch ? p[(long long)(c0 + e) * W] : S(0);
 #pragma unroll
-    for (int e = 0; e < 8; ++e)
+    for (int e = 0; e < 32; ++e)
       if (c0 + e < nch) {
         p[(long long)(c0 + e) * W] = acc;
         acc += v[e];
@@ -466,8 +466,13 @@ __device__ __forceinline__ double l1_den(const L1Args<S> &A, double mu, S sd, S 
   const long long n_pad = A.mn - n_in;
   double C0, Cc = 0.0;
   if constexpr (std::is_integral<S>::value) {
-    C0 = A.narrow ? (double)(A.mn * sd2 - sd * sd) : (double)((__int128)A.mn * sd2 - (__int128)sd * sd);
-    if (n_pad > 0) Cc = mu * ((double)((__int128)n_pad * n_in) * mu - 2.0 * (double)((__int128)sd * n_pad));
+    if (A.narrow) {  // the products below hold in 64 bits too: the same numbers
+      C0 = (double)(A.mn * sd2 - sd * sd);
+      if (n_pad > 0) Cc = mu * ((double)(n_pad * n_in) * mu - 2.0 * (double)(sd * n_pad));
+    } else {
+      C0 = (double)((__int128)A.mn * sd2 - (__int128)sd * sd);
+      if (n_pad > 0) Cc = mu * ((double)((__int128)n_pad * n_in) * mu - 2.0 * (double)((__int128)sd * n_pad));
+    }
   } else {
     C0 = (double)A.mn * sd2 - sd * sd;
     if (n_pad > 0) Cc = mu * ((double)n_pad * (double)n_in * mu - 2.0 * (sd * (double)n_pad));

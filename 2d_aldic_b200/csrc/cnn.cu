@@ -339,10 +339,8 @@ constexpr float kCorrScale = 0.08838834764831845f;  // 1 / sqrt(128)
 
 // x: the pairs in device memory; train keeps what the backward pass reads
 int forward(aldic_cnn *c, const void *x, int B, bool train, float *out, cudaStream_t st) {
-  const long long b = B;
   int rc;
-  const int splits = net_dense_splits(B);
-  if (splits > 1 && (rc = c->part.ensure(sizeof(float) * b * cnn::F3 * splits))) return rc;
+  if ((rc = c->part.ensure(net_dense_part(B)))) return rc;
   if ((rc = net_encode(x, B, c->Wb(0), c->Bv(0), c->Wb(1), c->Bv(1), kCorrScale, c->corr.p,
                        train ? c->e1.p : nullptr, train ? c->e2.p : nullptr, c->err.as<int>(), st)))
     return rc;

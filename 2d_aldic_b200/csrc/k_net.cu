@@ -293,28 +293,38 @@ __global__ void __launch_bounds__(kEncBlock, 2) k_encode(const __grid_constant__
 }
 
 // ------------------------------------------------------------------ k_dense
-// y[B x 256] = relu(corr[B x 4096] . W3^T + b3), out = y . W4^T + b4.  One CTA
-// per 128 rows, all 256 columns: 64-wide K steps of both operands by TMA into
-// a ring of four stages (one thread), products issued by another, 256 tensor
-// memory columns read by four warps.  With too few row tiles for the SMs the K
-// range is split over blockIdx.y and k_dense_out adds the partials; otherwise
-// the epilogue goes on to the output layer, a row a thread.
+// y[B x 256] = relu(corr[B x 4096] . W3^T + b3), out = y . W4^T + b4.  The K range
+// is summed in eight slices of 512, each in the tensor core's accumulator, and the
+// slices are added in FP32 in their order: the accumulator does not round every
+// addition to nearest, so a chain of 4096 loses more than eight of 512, and with
+// the same slices for every batch a pair's output does not depend on the batch it
+// comes in.  One CTA per 128 rows, all 256 columns: 64-wide K steps of both
+// operands by TMA into a ring of four stages (one thread), products issued by
+// another, a slice's 256 tensor memory columns read by eight warps (a row and half
+// of the columns a thread, their sums in its registers) under the next slice's
+// products.  With too few row tiles for the SMs (PART) each slice has a CTA of its own,
+// blockIdx.y, and k_dense_out adds them; otherwise the epilogue goes on to the output
+// layer, the second half of a row's sums after the first.
 // Bound: 48 KB of operands a step and SM through L2 (corr once, W3 by every
-// tile).  16384 rows: 52 us (ncu), 0.66 PFLOP/s; the generic product with its
-// split-K sum and the output layer took 560 us.
-constexpr int kDenseStages = 4, kDenseStage = (128 + kF) * 128, kDenseThreads = 192;
+// tile).  16384 rows: 47 us (ncu), 0.73 PFLOP/s; 52 us with one chain of 4096 read by
+// four warps at its end; the generic product with its split-K sum and the output layer
+// took 560 us.
+constexpr int kDenseStages = 4, kDenseStage = (128 + kF) * 128, kDenseThreads = 64 + 256;
+constexpr int kDenseSlices = 8, kSliceSteps = kCorr / 64 / kDenseSlices;
 
 struct DenseArgs {
   const float *b3, *W4, *b4;
   bf16 *y;
-  float *out, *part;         // part: [splits][B][256] when the K range is split
-  int B, steps;              // K steps a CTA
+  float *out, *part;         // part: [kDenseSlices][B][256] of PART
+  int B;
   int *err;
 };
 
 struct DenseShared {
   float W4[kF][kOut], b3[kF], b4[kOut];
-  uint64_t full[kDenseStages], empty[kDenseStages], done;
+  float o[kOut][128];        // the output layer's sums over the first half of a row
+  uint64_t full[kDenseStages], empty[kDenseStages];
+  uint64_t done[2], read[2]; // a slice's sums are there, and have been read
   uint32_t tmem;
   int failed;
 };
@@ -326,6 +336,7 @@ __device__ __forceinline__ void tma_2d(const CUtensorMap *m, uint32_t dst, uint6
       : "memory");
 }
 
+template <bool PART>
 __global__ void __launch_bounds__(kDenseThreads, 1) k_dense(const __grid_constant__ CUtensorMap mA,
                                                             const __grid_constant__ CUtensorMap mB,
                                                             const DenseArgs A) {
@@ -333,15 +344,19 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_dense(const __grid_constan
   unsigned char *ring = (unsigned char *)(((uintptr_t)dense_raw + 1023) & ~(uintptr_t)1023);
   DenseShared &S = *(DenseShared *)(ring + kDenseStages * kDenseStage);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * 128, k0 = blockIdx.y * A.steps;
-  if (warp == 0) tmem_alloc(&S.tmem, kF);
+  constexpr int slices = PART ? 1 : kDenseSlices, steps = slices * kSliceSteps;
+  const int m0 = blockIdx.x * 128, z0 = blockIdx.y;
+  if (warp == 0) tmem_alloc(&S.tmem, 2 * kF);
   if (tid == 0) {
     S.failed = 0;
     for (int s = 0; s < kDenseStages; ++s) {
       bar_init(&S.full[s], 1);
       bar_init(&S.empty[s], 1);
     }
-    bar_init(&S.done, 1);
+    for (int s = 0; s < 2; ++s) {
+      bar_init(&S.done[s], 1);
+      bar_init(&S.read[s], 8);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int q = tid; q < kF * kOut; q += kDenseThreads) S.W4[q % kF][q / kF] = A.W4[q];
@@ -354,7 +369,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_dense(const __grid_constan
   if (warp == 0) {
     if (lane == 0) {
       int k = 0;
-      for (; k < A.steps; ++k) {
+      for (; k < steps; ++k) {
         const int s = k % kDenseStages;
         if (k >= kDenseStages && !bar_wait(&S.empty[s], (k / kDenseStages - 1) & 1)) {
           S.failed = 1;
@@ -364,8 +379,8 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_dense(const __grid_constan
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&S.full[s])),
                      "r"(kDenseStage)
                      : "memory");
-        tma_2d(&mA, a, &S.full[s], 64 * (k0 + k), m0);
-        tma_2d(&mB, a + 128 * 128, &S.full[s], 64 * (k0 + k), 0);
+        tma_2d(&mA, a, &S.full[s], 64 * (z0 * kSliceSteps + k), m0);
+        tma_2d(&mB, a + 128 * 128, &S.full[s], 64 * (z0 * kSliceSteps + k), 0);
       }
       // every copy has landed before the CTA may end, also after a failed wait
       for (int q = k > kDenseStages ? k - kDenseStages : 0; q < k; ++q)
@@ -373,101 +388,135 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_dense(const __grid_constan
     }
   } else if (uniform(warp) == 1) {
     const uint32_t base = uniform(smem_u32(ring));
-    for (int k = 0; k < A.steps; ++k) {
-      const int s = k % kDenseStages;
-      if (!__all_sync(0xffffffffu, bar_wait(&S.full[s], (k / kDenseStages) & 1))) {
-        S.failed = 1;
-        break;
+    bool ok = true;
+    for (int z = 0, k = 0; z < slices && ok; ++z) {
+      const uint32_t d = tD + (z & 1) * kF;
+      if (z >= 2) {  // the slice before last has been read
+        ok = __all_sync(0xffffffffu, bar_wait(&S.read[z & 1], ((z >> 1) - 1) & 1));
+        tc_after_sync();
       }
-      tc_after_sync();
-      const uint64_t da = sdesc(base + s * kDenseStage), db = sdesc(base + s * kDenseStage + 128 * 128);
-      if (elect_one()) {
+      for (int q8 = 0; q8 < kSliceSteps && ok; ++q8, ++k) {
+        const int s = k % kDenseStages;
+        ok = __all_sync(0xffffffffu, bar_wait(&S.full[s], (k / kDenseStages) & 1));
+        if (!ok) break;
+        tc_after_sync();
+        const uint64_t da = sdesc(base + s * kDenseStage), db = sdesc(base + s * kDenseStage + 128 * 128);
+        if (elect_one()) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) mma_bf16(tD, da + 2 * q, db + 2 * q, idesc(kF), k > 0 || q > 0);
-        mma_commit(&S.empty[s]);
+          for (int q = 0; q < 4; ++q) mma_bf16(d, da + 2 * q, db + 2 * q, idesc(kF), q8 > 0 || q > 0);
+          mma_commit(&S.empty[s]);
+        }
+        __syncwarp();
       }
+      if (!ok) S.failed = 1;
+      if (elect_one()) mma_commit(&S.done[z & 1]);
       __syncwarp();
+      // after a failed wait: no product is under way when the CTA ends
+      if (!ok) bar_wait(&S.done[z & 1], (z >> 1) & 1);
     }
-    if (elect_one()) mma_commit(&S.done);
-    __syncwarp();
   } else {
-    const bool ok = __all_sync(0xffffffffu, bar_wait(&S.done, 0) && !*(volatile int *)&S.failed);
-    if (!ok) S.failed = 1;
-    tc_after_sync();
-    const int quarter = warp & 3, m = m0 + 32 * quarter + lane;
-    const uint32_t t = tD + ((uint32_t)(32 * quarter) << 16);
-    float o[kOut];
+    const int quarter = warp & 3, half = (warp - 2) >> 2, row = 32 * quarter + lane, m = m0 + row;
+    const uint32_t t = tD + ((uint32_t)(32 * quarter) << 16) + half * (kF / 2);
+    float sum[PART ? 1 : kF / 2] = {};
+    bool ok = true;
+    for (int z = 0; z < slices && ok; ++z) {
+      ok = __all_sync(0xffffffffu, bar_wait(&S.done[z & 1], (z >> 1) & 1) && !*(volatile int *)&S.failed);
+      if (!ok) break;
+      tc_after_sync();
 #pragma unroll
-    for (int k = 0; k < kOut; ++k) o[k] = S.b4[k];
-#pragma unroll 1
-    for (int c = 0; c < kF && ok; c += 32) {
-      float v[32];
+      for (int c = 0; c < kF / 2; c += 16) {
+        float v[16];
+        tmem_ld16(t + (z & 1) * kF + c, v);
+        if constexpr (PART) {
+          if (m < A.B) {
+            float4 *p = (float4 *)(A.part + ((long long)z0 * A.B + m) * kF + half * (kF / 2) + c);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) p[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+          }
+          __syncwarp();
+        } else {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) sum[c + k] += v[k];
+        }
+      }
+      tc_before_sync();
       __syncwarp();
-      tmem_ld32(t + c, v);
-      if (m >= A.B) continue;
-      if (A.part) {
-        float4 *p = (float4 *)(A.part + ((long long)blockIdx.y * A.B + m) * kF + c);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) p[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-        continue;
-      }
-      uint32_t w[16];
-#pragma unroll
-      for (int k = 0; k < 16; ++k)
-        w[k] = pack2(fmaxf(v[2 * k] + S.b3[c + 2 * k], 0.f), fmaxf(v[2 * k + 1] + S.b3[c + 2 * k + 1], 0.f));
-      uint4 *p = (uint4 *)(A.y + (long long)m * kF + c);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) p[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
-#pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        const float y = __uint_as_float(k & 1 ? w[k >> 1] & 0xffff0000u : w[k >> 1] << 16);
-        const float4 wa = *(const float4 *)&S.W4[c + k][0], wb = *(const float4 *)&S.W4[c + k][4];
-        o[0] += y * wa.x; o[1] += y * wa.y; o[2] += y * wa.z; o[3] += y * wa.w;
-        o[4] += y * wb.x; o[5] += y * wb.y; o[6] += y * wb.z; o[7] += y * wb.w;
-      }
+      if (lane == 0) bar_arrive(&S.read[z & 1]);
     }
-    if (ok && !A.part && m < A.B) {
-      float4 *p = (float4 *)(A.out + (long long)m * kOut);
-      p[0] = make_float4(o[0], o[1], o[2], o[3]);
-      p[1] = make_float4(o[4], o[5], o[6], o[7]);
+    if (!ok) S.failed = 1;
+    if constexpr (!PART) {
+      float o[kOut];
+#pragma unroll
+      for (int k = 0; k < kOut; ++k) o[k] = S.b4[k];
+      if (half) {
+        named_sync(1 + quarter, 64);  // the first half's sums
+#pragma unroll
+        for (int k = 0; k < kOut; ++k) o[k] = S.o[k][row];
+      }
+#pragma unroll
+      for (int c = 0; c < kF / 2; c += 8) {
+        const int n = half * (kF / 2) + c;
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          w[k] = pack2(fmaxf(sum[c + 2 * k] + S.b3[n + 2 * k], 0.f), fmaxf(sum[c + 2 * k + 1] + S.b3[n + 2 * k + 1], 0.f));
+        if (ok && m < A.B) *(uint4 *)(A.y + (long long)m * kF + n) = make_uint4(w[0], w[1], w[2], w[3]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float y = __uint_as_float(k & 1 ? w[k >> 1] & 0xffff0000u : w[k >> 1] << 16);
+          const float4 wa = *(const float4 *)&S.W4[n + k][0], wb = *(const float4 *)&S.W4[n + k][4];
+          o[0] += y * wa.x; o[1] += y * wa.y; o[2] += y * wa.z; o[3] += y * wa.w;
+          o[4] += y * wb.x; o[5] += y * wb.y; o[6] += y * wb.z; o[7] += y * wb.w;
+        }
+      }
+      if (!half) {
+#pragma unroll
+        for (int k = 0; k < kOut; ++k) S.o[k][row] = o[k];
+        named_sync(1 + quarter, 64);
+      } else if (ok && m < A.B) {
+        float4 *p = (float4 *)(A.out + (long long)m * kOut);
+        p[0] = make_float4(o[0], o[1], o[2], o[3]);
+        p[1] = make_float4(o[4], o[5], o[6], o[7]);
+      }
     }
   }
   tc_before_sync();
   __syncthreads();
   if (tid == 0 && S.failed) atomicExch(A.err, 3);
-  if (warp == 0) tmem_free(tD, kF);
+  if (warp == 0) tmem_free(tD, 2 * kF);
 }
 
-// the split layer's partials, added in split order; a warp a row, 8 columns a lane
-__global__ void __launch_bounds__(128) k_dense_out(const DenseArgs A, int splits) {
-  __shared__ __align__(16) float W4[kOut][kF];
+// the slices of the layer added in their order; a warp a row, 8 columns a lane,
+// then a thread an output of the block's four rows
+__global__ void __launch_bounds__(128) k_dense_out(const DenseArgs A) {
+  __shared__ float W4[kOut][kF + 1], y[4][kF];
   for (int q = threadIdx.x; q < kF * kOut; q += 128) W4[q / kF][q % kF] = A.W4[q];
-  __syncthreads();
-  const int b = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (b >= A.B) return;
-  float s[8] = {};
-  for (int z = 0; z < splits; ++z) {
-    const float4 *p = (const float4 *)(A.part + ((long long)z * A.B + b) * kF + 8 * lane);
-    const float4 u = p[0], v = p[1];
-    s[0] += u.x; s[1] += u.y; s[2] += u.z; s[3] += u.w;
-    s[4] += v.x; s[5] += v.y; s[6] += v.z; s[7] += v.w;
-  }
-  uint32_t w[4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b = blockIdx.x * 4 + warp;
+  if (b < A.B) {
+    float s[8] = {};
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
-    w[k] = pack2(fmaxf(s[2 * k] + A.b3[8 * lane + 2 * k], 0.f), fmaxf(s[2 * k + 1] + A.b3[8 * lane + 2 * k + 1], 0.f));
-  *(uint4 *)(A.y + (long long)b * kF + 8 * lane) = make_uint4(w[0], w[1], w[2], w[3]);
-  float mine = 0.f;
+    for (int z = 0; z < kDenseSlices; ++z) {
+      const float4 *p = (const float4 *)(A.part + ((long long)z * A.B + b) * kF + 8 * lane);
+      const float4 u = p[0], v = p[1];
+      s[0] += u.x; s[1] += u.y; s[2] += u.z; s[3] += u.w;
+      s[4] += v.x; s[5] += v.y; s[6] += v.z; s[7] += v.w;
+    }
+    uint32_t w[4];
 #pragma unroll
-  for (int o = 0; o < kOut; ++o) {
-    float t = 0.f;
+    for (int k = 0; k < 4; ++k)
+      w[k] = pack2(fmaxf(s[2 * k] + A.b3[8 * lane + 2 * k], 0.f), fmaxf(s[2 * k + 1] + A.b3[8 * lane + 2 * k + 1], 0.f));
+    *(uint4 *)(A.y + (long long)b * kF + 8 * lane) = make_uint4(w[0], w[1], w[2], w[3]);
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-      t += __uint_as_float(k & 1 ? w[k >> 1] & 0xffff0000u : w[k >> 1] << 16) * W4[o][8 * lane + k];
-    t = warp_sumf(t);
-    if (lane == o) mine = t + A.b4[o];
+      y[warp][8 * lane + k] = __uint_as_float(k & 1 ? w[k >> 1] & 0xffff0000u : w[k >> 1] << 16);
   }
-  if (lane < kOut) A.out[(long long)b * kOut + lane] = mine;
+  __syncthreads();
+  const int r = threadIdx.x / kOut, o = threadIdx.x % kOut, m = blockIdx.x * 4 + r;
+  if (r >= 4 || m >= A.B) return;
+  float t = A.b4[o];
+#pragma unroll 16
+  for (int k = 0; k < kF; ++k) t += y[r][k] * W4[o][k];
+  A.out[(long long)m * kOut + o] = t;
 }
 
 // rows x cols bf16 matrix, boxes of `box` rows x 64 columns in the 128-byte swizzle
@@ -521,28 +570,29 @@ int net_encode(const void *x, int B, const void *W1, const float *b1, const void
   return OK;
 }
 
-// splits of the K range: as many as keep the SMs busy, none once the row tiles do
-int net_dense_splits(int B) {
-  const int tiles = (B + 127) / 128;
-  int s = 1;
-  while (s < 16 && 2 * s * tiles <= 148) s *= 2;
-  return s;
-}
+// A CTA a slice while all of them run at once; beyond, the partials' way through
+// memory costs more than idle SMs (whole predictions, a CTA a slice against all: 256
+// pairs 56 / 64 us, 2048 74 / 83, 2500 88 / 83, 4096 111 / 108, 9000 197 / 152; two
+// or four slices a CTA lie between or above).
+bool dense_apart(int B) { return (B + 127) / 128 * kDenseSlices <= 148; }
+
+size_t net_dense_part(int B) { return dense_apart(B) ? sizeof(float) * kDenseSlices * kF * (size_t)B : 0; }
 
 int net_dense(const void *corr, int B, const void *W3, const float *b3, const float *W4, const float *b4,
               void *y, float *out, float *part, int *err, cudaStream_t st) {
   CUtensorMap mA, mB;
   int rc;
   if ((rc = make_map(&mA, corr, B, kCorr, 128)) || (rc = make_map(&mB, W3, kF, kCorr, kF))) return rc;
-  const int splits = net_dense_splits(B);
+  const bool apart = dense_apart(B);
   DenseArgs A;
   A.b3 = b3; A.W4 = W4; A.b4 = b4;
-  A.y = (bf16 *)y; A.out = out; A.part = splits > 1 ? part : nullptr;
-  A.B = B; A.steps = kCorr / 64 / splits; A.err = err;
+  A.y = (bf16 *)y; A.out = out; A.part = part;
+  A.B = B; A.err = err;
   const int smem = kDenseStages * kDenseStage + sizeof(DenseShared) + 1024;
-  ALDIC_CUDA(cudaFuncSetAttribute(k_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  k_dense<<<dim3((B + 127) / 128, splits), kDenseThreads, smem, st>>>(mA, mB, A);
-  if (splits > 1) k_dense_out<<<(B + 3) / 4, 128, 0, st>>>(A, splits);
+  auto *fn = apart ? k_dense<true> : k_dense<false>;
+  ALDIC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  fn<<<dim3((B + 127) / 128, apart ? kDenseSlices : 1), kDenseThreads, smem, st>>>(mA, mB, A);
+  if (apart) k_dense_out<<<(B + 3) / 4, 128, 0, st>>>(A);
   ALDIC_CUDA(cudaGetLastError());
   return OK;
 }

@@ -145,13 +145,6 @@ __device__ __forceinline__ void mma_u8_ta(uint32_t tmem_d, uint32_t tmem_a, uint
       "r"(tmem_a), "l"(db), "r"(id), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0));
 }
 
-__device__ __forceinline__ void bar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void named_sync(int id, int threads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
 // Four consecutive pixels from any address, read as aligned words
 template <typename T>
 struct Four {

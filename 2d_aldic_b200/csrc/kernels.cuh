@@ -232,11 +232,10 @@ int gemm_bf16(const GemmSrc &A, const GemmSrc &B, const GemmDst &D, int splits, 
               cudaStream_t st, int batches = 1);
 // the network's forward pass (k_net.cu): x [B][64][64][2] bf16, 16-byte aligned,
 // -> corr [B][64 x 64] (and the layers' activations e1, e2 [2B][64][128] unless
-// null); corr -> y [B][256] and out [B][8].  part: net_dense_splits(B) B 256
-// floats when that is over 1
+// null); corr -> y [B][256] and out [B][8].  part: net_dense_part(B) bytes
 int net_encode(const void *x, int B, const void *W1, const float *b1, const void *W2, const float *b2,
                float scale, void *corr, void *e1, void *e2, int *err, cudaStream_t st);
-int net_dense_splits(int B);
+size_t net_dense_part(int B);
 int net_dense(const void *corr, int B, const void *W3, const float *b3, const float *W4, const float *b4,
               void *y, float *out, float *part, int *err, cudaStream_t st);
 // learned initial guess (cnn.cu)

@@ -68,3 +68,15 @@ def test_forward_inputs(net):
     host = n.predict(x.float().cpu().numpy())
     np.testing.assert_array_equal(host, out.cpu().numpy())
     torch.testing.assert_close(out, _reference(torch, p, x), rtol=RTOL, atol=ATOL * float(out.abs().max()))
+
+
+def test_forward_does_not_depend_on_the_batch(net):
+    """A pair's output has the same bits in every batch: the dense layer's sums have
+    the same order whether its slices share a CTA or each has its own."""
+    import torch
+    n, _ = net
+    x = torch.randn((9601, 64, 64, 2), generator=torch.Generator(device="cuda").manual_seed(3), device="cuda")
+    x = x.to(torch.bfloat16)
+    whole = n.predict(x)
+    for B in (1, 127, 129, 2304, 2305, 9472):
+        torch.testing.assert_close(n.predict(x[9601 - B:]), whole[9601 - B:], rtol=0, atol=0)

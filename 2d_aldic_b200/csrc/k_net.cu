@@ -27,10 +27,20 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t *>(&h);
 }
-// the same with negative values to 0
+// the same with negative values and NaN to 0 (cvt's own relu keeps NaN)
 __device__ __forceinline__ uint32_t pack2_relu(float a, float b) {
   uint32_t r;
-  asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  asm("{\n\t.reg .b32 t;\n\tcvt.rn.bf16x2.f32 t, %1, %2;\n\tmax.bf16x2 %0, t, %3;\n\t}" : "=r"(r) : "f"(b), "f"(a), "r"(0));
+  return r;
+}
+
+// both sums in one instruction (16384 pairs: 233 us the call with two, 222 so)
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return r;
 }
 
@@ -168,8 +178,8 @@ __global__ void __launch_bounds__(kEncBlock, 2) k_encode(const __grid_constant__
           const float2 bb = bias[4 * q + j];
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
-            const float x = v[4 * j + 2 * k] + bb.x, y = v[4 * j + 2 * k + 1] + bb.y;
-            w[2 * j + k] = relu ? pack2_relu(x, y) : pack2(x, y);
+            const float2 x = add2(make_float2(v[4 * j + 2 * k], v[4 * j + 2 * k + 1]), bb);
+            w[2 * j + k] = relu ? pack2_relu(x.x, x.y) : pack2(x.x, x.y);
           }
         }
         tmem_st_16x16(tE + lanes + 32 * half + 16 * q, w);

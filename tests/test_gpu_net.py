@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 
 def _reference(torch, p, x):
-    """x: B x 64 x 64 x 2 bf16 on the GPU -> B x 8, FP32 sums."""
+    """x: B x 64 x 64 x 2 bf16 on the GPU -> B x 8, FP32 sums; ReLU of NaN is 0."""
+    relu = lambda t: torch.where(t > 0, t, torch.zeros_like(t))
     sizes = [(128, 64), (128, 128), (256, 4096), (8, 256)]
     o, L = 0, []
     for co, ci in sizes:
@@ -21,9 +22,9 @@ def _reference(torch, p, x):
 
     def enc(c):
         cells = x[..., c].float().view(B, 8, 8, 8, 8).permute(0, 1, 3, 2, 4).reshape(B, 64, 64)
-        return r(r(torch.relu(cells @ W[0].T + L[0][1])) @ W[1].T + L[1][1])
+        return r(r(relu(cells @ W[0].T + L[0][1])) @ W[1].T + L[1][1])
     corr = r((enc(0) @ enc(1).transpose(1, 2)) * 0.08838834764831845)
-    y = r(torch.relu(corr.reshape(B, 4096) @ W[2].T + L[2][1]))
+    y = r(relu(corr.reshape(B, 4096) @ W[2].T + L[2][1]))
     return y @ W[3].T + L[3][1]
 
 
@@ -80,3 +81,20 @@ def test_forward_does_not_depend_on_the_batch(net):
     whole = n.predict(x)
     for B in (1, 127, 129, 2304, 2305, 9472):
         torch.testing.assert_close(n.predict(x[9601 - B:]), whole[9601 - B:], rtol=0, atol=0)
+
+
+def test_forward_of_values_that_are_not_finite(net):
+    """A NaN pixel takes its cell's embedding to 0, an infinite one the pair's hidden
+    layer; the other pairs of the batch keep their bits."""
+    import torch
+    n, p = net
+    x = torch.randn((300, 64, 64, 2), generator=torch.Generator(device="cuda").manual_seed(8), device="cuda")
+    x = x.to(torch.bfloat16)
+    clean = n.predict(x)
+    x[3, 10, 20, 0] = x[140, 63, 63, 1] = x[299, :, :, 0] = float("nan")
+    x[5, 0, 0, 1], x[201, 33, 1, 0] = float("inf"), float("-inf")
+    out, ref = n.predict(x), _reference(torch, p, x)
+    assert bool(torch.isfinite(out).all())
+    torch.testing.assert_close(out, ref, rtol=RTOL, atol=ATOL * float(ref.abs().max()))
+    same = [b for b in range(300) if b not in (3, 140, 299, 5, 201)]
+    torch.testing.assert_close(out[same], clean[same], rtol=0, atol=0)

@@ -43,7 +43,7 @@ def _stale(target: str, deps: list[str]) -> bool:
 
 def build(verbose: bool = False, force: bool = False, extra: list[str] | None = None) -> str:
     os.makedirs(OBJ, exist_ok=True)
-    headers = [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith(".cuh")]
+    headers = [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith((".cuh", ".h"))]
     headers.append(os.path.join(ROOT, "include", "aldic_b200.h"))
     objs, jobs = [], []
     for s in SOURCES:

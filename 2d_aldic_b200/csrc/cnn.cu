@@ -27,6 +27,7 @@
 #include "../../include/aldic_b200.h"
 #include "aldic_internal.cuh"
 #include "kernels.cuh"
+#include "rules.h"
 
 namespace aldic {
 namespace cnn {
@@ -468,21 +469,31 @@ int check_err(aldic_cnn *c, cudaStream_t st, double *loss = nullptr) {
   return OK;
 }
 
-bool on_device(const void *p) {
-  cudaPointerAttributes at;
-  const bool dev = cudaPointerGetAttributes(&at, p) == cudaSuccess &&
-                   (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged);
+cudaPointerAttributes memory_of(const void *p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) at.type = cudaMemoryTypeUnregistered;
   cudaGetLastError();
-  return dev;
+  return at;
 }
+// in some GPU's memory
+bool on_device(const void *p) {
+  const cudaPointerAttributes at = memory_of(p);
+  return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
+}
+// where this network's kernels may use it
+bool in_place(const aldic_cnn *c, const void *p) {
+  const cudaPointerAttributes at = memory_of(p);
+  return memory_in_place((int)at.type, at.device, c->device);
+}
+static_assert(cudaMemoryTypeDevice == 2 && cudaMemoryTypeManaged == 3, "memory_in_place's types");
 
-// network input: fp32 (host or device) or bf16 patches -> *pairs, in device
+// network input: fp32 or bf16 patches on the host or any device -> *pairs, in device
 // memory: the caller's own where the kernels can read it (the call waits for
 // them before it returns), else a copy
 int load_input(aldic_cnn *c, const void *x, int x_bf16, int B, const void **pairs, cudaStream_t st) {
   const long long n = (long long)B * cnn::P * cnn::P * 2;
-  const bool dev = on_device(x);
-  if (x_bf16 && dev && (uintptr_t)x % 16 == 0) {
+  const bool here = in_place(c, x);
+  if (x_bf16 && here && (uintptr_t)x % 16 == 0) {
     *pairs = x;
     return OK;
   }
@@ -495,14 +506,14 @@ int load_input(aldic_cnn *c, const void *x, int x_bf16, int B, const void **pair
   }
   DevBuf tmp;
   const float *xd = (const float *)x;
-  if (!dev) {
+  if (!here) {
     if ((rc = tmp.ensure(4 * n))) return rc;
-    ALDIC_CUDA(cudaMemcpyAsync(tmp.p, x, 4 * n, cudaMemcpyHostToDevice, st));
+    ALDIC_CUDA(cudaMemcpyAsync(tmp.p, x, 4 * n, cudaMemcpyDefault, st));
     xd = tmp.as<float>();
   }
   k_f2bf<<<nblk(n), 256, 0, st>>>(xd, c->xin.as<bf16>(), n);
   ALDIC_CUDA(cudaGetLastError());
-  if (!dev) {
+  if (!here) {
     ALDIC_CUDA(cudaStreamSynchronize(st));
     tmp.release();
   }
@@ -668,7 +679,7 @@ int aldic_cnn_predict(aldic_cnn *c, const void *x, int x_bf16, int B, void *stre
   const void *pairs = nullptr;
   int rc = ensure(c, B, false);
   if (!rc) rc = load_input(c, x, x_bf16, B, &pairs, st);
-  const bool direct = on_device(out) && (uintptr_t)out % 16 == 0;
+  const bool direct = in_place(c, out) && (uintptr_t)out % 16 == 0;
   if (!rc) rc = forward(c, pairs, B, false, direct ? out : c->out.as<float>(), st);
   if (!rc && !direct && cudaMemcpyAsync(out, c->out.p, 4LL * B * cnn::NOUT, cudaMemcpyDefault, st) != cudaSuccess)
     rc = E_CUDA;

@@ -24,6 +24,7 @@ _SIGS = {
     "aldic_ctx_create": ([I32, P], I32),
     "aldic_ctx_destroy": ([P], I32),
     "aldic_ctx_set_stream": ([P, P], I32),
+    "aldic_ctx_set_wait_tries": ([P, C.c_uint], I32),
     "aldic_set_ref": ([P, P, I32, I32, I32, P, P], I32),
     "aldic_set_def": ([P, P, I32], I32),
     "aldic_set_fields": ([P, P, P, P, P, I32, I32], I32),

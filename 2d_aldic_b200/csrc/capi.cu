@@ -228,7 +228,6 @@ int ensure_grid_work(aldic_ctx *c, long long n) {
   c->gw.max_blocks = 148 * 8;
   if ((rc = c->gw_part.ensure(sizeof(double) * 2 * 4 * R * c->gw.max_blocks))) return rc;
   if ((rc = c->gw_mask.ensure(R * n))) return rc;
-  if ((rc = c->gw_misc.ensure(64))) return rc;
   double *v = c->gw_vec.as<double>();
   c->gw.x = v;
   c->gw.r = v + R * n;
@@ -246,19 +245,35 @@ int ensure_grid_work(aldic_ctx *c, long long n) {
   c->gw.mask = c->gw_mask.as<unsigned char>();
   unsigned int *misc = c->gw_misc.as<unsigned int>();
   c->gw.bar = misc;
-  c->gw.err = (int *)(misc + 2);
-  c->gw.iters_out = (int *)(misc + 3);
-  c->gw.gate = (int *)(misc + 4);
+  c->gw.err = (int *)(misc + 2);  // and the search's word
+  c->gw.iters_out = (int *)(misc + 4);
+  c->gw.gate = (int *)(misc + 6);
   c->gw.ticket = misc + 8;
   c->gw_n = n;
-  ALDIC_CUDA(cudaMemsetAsync(c->gw_misc.p, 0, 64, c->stream));
   return OK;
 }
 
-int check_grid_err(aldic_ctx *c) {
+int search_timed_out(aldic_ctx *c) {
+  cudaMemsetAsync(c->sw.err, 0, sizeof(int), c->stream);
+  set_error("integer search: a tensor-core wait timed out");
+  return E_TIMEOUT;
+}
+
+// waits for the stream and reads the search's status
+int check_search_err(aldic_ctx *c) {
   int err = 0;
-  ALDIC_CUDA(cudaMemcpyAsync(&err, c->gw.err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  ALDIC_CUDA(cudaMemcpyAsync(&err, c->sw.err, sizeof err, cudaMemcpyDeviceToHost, c->stream));
   ALDIC_CUDA(cudaStreamSynchronize(c->stream));
+  return err ? search_timed_out(c) : OK;
+}
+
+// waits for the stream and reads the grid solvers' status and the search's
+int check_grid_err(aldic_ctx *c) {
+  int both[2] = {0, 0};
+  ALDIC_CUDA(cudaMemcpyAsync(both, c->gw.err, sizeof both, cudaMemcpyDeviceToHost, c->stream));
+  ALDIC_CUDA(cudaStreamSynchronize(c->stream));
+  if (both[1]) return search_timed_out(c);
+  const int err = both[0];
   if (err == 1) {
     cudaMemsetAsync(c->gw.err, 0, sizeof(int), c->stream);
     set_error("grid solver: barrier wait timed out");
@@ -386,6 +401,9 @@ int aldic_ctx_create(int device, aldic_ctx **out) {
   if (!rc) rc = c->isums.ensure(sizeof(unsigned long long) * 2);
   if (!rc) rc = c->part.ensure(sizeof(double) * 1024);
   if (!rc) rc = c->queue.ensure(sizeof(unsigned int) * 4);
+  if (!rc) rc = c->gw_misc.ensure(64);
+  if (!rc && cudaMemsetAsync(c->gw_misc.p, 0, 64, c->stream) != cudaSuccess) rc = E_CUDA;
+  c->sw.err = c->gw_misc.as<int>() + 3;
   for (int k = 0; k < 8 && !rc; ++k)
     if (cudaEventCreate(&c->ev[k]) != cudaSuccess) rc = E_CUDA;
   cudaSetDevice(prev);
@@ -436,6 +454,14 @@ int aldic_ctx_set_stream(aldic_ctx *c, void *stream) {
   if (c->own_stream) cudaStreamDestroy(c->stream);
   c->stream = (cudaStream_t)stream;
   c->own_stream = false;
+  c->drop_graphs();
+  return OK;
+}
+
+int aldic_ctx_set_wait_tries(aldic_ctx *c, unsigned tries) {
+  ALDIC_CHECK(c, E_ARG, "null context");
+  Guard g(c);
+  c->sw.tries = tries;
   c->drop_graphs();
   return OK;
 }
@@ -719,7 +745,7 @@ int aldic_int_search(aldic_ctx *c, const int gridx[2], const int gridy[2], int w
     ALDIC_CUDA(cudaMemcpyAsync(qfactors, q.data(), sizeof(double) * 2 * n, cudaMemcpyDefault, c->stream));
     ALDIC_CUDA(cudaStreamSynchronize(c->stream));
   }
-  return finish(c, ax.staged || qfactors);
+  return ax.staged || qfactors ? check_search_err(c) : finish(c, false);
 }
 
 // Multigrid search shared by aldic_int_search_mg and the frame's

@@ -1188,7 +1188,7 @@ int tile_search(const uint8_t *f, const uint8_t *g, const SearchGeom &G, SearchW
   k_search_peak<<<pb, kPeakWarps * 32, 0, st>>>(K);
   ALDIC_CUDA(cudaGetLastError());
   // the points handed back: the per-point kernel over the device-side list
-  if ((rc = search_mma<uint8_t>(f, g, G, tab, fb, x, y, u, v, cc, st))) return rc;
+  if ((rc = search_mma<uint8_t>(f, g, G, tab, fb, x, y, u, v, cc, sw.err, sw.tries, st))) return rc;
   *used = true;
   return OK;
 }
@@ -1392,7 +1392,7 @@ int launch_search(const void *f, const void *g, const SearchGeom &G, double *x, 
       if (rc) return rc;
       uint4 *tab = tile_bufs(sw->buf.as<char>(), G.W, G.H, G.nx, G.ny, srch).tab;
       if ((rc = box_table<Px>((const Px *)g, G, tab, st)) ||
-          (rc = search_mma<Px>((const Px *)f, (const Px *)g, G, tab, nullptr, x, y, u, v, cc, st)))
+          (rc = search_mma<Px>((const Px *)f, (const Px *)g, G, tab, nullptr, x, y, u, v, cc, sw->err, sw->tries, st)))
         return rc;
     }
   } else {

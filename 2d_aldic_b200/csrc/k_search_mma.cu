@@ -120,7 +120,7 @@ MmaPlan mma_plan(const SearchGeom &G, int pl) {
 }
 
 struct MmaShared {
-  uint64_t full[kMmaSlots], empty[kMmaSlots], done;
+  uint64_t full[kMmaSlots], empty[kMmaSlots], done, drained;
   long long st, st2;
   long long part[4][2];            // a warp's share of st, st2
   int edge[4];                     // template sums: columns 0, tw - 1, rows 0, tw - 1
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kMmaBlock, 2)
     k_search_mma(const T *__restrict__ f, const T *__restrict__ g, const SearchGeom G, const MmaPlan P,
                  const uint4 *__restrict__ tab, const int *__restrict__ list, double *__restrict__ ox,
                  double *__restrict__ oy, double *__restrict__ ou, double *__restrict__ ov,
-                 double *__restrict__ occ) {
+                 double *__restrict__ occ, int *__restrict__ err, const uint32_t tries) {
   constexpr int PL = sizeof(T);
   using Wide = typename std::conditional<PL == 1, int, long long>::type;  // sums of products
   extern __shared__ unsigned char mma_raw[];
@@ -217,6 +217,7 @@ __global__ void __launch_bounds__(kMmaBlock, 2)
       bar_init(&S.empty[s], 1);
     }
     bar_init(&S.done, 1);
+    bar_init(&S.drained, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     S.top = 0u;
     S.nq = S.failed = 0;
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(kMmaBlock, 2)
   const long long mn = (long long)G.tw * G.tw;
   const double mu = *G.mu;
   auto wait = [&](uint64_t *bar, uint32_t parity) {
-    if (!*(volatile int *)&S.failed && !bar_wait(bar, parity)) S.failed = 1;
+    if (!*(volatile int *)&S.failed && !bar_wait(bar, parity, tries)) S.failed = 1;
   };
   auto pix = [&](int y, int x) {  // pixel of the padded region
     int v = 0;
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(kMmaBlock, 2)
           const int s = rc & 1, y0 = r * P.trows;
           wait(&S.full[s], (rc >> 1) & 1);
           tc_after_sync();
-          __syncwarp();
+          if (__any_sync(0xffffffffu, *(volatile int *)&S.failed)) break;  // no more products
           // the rows' descriptors: 8 PL further (16-byte units) a template row, 2
           // a K step, another block after 128 bytes
           uint64_t db = base + (uint64_t)(PL * 8 * y0);
@@ -330,6 +331,10 @@ __global__ void __launch_bounds__(kMmaBlock, 2)
           __syncwarp();
         }
       }
+    // no product is under way when the tensor memory goes, also after a failed wait
+    if (elect_one()) mma_commit(&S.drained);
+    __syncwarp();
+    bar_wait(&S.drained, 0);
   } else if (warp == kPeak) {
     for (int k = blockIdx.x; k < npts; k += gridDim.x) {
       named_sync(4, kMmaThreads + 32);  // the queue is complete
@@ -667,6 +672,7 @@ __global__ void __launch_bounds__(kMmaBlock, 2)
   }
   tc_before_sync();
   __syncthreads();
+  if (tid == 0 && S.failed) atomicExch(err, 3);
   if (warp == 0) tmem_free(tD, P.tcols);
 }
 
@@ -676,7 +682,7 @@ bool search_mma_fits(const SearchGeom &G, int bytes) { return bytes <= 2 && mma_
 
 template <typename T>
 int search_mma(const T *f, const T *g, const SearchGeom &G, const uint4 *tab, const int *list, double *x,
-               double *y, double *u, double *v, double *cc, cudaStream_t st) {
+               double *y, double *u, double *v, double *cc, int *err, unsigned tries, cudaStream_t st) {
   const MmaPlan P = mma_plan(G, sizeof(T));
   const int smem = P.total + 1024;
   int dev = 0, sms = 148;
@@ -685,15 +691,13 @@ int search_mma(const T *f, const T *g, const SearchGeom &G, const uint4 *tab, co
   ALDIC_CUDA(cudaFuncSetAttribute(k_search_mma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const long long npts = (long long)G.nx * G.ny;
   const int blocks = (int)std::min<long long>(npts, (long long)P.ctas * sms);
-  k_search_mma<T><<<blocks, kMmaBlock, smem, st>>>(f, g, G, P, tab, list, x, y, u, v, cc);
+  k_search_mma<T><<<blocks, kMmaBlock, smem, st>>>(f, g, G, P, tab, list, x, y, u, v, cc, err, tries);
   ALDIC_CUDA(cudaGetLastError());
   return OK;
 }
-template int search_mma<uint8_t>(const uint8_t *, const uint8_t *, const SearchGeom &, const uint4 *,
-                                 const int *, double *,
-                                 double *, double *, double *, double *, cudaStream_t);
-template int search_mma<uint16_t>(const uint16_t *, const uint16_t *, const SearchGeom &, const uint4 *,
-                                 const int *, double *,
-                                  double *, double *, double *, double *, cudaStream_t);
+template int search_mma<uint8_t>(const uint8_t *, const uint8_t *, const SearchGeom &, const uint4 *, const int *,
+                                 double *, double *, double *, double *, double *, int *, unsigned, cudaStream_t);
+template int search_mma<uint16_t>(const uint16_t *, const uint16_t *, const SearchGeom &, const uint4 *, const int *,
+                                  double *, double *, double *, double *, double *, int *, unsigned, cudaStream_t);
 
 }  // namespace aldic

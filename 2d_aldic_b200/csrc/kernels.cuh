@@ -33,6 +33,8 @@ int interp_f32(const float *F, long long M, long long N, long long P, const floa
 struct SearchWork {
   DevBuf buf;
   DevBuf big;  // per-CTA row sums and maps of search regions too large for shared memory
+  int *err = nullptr;          // 3 once a tensor-core wait has given up
+  unsigned tries = 1u << 22;   // polls of such a wait (kBarTries of tc.cuh)
   void release() {
     buf.release();
     big.release();
@@ -108,7 +110,7 @@ struct GridWork {
   double *part;          // per-block partial sums: 2 buffers of [4][nrhs][blocks]
   unsigned char *mask;   // per node flags (data present / unknown)
   unsigned int *bar;     // grid barrier {count, gen}
-  int *err;              // barrier / solver error flag
+  int *err;              // barrier / solver error flag; the integer search's word follows
   int *iters_out;        // PCG iterations used
   int max_blocks;
   int *gate = nullptr;   // k_local.cu's {gate, ticket}; the ticket is 0 between launches

@@ -27,11 +27,13 @@ __device__ __forceinline__ float fkey_inv(unsigned k) {
 // the tensor-core search of 8- (bytes 1) and 16-bit images: whether a geometry
 // fits it, and the search itself, over all grid points or those of list
 // {count, points...} (device memory).  tab: the window table of box_table.  f
-// and g are 4-byte aligned and may be read up to 16 bytes beyond the image.
+// and g are 4-byte aligned and may be read up to 16 bytes beyond the image.  *err
+// becomes 3 where a wait gave up (after `tries` polls); the points of that CTA that
+// were not done have NaN then.
 bool search_mma_fits(const SearchGeom &G, int bytes);
 template <typename T>
 int search_mma(const T *f, const T *g, const SearchGeom &G, const uint4 *tab, const int *list, double *x,
-               double *y, double *u, double *v, double *cc, cudaStream_t st);
+               double *y, double *u, double *v, double *cc, int *err, unsigned tries, cudaStream_t st);
 
 // tab[y W + x]: sums of g and g^2 over the tw x tw window with its first pixel
 // at (x, y) (0-based) and 1/sqrt(tw^2 sum g^2 - (sum g)^2), for every window of

@@ -76,9 +76,10 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
 // bounded wait on an mbarrier phase; false after a few seconds.  Each try may
 // suspend the thread for a microsecond: polling without it took a fifth of an
 // SM's issue slots where a dozen warps wait.
-__device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
+constexpr uint32_t kBarTries = 1u << 22;
+__device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity, uint32_t tries = kBarTries) {
   const uint32_t a = smem_u32(bar);
-  for (uint32_t it = 0; it < (1u << 22); ++it) {
+  for (uint32_t it = 0; it < tries; ++it) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred P1;\n\t"

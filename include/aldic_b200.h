@@ -79,6 +79,12 @@ ALDIC_API int aldic_ba_interp2_f32(const float *F, int64_t M, int64_t N, int64_t
 ALDIC_API int aldic_ctx_create(int device, aldic_ctx **out);
 ALDIC_API int aldic_ctx_destroy(aldic_ctx *ctx);
 ALDIC_API int aldic_ctx_set_stream(aldic_ctx *ctx, void *stream);
+/* Polls (of a microsecond at most) after which the integer search's kernel gives up a
+ * wait for its tensor cores; 4194304 unless set, 0 gives every wait up at once.  Such
+ * a search leaves NaN at the points it did not reach and is reported as
+ * ALDIC_E_TIMEOUT by the call or, where the call does not wait for its results
+ * (device arrays), by the next call on the context that reads a status. */
+ALDIC_API int aldic_ctx_set_wait_tries(aldic_ctx *ctx, unsigned tries);
 
 /* Reference image: funNormalizeImg.m:1 (ROI mean/std normalisation) and
  * funImgGradient.m:1 (7-tap gradients times the mask, DfCropWidth = 3).

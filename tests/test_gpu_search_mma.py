@@ -81,3 +81,33 @@ def test_full_scale_sums_bit_exact(aldic, oracle):
     _check(aldic, oracle, f >> 8, g >> 8, 20, 8, 9)
     b = (255 - (rng.random((150, 170)) < 0.02)).astype(np.uint8)
     _check(aldic, oracle, b, np.roll(b, (2, -1), (0, 1)), 20, 8, 9)
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16])
+def test_waits_that_give_up_are_an_error(aldic, oracle, synth, dtype):
+    """Every wait of the kernel gives up at once (no product is issued then): the call
+    fails, a frame whose start it was fails, device arrays carry NaN and the next
+    status tells; with the usual limit the context works on."""
+    import torch
+    f, g = _images(oracle, synth, dtype, 200, 180, 59)
+    ctx = aldic.Context(0)
+    search = lambda a, b: aldic.funIntegerSearch(a, b, 6, [1, 200], [1, 180], 21, 10, 0, 10, qfactors=False, ctx=ctx)
+    al = aldic.ALDIC(20, 10, 6, precision=aldic.FP32, ctx=ctx)
+    want = search(f, g)
+    al.set_images(f, g)
+    whole = al.frame()
+    aldic._lib.call("aldic_ctx_set_wait_tries", ctx.h, 0)
+    with pytest.raises(aldic.AldicError, match="timed out"):
+        search(f, g)
+    with pytest.raises(aldic.AldicError, match="timed out"):
+        al.frame()
+    out = search(torch.from_numpy(f).cuda(), torch.from_numpy(g).cuda())
+    torch.cuda.synchronize()
+    assert bool(torch.isnan(torch.as_tensor(out[2])).all())
+    aldic._lib.call("aldic_ctx_set_wait_tries", ctx.h, 1 << 22)
+    with pytest.raises(aldic.AldicError, match="timed out"):
+        search(f, g)                               # the word of the call before
+    for a, b in zip(search(f, g)[:4], want[:4]):
+        np.testing.assert_array_equal(a, b)
+    al.set_images(f, g)
+    np.testing.assert_array_equal(al.frame()["U"], whole["U"])

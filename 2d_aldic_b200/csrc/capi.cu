@@ -1730,7 +1730,7 @@ int aldic_qt_frame(aldic_ctx *c, const aldic_qt_frame_params *p, aldic_qt_mesh *
   ALDIC_CHECK(nx >= 2 && ny >= 2, E_ARG, "qt_frame: the search grid needs 2 x 2 nodes");
   const long long n0 = (long long)nx * ny;
   // ---- Section 3: whole-field search on the uniform grid, holes, Init
-  if ((rc = search_work_ensure(c->sw, W, H, nx, ny, srch, w, c->dtype))) return rc;
+  if ((rc = search_work_ensure(c->sw, c->dtype, W, H, nx, ny, w, step, srch))) return rc;
   auto &Q = c->qtf;
   if ((rc = Q.ugrid.ensure(sizeof(double) * (11 * n0 + 1024)))) return rc;
   double *sx = Q.ugrid.as<double>(), *sy = sx + n0, *su = sy + n0, *sv = su + n0, *scc = sv + n0;
@@ -2103,7 +2103,7 @@ int aldic_frame(aldic_ctx *c, const aldic_frame_params *p, double *x0, double *y
     return rc;
   // search work before any capture (a graph records its addresses)
   if ((qp.init == ALDIC_INIT_SEARCH || qp.init == ALDIC_INIT_GATED) &&
-      (rc = search_work_ensure(c->sw, c->W, c->H, M, N, p->search, p->winsize, c->dtype)))
+      (rc = search_work_ensure(c->sw, c->dtype, c->W, c->H, M, N, p->winsize, p->step, p->search)))
     return rc;
   // frame slab
   FrameBufs B;

@@ -1125,8 +1125,8 @@ int tile_dispatch(const TileArgs &A, const TilePlan &P, int step, cudaStream_t s
   return E_ARG;
 }
 
-// work slab: the window table (16 B per pixel), the hand-back list, then
-// per tile point (tiles hold at most 8 x 8 points, so (nx + 7) (ny + 7)
+// work slab: the window table (16 B per pixel), and for tiles the hand-back list,
+// then per tile point (tiles hold at most 8 x 8 points, so (nx + 7) (ny + 7)
 // bounds them) the correlation map (4 B per entry of the (2s+3)^2 map), the
 // template sums and the outer ring's window sums
 struct TileBufs {
@@ -1137,14 +1137,16 @@ struct TileBufs {
   uint2 *ringw;
   size_t bytes;
 };
-TileBufs tile_bufs(char *base, int W, int H, int nx, int ny, const int search[2]) {
-  const size_t cr = 2 * search[0] + 3, cc = 2 * search[1] + 3, slots = (size_t)(nx + 7) * (ny + 7);
-  TileBufs B;
+TileBufs tile_bufs(char *base, const SearchGeom &G, bool tiles) {
+  const size_t cr = G.cr, cc = G.cc, slots = (size_t)(G.nx + 7) * (G.ny + 7);
+  TileBufs B{};
   size_t o = 0;
   B.tab = reinterpret_cast<uint4 *>(base + o);
-  o += align16((size_t)W * H * sizeof(uint4));
+  o += align16((size_t)G.W * G.H * sizeof(uint4));
+  B.bytes = o;
+  if (!tiles) return B;
   B.fb = reinterpret_cast<int *>(base + o);
-  o += align16((size_t)((long long)nx * ny + 1) * sizeof(int));
+  o += align16((size_t)((long long)G.nx * G.ny + 1) * sizeof(int));
   B.cmap = reinterpret_cast<unsigned *>(base + o);
   o += align16(slots * cr * cc * sizeof(unsigned));
   B.subs = reinterpret_cast<TileSub *>(base + o);
@@ -1155,19 +1157,12 @@ TileBufs tile_bufs(char *base, int W, int H, int nx, int ny, const int search[2]
   return B;
 }
 
-// tiled 8-bit search; false in *used when the geometry has no tiled kernel
-int tile_search(const uint8_t *f, const uint8_t *g, const SearchGeom &G, SearchWork &sw,
-                double *x, double *y, double *u, double *v, double *cc, cudaStream_t st, bool *used) {
-  *used = false;
-  TilePlan P;
-  if (G.step % 4 || G.w % G.step || !tile_shape(G.step, G.w, G.sx, G.sy, P)) return OK;
+// tiled 8-bit search of a geometry that has a plan for it; B: its slab
+int tile_search(const uint8_t *f, const uint8_t *g, const SearchGeom &G, const TilePlan &P, const TileBufs &B,
+                const SearchWork &sw, double *x, double *y, double *u, double *v, double *cc, cudaStream_t st) {
   const int px1 = G.gx1 - 1, py1 = G.gy1 - 1;
-  if (px1 - G.sx - 1 < 0 || py1 - G.sy - 1 < 0) return OK;
   const long long npts = (long long)G.nx * G.ny;
-  const int srch[2] = {G.sx, G.sy};
-  int rc = search_work_ensure(sw, G.W, G.H, G.nx, G.ny, srch);
-  if (rc) return rc;
-  const TileBufs B = tile_bufs(sw.buf.as<char>(), G.W, G.H, G.nx, G.ny, srch);
+  int rc;
   uint4 *tab = B.tab;
   int *fb = B.fb;
   const long long mn = (long long)G.tw * G.tw;
@@ -1189,7 +1184,6 @@ int tile_search(const uint8_t *f, const uint8_t *g, const SearchGeom &G, SearchW
   ALDIC_CUDA(cudaGetLastError());
   // the points handed back: the per-point kernel over the device-side list
   if ((rc = search_mma<uint8_t>(f, g, G, tab, fb, x, y, u, v, cc, sw.err, sw.tries, st))) return rc;
-  *used = true;
   return OK;
 }
 
@@ -1359,6 +1353,12 @@ bool tiles_pay(const SearchGeom &G) {
   return (double)G.cr * G.cc * G.step * G.step * G.step < (G.w < 24 ? 2.5e6 : 1.85e6);
 }
 
+// whether a search goes by tiles, and their plan
+bool tiled(const SearchGeom &G, int bytes, TilePlan &P) {
+  return bytes == 1 && tiles_pay(G) && G.step % 4 == 0 && G.w % G.step == 0 &&
+         tile_shape(G.step, G.w, G.sx, G.sy, P);
+}
+
 template <typename T>
 int launch_search(const void *f, const void *g, const SearchGeom &G, double *x, double *y,
                   double *u, double *v, double *cc, double *pce, double *ppe, cudaStream_t st,
@@ -1379,20 +1379,18 @@ int launch_search(const void *f, const void *g, const SearchGeom &G, double *x, 
   // against 0.44; 16 bit 16/8/10 0.53 against 0.66, 50/25/30 0.26 against 1.16;
   // 320 x 340, 20/10/20 8 bit 0.119 against 0.127 ms
   if (sizeof(T) <= 2 && search_mma_fits(G, sizeof(T))) {
-    bool tiled = false;
-    if (sizeof(T) == 1 && sw && tiles_pay(G)) {
-      const int rc = tile_search((const uint8_t *)f, (const uint8_t *)g, G, *sw, x, y, u, v, cc, st, &tiled);
-      if (rc) return rc;
-    }
+    ALDIC_CHECK(sw != nullptr, E_ARG, "integer search: the context's work memory is needed");
+    TilePlan P;
+    const bool tiles = tiled(G, sizeof(T), P);
+    int rc = sw->buf.ensure(tile_bufs(nullptr, G, tiles).bytes);
+    if (rc) return rc;
+    const TileBufs B = tile_bufs(sw->buf.as<char>(), G, tiles);
     using Px = typename std::conditional<sizeof(T) == 1, uint8_t, uint16_t>::type;
-    if (!tiled) {
-      ALDIC_CHECK(sw != nullptr, E_ARG, "integer search: the context's work memory is needed");
-      const int srch[2] = {G.sx, G.sy};
-      int rc = search_work_ensure(*sw, G.W, G.H, G.nx, G.ny, srch);
-      if (rc) return rc;
-      uint4 *tab = tile_bufs(sw->buf.as<char>(), G.W, G.H, G.nx, G.ny, srch).tab;
-      if ((rc = box_table<Px>((const Px *)g, G, tab, st)) ||
-          (rc = search_mma<Px>((const Px *)f, (const Px *)g, G, tab, nullptr, x, y, u, v, cc, sw->err, sw->tries, st)))
+    if (tiles) {
+      if ((rc = tile_search((const uint8_t *)f, (const uint8_t *)g, G, P, B, *sw, x, y, u, v, cc, st))) return rc;
+    } else {
+      if ((rc = box_table<Px>((const Px *)g, G, B.tab, st)) ||
+          (rc = search_mma<Px>((const Px *)f, (const Px *)g, G, B.tab, nullptr, x, y, u, v, cc, sw->err, sw->tries, st)))
         return rc;
     }
   } else {
@@ -1470,27 +1468,31 @@ void geom_sizes(SearchGeom &G, int winsize, const int search[2]) {
 }
 
 template <typename T>
-size_t big_bytes(const SearchGeom &G) {
+int work_ensure(SearchWork &w, const SearchGeom &G) {
   using Tr = SearchTraits<T>;
   using S = typename SumT<Tr::integer>::type;
-  const bool small = (sizeof(T) <= 2 && search_mma_fits(G, sizeof(T))) ||
-                     SmemLayout<typename Tr::V, S>(G).total <= kSmemMax;
-  if (small) return 0;
+  if (sizeof(T) <= 2 && search_mma_fits(G, sizeof(T))) {
+    TilePlan P;
+    return w.buf.ensure(tile_bufs(nullptr, G, tiled(G, sizeof(T), P)).bytes);
+  }
+  if (SmemLayout<typename Tr::V, S>(G).total <= kSmemMax) return OK;
   const int npts = G.nx * G.ny;
-  return SmemLayout<typename Tr::V, S>(G, true).slot * (size_t)(npts < kBigBlocks ? npts : kBigBlocks);
+  return w.big.ensure(SmemLayout<typename Tr::V, S>(G, true).slot * (size_t)(npts < kBigBlocks ? npts : kBigBlocks));
 }
 
-int search_work_ensure(SearchWork &w, int W, int H, int nx, int ny, const int search[2], int winsize,
-                       int dtype) {
-  int rc = w.buf.ensure(tile_bufs(nullptr, W, H, nx, ny, search).bytes);
-  if (rc || winsize <= 0) return rc;
+int search_work_ensure(SearchWork &w, int dtype, int W, int H, int nx, int ny, int winsize, int step,
+                       const int search[2]) {
   SearchGeom G{};
+  G.W = W;
+  G.H = H;
   G.nx = nx;
   G.ny = ny;
+  G.step = step;
   geom_sizes(G, winsize, search);
-  const size_t b = dtype == 0 ? big_bytes<uint8_t>(G) : dtype == 1 ? big_bytes<uint16_t>(G)
-                 : dtype == 2 ? big_bytes<float>(G) : big_bytes<double>(G);
-  return b ? w.big.ensure(b) : OK;
+  return dtype == 0   ? work_ensure<uint8_t>(w, G)
+         : dtype == 1 ? work_ensure<uint16_t>(w, G)
+         : dtype == 2 ? work_ensure<float>(w, G)
+                      : work_ensure<double>(w, G);
 }
 
 int int_search(const void *f_raw, const void *g_raw, int dtype, int W, int H, const double *mu_g,

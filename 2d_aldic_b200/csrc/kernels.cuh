@@ -28,8 +28,9 @@ int interp_f32(const float *F, long long M, long long N, long long P, const floa
                const float *Y, long long n, float *Z, cudaStream_t st);
 
 // ---- k_search.cu
-// work of the tiled 8-bit search: the window table of the deformed image, the
-// list of points handed to the per-point kernel and the correlation maps
+// work of the 8- and 16-bit search: the window table of the deformed image, and of
+// the 8-bit tiles the list of points handed to the per-point kernel and the
+// correlation maps
 struct SearchWork {
   DevBuf buf;
   DevBuf big;  // per-CTA row sums and maps of search regions too large for shared memory
@@ -40,10 +41,10 @@ struct SearchWork {
     big.release();
   }
 };
-// work memory of a search geometry (with winsize > 0 and the image dtype also
-// the big-region slots), allocated ahead of any stream capture
-int search_work_ensure(SearchWork &w, int W, int H, int nx, int ny, const int search[2],
-                       int winsize = 0, int dtype = -1);
+// the work memory that int_search will use of a geometry, allocated ahead of any
+// stream capture
+int search_work_ensure(SearchWork &w, int dtype, int W, int H, int nx, int ny, int winsize, int step,
+                       const int search[2]);
 int search_dims(int W, int H, const int gridx[2], const int gridy[2], int winsize, int step,
                 const int search[2], int *nx, int *ny, int *gx1, int *gy1);
 int int_search(const void *f_raw, const void *g_raw, int dtype, int W, int H, const double *mu_g,

@@ -111,3 +111,24 @@ def test_waits_that_give_up_are_an_error(aldic, oracle, synth, dtype):
         np.testing.assert_array_equal(a, b)
     al.set_images(f, g)
     np.testing.assert_array_equal(al.frame()["U"], whole["U"])
+
+
+@pytest.mark.parametrize("dtype,step", [(np.uint16, 2), (np.uint8, 2), (np.uint8, 8)])
+def test_work_memory_is_what_the_path_reads(aldic, oracle, synth, dtype, step):
+    """Points on the tensor cores need a table of the image, not the tiles' map of every
+    point (2.7 GB here at step 2; the tiles of step 8 do not pay at this zone), in the
+    search by itself and in a frame, whose other arrays take 2 kB a node."""
+    import torch
+    W, H = 700, 690
+    f, g = _images(oracle, synth, dtype, W, H, 61)
+    ctx = aldic.Context(0)
+    ctx.set_ref(f)
+    ctx.set_def(g)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    x = aldic.funIntegerSearch(f, g, 40, [1, W], [1, H], 16, step, 0, step, qfactors=False, ctx=ctx)[0]
+    assert before - torch.cuda.mem_get_info()[0] < 128 << 20
+    al = aldic.ALDIC(16, step, 40, precision=aldic.FP32, n_admm=1, ctx=ctx)
+    al.set_images(f, g)
+    al.frame()
+    assert before - torch.cuda.mem_get_info()[0] < (256 << 20) + 2048 * x.size

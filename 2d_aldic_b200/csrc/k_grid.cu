@@ -698,6 +698,21 @@ __global__ void k_nodal_strain(int M, int N, double h, const double *__restrict_
                         *v = U[2 * q + 1];
                       },
                       out);
+    // the elements' strains take part with all of their nodes, so a displacement that
+    // is not finite makes NaN of its component at every node it shares an element
+    // with, also where the differences do not read it.  (The solved displacements
+    // of the other users of nodal_strain_node are finite everywhere or nowhere.)
+    double zu = 0.0, zv = 0.0;
+    for (int y = max(0, j - 1); y <= min(N - 1, j + 1); ++y)
+      for (int x = max(0, i - 1); x <= min(M - 1, i + 1); ++x) {
+        const long long q = (long long)y * M + x;
+        zu = fma(0.0, U[2 * q], zu);
+        zv = fma(0.0, U[2 * q + 1], zv);
+      }
+    out[0] += zu;
+    out[1] += zu;
+    out[2] += zv;
+    out[3] += zv;
     for (int c = 0; c < 4; ++c) F[4 * k + c] = out[c];
   }
 }

@@ -17,6 +17,7 @@
 #include "aldic_internal.cuh"
 #include "fe_node.cuh"
 #include "kernels.cuh"
+#include "rules.h"
 
 namespace aldic {
 
@@ -838,8 +839,7 @@ __global__ void __launch_bounds__(1024)
     *nconv = (int)t[4];
     const double m = t[4] ? (double)t[2] / d : nan;
     *meanit = m;
-    const double sd = t[4] > 1 ? sqrt((double)(t[4] * t[3] - t[2] * t[2]) / d / (double)(t[4] - 1))
-                               : (t[4] == 1 ? 0.0 : nan);
+    const double sd = t[4] > 1 ? sqrt(sample_variance(t[4], t[2], t[3])) : (t[4] == 1 ? 0.0 : nan);
     // Subpb1Quadtree.m:180 raises the threshold to at least `floor`
     // (MATLAB's max ignores a NaN); NaN floor = LocalICGN.m:128-131
     s_thr = isnan(floor) ? m + 0.15 * sd : fmax(m + 0.15 * sd, floor);

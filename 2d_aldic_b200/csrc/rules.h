@@ -16,4 +16,10 @@ ALDIC_RULE bool memory_in_place(int type, int where, int device) {
   return type == 3 || (type == 2 && where == device);
 }
 
+// Sample variance of `count` >= 2 whole numbers from their sum and sum of squares.
+// The difference is exact; its products pass 2^63 for some ten million subsets.
+ALDIC_RULE double sample_variance(long long count, long long sum, long long squares) {
+  return (double)((__int128)count * squares - (__int128)sum * sum) / (double)count / (double)(count - 1);
+}
+
 }  // namespace aldic

@@ -2,6 +2,7 @@
 import ctypes as C
 import os
 import subprocess
+from fractions import Fraction
 
 import pytest
 
@@ -9,6 +10,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SHIM = """
 #include "rules.h"
 extern "C" int in_place(int type, int where, int device) { return aldic::memory_in_place(type, where, device); }
+extern "C" double variance(long long n, long long s, long long q) { return aldic::sample_variance(n, s, q); }
 """
 
 
@@ -18,7 +20,10 @@ def rules(tmp_path_factory):
     (d / "shim.cpp").write_text(SHIM)
     subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "2d_aldic_b200", "csrc"),
                     str(d / "shim.cpp"), "-o", str(d / "rules.so")], check=True)
-    return C.CDLL(str(d / "rules.so"))
+    lib = C.CDLL(str(d / "rules.so"))
+    lib.variance.restype = C.c_double
+    lib.variance.argtypes = [C.c_longlong] * 3
+    return lib
 
 
 @pytest.mark.parametrize("device", [0, 1, 7])
@@ -29,3 +34,15 @@ def test_only_its_own_memory_is_used_in_place(rules, device):
         assert not rules.in_place(pinned, where, device)
         assert rules.in_place(dev, where, device) == (where == device)
         assert rules.in_place(managed, where, device)
+
+
+@pytest.mark.parametrize("n", [2, 59049, 30_000_000, 60_000_000, 2_000_000_000])
+@pytest.mark.parametrize("values", [(1, 99), (98, 99), (7, 7)])
+def test_variance_of_many_evaluation_counts(rules, n, values):
+    """Half of the subsets took one number of evaluations, half the other: exact up to
+    the last divisions' roundings also where n sum(v^2) has more than 63 bits."""
+    a, b = values
+    k = n // 2
+    s, q = k * a + (n - k) * b, k * a * a + (n - k) * b * b
+    want = Fraction(n * q - s * s, n * (n - 1))
+    assert rules.variance(n, s, q) == pytest.approx(float(want), rel=4 * 2.0 ** -53, abs=0)

@@ -651,11 +651,12 @@ int aldic_cnn_train_step(aldic_cnn *c, const void *x, int x_bf16, const float *t
     // what lies before and after it
     const long long o = aldic_cnn::off_w(2), e = o + cnn::NW[2], n = cnn::n_params();
     const float *g = c->grad.as<float>();
-    if (cudaStreamWaitEvent(c->copies, c->w3_ready, 0) != cudaSuccess ||
-        cudaMemcpyAsync(grads + o, g + o, 4 * (e - o), cudaMemcpyDefault, c->copies) != cudaSuccess ||
-        cudaMemcpyAsync(grads, g, 4 * o, cudaMemcpyDefault, st) != cudaSuccess ||
-        cudaMemcpyAsync(grads + e, g + e, 4 * (n - e), cudaMemcpyDefault, st) != cudaSuccess ||
-        cudaStreamSynchronize(c->copies) != cudaSuccess) {
+    const bool sent = cudaStreamWaitEvent(c->copies, c->w3_ready, 0) == cudaSuccess &&
+                      cudaMemcpyAsync(grads + o, g + o, 4 * (e - o), cudaMemcpyDefault, c->copies) == cudaSuccess &&
+                      cudaMemcpyAsync(grads, g, 4 * o, cudaMemcpyDefault, st) == cudaSuccess &&
+                      cudaMemcpyAsync(grads + e, g + e, 4 * (n - e), cudaMemcpyDefault, st) == cudaSuccess;
+    // waited for in any case: no copy is on its way to the caller's memory afterwards
+    if (cudaStreamSynchronize(c->copies) != cudaSuccess || !sent) {
       set_error("cnn_train_step: copying the gradients failed");
       rc = E_CUDA;
     }

@@ -49,6 +49,7 @@ struct FitArgs {
   double *b, *x, *part;
   unsigned char *mask;
   int *gate;                     // {gate, ticket}
+  int *iters;                    // most iterations of a solve so far
   unsigned int *bar;             // k_pcg's grid barrier words, reset here
   double lam2, rtol;
   double ca[kFitSteps], cb[kFitSteps];  // d <- ca d + cb D^-1 r
@@ -203,6 +204,7 @@ __global__ void __launch_bounds__(kFitThreads, 1) k_fit_tile(const __grid_consta
   }
   const int any2 = __syncthreads_or(need == 2), any1 = __syncthreads_or(need == 1);
   if (threadIdx.x == 0) {
+    atomicMax(A.iters, kFitSteps);
     A.gate[0] = any2 ? 2 : (any1 ? 1 : 0);
     A.gate[1] = 0;
     A.bar[0] = A.bar[1] = 0;
@@ -218,6 +220,7 @@ struct FillArgs {
   double *b, *x;
   unsigned char *mask;
   int *gate;
+  int *iters;  // most iterations of a solve so far
   unsigned int *bar;
   double rtol;
   int M, N, nf;
@@ -472,7 +475,8 @@ __global__ void __launch_bounds__(kFillThreads, 2) k_fill_tile(const __grid_cons
   __syncthreads();
   double alpha = 0.0, beta = 0.0, gi = 0.0, ai = 0.0, bnorm = 0.0;
   bool done = false;
-  for (int it = 0; it < kFillMaxit; ++it) {
+  int it = 0;
+  for (; it < kFillMaxit; ++it) {
     apply(r, w);
     double a0 = 0.0, a1 = 0.0;
 #pragma unroll
@@ -509,6 +513,7 @@ __global__ void __launch_bounds__(kFillThreads, 2) k_fill_tile(const __grid_cons
     if (threadIdx.x == 0) atomicExch(A.gate, 1);
     return;
   }
+  if (threadIdx.x == 0) atomicMax(A.iters, it);
 #pragma unroll
   for (int q = 0; q < kFillPer; ++q)
     if (threadIdx.x + q * kFillThreads < cnt) {
@@ -547,7 +552,7 @@ int fit_tiles(GridWork &w, int M, int N, int nf, const FieldMap &in, const Field
   A.bad = bad;
   A.b = w.b; A.x = w.x; A.mask = w.mask;
   A.part = w.r;  // k_pcg overwrites it only once the gate is set
-  A.gate = w.gate; A.bar = w.bar;
+  A.gate = w.gate; A.iters = w.iters_out; A.bar = w.bar;
   A.lam2 = lam2; A.rtol = rtol;
   fit_coefficients(A.ca, A.cb);
   for (int k = 0; k < 18; ++k) {
@@ -573,7 +578,7 @@ int fill_tiles(GridWork &w, int M, int N, int nf, const FieldMap &vals, const un
   A.vals = vals;
   A.bad = bad;
   A.b = w.b; A.x = w.x; A.mask = w.mask;
-  A.gate = w.gate; A.bar = w.bar;
+  A.gate = w.gate; A.iters = w.iters_out; A.bar = w.bar;
   A.rtol = rtol;
   A.M = M; A.N = N; A.nf = nf;
   const long long n = (long long)M * N;

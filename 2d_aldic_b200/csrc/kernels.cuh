@@ -112,7 +112,7 @@ struct GridWork {
   unsigned char *mask;   // per node flags (data present / unknown)
   unsigned int *bar;     // grid barrier {count, gen}
   int *err;              // barrier / solver error flag; the integer search's word follows
-  int *iters_out;        // PCG iterations used
+  int *iters_out;        // most iterations of a solve so far
   int max_blocks;
   int *gate = nullptr;   // k_local.cu's {gate, ticket}; the ticket is 0 between launches
   double *tmp = nullptr; // 12 M N doubles no solver touches

@@ -515,7 +515,8 @@ typedef struct {
    * search + Init, 2 IC-GN kernel, 3 LocalICGN post-processing, 4 Section 5
    * (beta, Subpb2, nodal strain), 5 ADMM iterations, 6 whole frame */
   double t_stage_ms[8];
-  int max_pcg_iters;        /* most PCG iterations taken by one node-grid solve */
+  int max_pcg_iters;        /* most iterations taken by one node-grid solve, of its tiles or of
+                             the grid-wide PCG where that went on */
   double node_grid[4];      /* the node grid used: {x, y of the first node, M, N} */
   double t_search_mg_ms;    /* host time of the multigrid search (ALDIC_INIT_SEARCH_MG) */
   int gated_init;           /* ALDIC_INIT_GATED: nodes started from the given guess */

@@ -101,3 +101,14 @@ def test_smooth_matches_oracle(aldic, oracle, M, N, nf):
     lib.call("aldic_smooth", aldic.default_context().h, M, N, nf, got.ctypes.data)
     ref = oracle.smooth_fields(M, N, v.reshape(-1).copy(), nf)
     np.testing.assert_allclose(got, ref, rtol=0, atol=1e-11 * np.linalg.norm(np.nan_to_num(v)) / (0.0214 * (np.pi / 24) ** 2))
+
+
+def test_frame_counts_the_iterations_of_its_solves(aldic, synth):
+    """Also where the tiles finish every solve: the fits take their fixed number of
+    steps, the refills' iterations are counted by the tile that takes most."""
+    f = synth.speckle(200, 180, 900, 3)
+    g = synth.warp(f, synth.uniform_affine(0.002, -0.001, 0.4, -0.3), 0.5, 3)
+    al = aldic.ALDIC(20, 10, 6, ctx=aldic.Context(0))
+    al.set_images(f, g)
+    its = [al.frame()["stats"]["max_pcg_iters"] for _ in range(3)]
+    assert its[0] >= 12 and its == its[:1] * 3

@@ -8,6 +8,7 @@
 // intrinsics so no FMA contraction changes the result.
 #include "aldic_internal.cuh"
 #include "kernels.cuh"
+#include "rules.h"
 
 namespace aldic {
 
@@ -142,13 +143,9 @@ int roi_stats(const void *img, int dtype, int W, const int roi[4], double *d_sta
 }
 
 // ------------------------------------------------------------------ normalise
-// (v - m) / s correctly rounded, s the same for every pixel: with y the
-// correctly rounded 1 / s and q a quotient within one unit in the last place,
-// q + (n - q s) y is the rounded quotient n / s (P. W. Markstein, "Computation
-// of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
-// Dev. 34, 1990; a divisor whose significand is all ones excepted).  Three
-// operations in place of a division's thirty; deviations out of the range where
-// no step under- or overflows, 0 or NaN among them, are divided by.
+// (v - m) / s correctly rounded, s the same for every pixel: rounded_quotient's five
+// operations in place of a division's thirty.  Deviations out of the range where no
+// step under- or overflows, 0 or NaN among them, are divided by.
 struct Norm {
   double m, s, y;
   bool by_product;
@@ -159,8 +156,7 @@ struct Norm {
   __device__ __forceinline__ double operator()(double v) const {
     const double n = __dsub_rn(v, m);
     if (!by_product || !(fabs(n) > 1e-100 && fabs(n) < 1e100)) return __ddiv_rn(n, s);
-    const double q = __dmul_rn(n, y);
-    return __fma_rn(__fma_rn(-q, s, n), y, q);
+    return rounded_quotient(n, s, y);
   }
 };
 

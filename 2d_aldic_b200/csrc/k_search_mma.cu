@@ -235,7 +235,9 @@ __global__ void __launch_bounds__(kMmaBlock, 2)
   const long long mn = (long long)G.tw * G.tw;
   const double mu = *G.mu;
   auto wait = [&](uint64_t *bar, uint32_t parity) {
-    if (!*(volatile int *)&S.failed && !bar_wait(bar, parity, tries)) S.failed = 1;
+    const bool ok = !*(volatile int *)&S.failed && bar_wait(bar, parity, tries);
+    if (!ok) S.failed = 1;
+    return ok;
   };
   auto pix = [&](int y, int x) {  // pixel of the padded region
     int v = 0;
@@ -310,9 +312,8 @@ __global__ void __launch_bounds__(kMmaBlock, 2)
         const uint32_t skip = (P.rows * 128 - 128) / 16;
         for (int r = 0; r < rounds; ++r, ++rc) {
           const int s = rc & 1, y0 = r * P.trows;
-          wait(&S.full[s], (rc >> 1) & 1);
+          if (!__all_sync(0xffffffffu, wait(&S.full[s], (rc >> 1) & 1))) break;  // no more products
           tc_after_sync();
-          if (__any_sync(0xffffffffu, *(volatile int *)&S.failed)) break;  // no more products
           // the rows' descriptors: 8 PL further (16-byte units) a template row, 2
           // a K step, another block after 128 bytes
           uint64_t db = base + (uint64_t)(PL * 8 * y0);

@@ -306,10 +306,10 @@ GemmSrc src(const void *p, int mode, long long rows, long long kdim, long long l
   return s;
 }
 
-GemmDst dst(void *p, long long M, long long N, long long ld, int fp32, const float *bias, int relu,
-            int mode = GEMM_ROW, const void *mask = nullptr) {
+GemmDst dst(void *p, long long M, long long N, long long ld, int fp32, int mode = GEMM_ROW,
+            const void *mask = nullptr) {
   GemmDst d;
-  d.p = p; d.M = M; d.N = N; d.ld = ld; d.fp32 = fp32; d.bias = bias; d.relu = relu; d.mode = mode;
+  d.p = p; d.M = M; d.N = N; d.ld = ld; d.fp32 = fp32; d.bias = nullptr; d.relu = 0; d.mode = mode;
   d.mask = (const bf16 *)mask; d.Hin = d.Win = d.C = d.ps = 0; d.split_stride = 0;
   return d;
 }
@@ -357,7 +357,7 @@ int weight_grad(aldic_cnn *c, const GemmSrc &A, const GemmSrc &Bm, float *g, cud
   const long long n = A.rows * Bm.rows;
   int rc;
   if (splits > 1 && (rc = c->part.ensure(sizeof(float) * n * splits))) return rc;
-  GemmDst d = dst(splits > 1 ? c->part.p : g, A.rows, Bm.rows, Bm.rows, 1, nullptr, 0);
+  GemmDst d = dst(splits > 1 ? c->part.p : g, A.rows, Bm.rows, Bm.rows, 1);
   d.split_stride = n;
   if ((rc = gemm_bf16(A, Bm, d, splits, c->err.as<int>(), st))) return rc;
   if (splits > 1) k_splitk_sum<<<nblk(n), 256, 0, st>>>(c->part.as<float>(), splits, n, g);
@@ -392,10 +392,10 @@ int backward(aldic_cnn *c, const void *x, int B, cudaStream_t st) {
   if ((rc = bias_grad(c, c->dz3.p, b, cnn::F3, c->gB(2), st))) return rc;
   if ((rc = gemm_bf16(src(c->dz3.p, GEMM_ROW, b, cnn::F3, cnn::F3),
                       src(c->Wb(2), GEMM_TRANS, cnn::K3, cnn::F3, cnn::K3),
-                      dst(c->dcorr.p, b, cnn::K3, cnn::K3, 0, nullptr, 0), 1, err, st)))
+                      dst(c->dcorr.p, b, cnn::K3, cnn::K3, 0), 1, err, st)))
     return rc;
   // C: d e2_f = s dcorr . e2_g,  d e2_g = s dcorr^T . e2_f  (one product per pair)
-  GemmDst df = dst(c->de2.p, cnn::CELLS, cnn::C2, cnn::C2, 0, nullptr, 0);
+  GemmDst df = dst(c->de2.p, cnn::CELLS, cnn::C2, cnn::C2, 0);
   df.scale = kCorrScale;
   df.bstride = fs;
   if ((rc = gemm_bf16(src(c->dcorr.p, GEMM_ROW, cnn::CELLS, cnn::CELLS, cnn::CELLS, 0, 0, 0, 0, cnn::K3),
@@ -415,7 +415,7 @@ int backward(aldic_cnn *c, const void *x, int B, cudaStream_t st) {
   if ((rc = bias_grad(c, c->de2.p, cells, cnn::C2, c->gB(1), st))) return rc;
   if ((rc = gemm_bf16(src(c->de2.p, GEMM_ROW, cells, cnn::C2, cnn::C2),
                       src(c->Wb(1), GEMM_TRANS, cnn::K2, cnn::C2, cnn::K2),
-                      dst(c->dz1.p, cells, cnn::C1, cnn::C1, 0, nullptr, 0, GEMM_ROW, c->e1.p), 1, err,
+                      dst(c->dz1.p, cells, cnn::C1, cnn::C1, 0, GEMM_ROW, c->e1.p), 1, err,
                       st)))
     return rc;
   // E1

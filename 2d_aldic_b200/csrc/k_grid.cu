@@ -891,8 +891,6 @@ __global__ void k_vsub2(const double *a1, const double *b1, double *o1, long lon
   }
 }
 
-// block partials of |a - b|^2; with copy, a <- b as it goes (the caller's
-// "old" vector refreshed in the same pass)
 // *res = sqrt(sum of the blocks' s) * scale: the last block to arrive adds the
 // partials in their order, so the result does not depend on which it is
 __device__ __forceinline__ void norm_finish(double s, double *part, unsigned int *ticket, double *res,
@@ -926,7 +924,8 @@ __device__ __forceinline__ void norm_finish(double s, double *part, unsigned int
   }
 }
 
-// |a - b| * scale, and with `copy` a = b
+// |a - b| * scale, and with `copy` a <- b as it goes (the caller's "old" vector
+// refreshed in the same pass)
 __global__ void k_diffnorm(double *a, const double *b, long long n, double *part, unsigned int *ticket,
                            double *res, double scale, bool copy) {
   double s = 0.0;

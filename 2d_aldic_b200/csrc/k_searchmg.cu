@@ -41,25 +41,19 @@ constexpr int kStrip = 8;                                          // last level
 constexpr int kMaxFinal = 80;  // largest last-level region side (about winsize + 1)
 constexpr int kMaxFFT = 8192;  // largest FFT length (ROI up to 4096 px per side)
 
+// S: window sums; V: a pixel in shared memory (of floats, and their sums of
+// products); G: a sum of products in memory
 template <typename P> struct MgT;
 template <> struct MgT<uint8_t> {
-  using S = long long;       // window sums
-  using V = unsigned int;    // shared-memory pixel
-  using A = unsigned int;    // per-thread product sums (<= 16 * 8 * 255^2)
-  using G = unsigned long long;
-  static constexpr bool integer = true;
-};
-template <> struct MgT<uint16_t> {
   using S = long long;
   using V = unsigned int;
-  using A = unsigned long long;
   using G = unsigned long long;
   static constexpr bool integer = true;
 };
+template <> struct MgT<uint16_t> : MgT<uint8_t> {};
 template <> struct MgT<float> {
   using S = double;
   using V = double;
-  using A = double;
   using G = double;
   static constexpr bool integer = false;
 };
@@ -759,7 +753,6 @@ __global__ void __launch_bounds__(224) k_mg_crop(const P *__restrict__ f, const 
                                                  int W, const MgReg *__restrict__ regs,
                                                  typename MgT<P>::G *__restrict__ acc) {
   using V = typename MgT<P>::V;
-  using A = typename MgT<P>::A;
   using G = typename MgT<P>::G;
   constexpr int kTile = CropCfg<P>::TILE, kSeg = CropCfg<P>::SW;
   constexpr int TS = kTile + 4;             // template row stride
@@ -791,7 +784,7 @@ __global__ void __launch_bounds__(224) k_mg_crop(const P *__restrict__ f, const 
   __syncthreads();
   const int oyi = threadIdx.x / kSegs, seg = threadIdx.x - oyi * kSegs;  // oy = oyi - 1
   const int xs = seg * kSeg;
-  A s[kCropR];
+  V s[kCropR];
 #pragma unroll
   for (int k = 0; k < kCropR; ++k) s[k] = 0;
   if (xs < nx) {
@@ -803,9 +796,9 @@ __global__ void __launch_bounds__(224) k_mg_crop(const P *__restrict__ f, const 
       for (int k = 0; k < kSeg + kCropR - 1; ++k) win[k] = dr[k];
 #pragma unroll
       for (int xx = 0; xx < kSeg; ++xx) {
-        const A t = (A)tr[xx];
+        const V t = tr[xx];
 #pragma unroll
-        for (int k = 0; k < kCropR; ++k) s[k] += t * (A)win[xx + k];
+        for (int k = 0; k < kCropR; ++k) s[k] += t * win[xx + k];
       }
     }
   }
@@ -913,7 +906,6 @@ __global__ void __launch_bounds__(256) k_mg_full(const P *__restrict__ f, const 
                                                  double *__restrict__ res) {
   using S = typename MgT<P>::S;
   using V = typename MgT<P>::V;
-  using A = typename MgT<P>::A;
   constexpr int PL = MgT<P>::integer ? sizeof(P) : 1;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[64];
@@ -1096,7 +1088,7 @@ __global__ void __launch_bounds__(256) k_mg_full(const P *__restrict__ f, const 
       const int oy = j - (b - 1), ox0 = i0 - (a - 1);
       const int ty0 = max(0, -oy), ty1 = min(b, dh - oy);
       const int txa = max(0, -(ox0 + kStrip - 1)), txb = min(a, dw - ox0);
-      A s[kStrip];
+      V s[kStrip];
 #pragma unroll
       for (int k = 0; k < kStrip; ++k) s[k] = 0;
       for (int ty = ty0; ty < ty1; ++ty) {
@@ -1111,7 +1103,7 @@ __global__ void __launch_bounds__(256) k_mg_full(const P *__restrict__ f, const 
 #pragma unroll
           for (int q = 0; q < 8; ++q)
 #pragma unroll
-            for (int k = 0; k < kStrip; ++k) s[k] += (A)tv[q] * (A)dv[q + k];
+            for (int k = 0; k < kStrip; ++k) s[k] += tv[q] * dv[q + k];
         }
       }
 #pragma unroll

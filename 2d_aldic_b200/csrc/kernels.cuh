@@ -15,10 +15,11 @@ int normalize(const void *img, int dtype, long long n, const double *d_stats, do
               float *o32, cudaStream_t st);
 int gradient(const double *f, const double *mask, int W, int H, double *gx64, double *gy64,
              float *gx32, float *gy32, cudaStream_t st);
-// row-cubic coefficients of the FP64 image g: W H float4, q[y W + x] =
-// (a0, a1, a2, a3) of row y's Keys cubic on floor column x
+// (img - mean) / std in FP64 and FP32, d_stats = {mean, std}, and its row cubics
 int normalize_cubic(const void *img, int dtype, int W, int H, const double *d_stats, double *o64, float *o32,
                     float4 *q, cudaStream_t st);
+// row-cubic coefficients of the FP64 image g: W H float4, q[y W + x] =
+// (a0, a1, a2, a3) of row y's Keys cubic on floor column x
 int row_cubic(const double *g, int W, int H, float4 *q, cudaStream_t st);
 // q[i] = (gx[i], gy[i]), n float2
 int grad_pairs(const float *gx, const float *gy, long long n, float2 *q, cudaStream_t st);
@@ -271,11 +272,11 @@ int fe_rhs(GridWork &w, int M, int N, double h, double beta, double mu, const do
 // beta part into fields 0-1, the mu part into 2-3 (for the beta sweep)
 int fe_rhs_parts(GridWork &w, int M, int N, double h, const double *U, const double *F,
                  const double *udual, const double *vdual, cudaStream_t st);
-// interleave w.x (2 fields from slot f0) into Uhat
 // The finite-element Subproblem 2 at beta (*beta_ptr if given): right-hand side and
 // direct solve (basis B of the mesh), Uhat interleaved; w.b, w.x, w.r are used
 int fe_solve(const FdmBasis &B, GridWork &w, double h, double beta, double mu, const double *beta_ptr,
              const double *U, const double *F, const double *ud, const double *vd, double *Uhat, cudaStream_t st);
+// interleave w.x (2 fields) into Uhat
 int fe_store(const GridWork &w, int M, int N, double *Uhat, cudaStream_t st);
 // nodal strain (funGlobal_NodalStrainAvg.m)
 int nodal_strain(int M, int N, double h, const double *U, double *F, cudaStream_t st);

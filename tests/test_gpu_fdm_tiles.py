@@ -48,20 +48,3 @@ def test_subpb2_tile_edges(aldic, M, N):
     got = aldic.Subpb2(mesh, beta, mu, U, F, ud, vd)
     want = _solve(M, N, h, beta, mu, U, F, ud, vd)
     np.testing.assert_allclose(got, want, rtol=0, atol=1e-10 * np.abs(want).max())
-
-
-@pytest.mark.parametrize("dtype", [np.float64, np.float32])
-def test_interp_border_and_inside_agree(aldic, oracle, dtype):
-    """Points of every kind in one call: far inside, on the last taps that lie
-    inside, one past them, beyond the image, not finite; two planes."""
-    rng = np.random.default_rng(5)
-    N, M = 37, 41
-    F = rng.standard_normal((2, N, M)).astype(dtype)
-    edge = np.array([-7, -4, -0.5, 0, 0.5, 1, 1.5, 2 - 1e-6, 2, 2.25, 3, 20.7], dtype)
-    hi = np.concatenate([edge, [np.nan, np.inf, -np.inf]]).astype(dtype)
-    X = np.concatenate([hi, N + 1 - edge, rng.uniform(0, N, 200).astype(dtype)]).astype(dtype)
-    Y = np.concatenate([hi, M + 1 - edge, rng.uniform(0, M, 200).astype(dtype)]).astype(dtype)
-    X, Y = (np.ascontiguousarray(a) for a in np.meshgrid(X, Y))
-    got = aldic.ba_interp2(F, X, Y)
-    for p in range(2):
-        np.testing.assert_array_equal(got[p], oracle.ba_interp2(F[p], X, Y))

@@ -103,6 +103,53 @@ def test_smooth_matches_oracle(aldic, oracle, M, N, nf):
     np.testing.assert_allclose(got, ref, rtol=0, atol=1e-11 * np.linalg.norm(np.nan_to_num(v)) / (0.0214 * (np.pi / 24) ** 2))
 
 
+def _smooth(aldic, M, N, v):
+    from importlib import import_module
+    out = np.ascontiguousarray(v.T).reshape(-1)    # fields interleaved
+    import_module("2d_aldic_b200._lib").call("aldic_smooth", aldic.default_context().h, M, N, len(v), out.ctypes.data)
+    return out.reshape(-1, len(v)).T
+
+
+@pytest.mark.parametrize("M,N", [(40, 33), (97, 70)])
+def test_smooth_goes_on_where_the_tiles_cannot_finish(aldic, oracle, M, N):
+    """A region without data that the tiles' fixed steps do not cross: the grid-wide
+    solver goes on from their result, and convolves."""
+    v = _data(M, N, 2, 7)
+    hole = np.zeros((N, M), bool)
+    hole[6:N - 6, 5:M - 7] = True
+    v[0, hole.reshape(-1)] = np.nan
+    ref = oracle.smooth_fields(M, N, np.ascontiguousarray(v.T).reshape(-1), 2).reshape(-1, 2).T
+    # lam2 (pi / (2 gap))^2 bounds the springs' smallest eigenvalue over the gap
+    tol = 1e-11 * np.linalg.norm(np.nan_to_num(v)) / (0.0214 * (np.pi / (2 * max(M, N))) ** 2)
+    np.testing.assert_allclose(_smooth(aldic, M, N, v), ref, rtol=0, atol=tol)
+
+
+@pytest.mark.parametrize("M,N", [(40, 33), (97, 70)])
+def test_smooth_of_infinite_data(aldic, oracle, M, N):
+    """An infinite value has no finite residual: its field stays as it was and is only
+    convolved, in both passes; the other field is smoothed as ever, and the next call
+    finds the gate and the tickets as they should be."""
+    v = _data(M, N, 2, 9)
+    want = oracle.smooth_fields(M, N, np.ascontiguousarray(v.T).reshape(-1), 2).reshape(-1, 2).T
+    clean = _smooth(aldic, M, N, v)
+    tol = 1e-11 * np.linalg.norm(v) / 0.886
+    np.testing.assert_allclose(clean, want, rtol=0, atol=tol)
+    w = v.copy()
+    w[0, M * (N // 2) + M // 3] = np.inf
+    e = np.exp([-4.0, -2.0, -4.0, -2.0, 0.0, -2.0, -4.0, -2.0, -4.0])
+
+    def conv(a):
+        pad = np.pad(a.reshape(N, M), 1)
+        one = np.pad(np.ones((N, M)), 1)
+        near = lambda q: [q[1 + dj:1 + dj + N, 1 + di:1 + di + M] for dj in (-1, 0, 1) for di in (-1, 0, 1)]
+        return (sum(c * b for c, b in zip(e, near(pad))) / sum(c * b for c, b in zip(e, near(one)))).reshape(-1)
+    got = _smooth(aldic, M, N, w)
+    # nine terms of at most max |v|, whose sum and division round ten times, in two passes
+    np.testing.assert_allclose(got[0], conv(conv(w[0])), rtol=0, atol=20 * 2.0 ** -53 * np.abs(v).max())
+    np.testing.assert_allclose(got[1], want[1], rtol=0, atol=tol)
+    np.testing.assert_array_equal(_smooth(aldic, M, N, v), clean)
+
+
 def test_frame_counts_the_iterations_of_its_solves(aldic, synth):
     """Also where the tiles finish every solve: the fits take their fixed number of
     steps, the refills' iterations are counted by the tile that takes most."""

@@ -243,7 +243,7 @@ int grad_pairs(const float *gx, const float *gy, long long n, float2 *q, cudaStr
 
 // Both at once: the normalised image and its row cubics, a row in segments of 256
 // columns, whose normalised values and the three beside them lie in shared memory.
-// Bound by memory: 4096 x 4096, 16 bit, writes 28 bytes a pixel; 103 us (the
+// Bound by memory: 4096 x 4096, 16 bit, writes 28 bytes a pixel; 104 us (the
 // copy rate allows 77), 146 us as two kernels that wrote the image and read it back.
 template <typename T>
 __global__ void __launch_bounds__(256)

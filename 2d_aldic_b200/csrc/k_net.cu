@@ -62,7 +62,7 @@ __device__ __forceinline__ uint32_t swz(int r, int c) { return r * 128 + ((c ^ (
 // KB each) and the weights (48 KB) are there.  The pair's 16 KB are loaded a
 // pair ahead, and the next embedding is issued with the correlation.  Eight
 // warps do the epilogues; a ninth only issues the products.
-// Tensor memory: D 128, C 64, E 64 columns.  16384 pairs: 164 us (ncu), against
+// Tensor memory: D 128, C 64, E 64 columns.  16384 pairs: 161 us (ncu), against
 // 62 us for their 24 KB each at the copy rate and 68 us for the products; a
 // pair's chain of three products and three epilogues is what is left (two CTAs
 // an SM hide half of it; 512 epilogue threads a CTA measured 6 % slower).  The
@@ -316,8 +316,8 @@ __global__ void __launch_bounds__(kEncBlock, 2) k_encode(const __grid_constant__
 // blockIdx.y, and k_dense_out adds them; otherwise the epilogue goes on to the output
 // layer, the second half of a row's sums after the first.
 // Bound: 48 KB of operands a step and SM through L2 (corr once, W3 by every
-// tile).  16384 rows: 47 us (ncu), 0.73 PFLOP/s; 52 us with one chain of 4096 read by
-// four warps at its end; the generic product with its split-K sum and the output layer
+// tile).  16384 rows: 47.6 us (ncu), 0.72 PFLOP/s; 50.2 us with one chain of 4096 read
+// by four warps at its end; the generic product with its split-K sum and the output layer
 // took 560 us.
 constexpr int kDenseStages = 4, kDenseStage = (128 + kF) * 128, kDenseThreads = 64 + 256;
 constexpr int kDenseSlices = 8, kSliceSteps = kCorr / 64 / kDenseSlices;

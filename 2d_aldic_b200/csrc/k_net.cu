@@ -86,7 +86,7 @@ struct EncShared {
   unsigned char out[kCells * 128];   // the correlation on its way to memory
   unsigned char W1[128 * 128];
   unsigned char W2[2][128 * 128];
-  uint64_t bar[4];                   // embedding, 1x1, correlation; x has landed
+  uint64_t bar[5];                   // embedding, 1x1, correlation; x has landed; all products ended
   uint32_t tmem;
   int failed;
 };
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kEncBlock, 2) k_encode(const __grid_constant__
   if (warp == 0) tmem_alloc(&S.tmem, 256);
   if (tid == 0) {
     S.failed = 0;
-    for (int k = 0; k < 4; ++k) bar_init(&S.bar[k], 1);
+    for (int k = 0; k < 5; ++k) bar_init(&S.bar[k], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // this warp's quarter of the tensor memory's lanes (rows) and half of the
@@ -294,6 +294,14 @@ __global__ void __launch_bounds__(kEncBlock, 2) k_encode(const __grid_constant__
   }
   tc_before_sync();
   __syncthreads();
+  if (S.failed) {  // the products under way end before the tensor memory goes
+    if (issuer) {
+      if (elect_one()) mma_commit(&S.bar[4]);
+      __syncwarp();
+      bar_wait(&S.bar[4], 0);
+    }
+    __syncthreads();
+  }
   if (issuer && lane == 0) {
     if (!S.failed) store(blockIdx.x + (A.B - 1 - (int)blockIdx.x) / (int)gridDim.x * (int)gridDim.x);
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");

@@ -332,10 +332,6 @@ __global__ void __launch_bounds__(kMmaBlock, 2)
           __syncwarp();
         }
       }
-    // no product is under way when the tensor memory goes, also after a failed wait
-    if (elect_one()) mma_commit(&S.drained);
-    __syncwarp();
-    bar_wait(&S.drained, 0);
   } else if (warp == kPeak) {
     for (int k = blockIdx.x; k < npts; k += gridDim.x) {
       named_sync(4, kMmaThreads + 32);  // the queue is complete
@@ -673,7 +669,15 @@ __global__ void __launch_bounds__(kMmaBlock, 2)
   }
   tc_before_sync();
   __syncthreads();
-  if (tid == 0 && S.failed) atomicExch(err, 3);
+  if (S.failed) {  // the products under way end before the tensor memory goes
+    if (uniform(warp) == kIssuer) {
+      if (elect_one()) mma_commit(&S.drained);
+      __syncwarp();
+      bar_wait(&S.drained, 0);
+    }
+    if (tid == 0) atomicExch(err, 3);
+    __syncthreads();
+  }
   if (warp == 0) tmem_free(tD, P.tcols);
 }
 
